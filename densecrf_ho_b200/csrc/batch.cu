@@ -711,6 +711,7 @@ int Batch::qp(const float* init, float* out, int max_iter, int* steps, double* e
     for (auto& t : terms) {
         key.push_back(t->lat->va.get());
         key.push_back(t->lat->vb.get());
+        key.push_back(t->lat->rows.get());
         key.push_back(t->lat.get());
         key.push_back((const void*)(uintptr_t)t->lat->dom_tile);
     }

@@ -110,6 +110,32 @@ inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
+// The same as a programmatic dependent launch: the kernel may be set up on the
+// SMs while its predecessor in the stream drains (it must call grid_wait()
+// before it touches global memory, and grid_release() lets its own successor
+// do the same).  For the filters' chains of kernels of a few microseconds,
+// whose launch gaps would otherwise be a third of their time.
+template <typename... KArgs, typename... Args>
+inline void launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                           Args&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    DCRF_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(std::forward<Args>(args))...));
+    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+}
+// All work before this grid in its stream has completed and is visible.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next grid of the stream may be set up once every block is here or done.
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Number of SMs of the current device (cached per process; one device per
 // process is the supported deployment).
 int sm_count();

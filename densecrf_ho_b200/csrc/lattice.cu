@@ -40,9 +40,10 @@ constexpr int kStages = 3;       // shared-memory ring depth, in chunks
 constexpr int kChunk = 32;       // entries per chunk (13 KB of ring per warp: 16 warps / SM)
 constexpr int kMaxOrderKey = (1 << 24) - 1;
 constexpr int kLongList = 64;    // lists longer than this use the staged warp kernels
-constexpr int kHugeList = 1024;  // lists longer than this get the finest ordered-splat split
+constexpr int kHugeList = 1024;  // lists longer than this get a block (plain) or the finest split (ordered splat)
 constexpr int kHugeLabels = 12;  // labels per block for those lists (120 threads)
 constexpr int kTB = 256;         // threads per block of the element-wise kernels
+constexpr int kSegPad = 4;       // entries past the splat lists' end that a paired load may touch
 
 template <int KW>
 struct Key {
@@ -298,14 +299,15 @@ __global__ void iota_copy_kernel(int E, const int* __restrict__ offset, int* __r
     vals[e] = e;
 }
 
+// A splat list's entry is (pixel, weight bits).
+__device__ __forceinline__ float entry_w(int2 e) { return __int_as_float(e.y); }
+
 __global__ void seg_fill_kernel(int E, int d1, const int* __restrict__ sorted_entries,
-                                const float* __restrict__ bary, int* __restrict__ seg_pix,
-                                float* __restrict__ seg_w) {
+                                const float* __restrict__ bary, int2* __restrict__ seg) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= E) return;
     const int e = sorted_entries[s];
-    seg_pix[s] = e / d1;
-    seg_w[s] = bary[e];
+    seg[s] = make_int2(e / d1, __float_as_int(bary[e]));
 }
 
 // ------------------------------------------------------------- filter --
@@ -346,23 +348,19 @@ __device__ __forceinline__ void cp_async_wait() {
 // Streams the list [s0, s1) of one vertex through the per-warp ring:
 // `vals_of(slot, e)` is this lane's staged word for entry e, and
 // consume(slot, n) is called once per chunk, in order.
-template <typename T, bool NORM, typename Consume>
+template <typename T, typename Consume>
 __device__ __forceinline__ void stream_list(int s0, int s1, int L, int k, bool act, int lane,
-                                            const int* __restrict__ seg_pix, const float* __restrict__ seg_w,
-                                            const T* __restrict__ src, const float* __restrict__ norm,
-                                            T (*ring)[kChunk][32], float (*mw)[kChunk], float (*mn)[kChunk],
+                                            const int2* __restrict__ seg,
+                                            const T* __restrict__ src, T (*ring)[kChunk][32], float (*mw)[kChunk],
                                             Consume&& consume) {
     const int nch = (s1 - s0 + kChunk - 1) / kChunk;
     auto pix_of = [&](int c) {
         const int base = s0 + c * kChunk;
-        return (c < nch && lane < s1 - base) ? seg_pix[base + lane] : 0;
+        return (c < nch && lane < s1 - base) ? seg[base + lane].x : 0;
     };
     auto issue = [&](int c, int pc) {
         const int slot = c % kStages, base = s0 + c * kChunk, n = min(kChunk, s1 - base);
-        if (lane < n) {
-            cp_async4(&mw[slot][lane], seg_w + base + lane);
-            if (NORM) cp_async4(&mn[slot][lane], norm + pc);
-        }
+        if (lane < n) cp_async4(&mw[slot][lane], &seg[base + lane].y);
         for (int e = 0; e < n; e++) {
             const int p = __shfl_sync(0xffffffffu, pc, e);
             if (act) cp_async4(&ring[slot][e][lane], src + (long)p * L + k);
@@ -391,586 +389,524 @@ __device__ __forceinline__ void stream_list(int s0, int s1, int L, int k, bool a
     __syncwarp();
 }
 
-template <bool PRE_NORM, int LC = 0>
+// The allocation-free filter's splat of the long lists (it may not hold the
+// padded rows of the splat below): rows as they are, one warp per vertex.
 __global__ void __launch_bounds__(32 * kStageWarps)
-    splat_kernel(int M, int Lrt, const int* __restrict__ order, const int* __restrict__ seg_start,
-                 const int* __restrict__ seg_pix, const float* __restrict__ seg_w, const float* __restrict__ in,
-                 const float* __restrict__ norm, float* __restrict__ vals, Live lv, int Lrow) {
-    const int L = LC ? LC : Lrt;
+    splat_kernel(int M, int L, const int* __restrict__ order, const int* __restrict__ seg_start,
+                 const int2* __restrict__ seg, const float* __restrict__ in,
+                 float* __restrict__ vals) {
     __shared__ float ring[kStageWarps][kStages][kChunk][32];
     __shared__ float mw[kStageWarps][kStages][kChunk];
-    __shared__ float mn[kStageWarps][kStages][kChunk];
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long total = live_total(lv, M);
-    // warp-uniform loop; the kernel has no block-wide barrier
-    for (long unit = (long)blockIdx.x * kStageWarps + wib; unit < total; unit += (long)gridDim.x * kStageWarps) {
-        const int v = order[live_unit(lv, unit)];
-        const int s0 = seg_start[v], s1 = seg_start[v + 1];
-        for (int kb = 0; kb < L; kb += 32) {
-            const int k = kb + lane;
-            const bool act = k < L;
-            float acc = 0.0f;
-            stream_list<float, PRE_NORM>(s0, s1, L, k, act, lane, seg_pix, seg_w, in, norm, ring[wib], mw[wib],
-                                         mn[wib], [&](int slot, int n) {
+    const int unit = blockIdx.x * kStageWarps + wib;
+    if (unit >= M) return;  // warp-uniform
+    const int v = order[unit];
+    const int s0 = seg_start[v], s1 = seg_start[v + 1];
+    for (int kb = 0; kb < L; kb += 32) {
+        const int k = kb + lane;
+        const bool act = k < L;
+        float acc = 0.0f;
+        stream_list<float>(s0, s1, L, k, act, lane, seg, in, ring[wib], mw[wib], [&](int slot, int n) {
 #pragma unroll 4
-                                             for (int e = 0; e < n; e++) {
-                                                 float x = ring[wib][slot][e][lane];
-                                                 if (PRE_NORM) x = fmul(x, mn[wib][slot][e]);
-                                                 acc = fadd(acc, fmul(mw[wib][slot][e], x));
-                                             }
-                                         });
-            if (act) vals[(long)(v + 1) * Lrow + k] = acc;
-        }
-        for (int k = L + lane; k < Lrow; k += 32) vals[(long)(v + 1) * Lrow + k] = 0.0f;  // row padding
+            for (int e = 0; e < n; e++) acc = fadd(acc, fmul(mw[wib][slot][e], ring[wib][slot][e][lane]));
+        });
+        if (act) vals[(long)(v + 1) * L + k] = acc;
     }
 }
 
-// The longest lists with L = 21: the cp.async ring of splat_kernel, kStages chunks
-// of 32 entries deep, but each lane copies its own entry's 21 values into a
-// [label][entry] ring (no shuffles, 21 copies per chunk instead of 32), and
-// lane k < 21 sums its label in entry order with float4 reads of four
-// entries' values, weights (and norms) at a time.
-constexpr int kRS = 36;  // ring row stride: float4-aligned, 4 banks apart per label
-template <bool PRE_NORM>
-__global__ void __launch_bounds__(32 * kStageWarps)
-    splat_ring21_kernel(int M, const int* __restrict__ order, const int* __restrict__ seg_start,
-                        const int* __restrict__ seg_pix, const float* __restrict__ seg_w,
-                        const float* __restrict__ in, const float* __restrict__ norm, float* __restrict__ vals,
-                        Live lv, int Lrow) {
-    constexpr int L = 21;
-    __shared__ __align__(16) float X[kStageWarps][kStages][L][kRS];
-    __shared__ __align__(16) float Wr[kStageWarps][kStages][kChunk];
-    __shared__ __align__(16) float Nr[kStageWarps][kStages][kChunk];
+// ... and of the short lists: one thread per (vertex, label).
+__global__ void splat_short_kernel(int n_short, int L, const int* __restrict__ order,
+                                   const int* __restrict__ seg_start, const int2* __restrict__ seg, const float* __restrict__ in,
+                                   float* __restrict__ vals) {
+    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long)n_short * L) return;
+    const int u = (int)(t / L), k = (int)(t - (long)u * L);
+    const int v = order[u];
+    const int s0 = seg_start[v], s1 = seg_start[v + 1];
+    float acc = 0.0f;
+#pragma unroll 4
+    for (int s = s0; s < s1; s++) acc = fadd(acc, fmul(entry_w(seg[s]), in[(long)seg[s].x * L + k]));
+    vals[(long)(v + 1) * L + k] = acc;
+}
+
+// ----------------------------------------------------------- row splat --
+// The plain splat, L > 2.  The input is copied once into rows of Q = ceil(L /
+// 4) float4 (pad_rows_kernel: labels past L are zero, the normalisation
+// factor already applied: fmul(x, norm) is the product the reference forms
+// before the splat), so that a list entry costs Q aligned 16-byte loads
+// instead of L scalar ones plus a norm gather.  L = 21, one warp instruction
+// per entry and label group:
+//   short lists  one thread per (vertex, four labels), kSplatU entries' rows
+//                in flight, the next entries' (pixel, weight) already loaded;
+//   long lists   one warp per vertex, a ring of kSplatStages chunks of 32
+//                entries filled with 16-byte cp.async (6 per lane and chunk
+//                for L = 21), lane = label for the sums: 1 shared-memory read
+//                + 1 multiply + 1 add per entry;
+//   huge lists   one block per vertex: the block's whole ring for one list
+//                (kHugeStages chunks of 64 entries), four warps copying and the
+//                first one adding.  A lone warp with two chunks of lookahead
+//                waits for its loads (about 840 cycles per 32 entries: the
+//                3607-entry list of a 640x480 bilateral lattice set the
+//                splat's 50 us); with five chunks of 64 in flight the chain of
+//                dependent adds is what is left.
+// All sum a (vertex, label)'s entries in list order from +0, one rounding per
+// product and per sum, as the reference's scatter does.
+constexpr int kSplatU = 4;        // entries in flight per thread (short lists)
+constexpr int kSplatWarps = 4;    // lists per block (long lists)
+constexpr int kSplatStages = 3;   // 9.4 KB of ring per warp at L = 21: 20 warps / SM
+constexpr int kSplatThreads = 32 * kSplatWarps;
+
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+// a + w x per half, the product and the sum each rounded: scalar products and
+// a packed sum.  A packed product feeding a packed sum was measured to come
+// out as one fused multiply-add (rounded once), which the reference's SSE2
+// arithmetic does not do.
+__device__ __forceinline__ unsigned long long add_mul2(unsigned long long a, float w, unsigned long long x) {
+    const float2 f = unpack2(x);
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(pack2(fmul(w, f.x), fmul(w, f.y))));
+    return r;
+}
+
+__device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr(sdst)), "l"(gsrc) : "memory");
+}
+
+// A batched solve's live slice tiles, or tiles of the whole pixel range: the
+// first pixel of tile u and its pixel count.
+__device__ __forceinline__ int tile_pixels(const Live& lv, const long* pix_base, long u, int tile, long N,
+                                           long& p0) {
+    long pend = N;
+    if (lv.n) {
+        long local;
+        const int img = live_locate(lv, u, local);
+        p0 = pix_base[img] + local * tile;
+        pend = pix_base[img + 1];
+    } else {
+        p0 = u * tile;
+    }
+    return (int)min((long)tile, pend - p0);
+}
+
+// rows[i][q] = (in[i][4q .. 4q+3] o norm[i]), zero past L: a tile of pixels per
+// warp, copied to shared memory as it lies (16 bytes at a time where the
+// pointer allows, vec) and written back in rows.  Bound by memory: 84 bytes
+// in, 96 out per pixel at L = 21.
+constexpr int kPadWarps = 4;
+template <int QC>
+__global__ void __launch_bounds__(32 * kPadWarps)
+    pad_rows_kernel(int N, int L, int Qrt, int tile, const float* __restrict__ in, const float* __restrict__ norm,
+                    float4* __restrict__ rows, Live lv, const long* __restrict__ pix_base, int vec) {
+    extern __shared__ __align__(16) unsigned char pad_smem[];
+    const int Q = QC ? QC : Qrt;
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long total = live_total(lv, M);
-    // warp-uniform loop; no block-wide barrier inside
-    for (long unit = (long)blockIdx.x * kStageWarps + wib; unit < total; unit += (long)gridDim.x * kStageWarps) {
-        const int v = order[live_unit(lv, unit)];
-        const int s0 = seg_start[v], s1 = seg_start[v + 1];
-        const int nch = (s1 - s0 + kChunk - 1) / kChunk;
-        auto pix_of = [&](int c) {
-            const int e = s0 + c * kChunk + lane;
-            return (c < nch && e < s1) ? seg_pix[e] : -1;
-        };
-        auto issue = [&](int c, int p) {
-            if (p < 0) return;  // past the end of the list: never summed
-            const int slot = c % kStages, e = s0 + c * kChunk + lane;
-            const float* row = in + (long)p * L;
-#pragma unroll
-            for (int k = 0; k < L; k++) cp_async4(&X[wib][slot][k][lane], row + k);
-            cp_async4(&Wr[wib][slot][lane], seg_w + e);
-            if (PRE_NORM) cp_async4(&Nr[wib][slot][lane], norm + p);
-        };
-        float acc = 0.0f;
-        int pcur = pix_of(0);
-#pragma unroll
-        for (int c = 0; c < kStages - 1; c++) {
-            const int pn = pix_of(c + 1);
-            issue(c, pcur);
-            cp_async_commit();
-            pcur = pn;
-        }
-        for (int c = 0; c < nch; c++) {
-            const int ci = c + kStages - 1;
-            const int pn = pix_of(ci + 1);
-            issue(ci, pcur);
-            cp_async_commit();
-            pcur = pn;
-            cp_async_wait<kStages - 1>();  // chunk c has landed (this lane's copies)
-            __syncwarp();                  // ... and every other lane's
-            const int slot = c % kStages, n = min(kChunk, s1 - (s0 + c * kChunk));
-            if (lane < L) {
-                const float4* xs = reinterpret_cast<const float4*>(&X[wib][slot][lane][0]);
-                const float4* ws = reinterpret_cast<const float4*>(&Wr[wib][slot][0]);
-                const float4* ns = reinterpret_cast<const float4*>(&Nr[wib][slot][0]);
-                const int n4 = n >> 2;
-                for (int q = 0; q < n4; q++) {
-                    float4 x = xs[q];
-                    const float4 w = ws[q];
-                    if (PRE_NORM) {
-                        const float4 nv = ns[q];
-                        x.x = fmul(x.x, nv.x);
-                        x.y = fmul(x.y, nv.y);
-                        x.z = fmul(x.z, nv.z);
-                        x.w = fmul(x.w, nv.w);
-                    }
-                    acc = fadd(acc, fmul(w.x, x.x));
-                    acc = fadd(acc, fmul(w.y, x.y));
-                    acc = fadd(acc, fmul(w.z, x.z));
-                    acc = fadd(acc, fmul(w.w, x.w));
-                }
-                for (int e = n4 << 2; e < n; e++) {
-                    float x = X[wib][slot][lane][e];
-                    if (PRE_NORM) x = fmul(x, Nr[wib][slot][e]);
-                    acc = fadd(acc, fmul(Wr[wib][slot][e], x));
-                }
-            }
-            __syncwarp();  // the slot is refilled kStages-1 chunks later
-        }
+    float* buf = reinterpret_cast<float*>(pad_smem) + (size_t)wib * ((tile * L + 3) & ~3);
+    grid_release();
+    grid_wait();
+    const long total = live_total(lv, ((long)N + tile - 1) / tile);
+    for (long u = (long)blockIdx.x * kPadWarps + wib; u < total; u += (long)gridDim.x * kPadWarps) {
+        long p0;
+        const int np = tile_pixels(lv, pix_base, u, tile, N, p0);
+        const long t0 = p0 * L;
+        const int ne = np * L, n4 = vec && (t0 & 3) == 0 ? ne >> 2 : 0;
+        for (int e = lane; e < n4; e += 32) cp_async16(buf + 4 * e, in + t0 + 4 * e);
+        for (int e = 4 * n4 + lane; e < ne; e += 32) cp_async4(buf + e, in + t0 + e);
+        cp_async_commit();
         cp_async_wait<0>();
         __syncwarp();
-        if (lane < L) vals[(long)(v + 1) * Lrow + lane] = acc;
-        else if (lane < Lrow) vals[(long)(v + 1) * Lrow + lane] = 0.0f;  // row padding
+        for (int it = lane; it < np * Q; it += 32) {
+            const int pl = it / Q, q = it - pl * Q, n = L - 4 * q;
+            const float* x = buf + pl * L + 4 * q;
+            float4 r = make_float4(x[0], n > 1 ? x[1] : 0.0f, n > 2 ? x[2] : 0.0f, n > 3 ? x[3] : 0.0f);
+            if (norm) {
+                const float s = norm[p0 + pl];
+                r.x = fmul(r.x, s);
+                r.y = n > 1 ? fmul(r.y, s) : 0.0f;
+                r.z = n > 2 ? fmul(r.z, s) : 0.0f;
+                r.w = n > 3 ? fmul(r.w, s) : 0.0f;
+            }
+            rows[(p0 * Q) + it] = r;
+        }
+        __syncwarp();  // buf is refilled
     }
 }
 
-// Lists of at most kHugeList entries: one warp per vertex, lane = label (in
-// chunks of 32 labels).  The list streams in chunks of 32 entries: each
-// lane loads one entry's pixel, weight and normalisation factor (coalesced,
-// the next chunk's while the current one is summed) and stores them as one
-// 16-byte record in shared memory; then every entry costs one broadcast
-// record read and one coalesced read of the pixel's L input values.  The
-// sum is the same in-order chain per (vertex, label) as splat_kernel's.
-template <bool PRE_NORM, int LC, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS)
-    splat_warp_kernel(int n, int Lrt, const int* __restrict__ order, const int* __restrict__ seg_start,
-                      const int* __restrict__ seg_pix, const float* __restrict__ seg_w,
-                      const float* __restrict__ in, const float* __restrict__ norm, float* __restrict__ vals,
-                      Live lv, int Lrow) {
-    const int L = LC ? LC : Lrt;
-    __shared__ float4 rec[WARPS][32];
-    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long total = live_total(lv, n);
-    // warp-uniform loop; no block-wide barrier inside
-    for (long unit = (long)blockIdx.x * WARPS + wib; unit < total; unit += (long)gridDim.x * WARPS) {
-        const int v = order[live_unit(lv, unit)];
+// The lists a splat launch covers: positions [first, first + count) of
+// `order`, or the live images' positions of the domain behind lv.
+struct SplatRange {
+    int first = 0, count = 0;
+    Live lv;
+};
+__device__ __forceinline__ int splat_vertex(const SplatRange& r, const int* __restrict__ order, long u) {
+    return order[r.lv.n ? live_unit(r.lv, u) : r.first + u];
+}
+
+// Thread t of nt of the short lists' part.
+template <int QC>
+__device__ __forceinline__ void splat_rows_short(const SplatRange& r, int Qrt, const int* __restrict__ order,
+                                                 const int* __restrict__ seg_start,
+                                                 const int2* __restrict__ seg,
+                                                 const float4* __restrict__ rows, float4* __restrict__ vals, long t0,
+                                                 long nt) {
+    const int Q = QC ? QC : Qrt;
+    const long total = live_total(r.lv, r.count) * Q;
+    for (long t = t0; t < total; t += nt) {
+        const long u = t / Q;
+        const int q = (int)(t - u * Q);
+        const int v = splat_vertex(r, order, u);
         const int s0 = seg_start[v], s1 = seg_start[v + 1];
-        float4* r = rec[wib];
-        for (int kb = 0; kb < L; kb += 32) {
-            const int k = kb + lane;
-            const bool act = k < L;
-            float acc = 0.0f;
-            int p = 0;
-            float w = 0.0f, nn = 1.0f;
-            auto fetch = [&](int base) {
-                const int e = base + lane;
-                if (e < s1) {
-                    p = seg_pix[e];
-                    w = seg_w[e];
-                    if (PRE_NORM) nn = norm[p];
+        unsigned long long a0 = 0ull, a1 = 0ull;
+        // four entries per step, loaded two at a time from an even position
+        // (those outside the list are not used)
+        const int4* seg2 = reinterpret_cast<const int4*>(seg);
+        int s = s0 & ~1;
+        int4 ea, eb;
+        if (s < s1) {
+            ea = seg2[s >> 1];
+            eb = seg2[(s >> 1) + 1];
+        }
+        for (; s < s1; s += kSplatU) {
+            int p[kSplatU] = {ea.x, ea.z, eb.x, eb.z};
+            const float w[kSplatU] = {__int_as_float(ea.y), __int_as_float(ea.w), __int_as_float(eb.y),
+                                      __int_as_float(eb.w)};
+            ulonglong2 x[kSplatU];
+#pragma unroll
+            for (int i = 0; i < kSplatU; i++) {  // no branch: the four loads go out together
+                if (s + i < s0 || s + i >= s1) p[i] = 0;
+                x[i] = *reinterpret_cast<const ulonglong2*>(rows + (long)p[i] * Q + q);
+            }
+            const int sn = (s + kSplatU < s1 ? s + kSplatU : s) >> 1;
+            ea = seg2[sn];
+            eb = seg2[sn + 1];
+#pragma unroll
+            for (int i = 0; i < kSplatU; i++)
+                if (s + i >= s0 && s + i < s1) {
+                    a0 = add_mul2(a0, w[i], x[i].x);
+                    a1 = add_mul2(a1, w[i], x[i].y);
+                }
+        }
+        *reinterpret_cast<ulonglong2*>(vals + (long)(v + 1) * Q + q) = make_ulonglong2(a0, a1);
+    }
+}
+
+// The sum of one staged chunk of n <= E entries of rows of nq float4: this
+// lane's label at xs, the weights at ws.
+template <int E>
+__device__ __forceinline__ float splat_sum_chunk(float acc, const float* xs, const float* ws, int nq, int n) {
+    if (n == E) {
+#pragma unroll
+        for (int g = 0; g < E / 4; g++) {
+            const float4 w = reinterpret_cast<const float4*>(ws)[g];
+            acc = fadd(acc, fmul(w.x, xs[(4 * g + 0) * 4 * nq]));
+            acc = fadd(acc, fmul(w.y, xs[(4 * g + 1) * 4 * nq]));
+            acc = fadd(acc, fmul(w.z, xs[(4 * g + 2) * 4 * nq]));
+            acc = fadd(acc, fmul(w.w, xs[(4 * g + 3) * 4 * nq]));
+        }
+    } else {
+#pragma unroll 4
+        for (int e = 0; e < n; e++) acc = fadd(acc, fmul(ws[e], xs[e * 4 * nq]));
+    }
+    return acc;
+}
+
+// Bytes of ring per warp for rows of nq float4 (at most 8 at a time).
+__host__ __device__ constexpr int splat_ring_bytes(int nq) { return kSplatStages * 32 * (nq * 16 + 4); }
+
+// Long lists: warp `unit0` of nw.
+template <int QC>
+__device__ __forceinline__ void splat_rows_long(const SplatRange& r, int Qrt, const int* __restrict__ order,
+                                                const int* __restrict__ seg_start, const int2* __restrict__ seg, const float4* __restrict__ rows,
+                                                float4* __restrict__ vals, unsigned char* ring, long unit0,
+                                                long nw) {
+    const int Q = QC ? QC : Qrt;
+    const int lane = threadIdx.x & 31;
+    const long total = live_total(r.lv, r.count);
+    for (long unit = unit0; unit < total; unit += nw) {  // warp-uniform
+        const int v = splat_vertex(r, order, unit);
+        const int s0 = seg_start[v], s1 = seg_start[v + 1];
+        const int nch = (s1 - s0 + 31) >> 5;
+        for (int qb = 0; qb < Q; qb += 8) {  // 32 labels at a time
+            const int nq = QC ? QC : min(8, Q - qb);
+            float4* X = reinterpret_cast<float4*>(ring);                            // [stage][entry][nq]
+            float* Wt = reinterpret_cast<float*>(X + kSplatStages * 32 * nq);       // [stage][entry]
+            auto pix_of = [&](int c) {
+                const int s = s0 + c * 32 + lane;
+                return (c < nch && s < s1) ? seg[s].x : 0;
+            };
+            auto issue = [&](int c, int pc) {
+                const int slot = c % kSplatStages, base = s0 + c * 32, n = min(32, s1 - base);
+                if (lane < n) cp_async4(Wt + slot * 32 + lane, &seg[base + lane].y);
+#pragma unroll
+                for (int i = 0; i < (QC ? QC : 8); i++) {
+                    if (!QC && i >= nq) break;
+                    const int idx = lane + 32 * i, e = idx / nq;
+                    const int p = __shfl_sync(0xffffffffu, pc, e);
+                    if (e < n) cp_async16(X + slot * 32 * nq + idx, rows + (long)p * Q + qb + (idx - e * nq));
                 }
             };
-            fetch(s0);
-            for (int c0 = s0; c0 < s1; c0 += 32) {
-                r[lane] = make_float4(__int_as_float(p), w, nn, 0.0f);
-                fetch(c0 + 32);  // in flight while this chunk is summed
-                __syncwarp();
-                const int cnt = min(32, s1 - c0);
-                if (act) {
-#pragma unroll 8
-                    for (int e = 0; e < cnt; e++) {
-                        const float4 q = r[e];
-                        float x = in[(long)__float_as_int(q.x) * L + k];
-                        if (PRE_NORM) x = fmul(x, q.z);
-                        acc = fadd(acc, fmul(q.y, x));
+            float acc = 0.0f;
+            int pcur = pix_of(0);
+#pragma unroll
+            for (int c = 0; c < kSplatStages - 1; c++) {
+                const int pn = pix_of(c + 1);
+                if (c < nch) issue(c, pcur);
+                cp_async_commit();
+                pcur = pn;
+            }
+            for (int c = 0; c < nch; c++) {
+                const int ci = c + kSplatStages - 1;
+                const int pn = pix_of(ci + 1);
+                if (ci < nch) issue(ci, pcur);
+                cp_async_commit();
+                pcur = pn;
+                cp_async_wait<kSplatStages - 1>();  // chunk c has landed (this lane's copies)
+                __syncwarp();                       // ... and every other lane's
+                const int slot = c % kSplatStages, n = min(32, s1 - (s0 + c * 32));
+                if (lane < 4 * nq)
+                    acc = splat_sum_chunk<32>(acc, reinterpret_cast<const float*>(X + slot * 32 * nq) + lane,
+                                              Wt + slot * 32, nq, n);
+                __syncwarp();  // the slot is refilled kSplatStages - 1 chunks later
+            }
+            cp_async_wait<0>();
+            __syncwarp();
+            if (lane < 4 * nq) reinterpret_cast<float*>(vals)[((long)(v + 1) * Q + qb) * 4 + lane] = acc;
+        }
+    }
+}
+
+// Huge lists: block b takes the b-th of the visiting order.
+constexpr int kHugeE = 64;                              // entries per chunk
+constexpr int kHugeStages = kSplatWarps * kSplatStages / 2;  // the four warps' rings as one
+template <int QC>
+__device__ __forceinline__ void splat_rows_huge(int b, int Qrt, const int* __restrict__ order,
+                                                const int* __restrict__ seg_start, const int2* __restrict__ seg, const float4* __restrict__ rows,
+                                                float4* __restrict__ vals, unsigned char* ring) {
+    const int Q = QC ? QC : Qrt;
+    const int t = threadIdx.x;
+    constexpr int kMax = kHugeE * 8 / kSplatThreads;  // copies per thread and chunk, at most
+    {
+        const int v = order[b];
+        const int s0 = seg_start[v], s1 = seg_start[v + 1];
+        const int nch = (s1 - s0 + kHugeE - 1) / kHugeE;
+        for (int qb = 0; qb < Q; qb += 8) {  // 32 labels at a time
+            const int nq = QC ? QC : min(8, Q - qb);
+            const int ncopy = kHugeE * nq;
+            float4* X = reinterpret_cast<float4*>(ring);                        // [stage][entry][nq]
+            float* Wt = reinterpret_cast<float*>(X + kHugeStages * ncopy);      // [stage][entry]
+            // this thread's copies: entry (t + i threads) / nq of each chunk;
+            // their pixels are loaded two chunks before their rows
+            auto pix = [&](int c, int (&p)[kMax]) {
+#pragma unroll
+                for (int i = 0; i < kMax; i++) {
+                    const int idx = t + i * kSplatThreads;
+                    p[i] = -1;
+                    if (idx < ncopy && c < nch) {
+                        const int s = s0 + c * kHugeE + idx / nq;
+                        if (s < s1) p[i] = seg[s].x;
                     }
                 }
-                __syncwarp();  // the records are rewritten next chunk
-            }
-            if (act) vals[(long)(v + 1) * Lrow + k] = acc;
-        }
-        for (int k = L + lane; k < Lrow; k += 32) vals[(long)(v + 1) * Lrow + k] = 0.0f;  // row padding
-    }
-}
-
-// Short lists (at most kLongList entries; the tail of `order`): one thread
-// per (vertex, label), the same in-order sum without staging.
-template <bool PRE_NORM, int LC = 0>
-__global__ void splat_short_kernel(int n_short, int Lrt, const int* __restrict__ order,
-                                   const int* __restrict__ seg_start, const int* __restrict__ seg_pix,
-                                   const float* __restrict__ seg_w, const float* __restrict__ in,
-                                   const float* __restrict__ norm, float* __restrict__ vals, Live lv, int Lrow) {
-    const int L = LC ? LC : Lrt;
-    const long total = live_total(lv, n_short) * Lrow;
-    for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
-        const long u = t / Lrow;
-        const int k = (int)(t - u * Lrow);
-        const int v = order[live_unit(lv, u)];
-        if (k >= L) {  // row padding
-            vals[(long)(v + 1) * Lrow + k] = 0.0f;
-            continue;
-        }
-        const int s0 = seg_start[v], s1 = seg_start[v + 1];
-        float acc = 0.0f;
-#pragma unroll 4
-        for (int s = s0; s < s1; s++) {
-            const int p = seg_pix[s];
-            float x = in[(long)p * L + k];
-            if (PRE_NORM) x = fmul(x, norm[p]);
-            acc = fadd(acc, fmul(seg_w[s], x));
-        }
-        vals[(long)(v + 1) * Lrow + k] = acc;
-    }
-}
-
-// Block-tiled splat for L = 21.  A block takes kTV consecutive lists of the
-// visiting order at a time (a tile) and stages their entries through shared
-// memory in slabs of kSL entries per list, so that hundreds of input rows
-// are in flight per block instead of a few per warp:
-//   1. the slab's (pixel, weight) pairs of the kTV lists (coalesced) and the
-//      next tile's list ranges are loaded one step ahead into registers and
-//      published to shared memory at the start of the step;
-//   2. thread (list g, label k) copies label k of every entry of list g with
-//      cp.async into a [list][entry][label] buffer: the 21 threads of a list
-//      read one entry's 84 contiguous bytes, and the list stride (693
-//      floats, 21 mod 32) makes one warp's writes and reads conflict-free;
-//      the record owners copy the entries' norms beside them;
-//   3. thread (g, k) adds the slab to its running sum in entry order.
-// The per-(vertex, label) chain is the same sequence of float operations as
-// in every other splat form, so the values are bit-identical.  Lists longer
-// than one slab take several slabs with the sum carried in a register; the
-// visiting order puts lists of similar length next to each other.
-constexpr int kTV = 12;           // lists per tile (12 x 21 = 252 worker threads)
-constexpr int kSL = 32;           // entries per list per slab
-constexpr int kTE = kTV * kSL;    // entry slots per slab
-constexpr int kXV = kSL * 21 + 21;  // floats per list in the row buffer (21 mod 32)
-constexpr int kRV = kSL + 1;      // per-list stride of the weight / norm arrays
-constexpr int kTileThreads = 256;
-constexpr int kTileBlocksPerSM = 5;
-template <bool PRE_NORM>
-__global__ void __launch_bounds__(kTileThreads)
-    splat_tile21_kernel(int count, const int* __restrict__ order, const int* __restrict__ seg_start,
-                        const int* __restrict__ seg_pix, const float* __restrict__ seg_w,
-                        const float* __restrict__ in, const float* __restrict__ norm, float* __restrict__ vals,
-                        Live lv, int Lrow) {
-    constexpr int L = 21;
-    __shared__ __align__(16) float X[kTV * kXV];
-    __shared__ float Ws[kTV * kRV], Ns[kTV * kRV];
-    __shared__ int Ps[kTV * kRV];
-    __shared__ int tv[2][kTV], ts0[2][kTV], tn[2][kTV];
-    const int t = threadIdx.x;
-    const int g = t / L, k = t - g * L;  // worker role (t < kTV * L)
-    const bool worker = t < kTV * L;
-    const long total = live_total(lv, count);
-    const long ntiles = (total + kTV - 1) / kTV;
-    // list range (v, s0, n) of slot t < kTV of a tile
-    auto load_meta = [&](long tile, int& v, int& s0, int& n) {
-        v = -1;
-        s0 = n = 0;
-        const long u = tile * kTV + t;
-        if (tile < ntiles && u < total) {
-            v = order[live_unit(lv, u)];
-            s0 = seg_start[v];
-            n = seg_start[v + 1] - s0;
-        }
-    };
-    // (pixel, weight) of this thread's record slots j = t, t + 256 of slab s
-    // of the tile whose ranges are in buffer b
-    int rp[2] = {0, 0};
-    float rw[2] = {0.0f, 0.0f};
-    auto fetch = [&](int b, int s) {
+            };
+            auto issue = [&](int c, const int (&p)[kMax]) {
+                if (c < nch) {
+                    const int slot = c % kHugeStages;
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int j = t + h * kTileThreads;
-            rp[h] = -1;
-            if (j < kTE) {
-                const int li = j / kSL, e = s * kSL + (j - li * kSL);
-                if (e < tn[b][li]) {
-                    rp[h] = seg_pix[ts0[b][li] + e];
-                    rw[h] = seg_w[ts0[b][li] + e];
+                    for (int i = 0; i < kMax; i++) {
+                        const int idx = t + i * kSplatThreads;
+                        if (idx < ncopy && p[i] >= 0)
+                            cp_async16(X + slot * ncopy + idx, rows + (long)p[i] * Q + qb + idx % nq);
+                    }
+                    const int s = s0 + c * kHugeE + t;
+                    if (t < kHugeE && s < s1) cp_async4(Wt + slot * kHugeE + t, &seg[s].y);
                 }
-            }
-        }
-    };
-    long tile = blockIdx.x;
-    if (tile >= ntiles) return;  // block-uniform
-    int mv = -1, ms0 = 0, mn = 0;
-    if (t < kTV) {
-        load_meta(tile, mv, ms0, mn);
-        tv[0][t] = mv;
-        ts0[0][t] = ms0;
-        tn[0][t] = mn;
-        load_meta(tile + gridDim.x, mv, ms0, mn);  // in flight during the first tile
-    }
-    __syncthreads();
-    fetch(0, 0);
-    for (int it = 0; tile < ntiles; it++, tile += gridDim.x) {  // block-uniform
-        const int b = it & 1;
-        int nmax = 0;
+                cp_async_commit();
+            };
+            int pa[kMax], pb[kMax];
+            pix(0, pa);
+            pix(1, pb);
+            auto step = [&](int c) {  // chunk c's copies, then the pixels of chunk c + 2
+                issue(c, pa);
 #pragma unroll
-        for (int i = 0; i < kTV; i++) nmax = max(nmax, tn[b][i]);
-        const int nslab = (nmax + kSL - 1) / kSL;
-        float acc = 0.0f;
-        for (int s = 0; s < nslab; s++) {
-            const bool last = s + 1 == nslab;
-            __syncthreads();  // the previous step's readers of Ps / Ws / Ns / X are done
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int j = t + h * kTileThreads;
-                if (j < kTE && rp[h] >= 0) {
-                    const int li = j / kSL, r = li * kRV + (j - li * kSL);
-                    Ps[r] = rp[h];
-                    Ws[r] = rw[h];
-                    if (PRE_NORM) cp_async4(&Ns[r], norm + rp[h]);
+                for (int i = 0; i < kMax; i++) pa[i] = pb[i];
+                pix(c + 2, pb);
+            };
+#pragma unroll 1
+            for (int c = 0; c < kHugeStages - 1; c++) step(c);
+            float acc = 0.0f;
+            for (int c = 0; c < nch; c++) {
+                cp_async_wait<kHugeStages - 2>();  // chunk c has landed (this thread's copies)
+                __syncthreads();                   // ... and everyone's; chunk c - 1 is summed
+                step(c + kHugeStages - 1);
+                if (t < 4 * nq) {
+                    const int slot = c % kHugeStages;
+                    acc = splat_sum_chunk<kHugeE>(acc, reinterpret_cast<const float*>(X + slot * ncopy) + t,
+                                                  Wt + slot * kHugeE, nq, min(kHugeE, s1 - (s0 + c * kHugeE)));
                 }
-            }
-            if (last && t < kTV) {  // the next tile's ranges, loaded during this one
-                tv[b ^ 1][t] = mv;
-                ts0[b ^ 1][t] = ms0;
-                tn[b ^ 1][t] = mn;
-            }
-            __syncthreads();
-            const int n = worker ? min(kSL, tn[b][g] - s * kSL) : 0;
-            if (n > 0) {
-                const float* src = in + k;
-                float* dst = &X[g * kXV + k];
-                const int* pp = &Ps[g * kRV];
-#pragma unroll 4
-                for (int e = 0; e < n; e++) cp_async4(dst + e * L, src + (long)pp[e] * L);
-            }
-            cp_async_commit();
-            // next step's records (and, after this tile, the following tile's
-            // ranges) in flight while this slab lands and is summed
-            if (!last) {
-                fetch(b, s + 1);
-            } else {
-                fetch(b ^ 1, 0);
-                if (t < kTV) load_meta(tile + 2L * gridDim.x, mv, ms0, mn);
             }
             cp_async_wait<0>();
-            __syncthreads();
-            if (n > 0) {
-                const float* xs = &X[g * kXV + k];
-                const float* ws = &Ws[g * kRV];
-                const float* ns = &Ns[g * kRV];
-#pragma unroll 4
-                for (int e = 0; e < n; e++) {
-                    float x = xs[e * L];
-                    if (PRE_NORM) x = fmul(x, ns[e]);
-                    acc = fadd(acc, fmul(ws[e], x));
-                }
-            }
-        }
-        if (worker && tv[b][g] >= 0) vals[(long)(tv[b][g] + 1) * Lrow + k] = acc;
-        for (int q = t; q < kTV * (Lrow - L); q += kTileThreads) {  // row padding
-            const int li = q / (Lrow - L);
-            if (tv[b][li] >= 0) vals[(long)(tv[b][li] + 1) * Lrow + L + (q - li * (Lrow - L))] = 0.0f;
+            __syncthreads();  // the ring is refilled
+            if (t < 4 * nq) reinterpret_cast<float*>(vals)[((long)(v + 1) * Q + qb) * 4 + t] = acc;
         }
     }
 }
 
-// ------------------------------------------------- bulk-copy (TMA) splat --
-// 1-D bulk copies (cp.async.bulk, the TMA engine; this GPU's own memory, no
-// multicast) complete on a shared-memory mbarrier.  Waits are bounded: a
-// wait that runs out counts itself in g_bulk_wait_timeouts and the filter's
-// output rows of that tile are written as NaN, so a result never silently
-// uses unfinished copies.
-__device__ unsigned long long g_bulk_wait_timeouts = 0;
-constexpr long kBulkWaitLimit = 1L << 24;  // try_wait polls (each suspends briefly): seconds
-
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory"); }
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(ok)
-        : "r"(smem_addr(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Waits for the phase with the given parity; false if the wait ran out.
-__device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsigned parity) {
-    for (long it = 0; it < kBulkWaitLimit; it++)
-        if (mbar_try_wait(bar, parity)) return true;
-    return false;
-}
-__device__ __forceinline__ void bulk_g2s(void* sdst, const void* gsrc, unsigned bytes, unsigned long long* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-            smem_addr(sdst)),
-        "l"(gsrc), "r"(bytes), "r"(smem_addr(bar))
-        : "memory");
-}
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
-
-// Splat for L = 21 whose input rows arrive by bulk copy.  The structure is
-// splat_tile21_kernel's (tiles of kTV lists, slabs of kSL entries, the next
-// tile's ranges and records prefetched), but the rows of a slab are fetched
-// per run of consecutive pixels in a list: one cp.async.bulk of the run's
-// 16-byte-aligned byte span (at most 96 bytes per entry) into a packed
-// shared-memory buffer, issued by the run's first entry.  The rows then
-// never pass through the L1 load pipeline, which bounds the other forms.
-// Each entry records where its row starts in the buffer.  A run whose
-// aligned span would end past the input (the last pixel, when 84 N is not a
-// multiple of 16) is copied with plain loads instead.  `in` must be 16-byte
-// aligned (the host checks it and uses another form otherwise).
-constexpr int kBulkFloats = kTE * 24;  // 96 bytes per entry slot at most
-constexpr int kBulkBlocksPerSM = 4;
-template <bool PRE_NORM>
-__global__ void __launch_bounds__(kTileThreads, kBulkBlocksPerSM)
-    splat_bulk21_kernel(int count, const int* __restrict__ order, const int* __restrict__ seg_start,
-                        const int* __restrict__ seg_pix, const float* __restrict__ seg_w,
-                        const float* __restrict__ in, int N, const float* __restrict__ norm,
-                        float* __restrict__ vals, Live lv, int Lrow) {
-    constexpr int L = 21;
-    __shared__ __align__(128) float X[kBulkFloats];
-    __shared__ float Ws[kTV * kRV], Ns[kTV * kRV];
-    __shared__ int Ps[kTV * kRV], Os[kTV * kRV];
-    __shared__ int tv[2][kTV], ts0[2][kTV], tn[2][kTV];
-    __shared__ unsigned s_space, s_tx;
-    __shared__ int s_timeout;
-    __shared__ __align__(8) unsigned long long bar;
-    const int t = threadIdx.x;
-    const int g = t / L, k = t - g * L;  // worker role (t < kTV * L)
-    const bool worker = t < kTV * L;
-    const long total = live_total(lv, count);
-    const long ntiles = (total + kTV - 1) / kTV;
-    const char* in_b = reinterpret_cast<const char*>(in);
-    const char* in_end = in_b + (size_t)N * L * sizeof(float);
-    auto load_meta = [&](long tile, int& v, int& s0, int& n) {
-        v = -1;
-        s0 = n = 0;
-        const long u = tile * kTV + t;
-        if (tile < ntiles && u < total) {
-            v = order[live_unit(lv, u)];
-            s0 = seg_start[v];
-            n = seg_start[v + 1] - s0;
-        }
-    };
-    int rp[2] = {0, 0};
-    float rw[2] = {0.0f, 0.0f};
-    auto fetch = [&](int b, int s) {
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int j = t + h * kTileThreads;
-            rp[h] = -1;
-            if (j < kTE) {
-                const int li = j / kSL, e = s * kSL + (j - li * kSL);
-                if (e < tn[b][li]) {
-                    rp[h] = seg_pix[ts0[b][li] + e];
-                    rw[h] = seg_w[ts0[b][li] + e];
-                }
-            }
-        }
-    };
-    long tile = blockIdx.x;
-    if (tile >= ntiles) return;  // block-uniform
-    if (t == 0) {
-        mbar_init(&bar, 1);
-        mbar_fence_init();
+// Blocks [0, huge_blocks) take the huge lists (the first of the visiting
+// order, longest first, so that the longest chain starts at once), the next
+// long_blocks the long ones and the others the short ones: one launch, the
+// short lists filling the SMs that the long chains leave idle.  A lattice
+// without long lists launches no such blocks and no shared memory.
+// A block per huge list pays while those lists are few enough to be all
+// resident and their chains set the launch's length (at most four per SM, a
+// single image: 640x480 bilateral 50 -> 30 us); where there are more, and in
+// batches, its one adding warp would leave the SMs idle (16 images of 512x512
+// have some 4000: 345 us against 276) and they count as long lists.
+constexpr int kHugePerSM = 4;
+template <int QC>
+__global__ void __launch_bounds__(kSplatThreads)
+    splat_rows_kernel(SplatRange rl, SplatRange rs, int huge_blocks, int long_blocks, int Q,
+                      const int* __restrict__ order, const int* __restrict__ seg_start,
+                      const int2* __restrict__ seg,
+                      const float4* __restrict__ rows, float4* __restrict__ vals, float4* __restrict__ other) {
+    extern __shared__ __align__(16) unsigned char splat_smem[];
+    grid_release();
+    grid_wait();
+    if (blockIdx.x == gridDim.x - 1)  // row 0 of both value buffers: what absent neighbours read
+        for (int q = threadIdx.x; q < (QC ? QC : Q); q += blockDim.x)
+            vals[q] = other[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    int b = blockIdx.x;
+    if (b < huge_blocks) {
+        splat_rows_huge<QC>(b, Q, order, seg_start, seg, rows, vals, splat_smem);
+        return;
     }
-    int mv = -1, ms0 = 0, mn = 0;
-    if (t < kTV) {
-        load_meta(tile, mv, ms0, mn);
-        tv[0][t] = mv;
-        ts0[0][t] = ms0;
-        tn[0][t] = mn;
-        load_meta(tile + gridDim.x, mv, ms0, mn);
+    b -= huge_blocks;
+    if (b < long_blocks) {
+        const int wib = threadIdx.x >> 5;
+        splat_rows_long<QC>(rl, Q, order, seg_start, seg, rows, vals,
+                            splat_smem + wib * splat_ring_bytes(QC ? QC : min(Q, 8)), (long)b * kSplatWarps + wib,
+                            (long)long_blocks * kSplatWarps);
+        return;
     }
-    __syncthreads();
-    fetch(0, 0);
-    unsigned phase = 0;
-    for (int it = 0; tile < ntiles; it++, tile += gridDim.x) {  // block-uniform
-        const int b = it & 1;
-        int nmax = 0;
+    b -= long_blocks;
+    splat_rows_short<QC>(rs, Q, order, seg_start, seg, rows, vals, (long)b * blockDim.x + threadIdx.x,
+                         (long)(gridDim.x - huge_blocks - long_blocks) * blockDim.x);
+}
+
+// The splat for L = 1, 2 (seqCompute; also every normalisation factor): the
+// same split of lists.  A long list's warp forms 128 products at a time (lane
+// = entry, the next 128 entries' values in flight) and lanes 0 .. L-1 add
+// them in entry order from shared memory; a short list takes one thread per
+// label.
+constexpr int kThinE = 128;  // entries per step of a long list
+
+template <int L>
+__global__ void __launch_bounds__(kSplatThreads)
+    splat_thin_kernel(SplatRange rl, SplatRange rs, int long_blocks, const int* __restrict__ order,
+                      const int* __restrict__ seg_start, const int2* __restrict__ seg, const float* __restrict__ in, const float* __restrict__ norm,
+                      float* __restrict__ vals, float* __restrict__ other) {
+    __shared__ __align__(16) float prod[kSplatWarps][L][kThinE];
+    constexpr int U = kThinE / 32;
+    grid_release();
+    grid_wait();
+    if (blockIdx.x == 0 && threadIdx.x < L) vals[threadIdx.x] = other[threadIdx.x] = 0.0f;  // absent neighbours
+    if ((int)blockIdx.x < long_blocks) {
+        const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const long total = live_total(rl.lv, rl.count);
+        for (long unit = (long)blockIdx.x * kSplatWarps + wib; unit < total;
+             unit += (long)long_blocks * kSplatWarps) {  // warp-uniform
+            const int v = splat_vertex(rl, order, unit);
+            const int s0 = seg_start[v], s1 = seg_start[v + 1];
+            int p[U];
+            float w[U], wc[U], x[U][L];
+            auto load_pw = [&](int c) {
 #pragma unroll
-        for (int i = 0; i < kTV; i++) nmax = max(nmax, tn[b][i]);
-        const int nslab = (nmax + kSL - 1) / kSL;
-        float acc = 0.0f;
-        bool bad = false;
-        for (int s = 0; s < nslab; s++) {
-            const bool last = s + 1 == nslab;
-            __syncthreads();  // the previous step's readers of the shared arrays are done
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int j = t + h * kTileThreads;
-                if (j < kTE && rp[h] >= 0) {
-                    const int li = j / kSL, r = li * kRV + (j - li * kSL);
-                    Ps[r] = rp[h];
-                    Ws[r] = rw[h];
-                    if (PRE_NORM) cp_async4(&Ns[r], norm + rp[h]);
+                for (int i = 0; i < U; i++) {
+                    const int s = min(c + i * 32 + lane, s1 - 1);
+                    const int2 e = seg[s];
+                    p[i] = e.x;
+                    w[i] = entry_w(e);
                 }
-            }
-            if (last && t < kTV) {
-                tv[b ^ 1][t] = mv;
-                ts0[b ^ 1][t] = ms0;
-                tn[b ^ 1][t] = mn;
-            }
-            if (t == 0) {
-                s_space = 0;
-                s_tx = 0;
-                s_timeout = 0;
-            }
-            __syncthreads();
-            // runs of consecutive pixels: the first entry of each places the
-            // run in the buffer and records every entry's row start
-            const char* rsrc[2] = {nullptr, nullptr};
-            unsigned rdst[2] = {0, 0}, rbytes[2] = {0, 0};
+            };
+            auto load_x = [&] {  // the values of the entries p, scaled; their weights become wc
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int j = t + h * kTileThreads;
-                if (j >= kTE || rp[h] < 0) continue;
-                const int li = j / kSL, el = j - li * kSL, base = li * kRV;
-                const int n = min(kSL, tn[b][li] - s * kSL);
-                const int p = Ps[base + el];
-                if (el > 0 && Ps[base + el - 1] == p - 1) continue;  // not a run start
-                int len = 1;
-                while (el + len < n && Ps[base + el + len] == p + len) len++;
-                const char* b0 = in_b + (size_t)p * (L * sizeof(float));
-                const char* b1 = b0 + (size_t)len * (L * sizeof(float));
-                const char* a0 = reinterpret_cast<const char*>(reinterpret_cast<uintptr_t>(b0) & ~(uintptr_t)15);
-                const char* a1 =
-                    reinterpret_cast<const char*>((reinterpret_cast<uintptr_t>(b1) + 15) & ~(uintptr_t)15);
-                const unsigned bytes = (unsigned)(a1 - a0);
-                const unsigned off = atomicAdd(&s_space, bytes);  // bytes and offsets: multiples of 16
-                const int row0 = (int)((off + (unsigned)(b0 - a0)) / sizeof(float));
-                for (int i = 0; i < len; i++) Os[base + el + i] = row0 + i * L;
-                if (a1 <= in_end) {
-                    atomicAdd(&s_tx, bytes);
-                    rsrc[h] = a0;
-                    rdst[h] = off;
-                    rbytes[h] = bytes;
-                } else {  // the span would pass the end of the input: plain loads
-                    for (int i = 0; i < len * L; i++) X[row0 + i] = in[(size_t)p * L + i];
-                }
-            }
-            fence_proxy_async_smem();  // this thread's generic writes of X before any async copy
-            __syncthreads();
-            // the phase's byte count before any copy can complete against it
-            if (t == 0) mbar_expect_tx(&bar, s_tx);
-            __syncthreads();
+                for (int i = 0; i < U; i++) {
+                    const float nn = norm ? norm[p[i]] : 1.0f;
+                    wc[i] = w[i];
 #pragma unroll
-            for (int h = 0; h < 2; h++)
-                if (rbytes[h]) bulk_g2s(reinterpret_cast<char*>(X) + rdst[h], rsrc[h], rbytes[h], &bar);
-            cp_async_commit();
-            if (!last) {
-                fetch(b, s + 1);
-            } else {
-                fetch(b ^ 1, 0);
-                if (t < kTV) load_meta(tile + 2L * gridDim.x, mv, ms0, mn);
-            }
-            cp_async_wait<0>();
-            if (!mbar_wait_bounded(&bar, phase)) s_timeout = 1;
-            phase ^= 1;
-            __syncthreads();
-            if (s_timeout) bad = true;
-            const int n = worker ? min(kSL, tn[b][g] - s * kSL) : 0;
-            if (n > 0) {
-                const int* os = &Os[g * kRV];
-                const float* ws = &Ws[g * kRV];
-                const float* ns = &Ns[g * kRV];
-#pragma unroll 4
-                for (int e = 0; e < n; e++) {
-                    float x = X[os[e] + k];
-                    if (PRE_NORM) x = fmul(x, ns[e]);
-                    acc = fadd(acc, fmul(ws[e], x));
+                    for (int k = 0; k < L; k++) {
+                        x[i][k] = in[(long)p[i] * L + k];
+                        if (norm) x[i][k] = fmul(x[i][k], nn);
+                    }
                 }
+            };
+            load_pw(s0);
+            load_x();
+            load_pw(s0 + kThinE);  // past the end: the last entry again
+            float acc = 0.0f;
+            for (int c = s0; c < s1; c += kThinE) {
+#pragma unroll
+                for (int i = 0; i < U; i++)
+#pragma unroll
+                    for (int k = 0; k < L; k++) prod[wib][k][i * 32 + lane] = fmul(wc[i], x[i][k]);
+                if (c + kThinE < s1) {  // in flight while this step is added
+                    load_x();
+                    load_pw(c + 2 * kThinE);
+                }
+                __syncwarp();
+                if (lane < L) {
+                    const int n = min(kThinE, s1 - c);
+                    const float* pr = prod[wib][lane];
+                    int e = 0;
+                    for (; e + 16 <= n; e += 16) {
+                        float4 q[4];
+#pragma unroll
+                        for (int g = 0; g < 4; g++) q[g] = reinterpret_cast<const float4*>(pr + e)[g];
+#pragma unroll
+                        for (int g = 0; g < 4; g++) {
+                            acc = fadd(acc, q[g].x);
+                            acc = fadd(acc, q[g].y);
+                            acc = fadd(acc, q[g].z);
+                            acc = fadd(acc, q[g].w);
+                        }
+                    }
+                    for (; e < n; e++) acc = fadd(acc, pr[e]);
+                }
+                __syncwarp();  // prod is rewritten next step
             }
+            if (lane < L) vals[(long)(v + 1) * L + lane] = acc;
         }
-        if (bad && t == 0) atomicAdd(&g_bulk_wait_timeouts, 1ull);
-        if (worker && tv[b][g] >= 0) vals[(long)(tv[b][g] + 1) * Lrow + k] = bad ? __int_as_float(0x7fc00000) : acc;
-        for (int q = t; q < kTV * (Lrow - L); q += kTileThreads) {  // row padding
-            const int li = q / (Lrow - L);
-            if (tv[b][li] >= 0) vals[(long)(tv[b][li] + 1) * Lrow + L + (q - li * (Lrow - L))] = 0.0f;
+    } else {
+        const long total = live_total(rs.lv, rs.count) * L;
+        const long nt = (long)(gridDim.x - long_blocks) * blockDim.x;
+        for (long t = (long)(blockIdx.x - long_blocks) * blockDim.x + threadIdx.x; t < total; t += nt) {
+            const long u = t / L;
+            const int k = (int)(t - u * L);
+            const int v = splat_vertex(rs, order, u);
+            const int s0 = seg_start[v], s1 = seg_start[v + 1];
+            float acc = 0.0f;
+            for (int s = s0; s < s1; s += 8) {
+                float y[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const int si = min(s + i, s1 - 1);
+                    const int2 e = seg[si];
+                    const int p = e.x;
+                    float x = in[(long)p * L + k];
+                    if (norm) x = fmul(x, norm[p]);
+                    y[i] = fmul(entry_w(e), x);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    if (s + i < s1) acc = fadd(acc, y[i]);
+            }
+            vals[(long)(v + 1) * L + k] = acc;
         }
     }
 }
@@ -982,8 +918,8 @@ __global__ void count_long_kernel(int M, const int* __restrict__ counts, int thr
     if ((threadIdx.x & 31) == 0 && b) atomicAdd(n, __popc(b));
 }
 
-// Class of a splat list by its length: 0 huge, 1 long, 2 short.
-__device__ __forceinline__ int list_class(int c) { return c > kHugeList ? 0 : c > kLongList ? 1 : 2; }
+// Class of a splat list by its length: 0 long, 1 short.
+__device__ __forceinline__ int list_class(int c) { return c > kLongList ? 0 : 1; }
 
 // Concatenated lattices: the key (class, image) of each position of the
 // length-sorted visiting order, for a second stable sort that groups each
@@ -1022,6 +958,8 @@ template <bool SEQ, int LC = 0>
 __global__ void blur_kernel(int M, int Lrt, const int2* __restrict__ nbr,
                             const float* __restrict__ src, float* __restrict__ dst, Live lv) {
     const int L = LC ? LC : Lrt;
+    grid_release();
+    grid_wait();
     const long total = live_total(lv, M) * L;
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
         const long u = t / L;
@@ -1041,11 +979,14 @@ __global__ void blur_kernel(int M, int Lrt, const int2* __restrict__ nbr,
 // one thread per (vertex, four labels), float4 loads of the vertex's row and
 // of its two neighbours' rows.  The same operations per element as
 // blur_kernel; the padding lanes hold zeros and stay zero.
-template <int Q>
+// SEQ: the half-sum in double, as blur_kernel<true> (the lattice gradient).
+template <int Q, bool SEQ = false>
 __global__ void blur4_kernel(int M, int Qrt, const int2* __restrict__ nbr, const float* __restrict__ src,
                              float* __restrict__ dst, Live lv) {
     const int Qn = Q ? Q : Qrt;
     const long lp = 4L * Qn;
+    grid_release();
+    grid_wait();
     const long total = live_total(lv, M) * Qn;
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
         const long u = t / Qn;
@@ -1055,11 +996,11 @@ __global__ void blur4_kernel(int M, int Qrt, const int2* __restrict__ nbr, const
         const float4 a = *reinterpret_cast<const float4*>(src + (long)(v + 1) * lp + 4 * q);
         const float4 x = *reinterpret_cast<const float4*>(src + (long)nb.x * lp + 4 * q);
         const float4 y = *reinterpret_cast<const float4*>(src + (long)nb.y * lp + 4 * q);
-        float4 r;
-        r.x = fadd(a.x, fmul(0.5f, fadd(x.x, y.x)));
-        r.y = fadd(a.y, fmul(0.5f, fadd(x.y, y.y)));
-        r.z = fadd(a.z, fmul(0.5f, fadd(x.z, y.z)));
-        r.w = fadd(a.w, fmul(0.5f, fadd(x.w, y.w)));
+        auto one = [](float c, float n1, float n2) {
+            const float s = fadd(n1, n2);
+            return SEQ ? (float)dadd((double)c, dmul(0.5, (double)s)) : fadd(c, fmul(0.5f, s));
+        };
+        const float4 r = make_float4(one(a.x, x.x, y.x), one(a.y, x.y, y.y), one(a.z, x.z, y.z), one(a.w, x.w, y.w));
         *reinterpret_cast<float4*>(dst + (long)(v + 1) * lp + 4 * q) = r;
     }
 }
@@ -1082,6 +1023,8 @@ __global__ void slice_kernel(int N, int Lrt, int drt, const int* __restrict__ of
                              float alpha, float* out, SliceEpilogue ep, Live lv) {
     const int L = LC ? LC : Lrt, d = DC ? DC : drt;
     const int d1 = d + 1;
+    grid_release();
+    grid_wait();
     const long total = live_total(lv, N) * L;
     for (long tl = (long)blockIdx.x * blockDim.x + threadIdx.x; tl < total; tl += (long)gridDim.x * blockDim.x) {
         const long u = tl / L;
@@ -1101,92 +1044,135 @@ __global__ void slice_kernel(int N, int Lrt, int drt, const int* __restrict__ of
     }
 }
 
-// Slice over rows padded to Lp = 4 Q floats (sseCompute, L > 2), a tile of
-// `tile` pixels per block (kSliceTile, fewer for very wide rows): the
-// tile's offsets, (barycentric * alpha) weights and normalisation factors
-// are staged once in shared memory (coalesced: they are contiguous), every
-// (pixel, four labels) item gathers the d+1 vertex rows with float4 loads
-// and applies the per-pixel part of the epilogue (norm, compatibility
-// scale), and the tile's L outputs per pixel -- contiguous in `out` --
-// leave through shared memory, coalesced, with the accumulation part
-// (base + coef * v).  Per element the arithmetic is slice_kernel's and
-// apply_epilogue's: acc = sum over j in order of (bary_j * alpha) *
-// value_j, from +0.
-constexpr int kSliceTile = 128;
-constexpr int kSliceThreads = 256;
-template <int DC, int Q, int LC>
-__global__ void __launch_bounds__(kSliceThreads)
-    slice4_kernel(int N, int Lrt, int Qrt, int drt, int tile, const int* __restrict__ offset,
-                  const float* __restrict__ bary, const float* __restrict__ vals, float alpha, float* out,
-                  SliceEpilogue ep, Live lv, const long* __restrict__ pix_base) {
+// Slice over rows of Q float4 (sseCompute, L > 2), a tile of pixels per warp
+// (no block barrier: the warps' loads overlap each other's sums).  The tile's
+// (row, barycentric * alpha) pairs and normalisation factors are staged in
+// shared memory and the accumulation base (out = base + coef * v) is copied
+// there asynchronously meanwhile; then lane (p, q) -- for L = 21 five pixels of
+// six 16-byte groups per instruction -- gathers its pixel's d+1 vertex rows
+// with 16-byte loads, applies the epilogue and leaves its four labels in shared
+// memory, and the tile, contiguous in `out`, is stored with 16-byte accesses
+// where the pointers allow (vec).  Per element the arithmetic is
+// slice_kernel's and apply_epilogue's: acc = sum over j in order of (bary_j *
+// alpha) * value_j, from +0.
+// DOT: `out` is not written; the warp's FP64 sum of dot[e] * v[e] goes to
+// partials[warp] instead.
+constexpr int kSliceWarps = 4;
+constexpr int kSliceTile = 20;  // pixels per warp tile (4 rounds of 5 at L = 21)
+template <int DC, int Q, int LC, bool DOT>
+__global__ void __launch_bounds__(32 * kSliceWarps)
+    slice_rows_kernel(int N, int Lrt, int Qrt, int drt, int tile, const int* __restrict__ offset,
+                      const float* __restrict__ bary, const float4* __restrict__ vals, float alpha, float* out,
+                      SliceEpilogue ep, Live lv, const long* __restrict__ pix_base, int vec,
+                      const float* __restrict__ dot, double* __restrict__ partials) {
     extern __shared__ __align__(16) unsigned char slice_smem[];
     const int d1 = (DC ? DC : drt) + 1, Qn = Q ? Q : Qrt, L = LC ? LC : Lrt;
-    const long lp = 4L * Qn;
-    int* s_off = reinterpret_cast<int*>(slice_smem);
-    float* s_wa = reinterpret_cast<float*>(s_off + tile * d1);
-    float* s_nrm = s_wa + tile * d1;
-    float* s_out = s_nrm + tile;
+    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tf = (tile * L + 3) & ~3;  // floats of the output tile
+    unsigned char* mine = slice_smem + (size_t)wib * ((tf * 4 + tile * (d1 * 8 + 8) + 15) & ~15);
+    float* s_out = reinterpret_cast<float*>(mine);               // [tile][L]
+    int2* s_ow = reinterpret_cast<int2*>(s_out + tf);            // [tile][d1]
+    float* s_nrm = reinterpret_cast<float*>(s_ow + tile * d1);   // [tile]
     const bool use_norm = ep.potts && ep.norm;
+    const float* base = DOT ? dot : ep.base;
+    const int ppr = Qn <= 32 ? 32 / Qn : 1;       // pixels per round (Qn <= 32)
+    const int lp = Qn <= 32 ? lane / Qn : 0;      // this lane's pixel of the round
+    const int q0 = Qn <= 32 ? lane - lp * Qn : lane;
+    double g = 0.0;
+    grid_release();
+    grid_wait();
     // Tiles: of the whole pixel range, or (live images) of each live image's
     // pixels, image by image (pix_base: its pixel offsets).
     const long total = live_total(lv, ((long)N + tile - 1) / tile);
-    for (long u = blockIdx.x; u < total; u += gridDim.x) {  // block-uniform
-        long p0, pend = N;
-        if (lv.n) {
-            long local;
-            const int img = live_locate(lv, u, local);
-            p0 = pix_base[img] + local * tile;
-            pend = pix_base[img + 1];
-        } else {
-            p0 = u * tile;
-        }
-        const int np = (int)min((long)tile, pend - p0);
-        for (int e = threadIdx.x; e < np * d1; e += blockDim.x) {
-            s_off[e] = offset[p0 * d1 + e];
-            s_wa[e] = fmul(bary[p0 * d1 + e], alpha);
-        }
-        if (use_norm)
-            for (int e = threadIdx.x; e < np; e += blockDim.x) s_nrm[e] = ep.norm[p0 + e];
-        __syncthreads();
-        for (int it = threadIdx.x; it < np * Qn; it += blockDim.x) {
-            const int pl = it / Qn, q = it - pl * Qn;
-            float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-            for (int j = 0; j < (DC ? DC + 1 : 17); j++) {
-                if (!DC && j >= d1) break;
-                const int o = s_off[pl * d1 + j];
-                const float wa = s_wa[pl * d1 + j];
-                const float4 v = *reinterpret_cast<const float4*>(vals + (long)(o + 1) * lp + 4 * q);
-                a[0] = fadd(a[0], fmul(wa, v.x));
-                a[1] = fadd(a[1], fmul(wa, v.y));
-                a[2] = fadd(a[2], fmul(wa, v.z));
-                a[3] = fadd(a[3], fmul(wa, v.w));
-            }
-            const int k0 = 4 * q;
-            float* so = s_out + pl * L + k0;
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                if (k0 + c >= L) break;
-                float v = a[c];
-                if (ep.potts) {
-                    if (use_norm) v = fmul(v, s_nrm[pl]);
-                    v = ep.scale_vec ? fmul(ep.scale_vec[k0 + c], v) : fmul(ep.scale, v);
-                }
-                so[c] = v;
-            }
-        }
-        __syncthreads();
+    for (long u = (long)blockIdx.x * kSliceWarps + wib; u < total; u += (long)gridDim.x * kSliceWarps) {
+        long p0;
+        const int np = tile_pixels(lv, pix_base, u, tile, N, p0);
         const long t0 = p0 * L;
         const int ne = np * L;
-        if (ep.base) {
-            for (int e = threadIdx.x; e < ne; e += blockDim.x)
-                out[t0 + e] = fadd(ep.base[t0 + e], fmul(ep.coef, s_out[e]));
-        } else if (ep.zero_base) {
-            for (int e = threadIdx.x; e < ne; e += blockDim.x) out[t0 + e] = fadd(0.0f, fmul(ep.coef, s_out[e]));
-        } else {
-            for (int e = threadIdx.x; e < ne; e += blockDim.x) out[t0 + e] = s_out[e];
+        const int n4 = vec && (t0 & 3) == 0 ? ne >> 2 : 0;  // whole 16-byte groups of the tile
+        if (base) {
+            for (int e = lane; e < n4; e += 32) cp_async16(s_out + 4 * e, base + t0 + 4 * e);
+            for (int e = 4 * n4 + lane; e < ne; e += 32) cp_async4(s_out + e, base + t0 + e);
         }
-        __syncthreads();  // the next tile restages the shared arrays
+        cp_async_commit();
+        for (int e = lane; e < np * d1; e += 32)
+            s_ow[e] = make_int2((offset[p0 * d1 + e] + 1) * Qn, __float_as_int(fmul(bary[p0 * d1 + e], alpha)));
+        if (use_norm)
+            for (int e = lane; e < np; e += 32) s_nrm[e] = ep.norm[p0 + e];
+        cp_async_wait<0>();
+        __syncwarp();
+        auto item = [&](int pl, int q) {
+            const int2* ow = s_ow + pl * d1;
+            const float4* vq = vals + q;
+            unsigned long long a0 = 0ull, a1 = 0ull;
+            auto add = [&](int2 e) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(vq + e.x);
+                const float wa = __int_as_float(e.y);
+                a0 = add_mul2(a0, wa, v.x);
+                a1 = add_mul2(a1, wa, v.y);
+            };
+            if (DC) {
+#pragma unroll
+                for (int j = 0; j < DC + 1; j++) add(ow[j]);
+            } else {
+                for (int j = 0; j < d1; j++) add(ow[j]);
+            }
+            const float2 lo = unpack2(a0), hi = unpack2(a1);
+            float v[4] = {lo.x, lo.y, hi.x, hi.y};
+            const int k0 = 4 * q;
+            float* so = s_out + pl * L + k0;
+            if (use_norm) {
+                const float nn = s_nrm[pl];
+#pragma unroll
+                for (int c = 0; c < 4; c++) v[c] = fmul(v[c], nn);
+            }
+            if (ep.potts) {
+                if (ep.scale_vec) {
+#pragma unroll
+                    for (int c = 0; c < 4; c++)
+                        if (k0 + c < L) v[c] = fmul(ep.scale_vec[k0 + c], v[c]);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 4; c++) v[c] = fmul(ep.scale, v[c]);
+                }
+            }
+            if (DOT) {
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    if (k0 + c < L) g += (double)so[c] * (double)v[c];
+                return;
+            }
+            if (base) {
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    if (k0 + c < L) so[c] = fadd(so[c], fmul(ep.coef, v[c]));
+            } else {
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    if (k0 + c < L) so[c] = ep.zero_base ? fadd(0.0f, fmul(ep.coef, v[c])) : v[c];
+            }
+        };
+        if (Qn <= 32) {
+            if (lp < ppr) {
+#pragma unroll 2
+                for (int pl = lp; pl < np; pl += ppr) item(pl, q0);
+            }
+        } else {
+            for (int pl = 0; pl < np; pl++)
+                for (int q = q0; q < Qn; q += 32) item(pl, q);
+        }
+        __syncwarp();
+        if (!DOT) {
+            float4* o4 = reinterpret_cast<float4*>(out + t0);
+            for (int e = lane; e < n4; e += 32) o4[e] = reinterpret_cast<const float4*>(s_out)[e];
+            for (int e = 4 * n4 + lane; e < ne; e += 32) out[t0 + e] = s_out[e];
+            __syncwarp();  // the next tile restages the shared arrays
+        }
+    }
+    if (DOT) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) g += __shfl_down_sync(0xffffffffu, g, o);
+        if (lane == 0) partials[(long)blockIdx.x * kSliceWarps + wib] = g;
     }
 }
 
@@ -1274,17 +1260,6 @@ __device__ __forceinline__ float ord_mask_upper(float cu, int b) {
     asm("sub.rn.sat.f32 %0, %1, %2;" : "=f"(m) : "f"((float)b + 1.0f), "f"(cu));
     return m;
 }
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(unsigned long long v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-
 template <bool UPPER>
 __device__ __forceinline__ void ord_accumulate(float (&acc)[kRes], float c, float w) {
 #pragma unroll
@@ -1307,7 +1282,7 @@ __device__ __forceinline__ void ord_consume(float (&acc)[kRes], const float (*ri
 // that the slice's per-label bin reads coalesce.
 __global__ void __launch_bounds__(32 * kStageWarps)
     ord_splat_kernel(int M, int L, const int* __restrict__ order, const int* __restrict__ seg_start,
-                     const int* __restrict__ seg_pix, const float* __restrict__ seg_w,
+                     const int2* __restrict__ seg,
                      const float2* __restrict__ bins, float* __restrict__ vals) {
     __shared__ float ring[kStageWarps][kStages][kChunk][32];
     __shared__ float mw[kStageWarps][kStages][kChunk];
@@ -1324,11 +1299,11 @@ __global__ void __launch_bounds__(32 * kStageWarps)
         float acc[kRes];
 #pragma unroll
         for (int b = 0; b < kRes; b++) acc[b] = 0.0f;
-        stream_list<float, false>(s0, s1, 2 * L, 2 * k + (upper ? 1 : 0), act, lane, seg_pix, seg_w, bf, nullptr,
-                                  ring[wib], mw[wib], nullptr, [&](int slot, int n) {
-                                      if (upper) ord_consume<true>(acc, ring[wib][slot], mw[wib][slot], lane, n);
-                                      else ord_consume<false>(acc, ring[wib][slot], mw[wib][slot], lane, n);
-                                  });
+        stream_list<float>(s0, s1, 2 * L, 2 * k + (upper ? 1 : 0), act, lane, seg, bf, ring[wib], mw[wib],
+                           [&](int slot, int n) {
+                               if (upper) ord_consume<true>(acc, ring[wib][slot], mw[wib][slot], lane, n);
+                               else ord_consume<false>(acc, ring[wib][slot], mw[wib][slot], lane, n);
+                           });
         if (act) {
             float* row = vals + ((long)(v + 1) * kOrdW + (upper ? kRes : 0)) * L + k;
 #pragma unroll
@@ -1393,8 +1368,7 @@ size_t ord_block_smem(int kb) {
 template <int G>
 __global__ void __launch_bounds__(kOrdBlockMaxL * G < 1024 ? kOrdBlockMaxL * G : 1024)
     ord_splat_block_kernel(int L, int kb, int kblocks, const int* __restrict__ order,
-                           const int* __restrict__ seg_start, const int* __restrict__ seg_pix,
-                           const float* __restrict__ seg_w, const float2* __restrict__ bins,
+                           const int* __restrict__ seg_start, const int2* __restrict__ seg, const float2* __restrict__ bins,
                            float* __restrict__ vals) {
     extern __shared__ __align__(16) float osm[];
     float* xr = osm;                            // [kOXS][kb][kORow]
@@ -1414,9 +1388,9 @@ __global__ void __launch_bounds__(kOrdBlockMaxL * G < 1024 ? kOrdBlockMaxL * G :
         if (c < nch && t < kOE) {
             const int slot = c % kOPS, e = s0 + c * kOE + t;
             if (e < s1) {
-                cp_async4(&pr[slot * kOE + t], seg_pix + e);
-                cp_async4(&wr[(slot * kOE + t) * 2], seg_w + e);
-                cp_async4(&wr[(slot * kOE + t) * 2 + 1], seg_w + e);
+                cp_async4(&pr[slot * kOE + t], &seg[e].x);
+                cp_async4(&wr[(slot * kOE + t) * 2], &seg[e].y);
+                cp_async4(&wr[(slot * kOE + t) * 2 + 1], &seg[e].y);
             } else {
                 pr[slot * kOE + t] = 0;
                 wr[(slot * kOE + t) * 2] = 0.0f;
@@ -1532,8 +1506,7 @@ __global__ void __launch_bounds__(kOrdBlockMaxL * G < 1024 ? kOrdBlockMaxL * G :
 // passes, without staging.
 template <int LC = 0>
 __global__ void ord_splat_short_kernel(int n_short, int Lrt, const int* __restrict__ order,
-                                       const int* __restrict__ seg_start, const int* __restrict__ seg_pix,
-                                       const float* __restrict__ seg_w, const float2* __restrict__ bins,
+                                       const int* __restrict__ seg_start, const int2* __restrict__ seg, const float2* __restrict__ bins,
                                        float* __restrict__ vals) {
     const int L = LC ? LC : Lrt;
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1550,8 +1523,8 @@ __global__ void ord_splat_short_kernel(int n_short, int Lrt, const int* __restri
     for (int b = 0; b < kRes; b++) lo[b] = up[b] = 0.0f;
 #pragma unroll 2
     for (int s = s0; s < s1; s++) {
-        const float2 x = bins[(long)seg_pix[s] * L + k];
-        const float w = seg_w[s];
+        const float2 x = bins[(long)seg[s].x * L + k];
+        const float w = entry_w(seg[s]);
         lo[0] = fadd(lo[0], w);
 #pragma unroll
         for (int b = 1; b < kRes; b++) lo[b] = __fmaf_rn(ord_mask_lower(x.x, b), w, lo[b]);
@@ -1932,9 +1905,8 @@ void build_impl(Lattice& L, const float* d_features) {
     launch(iota_copy_kernel, ceil_div(Ereal, kTB), kTB, 0, st, (int)Ereal, offset, skeys, svals);
     DCRF_LAUNCH_CHECK();
     radix_sort_pairs(skeys, svals, (int)Ereal, bits_for(M), L.sort, st);
-    int* seg_pix = L.seg_pix.ensure(Ereal);
-    float* seg_w = L.seg_w.ensure(Ereal);
-    launch(seg_fill_kernel, ceil_div(Ereal, kTB), kTB, 0, st, (int)Ereal, d1, svals, bary, seg_pix, seg_w);
+    int2* seg = L.seg.ensure(Ereal + kSegPad);
+    launch(seg_fill_kernel, ceil_div(Ereal, kTB), kTB, 0, st, (int)Ereal, d1, svals, bary, seg);
     // Splat visiting order: longest lists first.
     int* vorder = L.vorder.ensure(M);
     int* okeys = L.vorder_keys.ensure(M);
@@ -1955,6 +1927,20 @@ void build_impl(Lattice& L, const float* d_features) {
 
 }  // namespace
 
+// Row stride of the plain filter's value buffers: L padded to a multiple of
+// four (float4 rows) on the sseCompute path (L > 2); seqCompute (L <= 2)
+// keeps L.
+static int value_row(int L) { return L > 2 ? (L + 3) & ~3 : L; }
+
+// Blocks of a launch over `units` work items, `per_block` per block of
+// `threads` threads: all of them at once, or -- with live images, whose
+// units are counted on the device -- twice as many blocks as the SMs hold
+// at full occupancy, looping over them.
+static int unit_grid(long units, int per_block, bool live, int threads) {
+    const long g = std::max(1L, (units + per_block - 1) / per_block);
+    return live ? (int)std::min(g, (long)sm_count() * 2 * (2048 / threads)) : (int)g;
+}
+
 namespace {
 
 // ----------------------------------------------------- feature gradient --
@@ -1971,7 +1957,7 @@ struct GradScale {
 };
 
 template <int DM>
-__global__ void grad_slice_kernel(int N, int L, int d, const int* __restrict__ offset, const int* __restrict__ rank,
+__global__ void grad_slice_kernel(int N, int L, int Lp, int d, const int* __restrict__ offset, const int* __restrict__ rank,
                                   const float* __restrict__ vals, const float* __restrict__ x, float alpha,
                                   GradScale sf, float* __restrict__ df) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1994,7 +1980,7 @@ __global__ void grad_slice_kernel(int N, int L, int d, const int* __restrict__ o
 #pragma unroll
         for (int j = 0; j <= DM; j++)
             if (j <= d)
-                ra[j] = fsub(fadd(0.0f, fmul(alpha, vals[(long)o0[j] * L + k])), fmul(alpha, vals[(long)o1[j] * L + k]));
+                ra[j] = fsub(fadd(0.0f, fmul(alpha, vals[(long)o0[j] * Lp + k])), fmul(alpha, vals[(long)o1[j] * Lp + k]));
         const float xk = x[(long)i * L + k];
         float sm = ra[0];
 #pragma unroll
@@ -2014,33 +2000,28 @@ template <int DM>
 void gradient_impl(Lattice& lat, float* df, const float* a, const float* b, int L) {
     cudaStream_t st = lat.stream;
     const int N = lat.N, d = lat.d, M = lat.M;
-    lat.ensure_values((size_t)L);
+    const int Lp = value_row(L), Q = Lp / 4;
+    lat.ensure_values((size_t)Lp);
     DCRF_CUDA(cudaMemsetAsync(df, 0, sizeof(float) * (size_t)N * d, st));
     // scale_factor and alpha as the reference computes them (:1104-1111)
     GradScale sf{};
     const float inv_std_dev = std::sqrt(2.0 / 3.0) * (d + 1);
     for (int i = 0; i < d; i++) sf.s[i] = 1.0 / std::sqrt(double((i + 2) * (i + 1))) * inv_std_dev;
     const float alpha = 1.0f / (1 + std::pow(2.0f, (float)-d)) / (d + 1);
-    const int n_short = M - lat.n_long;
-    const long ML = (long)M * L, SL = (long)n_short * L;
+    const long ML = (long)M * L, MQ = (long)M * Q;
     for (int dir = 0; dir < 2; dir++) {
         const float* in = dir ? b : a;
         float *src = lat.va.get(), *dst = lat.vb.get();
-        if (lat.n_long)
-            launch(splat_kernel<false>, ceil_div(lat.n_long, kStageWarps), 32 * kStageWarps, 0, st, lat.n_long, L,
-                   lat.vorder.get(), lat.seg_start.get(), lat.seg_pix.get(), lat.seg_w.get(), in, nullptr, src,
-                   Live{}, L);
-        if (n_short)
-            launch(splat_short_kernel<false>, ceil_div(SL, kTB), kTB, 0, st, n_short, L,
-                   lat.vorder.get() + lat.n_long, lat.seg_start.get(), lat.seg_pix.get(), lat.seg_w.get(), in,
-                   nullptr, src, Live{}, L);
+        lat.splat(in, L, nullptr, src);
         for (int jj = 0; jj <= d; jj++) {
             const int j = dir ? d - jj : jj;
-            launch(blur_kernel<true>, ceil_div(ML, kTB), kTB, 0, st, M, L, lat.nbr.get() + (long)j * M, src, dst,
-                   Live{});
+            const int2* nb = lat.nbr.get() + (long)j * M;
+            if (L <= 2) launch_chained(blur_kernel<true>, ceil_div(ML, kTB), kTB, 0, st, M, L, nb, src, dst, Live{});
+            else if (Q == 6) launch_chained(blur4_kernel<6, true>, ceil_div(MQ, kTB), kTB, 0, st, M, Q, nb, src, dst, Live{});
+            else launch_chained(blur4_kernel<0, true>, ceil_div(MQ, kTB), kTB, 0, st, M, Q, nb, src, dst, Live{});
             std::swap(src, dst);
         }
-        launch(grad_slice_kernel<DM>, ceil_div(N, 128), 128, 0, st, N, L, d, lat.offset.get(), lat.rank.get(), src,
+        launch(grad_slice_kernel<DM>, ceil_div(N, 128), 128, 0, st, N, L, Lp, d, lat.offset.get(), lat.rank.get(), src,
                dir ? a : b, alpha, sf, df);
     }
     DCRF_LAUNCH_CHECK();
@@ -2067,6 +2048,11 @@ namespace {
 __global__ void add_offset_kernel(long n, const int* __restrict__ src, int add, int* __restrict__ dst) {
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) dst[t] = src[t] + add;
+}
+
+__global__ void seg_offset_kernel(long n, const int2* __restrict__ src, int add, int2* __restrict__ dst) {
+    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n) dst[t] = make_int2(src[t].x + add, src[t].y);
 }
 
 // Neighbour rows are vertex + 1, with 0 for "absent".
@@ -2108,8 +2094,7 @@ void Lattice::concat(const std::vector<const Lattice*>& parts) {
     int* rk = rank.ensure(E);
     float* by = bary.ensure(E);
     int* ss = seg_start.ensure(M + 1);
-    int* sp = seg_pix.ensure(E);
-    float* sw = seg_w.ensure(E);
+    int2* sg = seg.ensure(E + kSegPad);
     int2* nb = nbr.ensure((size_t)d1 * M);
     int* vi = vimg.ensure(std::max(M, 1));
     long pb = 0, vb_ = 0;
@@ -2127,8 +2112,7 @@ void Lattice::concat(const std::vector<const Lattice*>& parts) {
                 launch(nbr_offset_kernel, ceil_div(p->M, kTB), kTB, 0, st, (long)p->M,
                        p->nbr.get() + (long)j * p->M, (int)vb_, nb + (long)j * M + vb_);
         }
-        launch(add_offset_kernel, ceil_div(e, kTB), kTB, 0, st, e, p->seg_pix.get(), (int)pb, sp + eb);
-        DCRF_CUDA(cudaMemcpyAsync(sw + eb, p->seg_w.get(), sizeof(float) * e, cudaMemcpyDeviceToDevice, st));
+        launch(seg_offset_kernel, ceil_div(e, kTB), kTB, 0, st, e, (const int2*)p->seg.get(), (int)pb, sg + eb);
         if (p->M) launch(fill_int_kernel, ceil_div(p->M, kTB), kTB, 0, st, (long)p->M, part, vi + vb_);
         pb += p->N;
         vb_ += p->M;
@@ -2143,18 +2127,18 @@ void Lattice::concat(const std::vector<const Lattice*>& parts) {
     int* ok = vorder_keys.ensure(M);
     launch(order_key_kernel, ceil_div(M, kTB), kTB, 0, st, M, cnt, ok, vo);
     radix_sort_pairs(ok, vo, M, 24, sort, st);
-    // Then, stably, by (class, image): each class (huge, long, short lists)
-    // holds its lists image by image, longest first within an image, so
+    // Then, stably, by (class, image): each class (long, short lists) holds
+    // its lists image by image, longest first within an image, so
     // that an image's lists of a class are one contiguous range of the order
     // (the live-image domains of a batched solve).
     const int B = (int)parts.size();
     DevBuf<int> pci;
-    int* per_ci = pci.ensure((size_t)3 * B);
-    DCRF_CUDA(cudaMemsetAsync(per_ci, 0, sizeof(int) * 3 * B, st));
+    int* per_ci = pci.ensure((size_t)2 * B);
+    DCRF_CUDA(cudaMemsetAsync(per_ci, 0, sizeof(int) * 2 * B, st));
     launch(class_image_key_kernel, ceil_div(M, kTB), kTB, 0, st, M, (const int*)vo, (const int*)cnt,
            (const int*)vi, B, ok, per_ci);
     int kbits = 1;
-    while ((1L << kbits) < 3L * B) kbits++;
+    while ((1L << kbits) < 2L * B) kbits++;
     radix_sort_pairs(ok, vo, M, kbits, sort, st);
     int* dl = total.ensure(2);
     DCRF_CUDA(cudaMemsetAsync(dl, 0, 2 * sizeof(int), st));
@@ -2162,9 +2146,9 @@ void Lattice::concat(const std::vector<const Lattice*>& parts) {
     launch(count_long_kernel, ceil_div(M, kTB), kTB, 0, st, M, cnt, kHugeList, dl + 1);
     DCRF_LAUNCH_CHECK();
     int nl[2];
-    std::vector<int> hci((size_t)3 * B);
+    std::vector<int> hci((size_t)2 * B);
     DCRF_CUDA(cudaMemcpyAsync(nl, dl, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-    DCRF_CUDA(cudaMemcpyAsync(hci.data(), per_ci, sizeof(int) * 3 * B, cudaMemcpyDeviceToHost, st));
+    DCRF_CUDA(cudaMemcpyAsync(hci.data(), per_ci, sizeof(int) * 2 * B, cudaMemcpyDeviceToHost, st));
     DCRF_CUDA(cudaStreamSynchronize(st));  // also keeps &Ei alive until its copy ran
     n_long = nl[0];
     n_huge = nl[1];
@@ -2174,8 +2158,8 @@ void Lattice::concat(const std::vector<const Lattice*>& parts) {
     std::vector<long> hb((size_t)kDomains * (B + 1), 0);
     auto row = [&](int dom) { return hb.data() + (long)dom * (B + 1); };
     long pos = 0;
-    for (int c = 0; c < 3; c++) {
-        long* r = row(kDomHuge + c);
+    for (int c = 0; c < 2; c++) {
+        long* r = row(kDomLong + c);
         for (int i = 0; i < B; i++) {
             r[i] = pos;
             pos += hci[(size_t)c * B + i];
@@ -2238,15 +2222,12 @@ Lattice::~Lattice() {
 }
 
 void Lattice::ensure_values(size_t row_width) {
-    size_t need = (size_t)(M + 1) * row_width;
+    const size_t need = (size_t)(M + 1) * row_width;
     if (need > va_floats) {
         va.ensure(need);
         vb.ensure(need);
         va_floats = need;
     }
-    // Row 0 is the zero row that absent neighbours read.
-    DCRF_CUDA(cudaMemsetAsync(va.get(), 0, sizeof(float) * row_width, stream));
-    DCRF_CUDA(cudaMemsetAsync(vb.get(), 0, sizeof(float) * row_width, stream));
 }
 
 // ---------------------------------------------------------------------------
@@ -2305,11 +2286,11 @@ void Lattice::compute_noalloc(float* out, const float* in, int L, bool reverse) 
     const long ML = (long)M * L, NL = (long)N * L;
     const int n_short = M - n_long;
     if (n_long)
-        launch(splat_kernel<false>, ceil_div(n_long, kStageWarps), 32 * kStageWarps, 0, st, n_long, L,
-               vorder.get(), seg_start.get(), seg_pix.get(), seg_w.get(), in, nullptr, src, Live{}, L);
+        launch(splat_kernel, ceil_div(n_long, kStageWarps), 32 * kStageWarps, 0, st, n_long, L, vorder.get(),
+               seg_start.get(), seg.get(), in, src);
     if (n_short)
-        launch(splat_short_kernel<false>, ceil_div((long)n_short * L, kTB), kTB, 0, st, n_short, L,
-               vorder.get() + n_long, seg_start.get(), seg_pix.get(), seg_w.get(), in, nullptr, src, Live{}, L);
+        launch(splat_short_kernel, ceil_div((long)n_short * L, kTB), kTB, 0, st, n_short, L,
+               (const int*)vorder.get() + n_long, seg_start.get(), seg.get(), in, src);
     const bool seq = L <= 2;
     for (int jj = 0; jj <= d; jj++) {
         const int j = reverse ? d - jj : jj;
@@ -2336,100 +2317,55 @@ void Lattice::compute(float* out, const float* in, int L, bool reverse, const Sl
     slice(out, L, ep);
 }
 
-// Row stride of the plain filter's value buffers: L padded to a multiple of
-// four (float4 rows) on the sseCompute path (L > 2); seqCompute (L <= 2)
-// keeps L.
-static int value_row(int L) { return L > 2 ? (L + 3) & ~3 : L; }
-
-// Blocks of a launch over `units` work items, `per_block` per block of
-// `threads` threads: all of them at once, or -- with live images, whose
-// units are counted on the device -- twice as many blocks as the SMs hold
-// at full occupancy, looping over them.
-static int unit_grid(long units, int per_block, bool live, int threads) {
-    const long g = std::max(1L, (units + per_block - 1) / per_block);
-    return live ? (int)std::min(g, (long)sm_count() * 2 * (2048 / threads)) : (int)g;
+// Shared memory of the tiled slice: at most 10 KB per warp.
+constexpr int kSliceSmem = 10 << 10;
+static size_t slice_warp_bytes(int tile, int d, int L) {
+    return ((size_t)((tile * L + 3) & ~3) * 4 + (size_t)tile * ((d + 1) * 8 + 8) + 15) & ~(size_t)15;
+}
+static int slice_tile_max(int tile, int d, int L) {
+    while (tile > 1 && slice_warp_bytes(tile, d, L) > (size_t)kSliceSmem) tile = tile > 4 ? (tile / 2) & ~3 : tile - 1;
+    return tile;
 }
 
-// The warp splat (L = 21) over order[first, first + count) with `warps`
-// vertices per block; with live images, over domain `dom`'s live lists.
-static void splat_warp_range(const Lattice& lat, int warps, int dom, int first, int count, int L, int Lp,
-                             const float* in, const float* pre_norm, float* vals, cudaStream_t st) {
-    if (count <= 0) return;
-    const Live lv = lat.live_of(dom);
-    const int* order = lat.vorder.get() + (lv.n ? 0 : first);
-    auto go = [&](auto kern, int w) {
-        launch(kern, unit_grid(count, w, lv.n != nullptr, 32 * w), 32 * w, 0, st, count, L, order, lat.seg_start.get(),
-               lat.seg_pix.get(), lat.seg_w.get(), in, pre_norm, vals, lv, Lp);
-    };
-    if (pre_norm) {
-        if (warps == 2) go(splat_warp_kernel<true, 21, 2>, 2);
-        else if (warps == 8) go(splat_warp_kernel<true, 21, 8>, 8);
-        else go(splat_warp_kernel<true, 21, 4>, 4);
-    } else {
-        if (warps == 2) go(splat_warp_kernel<false, 21, 2>, 2);
-        else if (warps == 8) go(splat_warp_kernel<false, 21, 8>, 8);
-        else go(splat_warp_kernel<false, 21, 4>, 4);
-    }
-}
-
-// The tiled splat (L = 21) over order[first, first + count); with live
-// images, over domain `dom`'s live lists.
-static void splat_tile_range(const Lattice& lat, int dom, int first, int count, const float* in,
-                             const float* pre_norm, float* vals, int Lp, cudaStream_t st) {
-    if (count <= 0) return;
-    // 38 KB of static shared memory per block: ask for the largest carveout
-    // so that kTileBlocksPerSM blocks fit on an SM.
-    static const bool carveout = [] {
-        DCRF_CUDA(cudaFuncSetAttribute(splat_tile21_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                       (int)cudaSharedmemCarveoutMaxShared));
-        DCRF_CUDA(cudaFuncSetAttribute(splat_tile21_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                       (int)cudaSharedmemCarveoutMaxShared));
-        return true;
-    }();
-    (void)carveout;
-    const Live lv = lat.live_of(dom);
-    const bool live = lv.n != nullptr;
-    const int* order = lat.vorder.get() + (live ? 0 : first);
-    // persistent blocks: each walks its tiles with the next tile's ranges and
-    // records prefetched
-    const int grid = (int)std::min<long>((count + kTV - 1) / kTV, (long)sm_count() * kTileBlocksPerSM);
-    launch(pre_norm ? splat_tile21_kernel<true> : splat_tile21_kernel<false>,
-           grid, kTileThreads, 0, st, count, order, lat.seg_start.get(),
-           lat.seg_pix.get(), lat.seg_w.get(), in, pre_norm, vals, lv, Lp);
-}
-
-// Bounded waits of the bulk-copy splat that ran out, since the library
-// loaded (read from the current device).
-unsigned long long bulk_wait_timeouts() {
-    unsigned long long v = 0;
-    DCRF_CUDA(cudaMemcpyFromSymbol(&v, g_bulk_wait_timeouts, sizeof(v)));
-    return v;
-}
-
-// The bulk-copy splat (L = 21) over order[first, first + count) (or domain
-// `dom`'s live lists); inputs that are not 16-byte aligned take the tiled
-// splat, which computes the same values.
-static void splat_bulk_range(const Lattice& lat, int dom, int first, int count, const float* in,
-                             const float* pre_norm, float* vals, int Lp, cudaStream_t st) {
-    if (count <= 0) return;
-    if (reinterpret_cast<uintptr_t>(in) % 16 != 0) {
-        splat_tile_range(lat, dom, first, count, in, pre_norm, vals, Lp, st);
+// Splats `in` [N][L] (times pre_norm) into vals: rows of Q float4 (L > 2) or
+// of L floats.  With live images only their lists (and pixels).
+void Lattice::splat(const float* in, int L, const float* pre_norm, float* vals) {
+    cudaStream_t st = stream;
+    const bool live = live_n != nullptr;
+    const int n_short = M - n_long;
+    const SplatRange rs{n_long, n_short, live_of(kDomShort)};
+    float* other = vals == va.get() ? vb.get() : va.get();
+    if (L <= 2) {
+        const SplatRange rl{0, n_long, live_of(kDomLong)};
+        const int lb = n_long ? unit_grid(n_long, kSplatWarps, live, kSplatThreads) : 0;
+        const int sb = n_short ? unit_grid((long)n_short * L, kSplatThreads, live, kSplatThreads) : 0;
+        if (lb + sb)
+            launch_chained(L == 1 ? splat_thin_kernel<1> : splat_thin_kernel<2>, lb + sb, kSplatThreads, 0, st, rl, rs,
+                           lb, vorder.get(), seg_start.get(), seg.get(), in, pre_norm, vals,
+                           other);
         return;
     }
-    static const bool carveout = [] {
-        DCRF_CUDA(cudaFuncSetAttribute(splat_bulk21_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                       (int)cudaSharedmemCarveoutMaxShared));
-        DCRF_CUDA(cudaFuncSetAttribute(splat_bulk21_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                       (int)cudaSharedmemCarveoutMaxShared));
-        return true;
-    }();
-    (void)carveout;
-    const Live lv = lat.live_of(dom);
-    const bool live = lv.n != nullptr;
-    const int* order = lat.vorder.get() + (live ? 0 : first);
-    const int grid = (int)std::min<long>((count + kTV - 1) / kTV, (long)sm_count() * kBulkBlocksPerSM);
-    launch(pre_norm ? splat_bulk21_kernel<true> : splat_bulk21_kernel<false>, grid, kTileThreads, 0, st, count,
-           order, lat.seg_start.get(), lat.seg_pix.get(), lat.seg_w.get(), in, lat.N, pre_norm, vals, lv, Lp);
+    const int Q = value_row(L) / 4;
+    float4* rw = reinterpret_cast<float4*>(rows.ensure((size_t)N * Q * 4));
+    const int tile = live ? dom_tile : slice_tile_for(L);
+    require(tile > 0, DCRF_E_STATE, "splat: live images without prepare_live");
+    const size_t psmem = sizeof(float) * kPadWarps * (size_t)((tile * L + 3) & ~3);
+    launch_chained(Q == 6 ? pad_rows_kernel<6> : pad_rows_kernel<0>,
+                   unit_grid(N, tile * kPadWarps, live, 32 * kPadWarps), 32 * kPadWarps, psmem, st, N, L, Q, tile, in,
+                   pre_norm, rw, live_of(kDomTile),
+                   live ? (const long*)(dom_base.get() + (long)kDomPix * (images + 1)) : nullptr, (int)aligned16(in));
+    const int hb = !concatenated && n_huge <= kHugePerSM * sm_count() ? n_huge : 0;
+    const SplatRange rl{hb, n_long - hb, live_of(kDomLong)};
+    const int lb = rl.count ? unit_grid(rl.count, kSplatWarps, live, kSplatThreads) : 0;
+    const int sb = n_short ? unit_grid((long)n_short * Q, kSplatThreads, live, kSplatThreads) : 0;
+    const size_t smem = hb + lb ? (size_t)kSplatWarps * splat_ring_bytes(std::min(Q, 8)) : 0;
+    auto kern = Q == 6 ? splat_rows_kernel<6> : splat_rows_kernel<0>;
+    if (smem > 48 * 1024)  // opt-in size: a per-device function attribute, set on every such call
+        DCRF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (hb + lb + sb)
+        launch_chained(kern, hb + lb + sb, kSplatThreads, smem, st, rl, rs, hb, lb, Q, vorder.get(),
+                       seg_start.get(), seg.get(), (const float4*)rw,
+                       reinterpret_cast<float4*>(vals), reinterpret_cast<float4*>(other));
 }
 
 namespace {
@@ -2448,7 +2384,7 @@ bool autotune_enabled() {
 }
 }  // namespace
 
-void Lattice::tune_shape(const float* in, int L, const float* pre_norm) {
+void Lattice::tune_shape(int L) {
     shape_L = L;  // also when the defaults stay
     if (N < kTuneMinPixels || !autotune_enabled()) return;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -2488,60 +2424,16 @@ void Lattice::tune_shape(const float* in, int L, const float* pre_norm) {
     FilterShape best;
     float* src = va.get();
     float* dst = vb.get();
-    float tbest = 1e30f;
-    for (int kind = 0; kind < 6; kind++) {
-        for (int w : {2, 4, 8}) {
-            if ((kind == 0 || kind >= 3) && w != 4) continue;  // no warp splat in these forms
-            FilterShape fs = best;
-            fs.splat_kind = kind;
-            fs.splat_warps = w;
-            // as splat_blur runs it: beside the very long lists' splat on the side stream
-            const float t = timed([&] {
-                const bool fork = splat_huge_fork(in, L, pre_norm, src, false);
-                splat_rest(fs, in, L, pre_norm, src, false, st, nullptr);
-                if (fork) {
-                    DCRF_CUDA(cudaEventRecord(ev_join, aux));
-                    DCRF_CUDA(cudaStreamWaitEvent(st, ev_join, 0));
-                }
-            });
-            if (t < tbest) {
-                tbest = t;
-                best.splat_kind = kind;
-                best.splat_warps = w;
-            }
-        }
-    }
+    float tbest;
     const int Q = Lp / 4;
     const long MQ = (long)M * Q;
     tbest = 1e30f;
     for (int bt : {128, 256, 512}) {
         const float t = timed([&] {
-            launch(blur4_kernel<6>, ceil_div(MQ, bt), bt, 0, st, M, Q, nbr.get(), (const float*)src, dst, Live{});
+            launch_chained(blur4_kernel<6>, ceil_div(MQ, bt), bt, 0, st, M, Q, nbr.get(), (const float*)src, dst,
+                           Live{});
         });
         if (t < tbest) tbest = t, best.blur_threads = bt;
-    }
-    {
-        DevBuf<float> probe;  // the slice candidates write here, not to the caller's output
-        float* o = probe.ensure((size_t)N * L);
-        const float alpha = 1.0f / (1.0f + std::pow(2.0f, (float)-d));
-        const SliceEpilogue ep;
-        const int per_px = (d + 1) * 8 + 4 + L * 4;
-        tbest = 1e30f;
-        for (int tile : {64, 128, 256}) {
-            const int tl = std::max(1, std::min(tile, (40 << 10) / per_px));
-            const float t = timed([&] {
-                auto sl = [&](auto kern) {
-                    launch(kern, ceil_div(N, tl), kSliceThreads, (size_t)tl * per_px, st, N, L, Q, d, tl,
-                           offset.get(), bary.get(), (const float*)src, alpha, o, ep, Live{},
-                           (const long*)nullptr);
-                };
-                if (d == 5) sl(slice4_kernel<5, 6, 21>);
-                else if (d == 2) sl(slice4_kernel<2, 6, 21>);
-                else sl(slice4_kernel<0, 0, 0>);
-            });
-            if (t < tbest) tbest = t, best.slice_tile = tile;
-        }
-        DCRF_CUDA(cudaStreamSynchronize(st));  // before the probe buffer goes back
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -2551,119 +2443,17 @@ void Lattice::tune_shape(const float* in, int L, const float* pre_norm) {
     tune_cache().push_back({key, best});
 }
 
-void Lattice::splat_rest(const FilterShape& fs, const float* in, int L, const float* pre_norm, float* vals,
-                         bool live, cudaStream_t st, cudaStream_t st_short) {
-    const int Lp = value_row(L);
-    // live images: the short lists are their own domain, splatted on
-    // st_short (concurrent with the long lists) when the caller gives one
-    cudaStream_t sts = live && st_short ? st_short : st;
-    const int nh = n_huge, n_short = M - n_long;
-    const int kind = L == 21 ? fs.splat_kind : 0;
-    if (kind == 2 && !live) {
-        splat_warp_range(*this, fs.splat_warps, kDomLong, nh, M - nh, L, Lp, in, pre_norm, vals, st);
-        return;
-    }
-    if (kind == 3) {  // the tiled splat for every list up to the huge ones
-        if (!live) {
-            splat_tile_range(*this, kDomLong, nh, M - nh, in, pre_norm, vals, Lp, st);
-        } else {
-            splat_tile_range(*this, kDomLong, nh, n_long - nh, in, pre_norm, vals, Lp, st);
-            splat_tile_range(*this, kDomShort, n_long, n_short, in, pre_norm, vals, Lp, sts);
-        }
-        return;
-    }
-    if (kind == 5) {  // the bulk-copy splat for every list up to the huge ones
-        if (!live) {
-            splat_bulk_range(*this, kDomLong, nh, M - nh, in, pre_norm, vals, Lp, st);
-        } else {
-            splat_bulk_range(*this, kDomLong, nh, n_long - nh, in, pre_norm, vals, Lp, st);
-            splat_bulk_range(*this, kDomShort, n_long, n_short, in, pre_norm, vals, Lp, sts);
-        }
-        return;
-    }
-    if (kind == 4) {  // the staged warp splat for the long lists, the tiled splat for the short ones
-        if (n_long > nh) {
-            const Live lv = live ? live_of(kDomLong) : Live{};
-            launch(pre_norm ? splat_kernel<true, 21> : splat_kernel<false, 21>,
-                   unit_grid(n_long - nh, kStageWarps, live, 32 * kStageWarps), 32 * kStageWarps, 0, st, n_long - nh,
-                   L, vorder.get() + (live ? 0 : nh), seg_start.get(), seg_pix.get(), seg_w.get(), in, pre_norm, vals,
-                   lv, Lp);
-        }
-        splat_tile_range(*this, kDomShort, n_long, n_short, in, pre_norm, vals, Lp, sts);
-        return;
-    }
-    if (n_long > nh) {
-        if (kind >= 1) {
-            splat_warp_range(*this, fs.splat_warps, kDomLong, nh, n_long - nh, L, Lp, in, pre_norm, vals, st);
-        } else {
-            const Live lv = live ? live_of(kDomLong) : Live{};
-            launch(L == 21 ? (pre_norm ? splat_kernel<true, 21> : splat_kernel<false, 21>)
-                           : (pre_norm ? splat_kernel<true> : splat_kernel<false>),
-                   unit_grid(n_long - nh, kStageWarps, live, 32 * kStageWarps), 32 * kStageWarps, 0, st, n_long - nh, L,
-                   vorder.get() + (live ? 0 : nh), seg_start.get(), seg_pix.get(), seg_w.get(), in, pre_norm, vals,
-                   lv, Lp);
-        }
-    }
-    if (n_short) {
-        if (kind == 2) {  // live: the short lists are their own domain
-            splat_warp_range(*this, fs.splat_warps, kDomShort, n_long, n_short, L, Lp, in, pre_norm, vals, sts);
-        } else {
-            const Live lv = live ? live_of(kDomShort) : Live{};
-            launch(L == 21 ? (pre_norm ? splat_short_kernel<true, 21> : splat_short_kernel<false, 21>)
-                           : (pre_norm ? splat_short_kernel<true> : splat_short_kernel<false>),
-                   unit_grid((long)n_short * Lp, kTB, live, kTB), kTB, 0, sts, n_short, L, vorder.get() + (live ? 0 : n_long),
-                   seg_start.get(), seg_pix.get(), seg_w.get(), in, pre_norm, vals, lv, Lp);
-        }
-    }
-}
-
-// The lists longer than kHugeList (the first n_huge of the order) run on the
-// high-priority side stream while the others are splatted: with L = 21 by
-// the transposing ring (one warp's chain sets their time, and its three
-// chunks of copies in flight hide the load latency a lone warp cannot hide
-// otherwise), else by splat_kernel.  Forks the side stream from `stream`
-// when there are such lists or `fork_anyway`; the caller joins it.
-bool Lattice::splat_huge_fork(const float* in, int L, const float* pre_norm, float* vals, bool fork_anyway) {
-    const int nh = n_huge;
-    if (nh == 0 && !fork_anyway) return false;
-    const int Lp = value_row(L);
-    const bool live = live_n != nullptr;
-    ensure_aux();
-    DCRF_CUDA(cudaEventRecord(ev_fork, stream));
-    DCRF_CUDA(cudaStreamWaitEvent(aux, ev_fork, 0));
-    if (nh > 0) {
-        const Live lv = live_of(kDomHuge);
-        const int g = unit_grid(nh, kStageWarps, live, 32 * kStageWarps);
-        if (L == 21)
-            launch(pre_norm ? splat_ring21_kernel<true> : splat_ring21_kernel<false>, g, 32 * kStageWarps, 0, aux,
-                   nh, vorder.get(), seg_start.get(), seg_pix.get(), seg_w.get(), in, pre_norm, vals, lv, Lp);
-        else
-            launch(pre_norm ? splat_kernel<true> : splat_kernel<false>, g, 32 * kStageWarps, 0, aux, nh, L,
-                   vorder.get(), seg_start.get(), seg_pix.get(), seg_w.get(), in, pre_norm, vals, lv, Lp);
-    }
-    return true;
-}
-
 void Lattice::splat_blur(const float* in, int L, bool reverse, const float* pre_norm) {
     require(L >= 1, DCRF_E_ARG, "compute: L must be >= 1");
     const int Lp = value_row(L);
     ensure_values((size_t)Lp);
-    if (L == 21 && shape_L != L) tune_shape(in, L, pre_norm);
+    if (L == 21 && shape_L != L) tune_shape(L);
     cudaStream_t st = stream;
     const long ML = (long)M * L;
     float *src = va.get(), *dst = vb.get();
     // A batched solve's live images: only their lists, vertices and pixels.
     const bool live = live_n != nullptr;
-    // As in the ordered filter, the very long lists run on the side stream
-    // (splat_huge_fork).  With live images the short lists are a separate launch: it runs on the
-    // side stream too (after the very long lists), beside the long lists'.
-    const bool fork_short = live && M - n_long > 0 && n_long > n_huge;
-    const bool forked = splat_huge_fork(in, L, pre_norm, src, fork_short);
-    splat_rest(shape, in, L, pre_norm, src, live, st, fork_short ? aux : nullptr);
-    if (forked) {
-        DCRF_CUDA(cudaEventRecord(ev_join, aux));
-        DCRF_CUDA(cudaStreamWaitEvent(st, ev_join, 0));
-    }
+    splat(in, L, pre_norm, src);
     const bool seq = L <= 2;
     const int Q = Lp / 4;
     const long MQ = (long)M * Q;
@@ -2672,12 +2462,12 @@ void Lattice::splat_blur(const float* in, int L, bool reverse, const float* pre_
         const int j = reverse ? d - jj : jj;
         const int2* nb = nbr.get() + (long)j * M;
         if (seq) {
-            launch(blur_kernel<true>, unit_grid(ML, kTB, live, kTB), kTB, 0, st, M, L, nb, src, dst, lvv);
+            launch_chained(blur_kernel<true>, unit_grid(ML, kTB, live, kTB), kTB, 0, st, M, L, nb, src, dst, lvv);
         } else if (Q == 6) {
             const int bt = shape.blur_threads;
-            launch(blur4_kernel<6>, unit_grid(MQ, bt, live, bt), bt, 0, st, M, Q, nb, src, dst, lvv);
+            launch_chained(blur4_kernel<6>, unit_grid(MQ, bt, live, bt), bt, 0, st, M, Q, nb, src, dst, lvv);
         } else {
-            launch(blur4_kernel<0>, unit_grid(MQ, kTB, live, kTB), kTB, 0, st, M, Q, nb, src, dst, lvv);
+            launch_chained(blur4_kernel<0>, unit_grid(MQ, kTB, live, kTB), kTB, 0, st, M, Q, nb, src, dst, lvv);
         }
         std::swap(src, dst);
     }
@@ -2685,12 +2475,7 @@ void Lattice::splat_blur(const float* in, int L, bool reverse, const float* pre_
     plain_L = L;
 }
 
-int Lattice::slice_tile_for(int L) const {
-    // pixels per tile: kSliceTile (the tuned size for L = 21), fewer for very
-    // wide rows (40 KB of shared memory at most)
-    const int per_px = (d + 1) * 8 + 4 + L * 4;
-    return std::max(1, std::min(L == 21 ? shape.slice_tile : kSliceTile, (40 << 10) / per_px));
-}
+int Lattice::slice_tile_for(int L) const { return slice_tile_max(kSliceTile, d, L); }
 
 void Lattice::slice(float* out, int L, const SliceEpilogue& ep) {
     require(plain_vals && plain_L == L, DCRF_E_STATE, "slice: no splat_blur for this label count before it");
@@ -2700,23 +2485,26 @@ void Lattice::slice(float* out, int L, const SliceEpilogue& ep) {
     const float alpha = 1.0f / (1.0f + std::pow(2.0f, (float)-d));
     const bool live = live_n != nullptr;
     if (L <= 2) {
-        launch(slice_kernel<true, 0, 0>, unit_grid(NL, kTB, live, kTB), kTB, 0, st, N, L, d, offset.get(), bary.get(),
-               src, alpha, out, ep, live_of(kDomPix));
+        launch_chained(slice_kernel<true, 0, 0>, unit_grid(NL, kTB, live, kTB), kTB, 0, st, N, L, d, offset.get(),
+                       bary.get(), src, alpha, out, ep, live_of(kDomPix));
     } else {
         const int Q = value_row(L) / 4;
-        const int per_px = (d + 1) * 8 + 4 + L * 4;
         // live images: tiles of each image's pixels, the size prepare_live fixed
         const int tile = live ? dom_tile : slice_tile_for(L);
         require(tile > 0, DCRF_E_STATE, "slice: live images without prepare_live");
-        const size_t smem = (size_t)tile * per_px;
+        const size_t smem = kSliceWarps * slice_warp_bytes(tile, d, L);
+        const int vec = aligned16(out) && (!ep.base || aligned16(ep.base));
         const long* pix_base = live ? dom_base.get() + (long)kDomPix * (images + 1) : nullptr;
         auto sl = [&](auto kern) {
-            launch(kern, unit_grid(N, tile, live, kSliceThreads), kSliceThreads, smem, st, N, L, Q, d, tile, offset.get(),
-                   bary.get(), src, alpha, out, ep, live_of(kDomTile), pix_base);
+            launch_chained(kern, unit_grid(N, tile * kSliceWarps, live, 32 * kSliceWarps), 32 * kSliceWarps, smem, st, N,
+                           L, Q, d, tile, offset.get(), bary.get(), reinterpret_cast<const float4*>(src), alpha, out,
+                           ep, live_of(kDomTile), pix_base, vec, (const float*)nullptr, (double*)nullptr);
         };
-        if (d == 5 && L == 21) sl(slice4_kernel<5, 6, 21>);
-        else if (d == 2 && L == 21) sl(slice4_kernel<2, 6, 21>);
-        else sl(slice4_kernel<0, 0, 0>);
+        if (d == 5 && L == 21) sl(slice_rows_kernel<5, 6, 21, false>);
+        else if (d == 2 && L == 21) sl(slice_rows_kernel<2, 6, 21, false>);
+        else if (d == 5) sl(slice_rows_kernel<5, 0, 0, false>);
+        else if (d == 2) sl(slice_rows_kernel<2, 0, 0, false>);
+        else sl(slice_rows_kernel<0, 0, 0, false>);
     }
     DCRF_LAUNCH_CHECK();
 }
@@ -2756,6 +2544,9 @@ void Lattice::ord_splat_blur(const float2* bins, int L) {
     ensure_values(row);
     cudaStream_t st = stream;
     float *src = va.get(), *dst = vb.get();
+    // Row 0 is the zero row that absent neighbours read.
+    DCRF_CUDA(cudaMemsetAsync(src, 0, sizeof(float) * row, st));
+    DCRF_CUDA(cudaMemsetAsync(dst, 0, sizeof(float) * row, st));
     const int n_short = M - n_long;
     if (n_long && L <= kOrdBlockMaxL) {
         // Lists longer than kHugeList (the first n_huge of the order) are
@@ -2775,7 +2566,7 @@ void Lattice::ord_splat_blur(const float2* bins, int L) {
             if (smem > 48 * 1024)  // opt-in size: a per-device function attribute, set on every such call
                 DCRF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             launch(kern, count * kblocks, threads, smem, rs, L, kb, kblocks, vorder.get() + first,
-                   seg_start.get(), seg_pix.get(), seg_w.get(), bins, src);
+                   seg_start.get(), seg.get(), bins, src);
         };
         // The very long lists set the length of their kernel while leaving
         // most SMs idle; they run on a high-priority side stream, forked
@@ -2791,11 +2582,11 @@ void Lattice::ord_splat_blur(const float2* bins, int L) {
         run(ord_groups_cheapest(L), L, n_huge, n_long - n_huge, st);
     } else if (n_long) {
         launch(ord_splat_kernel, ceil_div(2L * n_long, kStageWarps), 32 * kStageWarps, 0, st, n_long, L,
-               vorder.get(), seg_start.get(), seg_pix.get(), seg_w.get(), bins, src);
+               vorder.get(), seg_start.get(), seg.get(), bins, src);
     }
     if (n_short)
         launch(ord_splat_short_kernel<0>, ceil_div((long)n_short * L, kTB), kTB, 0, st, n_short, L,
-               vorder.get() + n_long, seg_start.get(), seg_pix.get(), seg_w.get(), bins, src);
+               vorder.get() + n_long, seg_start.get(), seg.get(), bins, src);
     if (n_long && L <= kOrdBlockMaxL && n_huge > 0) DCRF_CUDA(cudaStreamWaitEvent(st, ev_join, 0));
     const int row4 = (int)(row / 4);
     for (int j = 0; j <= d; j++) {
@@ -2864,7 +2655,7 @@ void Lattice::ord_slice(float* out, const float2* bins, int L, const SliceEpilog
 // That is the reference's order per bin: its outside-pI loop runs over all
 // pixels before its pI loop.
 __global__ void ord_splat_restricted_kernel(int M, int L, const int* __restrict__ seg_start,
-                                            const int* __restrict__ seg_pix, const float* __restrict__ seg_w,
+                                            const int2* __restrict__ seg,
                                             const int* __restrict__ pos, const float2* __restrict__ ebins,
                                             const float2* __restrict__ rbins, float* __restrict__ stored,
                                             float* __restrict__ vals, unsigned char* __restrict__ active, int store) {
@@ -2879,13 +2670,13 @@ __global__ void ord_splat_restricted_kernel(int M, int L, const int* __restrict_
         for (int b = 0; b < kRes; b++) acc[b] = 0ull;
         bool any = false;
         for (int s = s0; s < s1; s++) {
-            const int p = seg_pix[s];
+            const int p = seg[s].x;
             if (pos[p] >= 0) {
                 any = true;
                 continue;
             }
             const float2 x = ebins[(long)p * L + k];
-            const float w = seg_w[s];
+            const float w = entry_w(seg[s]);
             const unsigned long long w2 = pack2(w, w);
 #pragma unroll
             for (int b = 0; b < kRes; b++) ord_step2(acc[b], x.x, x.y, (float)b, w2);
@@ -2903,10 +2694,10 @@ __global__ void ord_splat_restricted_kernel(int M, int L, const int* __restrict_
             acc[b] = pack2(stored[rowoff + (long)b * L], stored[rowoff + (long)(kRes + b) * L]);
     }
     for (int s = s0; s < s1; s++) {
-        const int ii = pos[seg_pix[s]];
+        const int ii = pos[seg[s].x];
         if (ii < 0) continue;
         const float2 x = rbins[(long)ii * L + k];
-        const float w = seg_w[s];
+        const float w = entry_w(seg[s]);
         const unsigned long long w2 = pack2(w, w);
 #pragma unroll
         for (int b = 0; b < kRes; b++) ord_step2(acc[b], x.x, x.y, (float)b, w2);
@@ -3003,7 +2794,7 @@ void Lattice::compute_ord_restricted(float* rout, const float* rQ, const int* pI
     DCRF_CUDA(cudaMemsetAsync(b, 0, sizeof(float) * cells, st));    // new_values_ starts zeroed
     if (M)
         launch(ord_splat_restricted_kernel, ceil_div((long)M * L, kTB), kTB, 0, st, M, L, seg_start.get(),
-               seg_pix.get(), seg_w.get(), (const int*)pos, eb, (const float2*)rb, stored, a, active, (int)store);
+               seg.get(), (const int*)pos, eb, (const float2*)rb, stored, a, active, (int)store);
     float *src = a, *dst = b;
     const int row4 = (int)(row / 4);
     for (int j = 0; j <= d; j++) {

@@ -7,8 +7,8 @@
 //   nbr[(d+1)*M]    int2 (n1+1, n2+1): blur neighbours of each vertex per axis,
 //                   shifted by one so that row 0 of a value buffer is the zero
 //                   row standing in for "absent" (src/permutohedral.cpp:490-516)
-//   seg_start[M+1], seg_pix[E], seg_w[E]   splat lists: for each vertex the
-//                   (pixel, weight) pairs that touch it, in increasing
+//   seg_start[M+1], seg[E]   splat lists: for each vertex the (pixel,
+//                   weight bits) pairs that touch it, in increasing
 //                   (pixel, remainder) order, E = N*(d+1).  Splatting then
 //                   gathers in exactly the order in which the reference's
 //                   scatter accumulates, without float atomics.
@@ -47,8 +47,6 @@ void rescaled_bins(float2* bins, const float* Q, long n, const float* qminmax, c
 int slice_grid(long n);
 // Capacity, in floats, of the fixed scratch array of compute_noalloc.
 size_t noalloc_scratch_floats();
-// Bounded device waits (bulk-copy splat) that ran out on the current device.
-unsigned long long bulk_wait_timeouts();
 
 // The units a filter launch covers.  Without `n`, every unit of the
 // launch's range.  With it (a batched solve), only the units of the images
@@ -93,24 +91,18 @@ __device__ __forceinline__ long live_unit(const Live& lv, long u) {
 }
 #endif
 
-// Launch shapes of the plain filter for L = 21 (Lattice::splat_blur /
-// slice).  Every shape computes the same arithmetic; only the speed
-// differs.  Lattice::tune_shape picks them by timing, once per device and
-// problem class (L, d, size), and caches the choice for the process.
+// Launch shapes of the plain filter for L = 21.  Every shape computes the
+// same arithmetic; only the speed differs.  Lattice::tune_shape picks the
+// blur's by timing, once per device and problem class (L, d, size), and
+// caches the choice for the process.  The splat and the slice have one form
+// each (splat_rows_kernel, slice_rows_kernel), faster than every form that
+// could be chosen before on every lattice measured; their fields are kept
+// because a pinned shape is read back as it was given.
 struct FilterShape {
-    // Splat of the lists up to the huge-list threshold (L = 21):
-    // 0 = staged splat_kernel for the long lists, one thread per (vertex,
-    //     label) for the short ones;
-    // 1 = warp splat for the long lists, the thread form for the short ones;
-    // 2 = warp splat for every list;
-    // 3 = tiled splat (splat_tile21_kernel) for every list;
-    // 4 = staged splat_kernel for the long lists, the tiled splat for the
-    //     short ones;
-    // 5 = bulk-copy splat (splat_bulk21_kernel) for every list.
-    int splat_kind = 0;
-    int splat_warps = 4;     // vertices (warps) per block of the warp splat: 2, 4 or 8
+    int splat_kind = 0;      // no effect
+    int splat_warps = 4;     // no effect
     int blur_threads = 256;  // threads per block of the float4 blur: 128, 256 or 512
-    int slice_tile = 128;    // pixels per block of the tiled slice: 64, 128 or 256
+    int slice_tile = 128;    // no effect
 };
 
 struct Lattice {
@@ -124,12 +116,14 @@ struct Lattice {
     cudaStream_t aux = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
 
-    DevBuf<int> offset, rank, seg_start, seg_pix;
+    DevBuf<int> offset, rank, seg_start;
+    DevBuf<int2> seg;
     DevBuf<int> vorder, vorder_keys;  // splat visiting order: longest lists first
-    DevBuf<float> bary, seg_w;
+    DevBuf<float> bary;
     DevBuf<int16_t> vkeys;
     DevBuf<int2> nbr;
     DevBuf<float> va, vb;    // filter value buffers
+    DevBuf<float> rows;      // the plain splat's input in rows of 16-byte groups, norm applied
     DevBuf<float2> obins;    // ordered filter: (c_lower, c_upper) per (pixel, label)
     size_t va_floats = 0;    // rows (M+1) * width currently zero-headed
 
@@ -143,10 +137,10 @@ struct Lattice {
     bool concatenated = false;  // built by concat(): no vertex keys
     DevBuf<int> vimg;           // concat(): image of each vertex
     // concat(): per-image work domains, kDomains rows of (images + 1) longs:
-    // the positions in vorder of each image's huge, long and short lists,
+    // the positions in vorder of each image's long and short lists,
     // its vertex ids, its slice tiles (tiles of dom_tile pixels, none
     // crossing an image) and its pixels.
-    enum { kDomHuge, kDomLong, kDomShort, kDomVert, kDomTile, kDomPix, kDomains };
+    enum { kDomLong, kDomShort, kDomVert, kDomTile, kDomPix, kDomains };
     int images = 0;
     std::vector<long> img_pixels;  // host: pixels of each image
     DevBuf<long> dom_base;
@@ -217,18 +211,12 @@ struct Lattice {
 
     void ensure_values(size_t row_width);
     void ensure_aux();
-    // Times the candidate shapes on this lattice with the input `in` (the
+    // Times the candidate shapes on this lattice (on its value buffers, the
     // first large call) unless the process has tuned this problem class
     // already; outputs are not touched.
-    void tune_shape(const float* in, int L, const float* pre_norm);
-    // Splat of every list after the first n_huge (whose splat runs on the
-    // side stream) into vals, in the form `fs` names; with live images the
-    // short lists' launch goes on st_short when one is given.
-    void splat_rest(const FilterShape& fs, const float* in, int L, const float* pre_norm, float* vals,
-                    bool live, cudaStream_t st, cudaStream_t st_short);
-    // Forks the side stream and splats the very long lists there (see
-    // lattice.cu); true when it forked (the caller joins ev_join).
-    bool splat_huge_fork(const float* in, int L, const float* pre_norm, float* vals, bool fork_anyway);
+    void tune_shape(int L);
+    // The splat of `in` [N][L] into the value buffer vals.
+    void splat(const float* in, int L, const float* pre_norm, float* vals);
 
     Lattice() = default;
     Lattice(const Lattice&) = delete;

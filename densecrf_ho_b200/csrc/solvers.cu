@@ -1403,6 +1403,7 @@ std::vector<const void*> Model::qp_graph_key(const float* Q, int max_iter) {
     for (const auto& t : terms) {
         k.push_back(t->lat->va.get());
         k.push_back(t->lat->vb.get());
+        k.push_back(t->lat->rows.get());
         k.push_back(t->norm.get());
         k.push_back(t->cw.get());
     }

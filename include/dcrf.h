@@ -135,15 +135,16 @@ dcrf_status dcrf_lattice_stream(dcrf_lattice lat, void** stream);
 /* Launch shapes of the 21-label plain filter (shape[4]: splat warps per
  * block in {2,4,8}, blur threads per block in {128,256,512}, slice pixels
  * per tile in {64,128,256}, splat form 0..5 as dcrf_batch_filter_shape
- * lists them).  The autotuner sets them on the first 21-label filter call of
- * a lattice of 2^18 pixels or more; set_filter_shape pins a shape instead
- * (that lattice is then never tuned).  Every shape computes bit-identical
- * values.  No counterpart in the reference. */
+ * lists them).  The autotuner sets the blur's on the first 21-label filter
+ * call of a lattice of 2^18 pixels or more; set_filter_shape pins a shape
+ * instead (that lattice is then never tuned).  The splat and the slice have
+ * one form each, faster than the forms these fields used to choose from: the
+ * other three values are read back as given and have no effect.  Every shape
+ * computes bit-identical values.  No counterpart in the reference. */
 dcrf_status dcrf_lattice_filter_shape(dcrf_lattice lat, int* shape);
 /* Number of bounded device waits that ran out on the current device since
- * the library was loaded (the bulk-copy splat waits for its copies with a
- * poll limit; a tile whose wait ran out writes NaN rows and counts here).
- * 0 in normal operation.  No counterpart in the reference. */
+ * the library was loaded.  Always 0: no kernel polls for its copies.  No
+ * counterpart in the reference. */
 dcrf_status dcrf_device_wait_timeouts(unsigned long long* count);
 dcrf_status dcrf_lattice_set_filter_shape(dcrf_lattice lat, const int* shape);
 
@@ -432,14 +433,11 @@ dcrf_status dcrf_batch_stream(dcrf_batch b, void** stream);
  * bit (no splat list, blur neighbour or slice crosses an image). */
 dcrf_status dcrf_batch_pairwise_apply(dcrf_batch b, int k, float* out, const float* in);
 dcrf_status dcrf_batch_pairwise_apply_dev(dcrf_batch b, int k, float* d_out, const float* d_in);
-/* The launch shapes the filter of term k uses, as the autotuner chose them
- * (shape[0] warp-splat vertices per block, [1] blur threads per block, [2]
- * slice pixels per block, [3] splat form: 0 staged long lists + thread-per-
- * label short lists, 1 warp splat for the long lists, 2 warp splat for
- * every list, 3 tiled splat for every list, 4 staged long lists + tiled
- * short lists, 5 bulk-copy splat for every list); the defaults until a
- * filter call of 2^18 pixels or more has
- * tuned them.  shape holds 4 ints.  No counterpart in the reference. */
+/* The launch shapes the filter of term k uses (shape[0] warp-splat vertices
+ * per block, [1] blur threads per block, [2] slice pixels per block, [3] splat
+ * form 0..5); only [1] has an effect (see dcrf_lattice_filter_shape), and it is
+ * the default until a filter call of 2^18 pixels or more has tuned it.
+ * shape holds 4 ints.  No counterpart in the reference. */
 dcrf_status dcrf_batch_filter_shape(dcrf_batch b, int k, int* shape);
 /* Pins term k's launch shapes (as dcrf_lattice_set_filter_shape). */
 dcrf_status dcrf_batch_set_filter_shape(dcrf_batch b, int k, const int* shape);
