@@ -1162,7 +1162,9 @@ __global__ void __launch_bounds__(32 * kSliceWarps)
                 for (int q = q0; q < Qn; q += 32) item(pl, q);
         }
         __syncwarp();
-        if (!DOT) {
+        if (DOT) {
+            __syncwarp();
+        } else {
             float4* o4 = reinterpret_cast<float4*>(out + t0);
             for (int e = lane; e < n4; e += 32) o4[e] = reinterpret_cast<const float4*>(s_out)[e];
             for (int e = 4 * n4 + lane; e < ne; e += 32) out[t0 + e] = s_out[e];
@@ -2507,6 +2509,26 @@ void Lattice::slice(float* out, int L, const SliceEpilogue& ep) {
         else sl(slice_rows_kernel<0, 0, 0, false>);
     }
     DCRF_LAUNCH_CHECK();
+}
+
+// Warps of slice_dot's grid: 12 blocks per SM fill it, each walking its tiles.
+int Lattice::dot_partials() { return sm_count() * 12 * kSliceWarps; }
+
+int Lattice::slice_dot(const float* dot, double* partials, int L, const SliceEpilogue& ep) {
+    require(plain_vals && plain_L == L && L > 2 && !ep.base, DCRF_E_STATE, "slice_dot: no splat_blur before it");
+    const int Q = value_row(L) / 4, tile = slice_tile_for(L);
+    const float alpha = 1.0f / (1.0f + std::pow(2.0f, (float)-d));
+    const int grid = std::min(ceil_div(N, tile * kSliceWarps), sm_count() * 12);
+    auto sl = [&](auto kern) {
+        launch_chained(kern, grid, 32 * kSliceWarps, kSliceWarps * slice_warp_bytes(tile, d, L), stream, N, L, Q, d,
+                       tile, offset.get(), bary.get(), reinterpret_cast<const float4*>(plain_vals), alpha,
+                       (float*)nullptr, ep, Live{}, (const long*)nullptr, (int)aligned16(dot), dot, partials);
+    };
+    if (d == 5 && L == 21) sl(slice_rows_kernel<5, 6, 21, true>);
+    else if (d == 2 && L == 21) sl(slice_rows_kernel<2, 6, 21, true>);
+    else sl(slice_rows_kernel<0, 0, 0, true>);
+    DCRF_LAUNCH_CHECK();
+    return grid * kSliceWarps;
 }
 
 void Lattice::compute_ord(float* out, const float* Q, int L, const SliceEpilogue& ep) {

@@ -172,6 +172,10 @@ struct Lattice {
     // plain_vals), then the slice.  Other work may run between them.
     void splat_blur(const float* in, int L, bool reverse, const float* pre_norm = nullptr);
     void slice(float* out, int L, const SliceEpilogue& ep);
+    // sum of dot[e] * (what slice() with ep, without a base, would write at e),
+    // as FP64 partials whose count is returned (at most dot_partials()); L > 2.
+    int slice_dot(const float* dot, double* partials, int L, const SliceEpilogue& ep);
+    static int dot_partials();
     const float* plain_vals = nullptr;
     int plain_L = 0;
     // The plain filter with its value buffers in a fixed device array instead

@@ -831,7 +831,7 @@ void Model::unary_init(float* Q) {
     require(has_unary, DCRF_E_STATE, "unary_init: no unary energy set");
     with_lc(L, [&](auto lc) {
         constexpr int LC = decltype(lc)::value;
-        launch(unary_init_kernel<LC>, ceil_div(N, 128), 128, 0, stream, N, L, unary.get(), Q);
+        launch_unary_init<LC>(N, L, unary.get(), Q, stream);
     });
     DCRF_LAUNCH_CHECK();
 }
