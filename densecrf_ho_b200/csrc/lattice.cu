@@ -26,24 +26,18 @@
 #include <string>
 #include <vector>
 
-#include "lattice.cuh"
+#include "lattice_device.cuh"
 
 namespace dcrf {
 
 namespace {
 
 constexpr int kEmpty = -1;
-constexpr int kRes = 10;       // RESOLUTION (include/permutohedral.h:41)
-constexpr int kOrdW = 2 * kRes;  // lower + upper bins per (vertex, label)
 constexpr int kStageWarps = 2;   // warps (splat lists) per splat block
 constexpr int kStages = 3;       // shared-memory ring depth, in chunks
 constexpr int kChunk = 32;       // entries per chunk (13 KB of ring per warp: 16 warps / SM)
 constexpr int kMaxOrderKey = (1 << 24) - 1;
-constexpr int kLongList = 64;    // lists longer than this use the staged warp kernels
-constexpr int kHugeList = 1024;  // lists longer than this get a block (plain) or the finest split (ordered splat)
 constexpr int kHugeLabels = 12;  // labels per block for those lists (120 threads)
-constexpr int kTB = 256;         // threads per block of the element-wise kernels
-constexpr int kSegPad = 4;       // entries past the splat lists' end that a paired load may touch
 
 template <int KW>
 struct Key {
@@ -299,9 +293,6 @@ __global__ void iota_copy_kernel(int E, const int* __restrict__ offset, int* __r
     vals[e] = e;
 }
 
-// A splat list's entry is (pixel, weight bits).
-__device__ __forceinline__ float entry_w(int2 e) { return __int_as_float(e.y); }
-
 __global__ void seg_fill_kernel(int E, int d1, const int* __restrict__ sorted_entries,
                                 const float* __restrict__ bary, int2* __restrict__ seg) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -329,21 +320,6 @@ __global__ void seg_fill_kernel(int E, int d1, const int* __restrict__ sorted_en
 // pixels or tiles) with a grid-stride loop: one pass with a full grid, or,
 // in a batched solve, the units of the images still running (Live) with a
 // grid sized for the device.
-
-__device__ __forceinline__ unsigned smem_addr(const void* p) {
-    return (unsigned)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void cp_async4(void* sdst, const void* gsrc) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_addr(sdst)), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void* sdst, const void* gsrc) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_addr(sdst)), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
 
 // Streams the list [s0, s1) of one vertex through the per-warp ring:
 // `vals_of(slot, e)` is this lane's staged word for entry e, and
@@ -455,31 +431,6 @@ constexpr int kSplatU = 4;        // entries in flight per thread (short lists)
 constexpr int kSplatWarps = 4;    // lists per block (long lists)
 constexpr int kSplatStages = 3;   // 9.4 KB of ring per warp at L = 21: 20 warps / SM
 constexpr int kSplatThreads = 32 * kSplatWarps;
-
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(unsigned long long v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-// a + w x per half, the product and the sum each rounded: scalar products and
-// a packed sum.  A packed product feeding a packed sum was measured to come
-// out as one fused multiply-add (rounded once), which the reference's SSE2
-// arithmetic does not do.
-__device__ __forceinline__ unsigned long long add_mul2(unsigned long long a, float w, unsigned long long x) {
-    const float2 f = unpack2(x);
-    unsigned long long r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(pack2(fmul(w, f.x), fmul(w, f.y))));
-    return r;
-}
-
-__device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr(sdst)), "l"(gsrc) : "memory");
-}
 
 // A batched solve's live slice tiles, or tiles of the whole pixel range: the
 // first pixel of tile u and its pixel count.
@@ -799,7 +750,8 @@ __global__ void __launch_bounds__(kSplatThreads)
                          (long)(gridDim.x - huge_blocks - long_blocks) * blockDim.x);
 }
 
-// The splat for L = 1, 2 (seqCompute; also every normalisation factor): the
+// The splat for L = 1, 2 (seqCompute; also every normalisation factor; `in`
+// null: ones): the
 // same split of lists.  A long list's warp forms 128 products at a time (lane
 // = entry, the next 128 entries' values in flight) and lanes 0 .. L-1 add
 // them in entry order from shared memory; a short list takes one thread per
@@ -841,7 +793,7 @@ __global__ void __launch_bounds__(kSplatThreads)
                     wc[i] = w[i];
 #pragma unroll
                     for (int k = 0; k < L; k++) {
-                        x[i][k] = in[(long)p[i] * L + k];
+                        x[i][k] = in ? in[(long)p[i] * L + k] : 1.0f;
                         if (norm) x[i][k] = fmul(x[i][k], nn);
                     }
                 }
@@ -898,7 +850,7 @@ __global__ void __launch_bounds__(kSplatThreads)
                     const int si = min(s + i, s1 - 1);
                     const int2 e = seg[si];
                     const int p = e.x;
-                    float x = in[(long)p * L + k];
+                    float x = in ? in[(long)p * L + k] : 1.0f;
                     if (norm) x = fmul(x, norm[p]);
                     y[i] = fmul(entry_w(e), x);
                 }
@@ -1003,16 +955,6 @@ __global__ void blur4_kernel(int M, int Qrt, const int2* __restrict__ nbr, const
         const float4 r = make_float4(one(a.x, x.x, y.x), one(a.y, x.y, y.y), one(a.z, x.z, y.z), one(a.w, x.w, y.w));
         *reinterpret_cast<float4*>(dst + (long)(v + 1) * lp + 4 * q) = r;
     }
-}
-
-__device__ __forceinline__ float apply_epilogue(float v, long t, int i, int k, const SliceEpilogue& ep) {
-    if (ep.potts) {
-        if (ep.norm) v = fmul(v, ep.norm[i]);
-        v = ep.scale_vec ? fmul(ep.scale_vec[k], v) : fmul(ep.scale, v);
-    }
-    if (ep.base) v = fadd(ep.base[t], fmul(ep.coef, v));
-    else if (ep.zero_base) v = fadd(0.0f, fmul(ep.coef, v));
-    return v;
 }
 
 // Slice: out(i, k) = sum_j (bary_ij * alpha) * value(o_ij, k) (sseCompute,
@@ -1178,670 +1120,6 @@ __global__ void __launch_bounds__(32 * kSliceWarps)
     }
 }
 
-// addSplitArray / sliceSplitArray bins (:548-589): the lower pass rounds
-// q*10 in float, the upper pass (q - 1e-9)*10 in double.
-// For q in [0, 1] these are the reference's indices; other values (which the
-// reference rejects with an assert) are clamped to a valid bin so no access
-// can leave the bin array.
-__device__ __forceinline__ int bin_lower(float q) {
-    int c = (int)floorf(fmul(q, (float)kRes));
-    c = c < kRes - 1 ? c : kRes - 1;
-    return c > 0 ? c : 0;
-}
-__device__ __forceinline__ int bin_upper(float q) {
-    int c = (int)floor(dmul(__dsub_rn((double)q, 1e-9), (double)kRes));
-    c = c > 0 ? c : 0;
-    return c < kRes - 1 ? c : kRes - 1;
-}
-
-// Ordered bins of every (pixel, label), computed once per ordered filter
-// (each pixel appears in d+1 splat lists and in the slice): the lower and
-// upper bin indices, held as floats (exact small integers) because the splat
-// compares them with float bin numbers.
-__device__ __forceinline__ float2 ord_bin_pair(float q) {
-    return make_float2((float)bin_lower(q), (float)bin_upper(q));
-}
-__device__ __forceinline__ int ord_lower_of(float2 b) { return (int)b.x; }
-__device__ __forceinline__ int ord_upper_of(float2 b) { return (int)b.y; }
-
-__global__ void ord_bins_kernel(long n, const float* __restrict__ Q, float2* __restrict__ bins) {
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    bins[t] = ord_bin_pair(Q[t]);
-}
-
-// The same, four elements per thread with 16-byte loads and stores (Q and
-// bins 16-byte aligned; n4 = n / 4 quads, the tail by ord_bins_kernel).
-__global__ void ord_bins4_kernel(long n4, const float4* __restrict__ Q, float4* __restrict__ bins) {
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n4) return;
-    const float4 q = Q[t];
-    const float2 a = ord_bin_pair(q.x), b = ord_bin_pair(q.y), c = ord_bin_pair(q.z), d = ord_bin_pair(q.w);
-    bins[2 * t] = make_float4(a.x, a.y, b.x, b.y);
-    bins[2 * t + 1] = make_float4(c.x, c.y, d.x, d.y);
-}
-
-// Each of the 10 bins accumulates, in entry order, the weights of the entries
-// that reach it: bins 0..c (lower pass) or c..9 (upper pass), addSplitArray
-// (:548-569).  Branch-free and bit-identical: the mask m = [c_lower >= b]
-// (lower) or [b >= c_upper] (upper) is exactly 1.0 or 0.0 (one PTX `set`,
-// NaN giving 0), so fma(m, w, acc) rounds acc + w once when the entry reaches
-// the bin and otherwise returns acc (acc + (+-0) = acc: the accumulator
-// starts at +0 and is never -0).
-__device__ __forceinline__ float step_ge(float a, float b) {  // a >= b ? 1 : 0
-    float r;
-    asm("set.ge.f32.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-
-// One entry into the bin-b pair (lower, upper) of packed accumulators:
-// acc = fma({[cl >= b], [b >= cu]}, w2, acc) with one f32x2 FMA, which rounds
-// each half exactly as fma.rn.f32 does.  w2 holds (w, w).  The bins are
-// small integers, so the masks are saturated sums: cl + (1 - b) and
-// (b + 1) - cu are exact integers, clamped to [0, 1] they are exactly the
-// comparisons (and a NaN would clamp to +0).  One `add.sat` per mask.
-__device__ __forceinline__ void ord_step2(unsigned long long& acc, float cl, float cu, float b,
-                                          unsigned long long w2) {
-    const float lo_c = 1.0f - b, up_c = b + 1.0f;  // exact; hoisted out of the entry loops
-    asm("{\n\t.reg .f32 ml, mu;\n\t.reg .b64 m;\n\t"
-        "add.rn.sat.f32 ml, %1, %3;\n\t"
-        "sub.rn.sat.f32 mu, %4, %2;\n\t"
-        "mov.b64 m, {ml, mu};\n\t"
-        "fma.rn.f32x2 %0, m, %5, %0;\n\t}"
-        : "+l"(acc)
-        : "f"(cl), "f"(cu), "f"(lo_c), "f"(up_c), "l"(w2));
-}
-// The single masks of ord_step2: [cl >= b] and [b >= cu] as 0.0 / 1.0.
-__device__ __forceinline__ float ord_mask_lower(float cl, int b) {
-    float m;
-    asm("add.rn.sat.f32 %0, %1, %2;" : "=f"(m) : "f"(cl), "f"(1.0f - (float)b));
-    return m;
-}
-__device__ __forceinline__ float ord_mask_upper(float cu, int b) {
-    float m;
-    asm("sub.rn.sat.f32 %0, %1, %2;" : "=f"(m) : "f"((float)b + 1.0f), "f"(cu));
-    return m;
-}
-template <bool UPPER>
-__device__ __forceinline__ void ord_accumulate(float (&acc)[kRes], float c, float w) {
-#pragma unroll
-    for (int b = 0; b < kRes; b++) {
-        const float m = UPPER ? step_ge((float)b, c) : step_ge(c, (float)b);
-        acc[b] = __fmaf_rn(m, w, acc[b]);
-    }
-}
-
-template <bool UPPER>
-__device__ __forceinline__ void ord_consume(float (&acc)[kRes], const float (*ring)[32], const float* mw, int lane,
-                                            int n) {
-#pragma unroll 2
-    for (int e = 0; e < n; e++) ord_accumulate<UPPER>(acc, ring[e][lane], mw[e]);
-}
-
-// Ordered splat, general L: one warp per (vertex, pass), streaming the
-// vertex's list as splat_kernel does.  A vertex row holds 20 bins x L
-// labels, bin-major ([v][bin][label]; bins [0,10) lower, [10,20) upper) so
-// that the slice's per-label bin reads coalesce.
-__global__ void __launch_bounds__(32 * kStageWarps)
-    ord_splat_kernel(int M, int L, const int* __restrict__ order, const int* __restrict__ seg_start,
-                     const int2* __restrict__ seg,
-                     const float2* __restrict__ bins, float* __restrict__ vals) {
-    __shared__ float ring[kStageWarps][kStages][kChunk][32];
-    __shared__ float mw[kStageWarps][kStages][kChunk];
-    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int unit = blockIdx.x * kStageWarps + wib;
-    if (unit >= 2 * M) return;  // warp-uniform
-    const int v = order[unit >> 1];
-    const bool upper = unit & 1;
-    const int s0 = seg_start[v], s1 = seg_start[v + 1];
-    const float* bf = reinterpret_cast<const float*>(bins);  // [pixel][label][lower, upper]
-    for (int kb = 0; kb < L; kb += 32) {
-        const int k = kb + lane;
-        const bool act = k < L;
-        float acc[kRes];
-#pragma unroll
-        for (int b = 0; b < kRes; b++) acc[b] = 0.0f;
-        stream_list<float>(s0, s1, 2 * L, 2 * k + (upper ? 1 : 0), act, lane, seg, bf, ring[wib], mw[wib],
-                           [&](int slot, int n) {
-                               if (upper) ord_consume<true>(acc, ring[wib][slot], mw[wib][slot], lane, n);
-                               else ord_consume<false>(acc, ring[wib][slot], mw[wib][slot], lane, n);
-                           });
-        if (act) {
-            float* row = vals + ((long)(v + 1) * kOrdW + (upper ? kRes : 0)) * L + k;
-#pragma unroll
-            for (int b = 0; b < kRes; b++) row[(long)b * L] = acc[b];
-        }
-    }
-}
-
-// Ordered splat of the long lists by blocks.  The 20 x L bin sums of a
-// vertex are 20 L independent in-order chains; thread (k, g) carries the
-// chains of label k, bins g*NB .. g*NB+NB-1, both passes, so a block shares
-// a long list's work and the longest lists no longer set the kernel's
-// length.
-//
-// The list streams through shared memory in chunks of kOE entries: the
-// pixel ids and weights of chunk c + 2 kODX and the (c_lower, c_upper) bins
-// of chunk c + kODX are copied with cp.async while chunk c is summed, one
-// block barrier per chunk.  Ring rows are label-major ([k][entry][lower,
-// upper], padded to an odd number of 16-byte units) so a thread reads two
-// entries per 16-byte load and eight consecutive labels hit distinct banks.
-// Weights are staged as (w, w) pairs; entries past the end of the list get
-// weight 0, which leaves every accumulator unchanged (the masks are 0 or 1
-// for any stale bin value).
-constexpr int kOE = 32;                 // entries per chunk
-constexpr int kODX = 4;                 // bins are copied kODX chunks ahead of use, pixel ids 2 kODX
-constexpr int kOXS = kODX + 1;          // bin ring slots (chunks c .. c+kODX)
-constexpr int kOPS = 2 * kODX + 1;      // pixel / weight ring slots (chunks c .. c+2 kODX)
-constexpr int kORow = 2 * kOE + 4;      // floats per ring row: 17 x 16 bytes
-constexpr int kOrdBlockMaxL = 160;      // larger L use ord_splat_kernel (shared-memory ring size)
-constexpr int kGroupChoices[] = {1, 2, 3, 5, 10};
-
-// Bin split with the fewest warp instructions per list entry: warps x (three
-// instructions per bin slot -- two masks and one f32x2 FMA -- + about two
-// for the shared-memory loads).
-int ord_groups_cheapest(int L) {
-    int best = 1;
-    long best_cost = -1;
-    for (int G : kGroupChoices) {
-        if (L * G > 1024) break;
-        const long warps = (L * G + 31) / 32, nb = (kRes + G - 1) / G;
-        const long cost = warps * (3 * nb + 2);
-        if (best_cost < 0 || cost <= best_cost) {
-            best = G;
-            best_cost = cost;
-        }
-    }
-    return best;
-}
-
-size_t ord_block_smem(int kb) {
-    return sizeof(float) * ((size_t)kOXS * kb * kORow + (size_t)kOPS * kOE * 2) + sizeof(int) * kOPS * kOE;
-}
-
-// G bin groups per label, NB = ceil(10 / G) bin slots per thread; slots past
-// bin 9 (when G does not divide 10) run on a dummy bin that is not stored.
-// Block b covers labels [k0, k0 + nk) of vertex order[b / kblocks], k0 =
-// (b % kblocks) * kb: a very long list can be shared by several blocks.
-// Compute threads are label-major (t = k * G + g), so the G threads reading
-// one label's bins sit in one warp and their shared-memory loads broadcast;
-// staging threads are entry-major (t = g * nk + k) so one warp's copies read
-// consecutive labels of one pixel.
-template <int G>
-__global__ void __launch_bounds__(kOrdBlockMaxL * G < 1024 ? kOrdBlockMaxL * G : 1024)
-    ord_splat_block_kernel(int L, int kb, int kblocks, const int* __restrict__ order,
-                           const int* __restrict__ seg_start, const int2* __restrict__ seg, const float2* __restrict__ bins,
-                           float* __restrict__ vals) {
-    extern __shared__ __align__(16) float osm[];
-    float* xr = osm;                            // [kOXS][kb][kORow]
-    float* wr = xr + (size_t)kOXS * kb * kORow;  // [kOPS][kOE][2]
-    int* pr = reinterpret_cast<int*>(wr + kOPS * kOE * 2);  // [kOPS][kOE]
-    constexpr int NB = (kRes + G - 1) / G;
-    const int t = threadIdx.x;
-    const int v = order[blockIdx.x / kblocks];
-    const int k0 = (blockIdx.x % kblocks) * kb, nk = min(kb, L - k0);
-    const int s0 = seg_start[v], s1 = seg_start[v + 1];
-    const int nch = (s1 - s0 + kOE - 1) / kOE;
-    const bool worker = t < nk * G;
-    const int k = t / G, g = t - k * G;      // compute role
-    const int sk = t % nk, sg = t / nk;      // staging role (sg < G for workers)
-
-    auto stage_pw = [&](int c) {  // pixel ids and weights of chunk c
-        if (c < nch && t < kOE) {
-            const int slot = c % kOPS, e = s0 + c * kOE + t;
-            if (e < s1) {
-                cp_async4(&pr[slot * kOE + t], &seg[e].x);
-                cp_async4(&wr[(slot * kOE + t) * 2], &seg[e].y);
-                cp_async4(&wr[(slot * kOE + t) * 2 + 1], &seg[e].y);
-            } else {
-                pr[slot * kOE + t] = 0;
-                wr[(slot * kOE + t) * 2] = 0.0f;
-                wr[(slot * kOE + t) * 2 + 1] = 0.0f;
-            }
-        }
-    };
-    // (c_lower, c_upper) of chunk c; needs chunk c's pixel ids in place.
-    // Staging thread (sk, sg) copies label k0 + sk of entries sg, sg + G, ...
-    // All pixel ids are read before the first copy is issued (the copies'
-    // memory clobber would otherwise order each read after the last copy).
-    auto stage_x = [&](int c) {
-        if (c >= nch || !worker) return;
-        constexpr int MX = (kOE + G - 1) / G;
-        const int slot = c % kOXS, ps = c % kOPS;
-        const int n = min(kOE, s1 - (s0 + c * kOE));
-        float* dst = &xr[((size_t)slot * kb + sk) * kORow];
-        const float2* src = bins + k0 + sk;
-        int pix[MX];
-#pragma unroll
-        for (int i = 0; i < MX; i++) {
-            const int e = sg + i * G;
-            pix[i] = e < n ? pr[ps * kOE + e] : 0;
-        }
-#pragma unroll
-        for (int i = 0; i < MX; i++) {
-            const int e = sg + i * G;
-            if (e < n) cp_async8(dst + 2 * e, src + (long)pix[i] * L);
-        }
-    };
-
-    // Group j (committed at iteration j; j < 0 in the prologue) holds the
-    // bins of chunk j + kODX and the pixel ids / weights of chunk j + 2 kODX.
-#pragma unroll
-    for (int c = 0; c < kODX; c++) stage_pw(c);
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncthreads();
-#pragma unroll
-    for (int c = 0; c < kODX; c++) {
-        stage_x(c);
-        stage_pw(c + kODX);
-        cp_async_commit();
-    }
-
-    // Bin g*NB + i's (lower, upper) sums as one packed pair: ord_step2 adds
-    // an entry to both with one f32x2 FMA (each half rounded as fma.rn.f32).
-    unsigned long long acc[NB];
-    float bf[NB];
-#pragma unroll
-    for (int i = 0; i < NB; i++) {
-        acc[i] = 0ull;
-        bf[i] = (float)(g * NB + i);
-    }
-    for (int c = 0; c < nch; c++) {
-        cp_async_wait<kODX - 1>();  // group c - kODX: bins of chunk c, pixel ids of chunk c + kODX
-        __syncthreads();            // ... everyone's copies; and chunk c-1's slots are free
-        stage_x(c + kODX);
-        stage_pw(c + 2 * kODX);
-        cp_async_commit();
-        if (worker) {
-            const float4* xs = reinterpret_cast<const float4*>(&xr[((size_t)(c % kOXS) * kb + k) * kORow]);
-            const ulonglong2* ws = reinterpret_cast<const ulonglong2*>(&wr[(c % kOPS) * kOE * 2]);
-            const int n2 = (min(kOE, s1 - (s0 + c * kOE)) + 1) >> 1;
-            // Batches of eight entries, the next batch's loads issued before
-            // this batch is summed.  A batch may run past n2 into the chunk's
-            // zero-weight tail (the ring rows hold kOE entries).
-            float4 x[4];      // (c_lower, c_upper) of entries 2 j, 2 j + 1
-            ulonglong2 w[4];  // ((w, w), (w, w)) of the same entries
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                x[j] = xs[j];
-                w[j] = ws[j];
-            }
-            for (int b0 = 0; b0 < n2; b0 += 4) {
-                float4 xn[4];
-                ulonglong2 wn[4];
-                const int nb0 = b0 + 4 < kOE / 2 ? b0 + 4 : b0;  // stays inside the ring row
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    xn[j] = xs[nb0 + j];
-                    wn[j] = ws[nb0 + j];
-                }
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-#pragma unroll
-                    for (int i = 0; i < NB; i++) ord_step2(acc[i], x[j].x, x[j].y, bf[i], w[j].x);
-#pragma unroll
-                    for (int i = 0; i < NB; i++) ord_step2(acc[i], x[j].z, x[j].w, bf[i], w[j].y);
-                }
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    x[j] = xn[j];
-                    w[j] = wn[j];
-                }
-            }
-        }
-    }
-    cp_async_wait<0>();
-    if (worker) {
-        float* row = vals + (long)(v + 1) * kOrdW * L + k0 + k;
-#pragma unroll
-        for (int i = 0; i < NB; i++) {
-            if (g * NB + i >= kRes) break;
-            const float2 r = unpack2(acc[i]);
-            row[(long)(g * NB + i) * L] = r.x;
-            row[(long)(kRes + g * NB + i) * L] = r.y;
-        }
-    }
-}
-
-// Ordered splat of the short lists: one thread per (vertex, label), both
-// passes, without staging.
-template <int LC = 0>
-__global__ void ord_splat_short_kernel(int n_short, int Lrt, const int* __restrict__ order,
-                                       const int* __restrict__ seg_start, const int2* __restrict__ seg, const float2* __restrict__ bins,
-                                       float* __restrict__ vals) {
-    const int L = LC ? LC : Lrt;
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)n_short * L) return;
-    const int u = (int)(t / L), k = (int)(t - (long)u * L);
-    const int v = order[u];
-    const int s0 = seg_start[v], s1 = seg_start[v + 1];
-    // Scalar chains: every entry reaches lower bin 0 (c_lower >= 0) and upper
-    // bin 9 (c_upper <= 9), plain adds there; the other 18 bins take a
-    // saturated-sum mask (exactly 0 or 1) and an FMA, fma(1, w, acc) being
-    // acc + w rounded once.
-    float lo[kRes], up[kRes];
-#pragma unroll
-    for (int b = 0; b < kRes; b++) lo[b] = up[b] = 0.0f;
-#pragma unroll 2
-    for (int s = s0; s < s1; s++) {
-        const float2 x = bins[(long)seg[s].x * L + k];
-        const float w = entry_w(seg[s]);
-        lo[0] = fadd(lo[0], w);
-#pragma unroll
-        for (int b = 1; b < kRes; b++) lo[b] = __fmaf_rn(ord_mask_lower(x.x, b), w, lo[b]);
-#pragma unroll
-        for (int b = 0; b < kRes - 1; b++) up[b] = __fmaf_rn(ord_mask_upper(x.y, b), w, up[b]);
-        up[kRes - 1] = fadd(up[kRes - 1], w);
-    }
-    float* row = vals + (long)(v + 1) * kOrdW * L + k;
-#pragma unroll
-    for (int b = 0; b < kRes; b++) {
-        row[(long)b * L] = lo[b];
-        row[(long)(kRes + b) * L] = up[b];
-    }
-}
-
-// Ordered blur: every bin independently, weightedAddSplitArray (:570-578).
-template <int R4>  // row width in float4 as a compile-time constant (0 = run-time row4r)
-__global__ void ord_blur_kernel(int M, int row4r, const int2* __restrict__ nbr,
-                                const float4* __restrict__ src, float4* __restrict__ dst) {
-    const int row4 = R4 ? R4 : row4r;
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)M * row4) return;
-    const int v = (int)(t / row4), c = (int)(t - (long)v * row4);
-    const int2 nb = nbr[v];
-    const float4 a = src[(long)(v + 1) * row4 + c];
-    const float4 p = src[(long)nb.x * row4 + c];
-    const float4 q = src[(long)nb.y * row4 + c];
-    float4 r;
-    r.x = fadd(a.x, fmul(0.5f, fadd(p.x, q.x)));
-    r.y = fadd(a.y, fmul(0.5f, fadd(p.y, q.y)));
-    r.z = fadd(a.z, fmul(0.5f, fadd(p.z, q.z)));
-    r.w = fadd(a.w, fmul(0.5f, fadd(p.w, q.w)));
-    dst[(long)(v + 1) * row4 + c] = r;
-}
-
-// Ordered slice: lower pass with weight -w*alpha, then upper with w*alpha
-// (:639-650, :687-696), accumulated into one value.  With GAP the LP's dual
-// gap terms are folded in: tmp = (alpha + u) - (v + su) for the final slice
-// value v, the clique term su (0 without cliques), and per-block sums of
-// tmp.Q and tmp.tmp (src/densecrf.cpp:725-729).
-// DC / LC: d and L as compile-time constants (0 = run-time drt / Lrt).
-template <bool GAP, int DC, int LC>
-__global__ void __launch_bounds__(kTB, 8) ord_slice_kernel(int N, int Lrt, int drt, const int* __restrict__ offset,
-                                 const float* __restrict__ bary, const float* __restrict__ vals,
-                                 const float2* __restrict__ bins, float alpha, float* out, SliceEpilogue ep,
-                                 GapFusion gf) {
-    const int L = LC ? LC : Lrt, d = DC ? DC : drt;
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    double g0 = 0.0, g1 = 0.0;
-    if (t < (long)N * L) {
-        const int i = (int)(t / L), k = (int)(t - (long)i * L);
-        const int d1 = d + 1;
-        const float2 bp = bins[t];
-        const int cl = ord_lower_of(bp), cu = ord_upper_of(bp);
-        float acc = 0.0f;
-#pragma unroll
-        for (int j = 0; j <= d; j++) {
-            const int o = offset[(long)i * d1 + j];
-            const float w = bary[(long)i * d1 + j];
-            acc = fadd(acc, fmul(vals[((long)(o + 1) * kOrdW + cl) * L + k], fmul(-w, alpha)));
-        }
-#pragma unroll
-        for (int j = 0; j <= d; j++) {
-            const int o = offset[(long)i * d1 + j];
-            const float w = bary[(long)i * d1 + j];
-            acc = fadd(acc, fmul(vals[((long)(o + 1) * kOrdW + kRes + cu) * L + k], fmul(w, alpha)));
-        }
-        const float v = apply_epilogue(acc, t, i, k, ep);
-        out[t] = v;
-        if (GAP) {
-            const float tmp = fsub(fadd(gf.alpha[t], gf.u[t]), fadd(v, gf.su ? gf.su[t] : 0.0f));
-            g0 = (double)tmp * (double)gf.Q[t];
-            g1 = (double)tmp * (double)tmp;
-        }
-    }
-    if (GAP) {
-        __shared__ double s0[kTB / 32], s1[kTB / 32];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            g0 += __shfl_down_sync(0xffffffffu, g0, o);
-            g1 += __shfl_down_sync(0xffffffffu, g1, o);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            s0[threadIdx.x >> 5] = g0;
-            s1[threadIdx.x >> 5] = g1;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double a = 0.0, b = 0.0;
-            for (int w = 0; w < kTB / 32; w++) {
-                a += s0[w];
-                b += s1[w];
-            }
-            gf.partials[blockIdx.x] = a;
-            gf.partials[gridDim.x + blockIdx.x] = b;
-        }
-    }
-}
-
-// One term of a fused two-term ordered slice.
-struct OrdSliceTerm {
-    const int* offset;
-    const float* bary;
-    const float* vals;
-    int d;
-    float alpha;
-    SliceEpilogue ep;
-};
-
-template <int DC>
-__device__ __forceinline__ float ord_slice_acc(const OrdSliceTerm& s, int i, int k, int L, int cl, int cu) {
-    const int d = DC ? DC : s.d, d1 = d + 1;
-    const int* __restrict__ off = s.offset + (long)i * d1;
-    const float* __restrict__ by = s.bary + (long)i * d1;
-    float acc = 0.0f;
-#pragma unroll
-    for (int j = 0; j <= d; j++)
-        acc = fadd(acc, fmul(s.vals[((long)(off[j] + 1) * kOrdW + cl) * L + k], fmul(-by[j], s.alpha)));
-#pragma unroll
-    for (int j = 0; j <= d; j++)
-        acc = fadd(acc, fmul(s.vals[((long)(off[j] + 1) * kOrdW + kRes + cu) * L + k], fmul(by[j], s.alpha)));
-    return acc;
-}
-
-// sa = t1's slice on top of t0's (Model::apply_ord_sum with two terms): v0 =
-// epilogue_0(slice_0) exactly as ord_slice_kernel writes it, then v0 +
-// coef_1 * scaled(slice_1) as ord_slice_kernel computes it from base = v0.
-// The value v0 never leaves the register; GAP as in ord_slice_kernel.
-template <bool GAP, int D0, int D1, int LC>
-__global__ void __launch_bounds__(kTB, 8) ord_slice_pair_kernel(int N, int Lrt, OrdSliceTerm t0, OrdSliceTerm t1,
-                                      const float2* __restrict__ bins, float* out, GapFusion gf) {
-    const int L = LC ? LC : Lrt;
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    double g0 = 0.0, g1 = 0.0;
-    if (t < (long)N * L) {
-        const int i = (int)(t / L), k = (int)(t - (long)i * L);
-        const float2 bp = bins[t];
-        const int cl = ord_lower_of(bp), cu = ord_upper_of(bp);
-        const float a0 = ord_slice_acc<D0>(t0, i, k, L, cl, cu);
-        const float a1 = ord_slice_acc<D1>(t1, i, k, L, cl, cu);
-        const float v0 = apply_epilogue(a0, t, i, k, t0.ep);
-        float s1 = a1;
-        if (t1.ep.potts) {
-            if (t1.ep.norm) s1 = fmul(s1, t1.ep.norm[i]);
-            s1 = t1.ep.scale_vec ? fmul(t1.ep.scale_vec[k], s1) : fmul(t1.ep.scale, s1);
-        }
-        const float v = fadd(v0, fmul(t1.ep.coef, s1));
-        out[t] = v;
-        if (GAP) {
-            const float tmp = fsub(fadd(gf.alpha[t], gf.u[t]), fadd(v, gf.su ? gf.su[t] : 0.0f));
-            g0 = (double)tmp * (double)gf.Q[t];
-            g1 = (double)tmp * (double)tmp;
-        }
-    }
-    if (GAP) {
-        __shared__ double s0[kTB / 32], s1[kTB / 32];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            g0 += __shfl_down_sync(0xffffffffu, g0, o);
-            g1 += __shfl_down_sync(0xffffffffu, g1, o);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            s0[threadIdx.x >> 5] = g0;
-            s1[threadIdx.x >> 5] = g1;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double a = 0.0, b = 0.0;
-            for (int w = 0; w < kTB / 32; w++) {
-                a += s0[w];
-                b += s1[w];
-            }
-            gf.partials[blockIdx.x] = a;
-            gf.partials[gridDim.x + blockIdx.x] = b;
-        }
-    }
-}
-
-// ord_slice_pair_kernel for the LP's common case (L = 21, a d = 2 and a
-// d = 5 term) with the per-pixel data staged: a block covers the same 256
-// elements (at most 14 pixels), and its pixels' offsets, alpha-scaled
-// barycentric weights and normalisation factors are loaded once, coalesced,
-// into shared memory instead of by each label's thread.  Element, block and
-// dual-gap partial sums are those of ord_slice_pair_kernel, so the values
-// are too: the lower pass's fmul(-w, alpha) is the exact negation of
-// fmul(w, alpha).
-template <bool GAP>
-__global__ void __launch_bounds__(kTB, 8) ord_slice_pair_staged(int N, OrdSliceTerm t0, OrdSliceTerm t1,
-                                                               const float2* __restrict__ bins, float* out,
-                                                               GapFusion gf) {
-    constexpr int L = 21, D0 = 3, D1 = 6, P = kTB / L + 2;  // pixels a block touches at most
-    __shared__ int so0[P * D0], so1[P * D1];
-    __shared__ float sw0[P * D0], sw1[P * D1], sn0[P], sn1[P];
-    const long NL = (long)N * L;
-    const long tb = (long)blockIdx.x * blockDim.x;
-    const long t = tb + threadIdx.x;
-    const int pf = (int)(tb / L);
-    const int np = (int)min((long)P, (long)N - pf);
-    for (int e = threadIdx.x; e < np * D0; e += blockDim.x) {
-        so0[e] = t0.offset[(long)pf * D0 + e];
-        sw0[e] = fmul(t0.bary[(long)pf * D0 + e], t0.alpha);
-    }
-    for (int e = threadIdx.x; e < np * D1; e += blockDim.x) {
-        so1[e] = t1.offset[(long)pf * D1 + e];
-        sw1[e] = fmul(t1.bary[(long)pf * D1 + e], t1.alpha);
-    }
-    if (threadIdx.x < np) {
-        if (t0.ep.norm) sn0[threadIdx.x] = t0.ep.norm[pf + threadIdx.x];
-        if (t1.ep.norm) sn1[threadIdx.x] = t1.ep.norm[pf + threadIdx.x];
-    }
-    __syncthreads();
-    double g0 = 0.0, g1 = 0.0;
-    if (t < NL) {
-        const int i = (int)(t / L), k = (int)(t - (long)i * L), li = i - pf;
-        const float2 bp = bins[t];
-        const int cl = ord_lower_of(bp), cu = ord_upper_of(bp);
-        float a0 = 0.0f, a1 = 0.0f;
-#pragma unroll
-        for (int j = 0; j < D0; j++)
-            a0 = fadd(a0, fmul(t0.vals[((long)(so0[li * D0 + j] + 1) * kOrdW + cl) * L + k], -sw0[li * D0 + j]));
-#pragma unroll
-        for (int j = 0; j < D0; j++)
-            a0 = fadd(a0, fmul(t0.vals[((long)(so0[li * D0 + j] + 1) * kOrdW + kRes + cu) * L + k], sw0[li * D0 + j]));
-#pragma unroll
-        for (int j = 0; j < D1; j++)
-            a1 = fadd(a1, fmul(t1.vals[((long)(so1[li * D1 + j] + 1) * kOrdW + cl) * L + k], -sw1[li * D1 + j]));
-#pragma unroll
-        for (int j = 0; j < D1; j++)
-            a1 = fadd(a1, fmul(t1.vals[((long)(so1[li * D1 + j] + 1) * kOrdW + kRes + cu) * L + k], sw1[li * D1 + j]));
-        float v0 = a0;
-        if (t0.ep.potts) {
-            if (t0.ep.norm) v0 = fmul(v0, sn0[li]);
-            v0 = t0.ep.scale_vec ? fmul(t0.ep.scale_vec[k], v0) : fmul(t0.ep.scale, v0);
-        }
-        if (t0.ep.base) v0 = fadd(t0.ep.base[t], fmul(t0.ep.coef, v0));
-        else if (t0.ep.zero_base) v0 = fadd(0.0f, fmul(t0.ep.coef, v0));
-        float s1 = a1;
-        if (t1.ep.potts) {
-            if (t1.ep.norm) s1 = fmul(s1, sn1[li]);
-            s1 = t1.ep.scale_vec ? fmul(t1.ep.scale_vec[k], s1) : fmul(t1.ep.scale, s1);
-        }
-        const float v = fadd(v0, fmul(t1.ep.coef, s1));
-        out[t] = v;
-        if (GAP) {
-            const float tmp = fsub(fadd(gf.alpha[t], gf.u[t]), fadd(v, gf.su ? gf.su[t] : 0.0f));
-            g0 = (double)tmp * (double)gf.Q[t];
-            g1 = (double)tmp * (double)tmp;
-        }
-    }
-    if (GAP) {
-        __shared__ double s0[kTB / 32], s1[kTB / 32];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            g0 += __shfl_down_sync(0xffffffffu, g0, o);
-            g1 += __shfl_down_sync(0xffffffffu, g1, o);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            s0[threadIdx.x >> 5] = g0;
-            s1[threadIdx.x >> 5] = g1;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double a = 0.0, b = 0.0;
-            for (int w = 0; w < kTB / 32; w++) {
-                a += s0[w];
-                b += s1[w];
-            }
-            gf.partials[blockIdx.x] = a;
-            gf.partials[gridDim.x + blockIdx.x] = b;
-        }
-    }
-}
-
-// Bins of rescale(Q) (src/eigen_utils.cpp:120-141) without materialising it:
-// rq = (Q - min) / (max - min), with min / max at qmm[0], qmm[1].
-__global__ void rescaled_bins_kernel(long n, const float* __restrict__ Q, const float* __restrict__ qmm,
-                                     float2* __restrict__ bins) {
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const float mn = qmm[0], range = fsub(qmm[1], qmm[0]);
-    float rq = fsub(Q[t], mn);
-    if (range > 0.0f) rq = rq / range;
-    bins[t] = ord_bin_pair(rq);
-}
-
-// The same, four elements per thread (as ord_bins4_kernel).
-__global__ void rescaled_bins4_kernel(long n4, const float4* __restrict__ Q, const float* __restrict__ qmm,
-                                      float4* __restrict__ bins) {
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n4) return;
-    const float mn = qmm[0], range = fsub(qmm[1], qmm[0]);
-    const float4 q = Q[t];
-    float r[4] = {fsub(q.x, mn), fsub(q.y, mn), fsub(q.z, mn), fsub(q.w, mn)};
-    if (range > 0.0f)
-#pragma unroll
-        for (int i = 0; i < 4; i++) r[i] = r[i] / range;
-    const float2 a = ord_bin_pair(r[0]), b = ord_bin_pair(r[1]), c = ord_bin_pair(r[2]), d = ord_bin_pair(r[3]);
-    bins[2 * t] = make_float4(a.x, a.y, b.x, b.y);
-    bins[2 * t + 1] = make_float4(c.x, c.y, d.x, d.y);
-}
-
-bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
-
-// Ordered-filter bins of Q [n]: four per thread where the pointers allow.
-void ord_bins(float2* bins, const float* Q, long n, cudaStream_t st) {
-    if (aligned16(Q) && aligned16(bins)) {
-        const long n4 = n / 4;
-        if (n4) launch(ord_bins4_kernel, ceil_div(n4, kTB), kTB, 0, st, n4, reinterpret_cast<const float4*>(Q),
-                       reinterpret_cast<float4*>(bins));
-        if (n > 4 * n4) launch(ord_bins_kernel, 1, kTB, 0, st, n - 4 * n4, Q + 4 * n4, bins + 4 * n4);
-    } else {
-        launch(ord_bins_kernel, ceil_div(n, kTB), kTB, 0, st, n, Q, bins);
-    }
-}
-
 int bits_for(int n) {  // bits needed to hold values 0..n-1
     int b = 0;
     while ((1LL << b) < (long long)n) b++;
@@ -1925,6 +1203,7 @@ void build_impl(Lattice& L, const float* d_features) {
     L.n_long = nl[0];
     L.n_huge = nl[1];
     L.va_floats = 0;
+    L.ord_T_ready = false;
 }
 
 }  // namespace
@@ -2178,6 +1457,7 @@ void Lattice::concat(const std::vector<const Lattice*>& parts) {
     DCRF_CUDA(cudaStreamSynchronize(st));  // hb is the copy's source
     dom_tile = 0;
     va_floats = 0;
+    ord_T_ready = false;
     concatenated = true;
 }
 
@@ -2445,6 +1725,27 @@ void Lattice::tune_shape(int L) {
     tune_cache().push_back({key, best});
 }
 
+// ord_T: row 0 the weights' sums per vertex in entry order, row j + 1 row j
+// blurred along axis j (each row M + 1 floats, the first zero).
+void Lattice::ensure_ord_totals() {
+    if (ord_T_ready) return;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    DCRF_CUDA(cudaStreamIsCapturing(stream, &cs));
+    const long rowT = M + 1;
+    float* T = ord_T.ensure((size_t)(d + 2) * rowT);
+    DCRF_CUDA(cudaMemsetAsync(T, 0, sizeof(float) * (d + 2) * rowT, stream));
+    const int n_short = M - n_long;
+    const SplatRange rl{0, n_long, Live{}}, rs{n_long, n_short, Live{}};
+    const int lb = ceil_div(n_long, kSplatWarps), sb = ceil_div(n_short, kSplatThreads);
+    launch_chained(splat_thin_kernel<1>, lb + sb, kSplatThreads, 0, stream, rl, rs, lb, vorder.get(), seg_start.get(),
+                   seg.get(), (const float*)nullptr, (const float*)nullptr, T, T + rowT);
+    for (int j = 0; j <= d; j++)
+        launch_chained(blur_kernel<false>, ceil_div(M, kTB), kTB, 0, stream, M, 1, nbr.get() + (long)j * M,
+                       T + j * rowT, T + (j + 1) * rowT, Live{});
+    DCRF_LAUNCH_CHECK();
+    ord_T_ready = cs == cudaStreamCaptureStatusNone;  // a captured launch has not run yet
+}
+
 void Lattice::splat_blur(const float* in, int L, bool reverse, const float* pre_norm) {
     require(L >= 1, DCRF_E_ARG, "compute: L must be >= 1");
     const int Lp = value_row(L);
@@ -2529,309 +1830,6 @@ int Lattice::slice_dot(const float* dot, double* partials, int L, const SliceEpi
     else sl(slice_rows_kernel<0, 0, 0, true>);
     DCRF_LAUNCH_CHECK();
     return grid * kSliceWarps;
-}
-
-void Lattice::compute_ord(float* out, const float* Q, int L, const SliceEpilogue& ep) {
-    require(L >= 1, DCRF_E_ARG, "compute_ord: L must be >= 1");
-    const long NL = (long)N * L;
-    float2* bins = obins.ensure((size_t)NL);
-    ord_bins(bins, Q, NL, stream);
-    compute_ord_bins(out, bins, L, ep, nullptr);
-}
-
-void rescaled_bins(float2* bins, const float* Q, long n, const float* qminmax, cudaStream_t st) {
-    if (aligned16(Q) && aligned16(bins)) {
-        const long n4 = n / 4;
-        if (n4) launch(rescaled_bins4_kernel, ceil_div(n4, kTB), kTB, 0, st, n4, reinterpret_cast<const float4*>(Q),
-                       qminmax, reinterpret_cast<float4*>(bins));
-        if (n > 4 * n4)
-            launch(rescaled_bins_kernel, 1, kTB, 0, st, n - 4 * n4, Q + 4 * n4, qminmax, bins + 4 * n4);
-    } else {
-        launch(rescaled_bins_kernel, ceil_div(n, kTB), kTB, 0, st, n, Q, qminmax, bins);
-    }
-    DCRF_LAUNCH_CHECK();
-}
-
-int slice_grid(long n) { return ceil_div(n, kTB); }
-
-void Lattice::compute_ord_bins(float* out, const float2* bins, int L, const SliceEpilogue& ep,
-                               const GapFusion* gap) {
-    ord_splat_blur(bins, L);
-    ord_slice(out, bins, L, ep, gap);
-}
-
-void Lattice::ord_splat_blur(const float2* bins, int L) {
-    require(L >= 1, DCRF_E_ARG, "compute_ord: L must be >= 1");
-    const size_t row = (size_t)L * kOrdW;
-    ensure_values(row);
-    cudaStream_t st = stream;
-    float *src = va.get(), *dst = vb.get();
-    // Row 0 is the zero row that absent neighbours read.
-    DCRF_CUDA(cudaMemsetAsync(src, 0, sizeof(float) * row, st));
-    DCRF_CUDA(cudaMemsetAsync(dst, 0, sizeof(float) * row, st));
-    const int n_short = M - n_long;
-    if (n_long && L <= kOrdBlockMaxL) {
-        // Lists longer than kHugeList (the first n_huge of the order) are
-        // shared by blocks of kHugeLabels labels x 10 bins, so that they
-        // finish early; the rest take one block per list with the bin split
-        // that issues the fewest instructions per entry.
-        auto run = [&](int G, int kb, int first, int count, cudaStream_t rs) {
-            if (count <= 0) return;
-            const int kblocks = (L + kb - 1) / kb;
-            const int threads = ((kb * G + 31) / 32) * 32;
-            const size_t smem = ord_block_smem(kb);
-            auto kern = G == 10 ? ord_splat_block_kernel<10>
-                      : G == 5  ? ord_splat_block_kernel<5>
-                      : G == 3  ? ord_splat_block_kernel<3>
-                      : G == 2  ? ord_splat_block_kernel<2>
-                                : ord_splat_block_kernel<1>;
-            if (smem > 48 * 1024)  // opt-in size: a per-device function attribute, set on every such call
-                DCRF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            launch(kern, count * kblocks, threads, smem, rs, L, kb, kblocks, vorder.get() + first,
-                   seg_start.get(), seg.get(), bins, src);
-        };
-        // The very long lists set the length of their kernel while leaving
-        // most SMs idle; they run on a high-priority side stream, forked
-        // after the value buffers are ready and joined before the blur, so
-        // the other splats (disjoint vertex rows) fill those SMs meanwhile.
-        if (n_huge > 0) {
-            ensure_aux();
-            DCRF_CUDA(cudaEventRecord(ev_fork, st));
-            DCRF_CUDA(cudaStreamWaitEvent(aux, ev_fork, 0));
-            run(10, kHugeLabels, 0, n_huge, aux);
-            DCRF_CUDA(cudaEventRecord(ev_join, aux));
-        }
-        run(ord_groups_cheapest(L), L, n_huge, n_long - n_huge, st);
-    } else if (n_long) {
-        launch(ord_splat_kernel, ceil_div(2L * n_long, kStageWarps), 32 * kStageWarps, 0, st, n_long, L,
-               vorder.get(), seg_start.get(), seg.get(), bins, src);
-    }
-    if (n_short)
-        launch(ord_splat_short_kernel<0>, ceil_div((long)n_short * L, kTB), kTB, 0, st, n_short, L,
-               vorder.get() + n_long, seg_start.get(), seg.get(), bins, src);
-    if (n_long && L <= kOrdBlockMaxL && n_huge > 0) DCRF_CUDA(cudaStreamWaitEvent(st, ev_join, 0));
-    const int row4 = (int)(row / 4);
-    for (int j = 0; j <= d; j++) {
-        auto kern = row4 == 105 ? ord_blur_kernel<105> : ord_blur_kernel<0>;  // 105 = 20 bins x 21 labels / 4
-        launch(kern, ceil_div((long)M * row4, kTB), kTB, 0, st, M, row4, nbr.get() + (long)j * M,
-               reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst));
-        std::swap(src, dst);
-    }
-    ord_vals = src;
-}
-
-void Lattice::ord_slice_pair(float* out, const float2* bins, int L, const Lattice& a, const SliceEpilogue& ea,
-                             const Lattice& b, const SliceEpilogue& eb, const GapFusion* gap) {
-    require(a.ord_vals && b.ord_vals, DCRF_E_STATE, "ord_slice_pair: no ord_splat_blur before it");
-    require(a.N == b.N, DCRF_E_ARG, "ord_slice_pair: lattices over different pixel counts");
-    const long NL = (long)a.N * L;
-    const OrdSliceTerm t0{a.offset.get(), a.bary.get(), a.ord_vals, a.d, 1.0f / (1.0f + std::pow(2.0f, (float)-a.d)),
-                          ea};
-    const OrdSliceTerm t1{b.offset.get(), b.bary.get(), b.ord_vals, b.d, 1.0f / (1.0f + std::pow(2.0f, (float)-b.d)),
-                          eb};
-    const GapFusion gf = gap ? *gap : GapFusion{};
-    auto sl = [&](auto kern) {
-        launch(kern, ceil_div(NL, kTB), kTB, 0, a.stream, a.N, L, t0, t1, bins, out, gf);
-    };
-    if (L == 21 && a.d == 2 && b.d == 5) {
-        launch(gap ? ord_slice_pair_staged<true> : ord_slice_pair_staged<false>, ceil_div(NL, kTB), kTB, 0,
-               a.stream, a.N, t0, t1, bins, out, gf);
-    } else if (gap) {
-        sl(ord_slice_pair_kernel<true, 0, 0, 0>);
-    } else {
-        sl(ord_slice_pair_kernel<false, 0, 0, 0>);
-    }
-    DCRF_LAUNCH_CHECK();
-}
-
-void Lattice::ord_slice(float* out, const float2* bins, int L, const SliceEpilogue& ep, const GapFusion* gap) {
-    require(ord_vals, DCRF_E_STATE, "ord_slice: no ord_splat_blur before it");
-    cudaStream_t st = stream;
-    const long NL = (long)N * L;
-    const float* src = ord_vals;
-    const float alpha = 1.0f / (1.0f + std::pow(2.0f, (float)-d));
-    const GapFusion gf = gap ? *gap : GapFusion{};
-    auto sl = [&](auto kern) {
-        launch(kern, ceil_div(NL, kTB), kTB, 0, st, N, L, d, offset.get(), bary.get(), src, bins, alpha, out, ep, gf);
-    };
-    if (gap) {
-        if (L == 21 && d == 5) sl(ord_slice_kernel<true, 5, 21>);
-        else if (L == 21 && d == 2) sl(ord_slice_kernel<true, 2, 21>);
-        else sl(ord_slice_kernel<true, 0, 0>);
-    } else {
-        if (L == 21 && d == 5) sl(ord_slice_kernel<false, 5, 21>);
-        else if (L == 21 && d == 2) sl(ord_slice_kernel<false, 2, 21>);
-        else sl(ord_slice_kernel<false, 0, 0>);
-    }
-    DCRF_LAUNCH_CHECK();
-}
-
-
-// ---------------------------------------------------------------------------
-// The restricted ordered filter (seqCompute_upper_minus_lower_ord_restricted,
-// src/permutohedral.cpp:702-900).
-//
-// Splat, per (vertex, label) and both passes: the vertex's list in pixel
-// order, first the pixels outside pI with their Q values (only in a store
-// call; the sums are then kept), then the pixels of pI with their rQ values.
-// That is the reference's order per bin: its outside-pI loop runs over all
-// pixels before its pI loop.
-__global__ void ord_splat_restricted_kernel(int M, int L, const int* __restrict__ seg_start,
-                                            const int2* __restrict__ seg,
-                                            const int* __restrict__ pos, const float2* __restrict__ ebins,
-                                            const float2* __restrict__ rbins, float* __restrict__ stored,
-                                            float* __restrict__ vals, unsigned char* __restrict__ active, int store) {
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)M * L) return;
-    const int v = (int)(t / L), k = (int)(t - (long)v * L);
-    const int s0 = seg_start[v], s1 = seg_start[v + 1];
-    const long rowoff = (long)(v + 1) * kOrdW * L + k;
-    unsigned long long acc[kRes];  // (lower, upper) sums of bin b
-    if (store) {
-#pragma unroll
-        for (int b = 0; b < kRes; b++) acc[b] = 0ull;
-        bool any = false;
-        for (int s = s0; s < s1; s++) {
-            const int p = seg[s].x;
-            if (pos[p] >= 0) {
-                any = true;
-                continue;
-            }
-            const float2 x = ebins[(long)p * L + k];
-            const float w = entry_w(seg[s]);
-            const unsigned long long w2 = pack2(w, w);
-#pragma unroll
-            for (int b = 0; b < kRes; b++) ord_step2(acc[b], x.x, x.y, (float)b, w2);
-        }
-#pragma unroll
-        for (int b = 0; b < kRes; b++) {
-            const float2 r = unpack2(acc[b]);
-            stored[rowoff + (long)b * L] = r.x;
-            stored[rowoff + (long)(kRes + b) * L] = r.y;
-        }
-        if (k == 0) active[v] = any ? 1 : 0;
-    } else {
-#pragma unroll
-        for (int b = 0; b < kRes; b++)
-            acc[b] = pack2(stored[rowoff + (long)b * L], stored[rowoff + (long)(kRes + b) * L]);
-    }
-    for (int s = s0; s < s1; s++) {
-        const int ii = pos[seg[s].x];
-        if (ii < 0) continue;
-        const float2 x = rbins[(long)ii * L + k];
-        const float w = entry_w(seg[s]);
-        const unsigned long long w2 = pack2(w, w);
-#pragma unroll
-        for (int b = 0; b < kRes; b++) ord_step2(acc[b], x.x, x.y, (float)b, w2);
-    }
-#pragma unroll
-    for (int b = 0; b < kRes; b++) {
-        const float2 r = unpack2(acc[b]);
-        vals[rowoff + (long)b * L] = r.x;
-        vals[rowoff + (long)(kRes + b) * L] = r.y;
-    }
-}
-
-// Blur of the active vertices only; the others keep whatever their row of dst
-// holds (:773-789: the reference's two buffers swap after every axis, so an
-// inactive vertex reads as 0 after odd axes and as its splat after even ones).
-__global__ void ord_blur_active_kernel(int M, int row4, const int2* __restrict__ nbr,
-                                       const unsigned char* __restrict__ active, const float4* __restrict__ src,
-                                       float4* __restrict__ dst) {
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)M * row4) return;
-    const int v = (int)(t / row4), c = (int)(t - (long)v * row4);
-    if (!active[v]) return;
-    const int2 nb = nbr[v];
-    const float4 a = src[(long)(v + 1) * row4 + c];
-    const float4 p = src[(long)nb.x * row4 + c];
-    const float4 q = src[(long)nb.y * row4 + c];
-    float4 r;
-    r.x = fadd(a.x, fmul(0.5f, fadd(p.x, q.x)));
-    r.y = fadd(a.y, fmul(0.5f, fadd(p.y, q.y)));
-    r.z = fadd(a.z, fmul(0.5f, fadd(p.z, q.z)));
-    r.w = fadd(a.w, fmul(0.5f, fadd(p.w, q.w)));
-    dst[(long)(v + 1) * row4 + c] = r;
-}
-
-// Slice at the pI pixels (:791-802, :885-896), as ord_slice_kernel does for
-// every pixel; out [nP][L] starts from 0.
-__global__ void ord_slice_restricted_kernel(int nP, int L, int d, const int* __restrict__ pI,
-                                            const int* __restrict__ offset, const float* __restrict__ bary,
-                                            const float* __restrict__ vals, const float2* __restrict__ rbins,
-                                            float alpha, float* out, SliceEpilogue ep) {
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)nP * L) return;
-    const int ii = (int)(t / L), k = (int)(t - (long)ii * L);
-    const int i = pI[ii], d1 = d + 1;
-    const float2 bp = rbins[t];
-    const int cl = ord_lower_of(bp), cu = ord_upper_of(bp);
-    float acc = 0.0f;
-    for (int j = 0; j <= d; j++) {
-        const int o = offset[(long)i * d1 + j];
-        const float w = bary[(long)i * d1 + j];
-        acc = fadd(acc, fmul(vals[((long)(o + 1) * kOrdW + cl) * L + k], fmul(-w, alpha)));
-    }
-    for (int j = 0; j <= d; j++) {
-        const int o = offset[(long)i * d1 + j];
-        const float w = bary[(long)i * d1 + j];
-        acc = fadd(acc, fmul(vals[((long)(o + 1) * kOrdW + kRes + cu) * L + k], fmul(w, alpha)));
-    }
-    out[t] = apply_epilogue(acc, t, i, k, ep);
-}
-
-__global__ void scatter_pos_kernel(int nP, const int* __restrict__ pI, int* __restrict__ pos) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < nP) pos[pI[t]] = t;
-}
-
-void Lattice::compute_ord_restricted(float* rout, const float* rQ, const int* pI, int nP, const float* Q, int L,
-                                     bool store, const SliceEpilogue& ep) {
-    require(L >= 1, DCRF_E_ARG, "compute_ord_restricted: L must be >= 1");
-    require(nP >= 0 && nP <= N, DCRF_E_ARG, "compute_ord_restricted: pI larger than the lattice");
-    require(store || r_L == L, DCRF_E_STATE,
-            "compute_ord_restricted: no stored splat for this label count (call with store first)");
-    require(!store || Q, DCRF_E_ARG, "compute_ord_restricted: store needs Q");
-    cudaStream_t st = stream;
-    const long row = (long)L * kOrdW, cells = (long)(M + 1) * row;
-    float* stored = r_stored.ensure((size_t)cells);
-    float* a = r_a.ensure((size_t)cells);
-    float* b = r_b.ensure((size_t)cells);
-    unsigned char* active = r_active.ensure((size_t)std::max(M, 1));
-    int* pos = r_pos.ensure((size_t)N);
-    float2* rb = r_bins.ensure((size_t)std::max<long>((long)nP * L, 1));
-    launch(fill_int_kernel, ceil_div(N, kTB), kTB, 0, st, (long)N, -1, pos);
-    if (nP) {
-        launch(scatter_pos_kernel, ceil_div(nP, kTB), kTB, 0, st, nP, pI, pos);
-        ord_bins(rb, rQ, (long)nP * L, st);
-    }
-    const float2* eb = nullptr;
-    if (store) {
-        float2* e = r_ebins.ensure((size_t)N * L);
-        ord_bins(e, Q, (long)N * L, st);
-        eb = e;
-        r_L = 0;  // until this call has stored its splat
-    }
-    DCRF_CUDA(cudaMemsetAsync(a, 0, sizeof(float) * row, st));      // row 0: the absent neighbour
-    DCRF_CUDA(cudaMemsetAsync(b, 0, sizeof(float) * cells, st));    // new_values_ starts zeroed
-    if (M)
-        launch(ord_splat_restricted_kernel, ceil_div((long)M * L, kTB), kTB, 0, st, M, L, seg_start.get(),
-               seg.get(), (const int*)pos, eb, (const float2*)rb, stored, a, active, (int)store);
-    float *src = a, *dst = b;
-    const int row4 = (int)(row / 4);
-    for (int j = 0; j <= d; j++) {
-        if (M)
-            launch(ord_blur_active_kernel, ceil_div((long)M * row4, kTB), kTB, 0, st, M, row4,
-                   nbr.get() + (long)j * M, (const unsigned char*)active, reinterpret_cast<const float4*>(src),
-                   reinterpret_cast<float4*>(dst));
-        std::swap(src, dst);
-    }
-    const float alpha = 1.0f / (1.0f + std::pow(2.0f, (float)-d));
-    if (nP)
-        launch(ord_slice_restricted_kernel, ceil_div((long)nP * L, kTB), kTB, 0, st, nP, L, d, pI, offset.get(),
-               bary.get(), (const float*)src, (const float2*)rb, alpha, rout, ep);
-    DCRF_LAUNCH_CHECK();
-    if (store) r_L = L;
 }
 
 }  // namespace dcrf

@@ -35,16 +35,19 @@ struct SliceEpilogue {
 // LP dual-gap sums folded into an ordered slice (see ord_slice_kernel).
 struct GapFusion {
     const float* alpha = nullptr;
-    const float* u = nullptr;
+    const float* u = nullptr;  // none: 0
     const float* Q = nullptr;
-    double* partials = nullptr;  // [2][slice_grid(N*L)]
+    double* partials = nullptr;  // [2][ord_slice_grid(N, L)]
     const float* su = nullptr;   // clique conditional gradient (lp_sp), or none
 };
 
-// Packed ordered-filter bin indices of rescale(Q) (min / max at qminmax[0..1]).
-void rescaled_bins(float2* bins, const float* Q, long n, const float* qminmax, cudaStream_t st);
-// Blocks of the element-wise slice kernels for n elements.
-int slice_grid(long n);
+// The ordered filter's bins of Q [N][L], or of rescale(Q) with its min / max at
+// qminmax[0..1] (null: Q itself), packed (see ordered.cu); their element count.
+void ordered_bins(unsigned short* bins, const float* Q, int N, int L, const float* qminmax, cudaStream_t st);
+size_t ordered_bins_size(long N, int L);
+constexpr int kOrdMaxL = 1 << 20;  // label counts of the ordered filter (int products stay in range)
+// Blocks (GapFusion partials) of an ordered slice.
+int ord_slice_grid(int N, int L);
 // Capacity, in floats, of the fixed scratch array of compute_noalloc.
 size_t noalloc_scratch_floats();
 
@@ -124,7 +127,14 @@ struct Lattice {
     DevBuf<int2> nbr;
     DevBuf<float> va, vb;    // filter value buffers
     DevBuf<float> rows;      // the plain splat's input in rows of 16-byte groups, norm applied
-    DevBuf<float2> obins;    // ordered filter: (c_lower, c_upper) per (pixel, label)
+    // Ordered filter (see ordered.cu): packed bins, masks of the stored quads,
+    // the up[0] plane, and per axis the blurred sums of each vertex's weights
+    // (T, a property of the lattice: computed on its first ordered call).
+    DevBuf<unsigned short> obins;
+    DevBuf<unsigned> ord_a, ord_b;
+    DevBuf<float> ord_plane, ord_T;
+    bool ord_T_ready = false;
+    void ensure_ord_totals();
     size_t va_floats = 0;    // rows (M+1) * width currently zero-headed
 
     // build scratch
@@ -183,17 +193,15 @@ struct Lattice {
     void compute_noalloc(float* out, const float* in, int L, bool reverse);
     // Ordered (upper minus lower, 10-bin) filter of Q in [0,1]; out = epilogue(v).
     void compute_ord(float* out, const float* Q, int L, const SliceEpilogue& ep);
-    // The same from precomputed packed bins (lower | upper << 8 per element).
-    void compute_ord_bins(float* out, const float2* bins, int L, const SliceEpilogue& ep, const GapFusion* gap);
-    // The same in two phases: splat + blur (leaves the vertex values in
-    // ord_vals), then the slice.  Other work may run between them.
-    void ord_splat_blur(const float2* bins, int L);
-    void ord_slice(float* out, const float2* bins, int L, const SliceEpilogue& ep, const GapFusion* gap);
+    // The same from packed bins in two phases: splat + blur (leaves the vertex
+    // values in ord_vals), then the slice.  Other work may run between them.
+    void ord_splat_blur(const unsigned short* bins, int L);
+    void ord_slice(float* out, const unsigned short* bins, int L, const SliceEpilogue& ep, const GapFusion* gap);
     // Both slices of a two-term sum in one pass: out = eb(b's slice) on top of
     // ea(a's slice), the arithmetic of ord_slice(a, ea with zero_base) then
     // ord_slice(b, eb with base = out); a and b share N and the bins, and each
     // has had its ord_splat_blur.  Runs on a's stream.
-    static void ord_slice_pair(float* out, const float2* bins, int L, const Lattice& a, const SliceEpilogue& ea,
+    static void ord_slice_pair(float* out, const unsigned short* bins, int L, const Lattice& a, const SliceEpilogue& ea,
                                const Lattice& b, const SliceEpilogue& eb, const GapFusion* gap);
     const float* ord_vals = nullptr;
 

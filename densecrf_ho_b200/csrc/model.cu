@@ -221,7 +221,7 @@ Model::Model(int W_, int H_, int L_) : W(W_), H(H_), N(W_ * H_), L(L_) {
     scal.ensure(1);
     // per-block partials: fixed-grid reductions, and the per-pixel / per-element
     // kernels that fold a reduction in (two values per block)
-    partials.ensure(std::max<size_t>((size_t)kRedBlocks * 16, 2 * (size_t)slice_grid((long)N * L) + 64));
+    partials.ensure(std::max<size_t>((size_t)kRedBlocks * 16, 2 * (size_t)std::max(ceil_div((long)N * L, 256), ord_slice_grid(N, L)) + 64));
 }
 
 Model::~Model() {
@@ -746,7 +746,7 @@ void Model::apply_sum(float* out, const float* in) {
 // a side stream while term 0's run on the model's stream; the slices, which
 // carry the accumulation, then run in term order.  `gap`: the dual-gap sums
 // folded into the last slice.
-void Model::apply_ord_sum(float* sa, const float2* bins, const GapFusion* gap) {
+void Model::apply_ord_sum(float* sa, const unsigned short* bins, const GapFusion* gap) {
     const int nt = (int)terms.size();
     if (nt >= 2) {
         if (!side) {
@@ -801,15 +801,6 @@ void Model::apply_ord_restricted(int k, float* rout, const float* rQ, const int*
                (const float*)nullptr, 1.0f, 0, rout);
         DCRF_LAUNCH_CHECK();
     }
-}
-
-void Model::apply_ord_bins(int k, float* out, const float2* bins, const float* base, bool zero_base,
-                           const GapFusion* gap) {
-    Term& t = *terms[k];
-    SliceEpilogue ep;
-    const CompatRoute r = route_compat(*this, t, ep, out, base, 1.0f, zero_base);
-    t.lat->compute_ord_bins(r.slice_out, bins, L, ep, r.matrix ? nullptr : gap);
-    finish_compat(*this, t, r, out, base, 1.0f, zero_base);
 }
 
 void Model::check_unit_range(const float* Q) {

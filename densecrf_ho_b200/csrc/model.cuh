@@ -112,7 +112,7 @@ struct Model {
     DevBuf<double> partials;
     DevBuf<SolverScalars> scal;
     DevBuf<int16_t> labels;
-    DevBuf<float2> lp_bins;  // ordered-filter bins of rescale(Q), shared by all terms
+    DevBuf<unsigned short> lp_bins;  // ordered-filter bins of rescale(Q), shared by all terms
     DevBuf<int> ipart;
     DevBuf<double> ho_pre;  // qp_sp: FP64 clique prefixes [2][R][L]
     DevBuf<double> ho_seg;  // qp_sp: FP64 per-segment totals of a clique prefix chain
@@ -142,7 +142,7 @@ struct Model {
     // out = base + coef * (-w K~ in)  (see SliceEpilogue).
     void apply(int k, bool nonorm, float* out, const float* in, const float* base = nullptr,
                float coef = 1.0f, bool zero_base = false);
-    void apply_ord_sum(float* sa, const float2* bins, const GapFusion* gap);
+    void apply_ord_sum(float* sa, const unsigned short* bins, const GapFusion* gap);
     // Replaces term k's Potts compatibility: kDiagonal (params: L weights)
     // or kMatrix (params: L x L column-major, used as 0.5 (m + m^T)).
     void set_compat(int k, int kind, const float* params);
@@ -185,8 +185,6 @@ struct Model {
     int parameters(int k, float* out) const;
     void set_parameters(int k, const float* v);
     int compat_gradient(int k, const float* b, const float* Q, float* out);
-    void apply_ord_bins(int k, float* out, const float2* bins, const float* base, bool zero_base,
-                        const GapFusion* gap);
     void apply_ord(int k, float* out, const float* rq, const float* base = nullptr,
                    bool zero_base = false);
     // out = sum_k apply_k(in), terms in order, their splats and blurs concurrent.

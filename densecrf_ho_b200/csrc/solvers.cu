@@ -523,7 +523,8 @@ __global__ void add_scaled_kernel(long n, float* __restrict__ a, const float* __
 // Y = multiplyC((alpha + u) - unary) + cur_Q (src/densecrf.cpp:627-635, 517-523).
 // With `pending`, the previous Frank-Wolfe iteration's update
 // alpha += delta (sa - alpha), u += delta (su - u) (:737-738) is applied here
-// first (and stored), saving a pass; su == nullptr means no cliques (su = 0).
+// first (and stored), saving a pass; su == nullptr means no cliques (su = 0,
+// and u == nullptr then: it starts at 0 and stays there).
 template <int LC>
 __global__ void lp_y_kernel(int N, int Lrt, float lambda, float cm, float* __restrict__ alpha,
                             float* __restrict__ u, const float* __restrict__ U,
@@ -539,12 +540,14 @@ __global__ void lp_y_kernel(int N, int Lrt, float lambda, float cm, float* __res
     for (int k = 0; k < PixVec<LC>::S; k++)
         if (k < L) {
             const long e = (long)i * L + k;
-            float a = alpha[e], uu = u[e];
+            float a = alpha[e], uu = u ? u[e] : 0.0f;
             if (pending) {
                 a = fadd(a, fmul(dl, fsub(sa[e], a)));
-                uu = fadd(uu, fmul(dl, fsub(su ? su[e] : 0.0f, uu)));
                 alpha[e] = a;
-                u[e] = uu;
+                if (u) {
+                    uu = fadd(uu, fmul(dl, fsub(su ? su[e] : 0.0f, uu)));
+                    u[e] = uu;
+                }
             }
             x[k] = fsub(fadd(a, uu), U[e]);
         }
@@ -668,14 +671,14 @@ __global__ void lp_q_kernel(int N, int Lrt, float lambda, const float* __restric
         for (int k = 0; k < PixVec<LC>::S; k++)
             if (k < L) {
                 const long e = (long)i * L + k;
-                bm[k] = fsub(fadd(fadd(alpha[e], u[e]), gamma[e]), U[e]);
+                bm[k] = fsub(fadd(fadd(alpha[e], u ? u[e] : 0.0f), gamma[e]), U[e]);
             }
         const float beta = (-col_sum<LC>(bm, L, i)) / (float)L;
 #pragma unroll
         for (int k = 0; k < PixVec<LC>::S; k++)
             if (k < L) {
                 const long e = (long)i * L + k;
-                const float x = fsub(fadd(fadd(fadd(alpha[e], beta), u[e]), gamma[e]), U[e]);
+                const float x = fsub(fadd(fadd(fadd(alpha[e], beta), u ? u[e] : 0.0f), gamma[e]), U[e]);
                 const float q = fadd(fmul(x, lambda), curQ[e]);
                 Q[e] = q;
                 mn = nan_min(mn, q);
@@ -712,7 +715,7 @@ __global__ void __launch_bounds__(32 * kTileWarps)
     lp_y_tiled(int N, float lambda, float cm, float* __restrict__ alpha, float* __restrict__ u,
                const float* __restrict__ U, const float* __restrict__ curQ, float* __restrict__ Y, bool pending,
                const float* __restrict__ sa, const float* __restrict__ su, const SolverScalars* __restrict__ sc) {
-    __shared__ float sm[kTileWarps][2][32 * LC];
+    __shared__ __align__(16) float sm[kTileWarps][2][32 * LC];
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long pix0 = ((long)blockIdx.x * kTileWarps + wib) * 32;
     if (pix0 >= N) return;
@@ -724,8 +727,8 @@ __global__ void __launch_bounds__(32 * kTileWarps)
     const float dl = pending ? sc->delta : 0.0f;
     float x[LC];
     // alpha (+ pending update)
-    tile_in<LC>(A, alpha, pix0, npix, lane);
-    if (pending) tile_in<LC>(B, sa, pix0, npix, lane);
+    tile_in4<LC>(A, alpha, pix0, npix, lane);
+    if (pending) tile_in4<LC>(B, sa, pix0, npix, lane);
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < LC; k++) {
@@ -737,27 +740,32 @@ __global__ void __launch_bounds__(32 * kTileWarps)
         x[k] = a;
     }
     __syncwarp();
-    if (pending) tile_out<LC>(A, alpha, pix0, npix, lane);
+    if (pending) tile_out4<LC>(A, alpha, pix0, npix, lane);
     __syncwarp();
     // u (+ pending update)
-    tile_in<LC>(A, u, pix0, npix, lane);
-    if (pending && su) tile_in<LC>(B, su, pix0, npix, lane);
-    __syncwarp();
+    if (u) {
+        tile_in4<LC>(A, u, pix0, npix, lane);
+        if (pending && su) tile_in4<LC>(B, su, pix0, npix, lane);
+        __syncwarp();
 #pragma unroll
-    for (int k = 0; k < LC; k++) {
-        float uu = ra[k];
-        if (pending) {
-            uu = fadd(uu, fmul(dl, fsub(su ? rb[k] : 0.0f, uu)));
-            ra[k] = uu;
+        for (int k = 0; k < LC; k++) {
+            float uu = ra[k];
+            if (pending) {
+                uu = fadd(uu, fmul(dl, fsub(su ? rb[k] : 0.0f, uu)));
+                ra[k] = uu;
+            }
+            x[k] = fadd(x[k], uu);
         }
-        x[k] = fadd(x[k], uu);
+        __syncwarp();
+        if (pending) tile_out4<LC>(A, u, pix0, npix, lane);
+        __syncwarp();
+    } else {
+#pragma unroll
+        for (int k = 0; k < LC; k++) x[k] = fadd(x[k], 0.0f);
     }
-    __syncwarp();
-    if (pending) tile_out<LC>(A, u, pix0, npix, lane);
-    __syncwarp();
     // x = (alpha + u) - unary;  Y = multiplyC(x) + cur_Q
-    tile_in<LC>(A, U, pix0, npix, lane);
-    tile_in<LC>(B, curQ, pix0, npix, lane);
+    tile_in4<LC>(A, U, pix0, npix, lane);
+    tile_in4<LC>(B, curQ, pix0, npix, lane);
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < LC; k++) x[k] = fsub(x[k], ra[k]);
@@ -765,7 +773,7 @@ __global__ void __launch_bounds__(32 * kTileWarps)
 #pragma unroll
     for (int k = 0; k < LC; k++) rb[k] = fadd(fmul(fadd(fmul(cm, s), x[k]), lambda), rb[k]);
     __syncwarp();
-    tile_out<LC>(B, Y, pix0, npix, lane);
+    tile_out4<LC>(B, Y, pix0, npix, lane);
 }
 
 template <int LC>
@@ -773,7 +781,7 @@ __global__ void __launch_bounds__(32 * kTileWarps)
     lp_q_tiled(int N, float lambda, const float* __restrict__ alpha, const float* __restrict__ u,
                const float* __restrict__ gamma, const float* __restrict__ U, const float* __restrict__ curQ,
                float* __restrict__ Q, double* __restrict__ partials) {
-    __shared__ float sm[kTileWarps][4][32 * LC];
+    __shared__ __align__(16) float sm[kTileWarps][4][32 * LC];
     __shared__ float smn[kTileWarps], smx[kTileWarps];
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long pix0 = ((long)blockIdx.x * kTileWarps + wib) * 32;
@@ -781,20 +789,20 @@ __global__ void __launch_bounds__(32 * kTileWarps)
     if (pix0 < N) {
         const int npix = (int)min(32L, (long)N - pix0);
         float* T[4] = {sm[wib][0], sm[wib][1], sm[wib][2], sm[wib][3]};
-        tile_in<LC>(T[0], alpha, pix0, npix, lane);
-        tile_in<LC>(T[1], u, pix0, npix, lane);
-        tile_in<LC>(T[2], gamma, pix0, npix, lane);
-        tile_in<LC>(T[3], U, pix0, npix, lane);
+        tile_in4<LC>(T[0], alpha, pix0, npix, lane);
+        if (u) tile_in4<LC>(T[1], u, pix0, npix, lane);
+        tile_in4<LC>(T[2], gamma, pix0, npix, lane);
+        tile_in4<LC>(T[3], U, pix0, npix, lane);
         __syncwarp();
         const float *ra = T[0] + lane * LC, *ru = T[1] + lane * LC, *rg = T[2] + lane * LC, *rU = T[3] + lane * LC;
         float t[LC];
 #pragma unroll
-        for (int k = 0; k < LC; k++) t[k] = fsub(fadd(fadd(ra[k], ru[k]), rg[k]), rU[k]);
+        for (int k = 0; k < LC; k++) t[k] = fsub(fadd(fadd(ra[k], u ? ru[k] : 0.0f), rg[k]), rU[k]);
         const float beta = (-col_sum<LC>(t, LC, pix0 + lane)) / (float)LC;
 #pragma unroll
-        for (int k = 0; k < LC; k++) t[k] = fsub(fadd(fadd(fadd(ra[k], beta), ru[k]), rg[k]), rU[k]);
+        for (int k = 0; k < LC; k++) t[k] = fsub(fadd(fadd(fadd(ra[k], beta), u ? ru[k] : 0.0f), rg[k]), rU[k]);
         __syncwarp();
-        tile_in<LC>(T[0], curQ, pix0, npix, lane);
+        tile_in4<LC>(T[0], curQ, pix0, npix, lane);
         __syncwarp();
         float* rq = T[0] + lane * LC;
         const bool act = lane < npix;
@@ -808,7 +816,7 @@ __global__ void __launch_bounds__(32 * kTileWarps)
             }
         }
         __syncwarp();
-        tile_out<LC>(T[0], Q, pix0, npix, lane);
+        tile_out4<LC>(T[0], Q, pix0, npix, lane);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -835,7 +843,7 @@ __global__ void __launch_bounds__(32 * kTileWarps)
     lp_gamma_tiled(int N, GammaConsts gc, const float* __restrict__ Y, float* __restrict__ gamma,
                    const SolverScalars* __restrict__ sc, double* __restrict__ partials) {
     if (sc->stop) return;  // uniform across the grid
-    __shared__ float sm[kTileWarps][2][32 * LC];
+    __shared__ __align__(16) float sm[kTileWarps][2][32 * LC];
     __shared__ double s32[32];
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long pix0 = ((long)blockIdx.x * kTileWarps + wib) * 32;
@@ -844,8 +852,8 @@ __global__ void __launch_bounds__(32 * kTileWarps)
         const int npix = (int)min(32L, (long)N - pix0);
         float* G = sm[wib][0];
         float* Yt = sm[wib][1];
-        tile_in<LC>(G, gamma, pix0, npix, lane);
-        tile_in<LC>(Yt, Y, pix0, npix, lane);
+        tile_in4<LC>(G, gamma, pix0, npix, lane);
+        tile_in4<LC>(Yt, Y, pix0, npix, lane);
         __syncwarp();
         float* rg = G + lane * LC;
         const float* ry = Yt + lane * LC;
@@ -875,7 +883,7 @@ __global__ void __launch_bounds__(32 * kTileWarps)
         const float d2 = eig_sum_ct<LC, 0>(t);
         if (lane < npix) acc = (double)(float)dadd(dmul(0.5, (double)d1), (double)d2);
         __syncwarp();
-        tile_out<LC>(G, gamma, pix0, npix, lane);
+        tile_out4<LC>(G, gamma, pix0, npix, lane);
     }
     const double tot = block_sum_any(acc, s32);
     if (threadIdx.x == 0) partials[blockIdx.x] = tot;
@@ -885,7 +893,7 @@ template <int LC>
 __global__ void __launch_bounds__(32 * kTileWarps)
     qp_direction_tiled(int N, const float* __restrict__ grad, const float* __restrict__ Q,
                        const float* __restrict__ U, float* __restrict__ sx, double* __restrict__ partials) {
-    __shared__ float sm[kTileWarps][3][32 * LC];
+    __shared__ __align__(16) float sm[kTileWarps][3][32 * LC];
     __shared__ double s32[32];
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long pix0 = ((long)blockIdx.x * kTileWarps + wib) * 32;
@@ -893,9 +901,9 @@ __global__ void __launch_bounds__(32 * kTileWarps)
     if (pix0 < N) {
         const int npix = (int)min(32L, (long)N - pix0);
         float *Gt = sm[wib][0], *Qt = sm[wib][1], *Ut = sm[wib][2];
-        tile_in<LC>(Gt, grad, pix0, npix, lane);
-        tile_in<LC>(Qt, Q, pix0, npix, lane);
-        tile_in<LC>(Ut, U, pix0, npix, lane);
+        tile_in4<LC>(Gt, grad, pix0, npix, lane);
+        tile_in4<LC>(Qt, Q, pix0, npix, lane);
+        tile_in4<LC>(Ut, U, pix0, npix, lane);
         __syncwarp();
         const float* rg = Gt + lane * LC;
         float* rq = Qt + lane * LC;
@@ -916,7 +924,7 @@ __global__ void __launch_bounds__(32 * kTileWarps)
             if (act) acc += (double)ru[k] * (double)s;
         }
         __syncwarp();
-        tile_out<LC>(Qt, sx, pix0, npix, lane);
+        tile_out4<LC>(Qt, sx, pix0, npix, lane);
     }
     const double tot = block_sum_any(acc, s32);
     if (threadIdx.x == 0) partials[blockIdx.x] = tot;
@@ -928,7 +936,7 @@ __global__ void lp_gap_kernel(long n, const float* __restrict__ alpha, const flo
                               const float* __restrict__ Q, double* __restrict__ partials) {
     double v[2] = {0.0, 0.0};
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-        const float tmp = fsub(fadd(alpha[t], u[t]), fadd(sa[t], su ? su[t] : 0.0f));
+        const float tmp = fsub(fadd(alpha[t], u ? u[t] : 0.0f), fadd(sa[t], su ? su[t] : 0.0f));
         v[0] += (double)tmp * (double)Q[t];
         v[1] += (double)tmp * (double)tmp;
     }
@@ -1625,12 +1633,12 @@ int Model::lp(const float* init, float* out, const dcrf_lp_params& p, dcrf_solve
     float* Q = buf(0);
     float* bestQ = out;
     float* alpha = buf(1);
-    float* u = buf(2);
+    float* u = R > 0 ? buf(2) : nullptr;  // 0 throughout without cliques
     float* sa = buf(3);
     float* su = R > 0 ? buf(4) : nullptr;
     float* gamma = buf(5);
     float* curQ = buf(6);
-    float2* bins = lp_bins.ensure(NL);
+    unsigned short* bins = lp_bins.ensure(ordered_bins_size(N, L));
     float* Y = buf(8);
     int16_t* lab = labels.ensure(N);
     SolverScalars* sc = scal.get();
@@ -1734,7 +1742,7 @@ int Model::lp(const float* init, float* out, const dcrf_lp_params& p, dcrf_solve
                 launch(minmax_finish_kernel, 1, 1024, 0, stream, part, pg, sc);
             }
         });
-        rescaled_bins(bins, Q, NL, &sc->qmin, stream);
+        ordered_bins(bins, Q, N, L, &sc->qmin, stream);
         // Clique conditional gradient su (computeUCondGrad), before the
         // ordered filters so that the dual-gap sums can ride along the
         // last term's slice with su included.
@@ -1766,7 +1774,7 @@ int Model::lp(const float* init, float* out, const dcrf_lp_params& p, dcrf_solve
         apply_ord_sum(sa, bins, fuse_gap ? &gf : nullptr);
         if (nt == 0) DCRF_CUDA(cudaMemsetAsync(sa, 0, sizeof(float) * NL, stream));
         if (fuse_gap) {
-            launch(finalize_large_kernel, 2, 1024, 0, stream, part, slice_grid(NL), 0, sc);
+            launch(finalize_large_kernel, 2, 1024, 0, stream, part, ord_slice_grid(N, L), 0, sc);
         } else {
             launch(lp_gap_kernel, kRedBlocks, kRedThreads, 0, stream, NL, alpha, u, sa, su, Q, part);
             launch(finalize_sums_kernel, 1, 64, 0, stream, part, kRedBlocks, 2, 0, sc);
@@ -1862,7 +1870,7 @@ int Model::lp(const float* init, float* out, const dcrf_lp_params& p, dcrf_solve
         launch(fill_float_kernel, ceil_div(NL, 256), 256, 0, stream, NL, 1.0f, gamma);
         DCRF_CUDA(cudaMemcpyAsync(curQ, Q, sizeof(float) * NL, cudaMemcpyDeviceToDevice, stream));
         DCRF_CUDA(cudaMemsetAsync(alpha, 0, sizeof(float) * NL, stream));
-        DCRF_CUDA(cudaMemsetAsync(u, 0, sizeof(float) * NL, stream));
+        if (u) DCRF_CUDA(cudaMemsetAsync(u, 0, sizeof(float) * NL, stream));
         int pit = 0;
         do {
             ++pit;
