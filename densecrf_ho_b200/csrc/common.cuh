@@ -48,8 +48,15 @@ void* dev_alloc(size_t bytes, size_t* got);
 // that frees or allocates waits until another thread's capture has ended.
 std::recursive_mutex& capture_mutex();
 void dev_release(void* p, size_t bytes) noexcept;
-// Frees the cached blocks of the current device, or of every device
-// (dcrf_release_cached_memory).
+// Page-locked host memory for a handle's read-backs, kPinnedSlot bytes, from
+// slabs kept for the next handle (memory.cu): cudaMallocHost and cudaFreeHost
+// took 2.0 of the 2.1 ms of creating a model and most of its 0.8 ms of
+// destruction.  pinned_release's caller has waited for the copies into it.
+constexpr size_t kPinnedSlot = 1024;
+void* pinned_alloc();
+void pinned_release(void* p) noexcept;
+// Frees the cached blocks of the current device, or of every device, and the
+// page-locked slabs no handle uses (dcrf_release_cached_memory).
 void dev_trim(bool all_devices) noexcept;
 // A budget on the bytes held by live DevBufs (0 = none): a request beyond it
 // fails with DCRF_E_NOMEM on the host, before any device call.

@@ -174,6 +174,69 @@ void* dev_alloc(size_t bytes, size_t* got) {
     return p;
 }
 
+// Slabs of kPinnedSlots slots.  A slab whose slots are all free again is
+// freed, except one (64 KiB) that stays for the next handle.
+namespace {
+constexpr int kPinnedSlots = 64;
+struct PinnedSlab {
+    char* p;
+    std::vector<int> free_slots;
+};
+std::mutex g_pinned_mu;
+std::vector<PinnedSlab>& pinned_slabs() {
+    static auto* s = new std::vector<PinnedSlab>();  // never destroyed: the process exit frees the memory
+    return *s;
+}
+// Frees the slabs without a slot in use, the first `keep` of them excepted.
+// Caller holds g_pinned_mu.
+void trim_pinned(int keep) noexcept {
+    auto& s = pinned_slabs();
+    for (size_t i = 0; i < s.size();) {
+        if ((int)s[i].free_slots.size() < kPinnedSlots || keep-- > 0) {
+            i++;
+            continue;
+        }
+        cudaFreeHost(s[i].p);
+        s[i] = std::move(s.back());
+        s.pop_back();
+    }
+}
+}  // namespace
+
+void* pinned_alloc() {
+    // cudaHostAlloc is not allowed beside another thread's stream capture
+    std::lock_guard<std::recursive_mutex> cap(capture_mutex());
+    std::lock_guard<std::mutex> lk(g_pinned_mu);
+    auto& s = pinned_slabs();
+    for (auto& b : s)
+        if (!b.free_slots.empty()) {
+            const int i = b.free_slots.back();
+            b.free_slots.pop_back();
+            return b.p + (size_t)i * kPinnedSlot;
+        }
+    PinnedSlab b;
+    void* p = nullptr;
+    DCRF_CUDA(cudaHostAlloc(&p, kPinnedSlots * kPinnedSlot, cudaHostAllocPortable));
+    b.p = static_cast<char*>(p);
+    for (int i = kPinnedSlots - 1; i > 0; i--) b.free_slots.push_back(i);
+    s.push_back(std::move(b));
+    return p;
+}
+
+void pinned_release(void* p) noexcept {
+    if (!p) return;
+    std::lock_guard<std::recursive_mutex> cap(capture_mutex());
+    std::lock_guard<std::mutex> lk(g_pinned_mu);
+    for (auto& b : pinned_slabs()) {
+        const char* q = static_cast<const char*>(p);
+        if (q >= b.p && q < b.p + kPinnedSlots * kPinnedSlot) {
+            b.free_slots.push_back((int)((q - b.p) / kPinnedSlot));
+            break;
+        }
+    }
+    trim_pinned(1);
+}
+
 void set_device_memory_limit(size_t bytes) {
     std::lock_guard<std::mutex> lk(g_mu);
     g_limit = bytes;
@@ -214,6 +277,10 @@ void dev_trim(bool all_devices) noexcept {
     std::lock_guard<std::recursive_mutex> cap(capture_mutex());
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return;
+    if (all_devices) {
+        std::lock_guard<std::mutex> lk(g_pinned_mu);
+        trim_pinned(0);
+    }
     {
         std::vector<int> devs;
         {

@@ -217,11 +217,14 @@ __global__ void fill_ones_kernel(long n, float* x) {
 Model::Model(int W_, int H_, int L_) : W(W_), H(H_), N(W_ * H_), L(L_) {
     DCRF_CUDA(cudaGetDevice(&device));
     DCRF_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-    DCRF_CUDA(cudaMallocHost(&h_scal, sizeof(SolverScalars)));
     scal.ensure(1);
     // per-block partials: fixed-grid reductions, and the per-pixel / per-element
     // kernels that fold a reduction in (two values per block)
-    partials.ensure(std::max<size_t>((size_t)kRedBlocks * 16, 2 * (size_t)std::max(ceil_div((long)N * L, 256), ord_slice_grid(N, L)) + 64));
+    partials.ensure(std::max<size_t>((size_t)kRedBlocks * 16,
+                                     2 * (size_t)std::max(ceil_div((long)N * L, 256), ord_slice_grid(N, L)) + 64));
+    static_assert(sizeof(SolverScalars) <= kPinnedSlot, "one slot per model");
+    h_scal = static_cast<SolverScalars*>(pinned_alloc());
+    std::memset(h_scal, 0, sizeof(SolverScalars));
 }
 
 Model::~Model() {
@@ -235,7 +238,7 @@ Model::~Model() {
     drop_qp_graph();
     if (gstream) cudaStreamDestroy(gstream);
     terms.clear();
-    if (h_scal) cudaFreeHost(h_scal);
+    pinned_release(h_scal);
     if (stream) cudaStreamDestroy(stream);
 }
 

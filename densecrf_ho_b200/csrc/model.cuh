@@ -82,6 +82,7 @@ struct Model {
     // iteration; gen counts the changes to the model that a graph may hold.
     cudaGraphExec_t qp_graph = nullptr;
     std::vector<const void*> qp_key;
+    std::vector<const void*> qp_seen;  // key of the last solve
     unsigned long long qp_graph_kernels = 0;
     bool qp_graph_failed = false;
     unsigned long long gen = 0;

@@ -1593,8 +1593,14 @@ int Model::qp(const float* init, float* out, int max_iter, double* energy_out) {
     // condition qp_cond_kernel sets -- until the stop rule fires, or kQpChunk
     // iterations per launch, after which the host looks at the stop flag and
     // launches it again.  The graph is kept for later solves with the same
-    // buffers and model.
+    // buffers and model.  Capturing and instantiating it costs as much as some
+    // ten eager iterations of a small image (0.6 ms), and a model made for one
+    // image solves once, usually in 3 to 6 iterations: the first solve with a
+    // key runs eagerly for kQpEager iterations before it builds the graph.
+    constexpr int kQpEager = 8;
     const std::vector<const void*> key = qp_graph_key(Q, max_iter);
+    const bool again = key == qp_seen;
+    qp_seen = key;
     int guard = 0;
     while (!h_scal->stop) {
         require(++guard < (1 << 26), DCRF_E_TIMEOUT, "qp: iteration cap reached");
@@ -1606,7 +1612,7 @@ int Model::qp(const float* init, float* out, int max_iter, double* energy_out) {
         }
         qp_iter();
         fetch_scalars();
-        if (!h_scal->stop && !qp_graph_failed && graphs_enabled()) {
+        if (!h_scal->stop && (again || guard >= kQpEager) && !qp_graph_failed && graphs_enabled()) {
             try {
                 build_qp_graph(qp_iter);
                 qp_key = key;
