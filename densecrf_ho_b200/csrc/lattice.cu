@@ -113,73 +113,106 @@ __device__ __forceinline__ float cvt_rne(float v) {
     return (float)__float2int_rn(v);
 }
 
-// K1: one thread per (padded) pixel.
-template <int DM>
-__global__ void elevate_kernel(const float* __restrict__ feat, int N, int Np, int d,
-                               const float* __restrict__ scale, int4* __restrict__ ekeys,
-                               int* __restrict__ rank_out, float* __restrict__ bary_out) {
+// K1: one thread per (padded) pixel.  DC: d as a compile-time constant, so that
+// every per-pixel array lives in registers (with run-time indexes they were in
+// local memory: 56 us for 640x480, d = 5), or 0 (d <= DM).
+struct ElevateScale {
+    float s[16];  // scale_factor_ per coordinate
+};
+template <int DM, int DC>
+__global__ void elevate_kernel(const float* __restrict__ feat, int N, int Np, int drt, ElevateScale scale,
+                               int4* __restrict__ ekeys, int* __restrict__ rank_out, float* __restrict__ bary_out) {
     constexpr int KW = (DM + 7) / 8;
+    constexpr int U = DC ? DC : DM;  // loop bounds; run-time d stops earlier
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= Np) return;
+    const int d = DC ? DC : drt;
     const int d1 = d + 1;
     const float invdp1 = 1.0f / (float)d1, dp1 = (float)d1;
-    float f[DM], el[DM + 1], rem0[DM + 1], rk[DM + 1], b[DM + 2];
-    for (int j = 0; j < d; j++) f[j] = k < N ? feat[(long)k * d + j] : 0.0f;
+    float f[U], el[U + 1], rem0[U + 1], rk[U + 1], b[U + 2];
+#pragma unroll
+    for (int j = 0; j < U; j++)
+        if (j < d) f[j] = k < N ? feat[(long)k * d + j] : 0.0f;
     // Elevation (:213-219): sm accumulates from the last coordinate down.
     float sm = 0.0f;
-    for (int j = d; j > 0; j--) {
-        float cf = fmul(f[j - 1], scale[j - 1]);
-        el[j] = fsub(sm, fmul((float)j, cf));
-        sm = fadd(sm, cf);
-    }
+#pragma unroll
+    for (int j = U; j > 0; j--)
+        if (j <= d) {
+            const float cf = fmul(f[j - 1], scale.s[j - 1]);
+            el[j] = fsub(sm, fmul((float)j, cf));
+            sm = fadd(sm, cf);
+        }
     el[0] = sm;
     // Closest 0-coloured simplex (:222-232).
     float sum = 0.0f;
-    for (int i = 0; i <= d; i++) {
-        float v = cvt_rne(fmul(invdp1, el[i]));
-        rem0[i] = fmul(v, dp1);
-        sum = fadd(sum, v);
-    }
-    // Rank (:235-245).
-    for (int i = 0; i <= d; i++) rk[i] = 0.0f;
-    for (int i = 0; i < d; i++) {
-        float di = fsub(el[i], rem0[i]);
-        for (int j = i + 1; j <= d; j++) {
-            float dj = fsub(el[j], rem0[j]);
-            float c = (di < dj) ? 1.0f : 0.0f;
-            rk[i] = fadd(rk[i], c);
-            rk[j] = fadd(rk[j], fsub(1.0f, c));
+#pragma unroll
+    for (int i = 0; i <= U; i++)
+        if (i <= d) {
+            const float v = cvt_rne(fmul(invdp1, el[i]));
+            rem0[i] = fmul(v, dp1);
+            sum = fadd(sum, v);
         }
-    }
+    // Rank (:235-245).
+#pragma unroll
+    for (int i = 0; i <= U; i++) rk[i] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < U; i++)
+        if (i < d) {
+            const float di = fsub(el[i], rem0[i]);
+#pragma unroll
+            for (int j = i + 1; j <= U; j++)
+                if (j <= d) {
+                    const float dj = fsub(el[j], rem0[j]);
+                    const float c = (di < dj) ? 1.0f : 0.0f;
+                    rk[i] = fadd(rk[i], c);
+                    rk[j] = fadd(rk[j], fsub(1.0f, c));
+                }
+        }
     // Back onto the plane (:248-254).
-    for (int i = 0; i <= d; i++) {
-        rk[i] = fadd(rk[i], sum);
-        float add = rk[i] < 0.0f ? dp1 : 0.0f;
-        float sub = rk[i] >= dp1 ? dp1 : 0.0f;
-        float t = fsub(add, sub);
-        rk[i] = fadd(rk[i], t);
-        rem0[i] = fadd(rem0[i], t);
-    }
+#pragma unroll
+    for (int i = 0; i <= U; i++)
+        if (i <= d) {
+            rk[i] = fadd(rk[i], sum);
+            const float add = rk[i] < 0.0f ? dp1 : 0.0f;
+            const float sub = rk[i] >= dp1 ? dp1 : 0.0f;
+            const float t = fsub(add, sub);
+            rk[i] = fadd(rk[i], t);
+            rem0[i] = fadd(rem0[i], t);
+        }
     // Barycentric coordinates (:257-275).
-    for (int i = 0; i < d + 2; i++) b[i] = 0.0f;
-    for (int i = 0; i <= d; i++) {
-        float v = fmul(fsub(el[i], rem0[i]), invdp1);
-        int p = (int)fsub((float)d, rk[i]);
-        p = min(max(p, 0), d);  // in range for finite features; guards NaN input
-        b[p] = fadd(b[p], v);
-        b[p + 1] = fsub(b[p + 1], v);
-    }
-    b[0] = fadd(b[0], fadd(1.0f, b[d + 1]));
+#pragma unroll
+    for (int i = 0; i < U + 2; i++) b[i] = 0.0f;
+#pragma unroll
+    for (int i = 0; i <= U; i++)
+        if (i <= d) {
+            const float v = fmul(fsub(el[i], rem0[i]), invdp1);
+            int p = (int)fsub((float)d, rk[i]);
+            p = min(max(p, 0), d);  // in range for finite features; guards NaN input
+#pragma unroll
+            for (int q = 0; q < U + 2; q++) {
+                if (q == p) b[q] = fadd(b[q], v);
+                if (q == p + 1) b[q] = fsub(b[q], v);
+            }
+        }
+    float last = 0.0f;  // b[d + 1]
+#pragma unroll
+    for (int q = 0; q < U + 2; q++)
+        if (q == d1) last = b[q];
+    b[0] = fadd(b[0], fadd(1.0f, last));
     // Keys of the d+1 vertices (:280-287); canonical simplex (:183-188).
-    for (int r = 0; r <= d; r++) {
+#pragma unroll
+    for (int r = 0; r <= U; r++) {
+        if (r > d) break;
         Key<KW> key;
         key_zero(key);
-        for (int i = 0; i < d; i++) {
-            int ri = (int)rk[i];
-            int canon = (ri <= d - r) ? r : r - d1;
-            key_set(key, i, (int16_t)(int)fadd(rem0[i], (float)canon));
-        }
-        long e = (long)k * d1 + r;
+#pragma unroll
+        for (int i = 0; i < U; i++)
+            if (i < d) {
+                const int ri = (int)rk[i];
+                const int canon = (ri <= d - r) ? r : r - d1;
+                key_set(key, i, (int16_t)(int)fadd(rem0[i], (float)canon));
+            }
+        const long e = (long)k * d1 + r;
 #pragma unroll
         for (int w = 0; w < KW; w++) ekeys[e * KW + w] = key.w[w];
         if (k < N) {
@@ -208,19 +241,13 @@ __global__ void insert_kernel(const int4* __restrict__ ekeys, int E, int* table,
             cur = old;
         }
         if (key_eq(load_key<KW>(ekeys, cur), key)) {
-            atomicMin(table + h, e);
+            // the slot only ever gets smaller: once it is at most e, e has no part in it
+            if (cur > e) atomicMin(table + h, e);
             entry_slot[e] = (int)h;
             return;
         }
         h = (h + 1) & mask;
     }
-}
-
-__global__ void first_flag_kernel(int E, const int* __restrict__ entry_slot,
-                                  const int* __restrict__ table, int* __restrict__ flag) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
-    flag[e] = table[entry_slot[e]] == e ? 1 : 0;
 }
 
 // K3: vertex ids and vertex keys.
@@ -280,25 +307,20 @@ __global__ void neighbor_kernel(int M, int d, const int16_t* __restrict__ vkeys,
     nbr[t] = make_int2(i1 + 1, i2 + 1);
 }
 
-__global__ void count_kernel(int E, const int* __restrict__ offset, int* __restrict__ counts) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e < E) atomicAdd(counts + offset[e], 1);
-}
-
-__global__ void iota_copy_kernel(int E, const int* __restrict__ offset, int* __restrict__ keys,
-                                 int* __restrict__ vals) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
-    keys[e] = offset[e];
-    vals[e] = e;
-}
-
-__global__ void seg_fill_kernel(int E, int d1, const int* __restrict__ sorted_entries,
-                                const float* __restrict__ bary, int2* __restrict__ seg) {
+// K5: the splat lists from the entries sorted by vertex: (pixel, weight) pairs,
+// and every list's start where the vertex changes (vertices without entries --
+// those only padding pixels touch -- start where the next list does).
+__global__ void seg_fill_kernel(int E, int M, int d1, const int* __restrict__ sorted_vertices,
+                                const int* __restrict__ sorted_entries, const float* __restrict__ bary,
+                                int2* __restrict__ seg, int* __restrict__ seg_start) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= E) return;
-    const int e = sorted_entries[s];
-    seg[s] = make_int2(e / d1, __float_as_int(bary[e]));
+    if (s > E) return;
+    const int v = s < E ? sorted_vertices[s] : M, before = s > 0 ? sorted_vertices[s - 1] : -1;
+    for (int u = before + 1; u <= v; u++) seg_start[u] = s;
+    if (s < E) {
+        const int e = sorted_entries[s];
+        seg[s] = make_int2(e / d1, __float_as_int(bary[e]));
+    }
 }
 
 // ------------------------------------------------------------- filter --
@@ -863,13 +885,6 @@ __global__ void __launch_bounds__(kSplatThreads)
     }
 }
 
-__global__ void count_long_kernel(int M, const int* __restrict__ counts, int threshold, int* __restrict__ n) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool is_long = v < M && counts[v] > threshold;
-    const unsigned b = __ballot_sync(0xffffffffu, is_long);
-    if ((threadIdx.x & 31) == 0 && b) atomicAdd(n, __popc(b));
-}
-
 // Class of a splat list by its length: 0 long, 1 short.
 __device__ __forceinline__ int list_class(int c) { return c > kLongList ? 0 : 1; }
 
@@ -877,13 +892,13 @@ __device__ __forceinline__ int list_class(int c) { return c > kLongList ? 0 : 1;
 // length-sorted visiting order, for a second stable sort that groups each
 // class's lists by image (longest first within an image), and the number of
 // lists per (class, image).
-__global__ void class_image_key_kernel(int M, const int* __restrict__ order, const int* __restrict__ counts,
+__global__ void class_image_key_kernel(int M, const int* __restrict__ order, const int* __restrict__ seg_start,
                                        const int* __restrict__ vimg, int images, int* __restrict__ keys,
                                        int* __restrict__ per_class_image) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= M) return;
     const int v = order[p];
-    const int key = list_class(counts[v]) * images + vimg[v];
+    const int key = list_class(seg_start[v + 1] - seg_start[v]) * images + vimg[v];
     keys[p] = key;
     atomicAdd(&per_class_image[key], 1);
 }
@@ -894,14 +909,28 @@ __global__ void class_image_key_kernel(int M, const int* __restrict__ order, con
 // order (first occurrence), so consecutive short lists gather rows of nearby
 // pixels and each input row is fetched from DRAM about once although d + 1
 // lists read it (sorting the short lists by length too scattered them over
-// the whole image).
-__global__ void order_key_kernel(int M, const int* __restrict__ counts, int* __restrict__ keys,
-                                 int* __restrict__ vals) {
+// the whole image).  Lengths count to a sixteenth of a power of two, which
+// keeps the classes apart (64 and 1024 are powers of two) and the key in one
+// 8-bit radix pass; three passes over exact lengths took 15 launches.  Also
+// counts the lists over kLongList and kHugeList entries (n[0], n[1]).
+constexpr int kOrderBits = 8;
+__global__ void order_key_kernel(int M, const int* __restrict__ seg_start, int* __restrict__ keys,
+                                 int* __restrict__ n) {
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= M) return;
-    const int c = counts[v];
-    keys[v] = c > kLongList ? kMaxOrderKey - min(c, kMaxOrderKey) : kMaxOrderKey;
-    vals[v] = v;
+    const int c = v < M ? seg_start[v + 1] - seg_start[v] : 0;
+    if (v < M) {
+        int key = 255;
+        if (c > kLongList) {
+            const int x = c - 1, e = 31 - __clz(x);  // x >= 64
+            key = 254 - min((e - 6) * 16 + ((x >> (e - 4)) & 15), 254);
+        }
+        keys[v] = key;
+    }
+    const unsigned l = __ballot_sync(0xffffffffu, c > kLongList), h = __ballot_sync(0xffffffffu, c > kHugeList);
+    if ((threadIdx.x & 31) == 0) {
+        if (l) atomicAdd(n, __popc(l));
+        if (h) atomicAdd(n + 1, __popc(h));
+    }
 }
 
 // One blur pass along one lattice axis: new = old + 1/2 (n1 + n2).  seqCompute
@@ -1136,29 +1165,24 @@ void build_impl(Lattice& L, const float* d_features) {
     require(E < (1L << 30), DCRF_E_ARG, "lattice too large (N*(d+1) >= 2^30)");
 
     // scale_factor (:190-194): computed in double, rounded to float.
-    std::vector<float> scale(d);
+    ElevateScale scale{};
     const float inv_std_dev = (float)(std::sqrt(2.0 / 3.0) * (d + 1));
-    for (int i = 0; i < d; i++) scale[i] = (float)(1.0 / std::sqrt((double)((i + 2) * (i + 1))) * inv_std_dev);
-    float* dscale = L.fscale.ensure(d);
-    DCRF_CUDA(cudaMemcpyAsync(dscale, scale.data(), sizeof(float) * d, cudaMemcpyHostToDevice, st));
+    for (int i = 0; i < d; i++) scale.s[i] = (float)(1.0 / std::sqrt((double)((i + 2) * (i + 1))) * inv_std_dev);
 
     int4* ekeys = L.ekeys.ensure((size_t)E * KW);
     int* rank = L.rank.ensure(Ereal);
     float* bary = L.bary.ensure(Ereal);
-    launch(elevate_kernel<DM>, ceil_div(Np, kTB), kTB, 0, st, d_features, N, Np, d, dscale, ekeys, rank, bary);
-    DCRF_LAUNCH_CHECK();
-
     unsigned cap = 1;
     while ((long)cap < 2 * E) cap <<= 1;
     int* table = L.table.ensure(cap);
     DCRF_CUDA(cudaMemsetAsync(table, 0xff, sizeof(int) * cap, st));
+    launch(d == DM ? elevate_kernel<DM, DM> : elevate_kernel<DM, 0>, ceil_div(Np, 128), 128, 0, st, d_features, N, Np,
+           d, scale, ekeys, rank, bary);
     int* eslot = L.entry_slot.ensure(E);
     launch(insert_kernel<KW>, ceil_div(E, kTB), kTB, 0, st, ekeys, (int)E, table, cap - 1, eslot);
     int* flags = L.flags.ensure(E);
-    launch(first_flag_kernel, ceil_div(E, kTB), kTB, 0, st, (int)E, eslot, table, flags);
-    DCRF_LAUNCH_CHECK();
-    int* dtotal = L.total.ensure(1);
-    exclusive_scan(flags, flags, (int)E, dtotal, L.scan, st);
+    int* dtotal = L.total.ensure(4);
+    first_flags_scan(eslot, table, (int)E, flags, dtotal, L.scan, st);
     int M = 0;
     DCRF_CUDA(cudaMemcpyAsync(&M, dtotal, sizeof(int), cudaMemcpyDeviceToHost, st));
     DCRF_CUDA(cudaStreamSynchronize(st));
@@ -1174,32 +1198,16 @@ void build_impl(Lattice& L, const float* d_features) {
                                                                      ekeys, slot_vid, nbr);
     DCRF_LAUNCH_CHECK();
 
-    // Splat lists: per-vertex counts -> starts; stable sort of entries by vertex.
-    int* counts = L.counts.ensure((size_t)M + 1);
-    DCRF_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * ((size_t)M + 1), st));
-    launch(count_kernel, ceil_div(Ereal, kTB), kTB, 0, st, (int)Ereal, offset, counts);
+    // Splat lists: stable sort of the entries by vertex, then the lists' starts.
     int* seg_start = L.seg_start.ensure((size_t)M + 1);
-    exclusive_scan(counts, seg_start, M + 1, nullptr, L.scan, st);
-    int* skeys = L.sort_keys.ensure(Ereal);
-    int* svals = L.sort_vals.ensure(Ereal);
-    launch(iota_copy_kernel, ceil_div(Ereal, kTB), kTB, 0, st, (int)Ereal, offset, skeys, svals);
-    DCRF_LAUNCH_CHECK();
-    radix_sort_pairs(skeys, svals, (int)Ereal, bits_for(M), L.sort, st);
+    const int *sorted_v, *sorted_e;
+    radix_sort_index(offset, (int)Ereal, bits_for(M), L.sort_keys.ensure(Ereal), L.sort_vals.ensure(Ereal), &sorted_v,
+                     &sorted_e, L.sort, st);
     int2* seg = L.seg.ensure(Ereal + kSegPad);
-    launch(seg_fill_kernel, ceil_div(Ereal, kTB), kTB, 0, st, (int)Ereal, d1, svals, bary, seg);
-    // Splat visiting order: longest lists first.
-    int* vorder = L.vorder.ensure(M);
-    int* okeys = L.vorder_keys.ensure(M);
-    launch(order_key_kernel, ceil_div(M, kTB), kTB, 0, st, M, counts, okeys, vorder);
-    radix_sort_pairs(okeys, vorder, M, 24, L.sort, st);
-    int* dlong = L.total.ensure(2);
-    DCRF_CUDA(cudaMemsetAsync(dlong, 0, 2 * sizeof(int), st));
-    launch(count_long_kernel, ceil_div(M, kTB), kTB, 0, st, M, counts, kLongList, dlong);
-    launch(count_long_kernel, ceil_div(M, kTB), kTB, 0, st, M, counts, kHugeList, dlong + 1);
-    DCRF_LAUNCH_CHECK();
+    launch(seg_fill_kernel, ceil_div(Ereal + 1, kTB), kTB, 0, st, (int)Ereal, M, d1, sorted_v, sorted_e,
+           (const float*)bary, seg, seg_start);
     int nl[2];
-    DCRF_CUDA(cudaMemcpyAsync(nl, dlong, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-    DCRF_CUDA(cudaStreamSynchronize(st));
+    L.visiting_order(nl);
     L.n_long = nl[0];
     L.n_huge = nl[1];
     L.va_floats = 0;
@@ -1349,12 +1357,22 @@ __global__ void fill_int_kernel(long n, int v, int* __restrict__ x) {
     if (t < n) x[t] = v;
 }
 
-__global__ void seg_count_kernel(int M, const int* __restrict__ seg_start, int* __restrict__ counts) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < M) counts[v] = seg_start[v + 1] - seg_start[v];
-}
-
 }  // namespace
+
+// vorder from seg_start (see order_key_kernel); nl: the lists over kLongList and
+// kHugeList entries.  Waits for the stream.
+void Lattice::visiting_order(int (&nl)[2]) {
+    int* dl = total.ensure(4);
+    DCRF_CUDA(cudaMemsetAsync(dl, 0, 2 * sizeof(int), stream));
+    int* ok = vorder_keys.ensure(std::max(M, 1));
+    int* vo = vorder.ensure(std::max(M, 1));
+    launch(order_key_kernel, ceil_div(M, kTB), kTB, 0, stream, M, (const int*)seg_start.get(), ok, dl);
+    const int *sk, *sv;
+    radix_sort_index(ok, M, kOrderBits, ok, vo, &sk, &sv, sort, stream);
+    if (sv != vo) DCRF_CUDA(cudaMemcpyAsync(vo, sv, sizeof(int) * M, cudaMemcpyDeviceToDevice, stream));
+    DCRF_CUDA(cudaMemcpyAsync(nl, dl, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream));
+    DCRF_CUDA(cudaStreamSynchronize(stream));
+}
 
 void Lattice::concat(const std::vector<const Lattice*>& parts) {
     require(!parts.empty(), DCRF_E_ARG, "lattice concat: no parts");
@@ -1402,12 +1420,10 @@ void Lattice::concat(const std::vector<const Lattice*>& parts) {
     const int Ei = (int)E;
     DCRF_CUDA(cudaMemcpyAsync(ss + M, &Ei, sizeof(int), cudaMemcpyHostToDevice, st));
     // Longest lists first, over all images.
-    int* cnt = counts.ensure(std::max(M, 1));
-    launch(seg_count_kernel, ceil_div(M, kTB), kTB, 0, st, M, ss, cnt);
-    int* vo = vorder.ensure(M);
-    int* ok = vorder_keys.ensure(M);
-    launch(order_key_kernel, ceil_div(M, kTB), kTB, 0, st, M, cnt, ok, vo);
-    radix_sort_pairs(ok, vo, M, 24, sort, st);
+    int nl[2];
+    visiting_order(nl);
+    int* vo = vorder.get();
+    int* ok = vorder_keys.get();
     // Then, stably, by (class, image): each class (long, short lists) holds
     // its lists image by image, longest first within an image, so
     // that an image's lists of a class are one contiguous range of the order
@@ -1416,19 +1432,13 @@ void Lattice::concat(const std::vector<const Lattice*>& parts) {
     DevBuf<int> pci;
     int* per_ci = pci.ensure((size_t)2 * B);
     DCRF_CUDA(cudaMemsetAsync(per_ci, 0, sizeof(int) * 2 * B, st));
-    launch(class_image_key_kernel, ceil_div(M, kTB), kTB, 0, st, M, (const int*)vo, (const int*)cnt,
+    launch(class_image_key_kernel, ceil_div(M, kTB), kTB, 0, st, M, (const int*)vo, (const int*)ss,
            (const int*)vi, B, ok, per_ci);
     int kbits = 1;
     while ((1L << kbits) < 2L * B) kbits++;
     radix_sort_pairs(ok, vo, M, kbits, sort, st);
-    int* dl = total.ensure(2);
-    DCRF_CUDA(cudaMemsetAsync(dl, 0, 2 * sizeof(int), st));
-    launch(count_long_kernel, ceil_div(M, kTB), kTB, 0, st, M, cnt, kLongList, dl);
-    launch(count_long_kernel, ceil_div(M, kTB), kTB, 0, st, M, cnt, kHugeList, dl + 1);
     DCRF_LAUNCH_CHECK();
-    int nl[2];
     std::vector<int> hci((size_t)2 * B);
-    DCRF_CUDA(cudaMemcpyAsync(nl, dl, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
     DCRF_CUDA(cudaMemcpyAsync(hci.data(), per_ci, sizeof(int) * 2 * B, cudaMemcpyDeviceToHost, st));
     DCRF_CUDA(cudaStreamSynchronize(st));  // also keeps &Ei alive until its copy ran
     n_long = nl[0];
@@ -1483,24 +1493,6 @@ void Lattice::build(const float* d_features, int d_, int N_) {
     else if (d <= 5) build_impl<5>(*this, d_features);
     else if (d <= 8) build_impl<8>(*this, d_features);
     else build_impl<16>(*this, d_features);
-}
-
-void Lattice::ensure_aux() {
-    if (aux) return;
-    int lo = 0, hi = 0;
-    DCRF_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-    DCRF_CUDA(cudaStreamCreateWithPriority(&aux, cudaStreamNonBlocking, hi));
-    DCRF_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-    DCRF_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
-}
-
-Lattice::~Lattice() {
-    if (aux) {
-        cudaStreamSynchronize(aux);
-        cudaEventDestroy(ev_fork);
-        cudaEventDestroy(ev_join);
-        cudaStreamDestroy(aux);
-    }
 }
 
 void Lattice::ensure_values(size_t row_width) {

@@ -115,9 +115,6 @@ struct Lattice {
     int n_long = 0;  // vertices whose splat list exceeds the staging threshold
     int n_huge = 0;  // ... and the (leading) ones whose list is very long
     cudaStream_t stream = nullptr;  // borrowed
-    // side stream (highest priority) for splat work that overlaps the rest
-    cudaStream_t aux = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
 
     DevBuf<int> offset, rank, seg_start;
     DevBuf<int2> seg;
@@ -139,8 +136,7 @@ struct Lattice {
 
     // build scratch
     DevBuf<int4> ekeys;
-    DevBuf<int> table, entry_slot, flags, slot_vid, sort_keys, sort_vals, counts, total;
-    DevBuf<float> fscale;
+    DevBuf<int> table, entry_slot, flags, slot_vid, sort_keys, sort_vals, total;
     ScanScratch scan;
     SortScratch sort;
 
@@ -222,7 +218,7 @@ struct Lattice {
     void gradient(float* df, const float* a, const float* b, int L);
 
     void ensure_values(size_t row_width);
-    void ensure_aux();
+    void visiting_order(int (&nl)[2]);
     // Times the candidate shapes on this lattice (on its value buffers, the
     // first large call) unless the process has tuned this problem class
     // already; outputs are not touched.
@@ -233,7 +229,6 @@ struct Lattice {
     Lattice() = default;
     Lattice(const Lattice&) = delete;
     Lattice& operator=(const Lattice&) = delete;
-    ~Lattice();
 };
 
 }  // namespace dcrf

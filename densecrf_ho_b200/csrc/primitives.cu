@@ -1,4 +1,6 @@
 // Deterministic device-wide integer primitives (no float atomics anywhere).
+#include <algorithm>
+
 #include "primitives.cuh"
 
 namespace dcrf {
@@ -106,62 +108,125 @@ constexpr int kSortItems = 16;
 constexpr int kSortTile = kSortThreads * kSortItems;
 constexpr int kRadix = 256;
 
-__global__ void radix_hist_kernel(const int* __restrict__ keys, int n, int shift, int ntiles,
-                                  int* __restrict__ hist) {
+// Histogram of one digit per tile; all of a thread's keys are loaded before
+// they are counted.
+__global__ void __launch_bounds__(kSortThreads)
+    radix_hist_kernel(const int* __restrict__ keys, int n, int shift, int ntiles, int* __restrict__ hist) {
     __shared__ int h[kRadix];
     for (int i = threadIdx.x; i < kRadix; i += blockDim.x) h[i] = 0;
     __syncthreads();
-    long base = (long)blockIdx.x * kSortTile;
-    for (int i = threadIdx.x; i < kSortTile; i += kSortThreads) {
-        long idx = base + i;
-        if (idx < n) atomicAdd(&h[(keys[idx] >> shift) & (kRadix - 1)], 1);
+    const long base = (long)blockIdx.x * kSortTile;
+    int k[kSortItems];
+#pragma unroll
+    for (int i = 0; i < kSortItems; i++) {
+        const long idx = base + i * kSortThreads + threadIdx.x;
+        k[i] = idx < n ? (keys[idx] >> shift) & (kRadix - 1) : -1;
     }
+#pragma unroll
+    for (int i = 0; i < kSortItems; i++)
+        if (k[i] >= 0) atomicAdd(&h[k[i]], 1);
     __syncthreads();
     for (int i = threadIdx.x; i < kRadix; i += blockDim.x) hist[(long)i * ntiles + blockIdx.x] = h[i];
 }
 
-// Stable scatter: within a tile, elements are ranked among equal digits in
-// index order (warp match + per-warp counts), then placed after the tiles
-// before it (digit-major scanned histogram).
-__global__ void radix_scatter_kernel(const int* __restrict__ keys_in, const int* __restrict__ vals_in,
-                                     int n, int shift, int ntiles, const int* __restrict__ offs,
-                                     int* __restrict__ keys_out, int* __restrict__ vals_out) {
-    __shared__ int running[kRadix];
-    __shared__ int wcnt[kSortThreads / 32][kRadix];
-    for (int i = threadIdx.x; i < kRadix; i += blockDim.x) {
-        running[i] = 0;
-        for (int w = 0; w < kSortThreads / 32; w++) wcnt[w][i] = 0;
+// One block per digit: exclusive scan of the digit's tile counts in place, its
+// total to hist[kRadix * ntiles + digit].  The scatter adds the totals of the
+// smaller digits, so the scan needs one launch.
+__global__ void __launch_bounds__(kScanThreads) radix_row_scan_kernel(int* __restrict__ hist, int ntiles) {
+    __shared__ int wt[kScanThreads / 32];
+    int* row = hist + (long)blockIdx.x * ntiles;
+    int carry = 0;
+    for (int base = 0; base < ntiles; base += kScanThreads) {
+        const int i = base + threadIdx.x;
+        const int v = i < ntiles ? row[i] : 0;
+        int tot;
+        const int ex = block_exclusive_scan(v, wt, &tot);
+        if (i < ntiles) row[i] = carry + ex;
+        carry += tot;
+        __syncthreads();  // wt is rewritten
+    }
+    if (threadIdx.x == 0) hist[(long)kRadix * ntiles + blockIdx.x] = carry;
+}
+
+// Stable scatter.  Each warp ranks 512 consecutive elements of the tile among
+// equal digits in index order (warp match + its own counts, no block barrier),
+// then the warps' counts are scanned per digit and every element goes after
+// the tiles and warps before it.  vals_in null: the value is the index.
+__global__ void __launch_bounds__(kSortThreads)
+    radix_scatter_kernel(const int* __restrict__ keys_in, const int* __restrict__ vals_in, int n, int shift,
+                         int ntiles, const int* __restrict__ offs, int* __restrict__ keys_out,
+                         int* __restrict__ vals_out) {
+    constexpr int W = kSortThreads / 32;
+    __shared__ int cnt[W][kRadix];
+    __shared__ int wt[kScanThreads / 32];
+    static_assert(kSortThreads == kRadix && kScanThreads == kSortThreads, "thread d owns digit d");
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, t = threadIdx.x;
+#pragma unroll
+    for (int i = 0; i < W; i++) cnt[i][t] = 0;
+    const long base = (long)blockIdx.x * kSortTile + (long)w * (kSortTile / W);
+    int key[kSortItems], rank[kSortItems];
+#pragma unroll
+    for (int i = 0; i < kSortItems; i++) {
+        const long idx = base + i * 32 + lane;
+        key[i] = idx < n ? keys_in[idx] : 0;
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const unsigned lt_mask = (1u << lane) - 1u;
-    long base = (long)blockIdx.x * kSortTile;
-    for (int it = 0; it < kSortItems; it++) {
-        long idx = base + (long)it * kSortThreads + threadIdx.x;
-        bool valid = idx < n;
-        int key = valid ? keys_in[idx] : 0;
-        int val = valid ? vals_in[idx] : 0;
-        int dig = valid ? ((key >> shift) & (kRadix - 1)) : kRadix;
-        unsigned peers = __match_any_sync(kFull, dig);
-        int rank = __popc(peers & lt_mask);
-        bool leader = (__ffs(peers) - 1) == lane;
-        int cnt = __popc(peers);
-        if (valid && leader) wcnt[w][dig] = cnt;
-        __syncthreads();
-        if (valid) {
-            int pos = running[dig] + rank;
-            for (int ww = 0; ww < w; ww++) pos += wcnt[ww][dig];
-            long o = (long)offs[(long)dig * ntiles + blockIdx.x] + pos;
-            keys_out[o] = key;
-            vals_out[o] = val;
-        }
-        __syncthreads();
-        if (valid && leader) {
-            atomicAdd(&running[dig], cnt);
-            wcnt[w][dig] = 0;
-        }
-        __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kSortItems; i++) {
+        const bool valid = base + i * 32 + lane < n;
+        const int dig = valid ? (key[i] >> shift) & (kRadix - 1) : kRadix;
+        const unsigned peers = __match_any_sync(kFull, dig);
+        rank[i] = __popc(peers & ((1u << lane) - 1u)) + (valid ? cnt[w][dig] : 0);
+        __syncwarp();
+        if (valid && (__ffs(peers) - 1) == lane) cnt[w][dig] += __popc(peers);
+        __syncwarp();
     }
+    __syncthreads();
+    {  // thread t: digit t's base over the digits, tiles and warps before it
+        int tot;
+        const int total = offs[(long)kRadix * ntiles + t];
+        int run = block_exclusive_scan(total, wt, &tot) + offs[(long)t * ntiles + blockIdx.x];
+#pragma unroll
+        for (int i = 0; i < W; i++) {
+            const int c = cnt[i][t];
+            cnt[i][t] = run;
+            run += c;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kSortItems; i++) {
+        const long idx = base + i * 32 + lane;
+        if (idx < n) {
+            const int o = cnt[w][(key[i] >> shift) & (kRadix - 1)] + rank[i];
+            keys_out[o] = key[i];
+            vals_out[o] = vals_in ? vals_in[idx] : (int)idx;
+        }
+    }
+}
+
+// First flags (lattice.cu): flag[e] = [table[slot[e]] == e] and their sums per
+// scan tile, in one pass.
+__global__ void flag_reduce_kernel(const int* __restrict__ slot, const int* __restrict__ table, int n,
+                                   int* __restrict__ flag, int* __restrict__ bsum) {
+    __shared__ int wt[kScanThreads / 32];
+    const long base = (long)blockIdx.x * kScanTile;
+    int s = 0, f[kScanItems];
+#pragma unroll
+    for (int i = 0; i < kScanItems; i++) {
+        const long e = base + i * kScanThreads + threadIdx.x;
+        f[i] = e < n ? slot[e] : -1;
+    }
+#pragma unroll
+    for (int i = 0; i < kScanItems; i++) {
+        const long e = base + i * kScanThreads + threadIdx.x;
+        f[i] = f[i] >= 0 && table[f[i]] == (int)e;
+        s += f[i];
+        if (e < n) flag[e] = f[i];
+    }
+    int tot;
+    block_exclusive_scan(s, wt, &tot);
+    if (threadIdx.x == 0) bsum[blockIdx.x] = tot;
 }
 
 }  // namespace
@@ -179,27 +244,54 @@ void exclusive_scan(const int* in, int* out, int n, int* d_total, ScanScratch& s
     DCRF_LAUNCH_CHECK();
 }
 
+void first_flags_scan(const int* slot, const int* table, int n, int* ranks, int* d_total, ScanScratch& s,
+                      cudaStream_t st) {
+    const int nb = ceil_div(n, kScanTile);
+    int* bs = s.block_sums.ensure(nb);
+    launch(flag_reduce_kernel, nb, kScanThreads, 0, st, slot, table, n, ranks, bs);
+    launch(scan_top_kernel, 1, kScanThreads, 0, st, bs, nb, d_total);
+    launch(scan_apply_kernel, nb, kScanThreads, 0, st, (const int*)ranks, ranks, n, (const int*)bs);
+    DCRF_LAUNCH_CHECK();
+}
+
+// Sorts (kin, vin) -- vin null: the indexes -- by passes that write alternately
+// to `a` and `b` buffers; returns true when the result is in a.
+static bool radix_passes(const int* kin, const int* vin, int* ka, int* va, int* kb, int* vb, int n, int key_bits,
+                         SortScratch& s, cudaStream_t st) {
+    const int ntiles = ceil_div(n, kSortTile);
+    int* hist = s.hist.ensure((size_t)kRadix * (ntiles + 1));
+    bool to_a = true;
+    for (int shift = 0; shift < key_bits; shift += 8) {
+        int *ko = to_a ? ka : kb, *vo = to_a ? va : vb;
+        launch(radix_hist_kernel, ntiles, kSortThreads, 0, st, kin, n, shift, ntiles, hist);
+        launch(radix_row_scan_kernel, kRadix, kScanThreads, 0, st, hist, ntiles);
+        launch(radix_scatter_kernel, ntiles, kSortThreads, 0, st, kin, vin, n, shift, ntiles, (const int*)hist, ko,
+               vo);
+        kin = ko;
+        vin = vo;
+        to_a = !to_a;
+    }
+    DCRF_LAUNCH_CHECK();
+    return !to_a;
+}
+
 void radix_sort_pairs(int* keys, int* vals, int n, int key_bits, SortScratch& s, cudaStream_t st) {
     if (n <= 1 || key_bits <= 0) return;
-    int ntiles = ceil_div(n, kSortTile);
     int* ka = s.keys_alt.ensure(n);
     int* va = s.vals_alt.ensure(n);
-    int* hist = s.hist.ensure((size_t)kRadix * ntiles);
-    int *kin = keys, *vin = vals, *kout = ka, *vout = va;
-    int passes = 0;
-    for (int shift = 0; shift < key_bits; shift += 8, passes++) {
-        launch(radix_hist_kernel, ntiles, kSortThreads, 0, st, kin, n, shift, ntiles, hist);
-        exclusive_scan(hist, hist, kRadix * ntiles, nullptr, s.scan, st);
-        launch(radix_scatter_kernel, ntiles, kSortThreads, 0, st, kin, vin, n, shift, ntiles, hist, kout,
-                                                             vout);
-        DCRF_LAUNCH_CHECK();
-        std::swap(kin, kout);
-        std::swap(vin, vout);
+    if (radix_passes(keys, vals, ka, va, keys, vals, n, key_bits, s, st)) {
+        DCRF_CUDA(cudaMemcpyAsync(keys, ka, sizeof(int) * n, cudaMemcpyDeviceToDevice, st));
+        DCRF_CUDA(cudaMemcpyAsync(vals, va, sizeof(int) * n, cudaMemcpyDeviceToDevice, st));
     }
-    if (kin != keys) {
-        DCRF_CUDA(cudaMemcpyAsync(keys, kin, sizeof(int) * n, cudaMemcpyDeviceToDevice, st));
-        DCRF_CUDA(cudaMemcpyAsync(vals, vin, sizeof(int) * n, cudaMemcpyDeviceToDevice, st));
-    }
+}
+
+void radix_sort_index(const int* keys, int n, int key_bits, int* kbuf, int* vbuf, const int** keys_out,
+                      const int** vals_out, SortScratch& s, cudaStream_t st) {
+    int* ka = s.keys_alt.ensure(std::max(n, 1));
+    int* va = s.vals_alt.ensure(std::max(n, 1));
+    const bool in_a = radix_passes(keys, nullptr, ka, va, kbuf, vbuf, n, std::max(key_bits, 1), s, st);
+    *keys_out = in_a ? ka : kbuf;
+    *vals_out = in_a ? va : vbuf;
 }
 
 }  // namespace dcrf

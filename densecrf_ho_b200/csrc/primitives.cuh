@@ -15,6 +15,11 @@ struct ScanScratch {
 void exclusive_scan(const int* in, int* out, int n, int* d_total, ScanScratch& s,
                     cudaStream_t st);
 
+// ranks[e] = number of e' < e with table[slot[e']] == e' (exclusive scan of the
+// first-occurrence flags); their total to d_total.
+void first_flags_scan(const int* slot, const int* table, int n, int* ranks, int* d_total, ScanScratch& s,
+                      cudaStream_t st);
+
 struct SortScratch {
     DevBuf<int> keys_alt, vals_alt, hist;
     ScanScratch scan;
@@ -25,5 +30,9 @@ struct SortScratch {
 // sort of (vertex id, entry index) pairs yields per-vertex entry lists in
 // increasing entry order.
 void radix_sort_pairs(int* keys, int* vals, int n, int key_bits, SortScratch& s, cudaStream_t st);
+// The same with the values 0 .. n-1 and the keys left as they are: the sorted
+// keys and indexes are returned in buffers of the scratch or in kbuf / vbuf [n].
+void radix_sort_index(const int* keys, int n, int key_bits, int* kbuf, int* vbuf, const int** keys_out,
+                      const int** vals_out, SortScratch& s, cudaStream_t st);
 
 }  // namespace dcrf
