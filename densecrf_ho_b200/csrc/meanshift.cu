@@ -11,7 +11,7 @@
 //      joint domain (x, y) / sigmaS, (L, u, v) / sigmaR, the neighbours found
 //      through a grid of unit buckets over (x, y, L), sums in double
 //      precision (NewNonOptimizedFilter, :3555-3907) -- the data-parallel
-//      step, one GPU thread per pixel (ms_filter_kernel);
+//      step, on the GPU (ms_filter_kernel);
 //   3. 8-connected labelling of the filtered image, colours closer than 0.1
 //      in every channel joining (Connect / Fill, :1166-1330);
 //   4. transitive closure over the region adjacency graph, joining adjacent
@@ -49,86 +49,114 @@ struct MsGrid {
     float sigma_s = 0.0f, sigma_r = 0.0f;
 };
 
-// One window shift at yk: Mh = mean of the points within the unit window
-// minus yk (zero when the window is empty).  The 27 buckets around yk's are
-// visited x-offset outermost, L-offset innermost, and each bucket's points
-// in decreasing pixel order -- the order EDISON's prepended bucket lists
-// walk -- so the double sums are the reference's.
-__device__ void ms_shift(const MsGrid& g, const double* __restrict__ cand, const int* __restrict__ bstart,
-                         const double (&yk)[kMsDim], double (&Mh)[kMsDim]) {
-#pragma unroll
-    for (int j = 0; j < kMsDim; j++) Mh[j] = 0.0;
-    double wsum = 0.0;
-    const int c1 = (int)yk[0] + 1, c2 = (int)yk[1] + 1, c3 = (int)__dsub_rn(yk[2], g.smin) + 1;
-    const int nb = g.nb1 * g.nb2 * g.nb3;
-    const int cb = c1 + g.nb1 * (c2 + g.nb2 * c3);
-    for (int a = -1; a <= 1; a++)
-        for (int b = -1; b <= 1; b++)
-            for (int c = -1; c <= 1; c++) {
-                const int bk = cb + a + g.nb1 * (b + g.nb2 * c);
-                if (bk < 0 || bk >= nb) continue;  // a window inside the data never leaves the grid
-                const int e1 = bstart[bk + 1];
-                for (int k = bstart[bk]; k < e1; k++) {
-                    const double* s = cand + (long)k * kMsDim;
-                    double el = __dsub_rn(s[0], yk[0]);
-                    double diff = __dmul_rn(el, el);
-                    el = __dsub_rn(s[1], yk[1]);
-                    diff = __dadd_rn(diff, __dmul_rn(el, el));
-                    if (diff < 1.0) {
-                        el = __dsub_rn(s[2], yk[2]);
-                        diff = yk[2] > g.hi_l ? __dmul_rn(__dmul_rn(4.0, el), el) : __dmul_rn(el, el);
-                        el = __dsub_rn(s[3], yk[3]);
-                        diff = __dadd_rn(diff, __dmul_rn(el, el));
-                        el = __dsub_rn(s[4], yk[4]);
-                        diff = __dadd_rn(diff, __dmul_rn(el, el));
-                        if (diff < 1.0) {  // uniform kernel, weight 1
-#pragma unroll
-                            for (int j = 0; j < kMsDim; j++) Mh[j] = __dadd_rn(Mh[j], s[j]);
-                            wsum = __dadd_rn(wsum, 1.0);
-                        }
-                    }
-                }
-            }
-    if (wsum > 0.0) {
-#pragma unroll
-        for (int j = 0; j < kMsDim; j++) Mh[j] = __dsub_rn(__ddiv_rn(Mh[j], wsum), yk[j]);
-    } else {
-#pragma unroll
-        for (int j = 0; j < kMsDim; j++) Mh[j] = 0.0;
-    }
-}
+constexpr int kMsLanes = 8;  // lanes that work on one pixel (ms_filter_kernel)
 
-// Mode seeking from every pixel: shift until the squared shift (the first
-// one unscaled, later ones rescaled to pixel and colour units) drops below
-// kMsEpsilon or kMsLimit iterations ran; out = the mode's colour times
-// sigmaR, rounded to float.
-__global__ void ms_filter_kernel(MsGrid g, const double* __restrict__ pts, const double* __restrict__ cand,
-                                 const int* __restrict__ bstart, float* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= g.N) return;
-    double yk[kMsDim], Mh[kMsDim];
-#pragma unroll
-    for (int j = 0; j < kMsDim; j++) yk[j] = pts[(long)i * kMsDim + j];
-    ms_shift(g, cand, bstart, yk, Mh);
-    double mv = 0.0;
-#pragma unroll
-    for (int j = 0; j < kMsDim; j++) mv = __dadd_rn(mv, __dmul_rn(Mh[j], Mh[j]));
+// Mode seeking from every pixel: shift the window until the squared shift
+// (the first one unscaled, later ones rescaled to pixel and colour units)
+// drops below kMsEpsilon or kMsLimit shifts were made; out = the mode's
+// colour times sigmaR, rounded to float.  A shift's target is the mean of the
+// points within the unit window (no shift where it holds none).
+//
+// The 27 buckets around the window are visited x-offset outermost, L-offset
+// innermost, and each bucket's points in decreasing pixel order -- the order
+// EDISON's prepended bucket lists walk -- so the double sums are the
+// reference's.  The buckets lie L-major in memory, so the three L offsets of
+// one (x, y) offset are one run of candidates: nine runs a shift.
+//
+// kMsLanes lanes work on one pixel: each tests one candidate, and lanes 0..4
+// then add one coordinate each of the accepted ones in order (-0.0 takes a
+// rejected one's place: it changes no sum).  The pixels of a warp walk their
+// runs in lockstep, and all lanes keep the window's position.
+//
+// Bound by FP64 issue and, with one thread a pixel as before, by the chain of
+// a slow pixel's up to 100 shifts of hundreds of dependent tests.  The whole
+// call, host preparation and copies included, radii 8 and 16 (range 8), one
+// thread a pixel -> now: 64x48 1.9 -> 0.5 and 9.6 -> 1.7 ms, 320x240 12.4 ->
+// 5.8 and 50.9 -> 13.4 ms, 640x480 33.5 -> 22.3 and 121 -> 55 ms.  16 or 32
+// lanes a pixel, measured without the two early ends of a step: 6.7 and 7.9
+// ms where 8 lanes took 6.5 (320x240, radius 8), 84 and 114 where 8 took 74
+// (640x480, radius 16).
+__global__ void __launch_bounds__(128)
+    ms_filter_kernel(MsGrid g, const double* __restrict__ pts, const double* __restrict__ cand,
+                     const int* __restrict__ bstart, float* __restrict__ out) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & (kMsLanes - 1);
+    const int base = threadIdx.x & 31 & ~(kMsLanes - 1);  // the group's first lane in its warp
+    const int i = blockIdx.x * (128 / kMsLanes) + threadIdx.x / kMsLanes;
+    const int jl = lane < kMsDim ? lane : 0;
+    const int nb = g.nb1 * g.nb2 * g.nb3;
     const double ss = g.sigma_s, sr = g.sigma_r;
-    int it = 1;
-    while (mv >= kMsEpsilon && it < kMsLimit) {
+    bool live = i < g.N;
+    double yk[kMsDim];
 #pragma unroll
-        for (int j = 0; j < kMsDim; j++) yk[j] = __dadd_rn(yk[j], Mh[j]);
-        ms_shift(g, cand, bstart, yk, Mh);
-        mv = __dmul_rn(__dmul_rn(__dadd_rn(__dmul_rn(Mh[0], Mh[0]), __dmul_rn(Mh[1], Mh[1])), ss), ss);
-        const double cr =
-            __dadd_rn(__dadd_rn(__dmul_rn(Mh[2], Mh[2]), __dmul_rn(Mh[3], Mh[3])), __dmul_rn(Mh[4], Mh[4]));
-        mv = __dadd_rn(mv, __dmul_rn(__dmul_rn(cr, sr), sr));
-        it++;
+    for (int j = 0; j < kMsDim; j++) yk[j] = live ? pts[(long)i * kMsDim + j] : 0.0;
+    for (int it = 1;; it++) {
+        const int c1 = (int)yk[0] + 1, c2 = (int)yk[1] + 1, c3 = (int)__dsub_rn(yk[2], g.smin) + 1;
+        const int cb = c3 + g.nb3 * (c2 + g.nb2 * c1);
+        const double l4 = yk[2] > g.hi_l ? 4.0 : 1.0;
+        double sum = 0.0;  // of coordinate jl
+        int cnt = 0;
+        for (int r = 0; r < 9; r++) {
+            const int bk = cb + g.nb3 * ((r % 3 - 1) + g.nb2 * (r / 3 - 1));
+            const bool in = live && bk >= 1 && bk < nb - 1;  // a window inside the data never leaves the grid
+            int k = in ? bstart[bk - 1] : 0;
+            const int e = in ? bstart[bk + 2] : 0;
+            for (; __any_sync(kAll, k < e); k += kMsLanes) {
+                const double* s = cand + (long)min(k + lane, max(e - 1, 0)) * kMsDim;
+                double el = __dsub_rn(s[0], yk[0]);
+                double diff = __dmul_rn(el, el);
+                el = __dsub_rn(s[1], yk[1]);
+                diff = __dadd_rn(diff, __dmul_rn(el, el));
+                bool ok = k + lane < e && diff < 1.0;
+                // A step is mostly one row of a bucket, in or out for the
+                // neighbouring pixels of a warp alike.
+                if (!__any_sync(kAll, ok)) continue;
+                // reads past the run's end stay inside the candidates' padding
+                const double* q = cand + (long)min(k, e) * kMsDim + jl;
+                double v[kMsLanes];
+#pragma unroll
+                for (int c = 0; c < kMsLanes; c++) v[c] = q[c * kMsDim];
+                el = __dsub_rn(s[2], yk[2]);
+                diff = __dmul_rn(__dmul_rn(l4, el), el);  // times 1 is exact
+                el = __dsub_rn(s[3], yk[3]);
+                diff = __dadd_rn(diff, __dmul_rn(el, el));
+                el = __dsub_rn(s[4], yk[4]);
+                diff = __dadd_rn(diff, __dmul_rn(el, el));
+                ok = ok && diff < 1.0;
+                const unsigned all = __ballot_sync(kAll, ok), m = all >> base;
+                if (all == 0u) continue;
+                cnt += __popc(m & (kAll >> (32 - kMsLanes)));
+#pragma unroll
+                for (int c = 0; c < kMsLanes; c++) sum = __dadd_rn(sum, m >> c & 1u ? v[c] : -0.0);
+            }
+        }
+        double Mh[kMsDim];
+#pragma unroll
+        for (int j = 0; j < kMsDim; j++) {
+            const double t = __shfl_sync(kAll, sum, base + j);
+            Mh[j] = cnt > 0 ? __dsub_rn(__ddiv_rn(t, (double)cnt), yk[j]) : 0.0;
+        }
+        double mv = 0.0;
+        if (it == 1) {
+#pragma unroll
+            for (int j = 0; j < kMsDim; j++) mv = __dadd_rn(mv, __dmul_rn(Mh[j], Mh[j]));
+        } else {
+            mv = __dmul_rn(__dmul_rn(__dadd_rn(__dmul_rn(Mh[0], Mh[0]), __dmul_rn(Mh[1], Mh[1])), ss), ss);
+            const double cr =
+                __dadd_rn(__dadd_rn(__dmul_rn(Mh[2], Mh[2]), __dmul_rn(Mh[3], Mh[3])), __dmul_rn(Mh[4], Mh[4]));
+            mv = __dadd_rn(mv, __dmul_rn(__dmul_rn(cr, sr), sr));
+        }
+        if (live) {
+#pragma unroll
+            for (int j = 0; j < kMsDim; j++) yk[j] = __dadd_rn(yk[j], Mh[j]);
+            live = mv >= kMsEpsilon && it < kMsLimit;
+        }
+        if (!__any_sync(kAll, live)) break;
     }
-#pragma unroll
-    for (int j = 0; j < kMsDim; j++) yk[j] = __dadd_rn(yk[j], Mh[j]);
-#pragma unroll
-    for (int j = 0; j < 3; j++) out[(long)i * 3 + j] = (float)__dmul_rn(yk[j + 2], sr);
+    if (lane < 3 && i < g.N) {
+        const double y = lane == 0 ? yk[2] : lane == 1 ? yk[3] : yk[4];
+        out[(long)i * 3 + lane] = (float)__dmul_rn(y, sr);
+    }
 }
 
 // ---------------------------------------------------------------- host --
@@ -441,13 +469,13 @@ void meanshift_filter(const uint8_t* rgb, int W, int H, int spatial_radius, floa
     for (int i = 0; i < N; i++) {
         const double* p = &pts[(size_t)kMsDim * i];
         const int c1 = (int)p[0] + 1, c2 = (int)p[1] + 1, c3 = (int)(p[2] - g.smin) + 1;
-        bucket[i] = c1 + g.nb1 * (c2 + g.nb2 * c3);
+        bucket[i] = c3 + g.nb3 * (c2 + g.nb2 * c1);  // L-major: ms_filter_kernel's runs
         bstart[bucket[i] + 1]++;
     }
     for (long b = 0; b < nb; b++) bstart[b + 1] += bstart[b];
     // within a bucket, decreasing pixel order (EDISON prepends to its lists)
     std::vector<int> fill(bstart.begin(), bstart.end() - 1);
-    std::vector<double> cand((size_t)kMsDim * N);
+    std::vector<double> cand((size_t)kMsDim * (N + kMsLanes));  // a group reads whole steps
     for (int i = N - 1; i >= 0; i--) {
         const int slot = fill[bucket[i]]++;
         std::memcpy(&cand[(size_t)kMsDim * slot], &pts[(size_t)kMsDim * i], sizeof(double) * kMsDim);
@@ -463,7 +491,7 @@ void meanshift_filter(const uint8_t* rgb, int W, int H, int spatial_radius, floa
     DCRF_CUDA(cudaMemcpyAsync(d_bstart.ensure(bstart.size()), bstart.data(), sizeof(int) * bstart.size(),
                               cudaMemcpyHostToDevice, stream));
     float* out = d_out.ensure((size_t)3 * N);
-    launch(ms_filter_kernel, ceil_div(N, 128), 128, 0, stream, g, (const double*)d_pts.get(),
+    launch(ms_filter_kernel, ceil_div(N, 128 / kMsLanes), 128, 0, stream, g, (const double*)d_pts.get(),
            (const double*)d_cand.get(), (const int*)d_bstart.get(), out);
     DCRF_LAUNCH_CHECK();
     DCRF_CUDA(cudaMemcpyAsync(filtered, out, sizeof(float) * 3 * N, cudaMemcpyDeviceToHost, stream));
