@@ -2,6 +2,7 @@
 #pragma once
 #include <type_traits>
 
+#include "lattice_device.cuh"
 #include "reduce.cuh"
 
 namespace dcrf {
@@ -62,6 +63,23 @@ __device__ __forceinline__ void tile_in4(float* buf, const float* __restrict__ g
         for (int j = 0; j < (8 * LC + 31) / 32; j++) {
             const int idx = j * 32 + lane;
             if (idx < 8 * LC) reinterpret_cast<float4*>(buf)[idx] = src[idx];
+        }
+    } else {
+        tile_in<LC>(buf, g, pix0, npix, lane);
+    }
+}
+// The same without a register in between: the copies are in flight until
+// cp_async_commit and cp_async_wait, so that a warp has several tiles' bytes
+// on their way at once.
+template <int LC>
+__device__ __forceinline__ void tile_in4_async(float* buf, const float* __restrict__ g, long pix0, int npix,
+                                               int lane) {
+    if (npix == 32 && (reinterpret_cast<uintptr_t>(g) & 15) == 0) {
+        const float4* src = reinterpret_cast<const float4*>(g + pix0 * LC);
+#pragma unroll
+        for (int j = 0; j < (8 * LC + 31) / 32; j++) {
+            const int idx = j * 32 + lane;
+            if (idx < 8 * LC) cp_async16(reinterpret_cast<float4*>(buf) + idx, src + idx);
         }
     } else {
         tile_in<LC>(buf, g, pix0, npix, lane);

@@ -609,49 +609,59 @@ __global__ void lp_gamma_kernel(int N, int Lrt, GammaConsts gc, const float* __r
     block_sum_store<1>(v, partials);
 }
 
-// |qp_value - qp_value1| < qp_tol test (:670-674).
-// Launched with one block of any multiple of 32 threads.
-__global__ void lp_gamma_check_kernel(const double* __restrict__ partials, int nblk, float qp_tol,
-                                      SolverScalars* sc) {
-    if (sc->stop) return;
-    __shared__ double s32[32];
-    double s = 0.0;
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x) s += partials[b];
-    s = block_sum_any(s, s32);
-    if (threadIdx.x == 0) {
-        const float qv1 = (float)s;
-        sc->steps++;
-        sc->gamma_sum++;
-        if (fabsf(fsub(sc->qp_value, qv1)) < qp_tol) sc->stop = 1;
-        else sc->qp_value = qv1;
-    }
-}
-
-// The same test as the exit condition of a graph's `while` node: the loop
-// goes on while the iterate has not converged and fewer than max_iter
-// iterations have run (the body always runs at least once).
-__global__ void lp_gamma_check_cond_kernel(const double* __restrict__ partials, int nblk, float qp_tol,
-                                           SolverScalars* sc, int max_iter, cudaGraphConditionalHandle h) {
-    __shared__ double s32[32];
-    double s = 0.0;
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x) s += partials[b];
-    s = block_sum_any(s, s32);
-    if (threadIdx.x == 0) {
-        if (!sc->stop) {
-            const float qv1 = (float)s;
-            sc->steps++;
-            sc->gamma_sum++;
-            if (fabsf(fsub(sc->qp_value, qv1)) < qp_tol) sc->stop = 1;
-            else sc->qp_value = qv1;
-        }
-        cudaGraphSetConditional(h, (!sc->stop && sc->steps < max_iter) ? 1u : 0u);
-    }
-}
-
 __global__ void lp_gamma_reset_kernel(SolverScalars* sc) {
     sc->stop = 0;
     sc->steps = 0;
     sc->qp_value = FLT_MAX;
+}
+
+// The |qp_value - qp_value1| < qp_tol test (:670-674) of one iteration's
+// objective; thread 0 only.
+__device__ __forceinline__ void lp_gamma_test(SolverScalars* sc, double s, float qp_tol) {
+    const float qv1 = (float)s;
+    sc->steps++;
+    sc->gamma_sum++;
+    if (fabsf(fsub(sc->qp_value, qv1)) < qp_tol) sc->stop = 1;
+    else sc->qp_value = qv1;
+}
+
+__device__ __forceinline__ double lp_partials_sum(const double* __restrict__ partials, int nblk, double* s32) {
+    double s = 0.0;
+    for (int b = threadIdx.x; b < nblk; b += blockDim.x) s += partials[b];
+    return block_sum_any(s, s32);
+}
+
+// The test after a single iteration.  With COND it sets the condition of a
+// graph's `while` node: the loop goes on while the iterate has not converged
+// and fewer than max_iter iterations have run.  Launched with one block of
+// any multiple of 32 threads.
+template <bool COND>
+__global__ void lp_gamma_check_kernel(const double* __restrict__ partials, int nblk, float qp_tol, SolverScalars* sc,
+                                      int max_iter, cudaGraphConditionalHandle h) {
+    if (!COND && sc->stop) return;
+    __shared__ double s32[32];
+    const double s = lp_partials_sum(partials, nblk, s32);
+    if (threadIdx.x == 0) {
+        if (!sc->stop) lp_gamma_test(sc, s, qp_tol);
+        if constexpr (COND) cudaGraphSetConditional(h, (!sc->stop && sc->steps < max_iter) ? 1u : 0u);
+    }
+}
+
+// The reset and the tests of lp_y_tiled's two iterations.
+template <bool COND>
+__global__ void lp_gamma_pair_kernel(const double* __restrict__ partials, int nblk, float qp_tol, SolverScalars* sc,
+                                     int max_iter, cudaGraphConditionalHandle h) {
+    __shared__ double s32[2][32];
+    const double s1 = lp_partials_sum(partials, nblk, s32[0]);
+    const double s2 = lp_partials_sum(partials + nblk, nblk, s32[1]);
+    if (threadIdx.x == 0) {
+        sc->stop = 0;
+        sc->steps = 0;
+        sc->qp_value = FLT_MAX;
+        lp_gamma_test(sc, s1, qp_tol);
+        if (!sc->stop) lp_gamma_test(sc, s2, qp_tol);
+        if constexpr (COND) cudaGraphSetConditional(h, (!sc->stop && sc->steps < max_iter) ? 1u : 0u);
+    }
 }
 
 // beta = -colsum(alpha + u + gamma - unary) / L (:684-691);
@@ -710,72 +720,154 @@ __global__ void lp_q_kernel(int N, int Lrt, float lambda, const float* __restric
 // Same arithmetic as lp_y_kernel / lp_q_kernel / lp_gamma_kernel /
 // qp_direction_kernel, one warp per 32 pixels, rows staged in shared memory.
 
+// One qp-gamma iteration of one pixel: g = the new gamma, returns the pixel's
+// objective as the reference's float.
 template <int LC>
-__global__ void __launch_bounds__(32 * kTileWarps)
-    lp_y_tiled(int N, float lambda, float cm, float* __restrict__ alpha, float* __restrict__ u,
-               const float* __restrict__ U, const float* __restrict__ curQ, float* __restrict__ Y, bool pending,
-               const float* __restrict__ sa, const float* __restrict__ su, const SolverScalars* __restrict__ sc) {
-    __shared__ __align__(16) float sm[kTileWarps][2][32 * LC];
-    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long pix0 = ((long)blockIdx.x * kTileWarps + wib) * 32;
-    if (pix0 >= N) return;
-    const int npix = (int)min(32L, (long)N - pix0);
-    float* A = sm[wib][0];
-    float* B = sm[wib][1];
-    float* ra = A + lane * LC;
-    float* rb = B + lane * LC;
-    const float dl = pending ? sc->delta : 0.0f;
-    float x[LC];
-    // alpha (+ pending update)
-    tile_in4<LC>(A, alpha, pix0, npix, lane);
-    if (pending) tile_in4<LC>(B, sa, pix0, npix, lane);
-    __syncwarp();
+__device__ __forceinline__ float gamma_row(const GammaConsts& gc, float (&g)[LC], const float (&y)[LC]) {
+    float t[LC];
+    const float s = eig_sum_ct<LC, 0>(g);
 #pragma unroll
     for (int k = 0; k < LC; k++) {
-        float a = ra[k];
-        if (pending) {
-            a = fadd(a, fmul(dl, fsub(rb[k], a)));
-            ra[k] = a;
-        }
-        x[k] = a;
+        const float ph = (-y[k] < 0.0f) ? 0.0f : -y[k];  // std::max(-Y, 0)
+        const float nh = (y[k] < 0.0f) ? 0.0f : y[k];    // std::max(Y, 0)
+        float st = fadd(fmul(fsub(s, g[k]), gc.c0), ph);
+        st = fadd(st, gc.delta);
+        float tt = fmul(fadd(fmul(gc.c1, s), fmul(gc.c2, g[k])), gc.lambda);
+        tt = fadd(tt, nh);
+        tt = fadd(tt, gc.delta);
+        g[k] = fmul(g[k], st / tt);
     }
-    __syncwarp();
-    if (pending) tile_out4<LC>(A, alpha, pix0, npix, lane);
-    __syncwarp();
-    // u (+ pending update)
-    if (u) {
-        tile_in4<LC>(A, u, pix0, npix, lane);
-        if (pending && su) tile_in4<LC>(B, su, pix0, npix, lane);
+    const float s2 = eig_sum_ct<LC, 0>(g);
+#pragma unroll
+    for (int k = 0; k < LC; k++) t[k] = fmul(g[k], fmul(fadd(fmul(gc.cm, s2), g[k]), gc.lambda));
+    const float d1 = eig_sum_ct<LC, 0>(t);
+#pragma unroll
+    for (int k = 0; k < LC; k++) t[k] = fmul(g[k], y[k]);
+    const float d2 = eig_sum_ct<LC, 0>(t);
+    return (float)dadd(dmul(0.5, (double)d1), (double)d2);
+}
+
+// lp_y_kernel's step, and with GAMMA the first two qp-gamma iterations on the
+// rows it holds anyway (lp_gamma_pair_kernel tests them; partials[b] and
+// partials[gridDim.x + b] are their objectives): gamma is read and written
+// once instead of twice and Y not read again, the objectives' sums are the
+// ones lp_gamma_tiled forms.
+//
+// Bound by memory: eight arrays of N L floats in or out (U, cur_Q, sa, alpha
+// and gamma in, alpha, Y and gamma out), ten with cliques; the tiles that fit
+// are on their way before the first is used.  640x480, 21 labels: 42 us with
+// its 5 us of tests, where lp_y, the reset and two launches of lp_gamma_tiled
+// with their tests took 73.  A third array pass over gamma and Y by
+// lp_gamma_tiled runs in about four of ten iterations, 16.6 -> 11.6 us there
+// through tile_in4_async.
+template <int LC, bool GAMMA>
+__global__ void __launch_bounds__(32 * kTileWarps)
+    lp_y_tiled(int N, GammaConsts gc, float* __restrict__ alpha, float* __restrict__ u, const float* __restrict__ U,
+               const float* __restrict__ curQ, float* __restrict__ Y, bool pending, const float* __restrict__ sa,
+               const float* __restrict__ su, const SolverScalars* __restrict__ sc, float* __restrict__ gamma,
+               double* __restrict__ partials) {
+    __shared__ __align__(16) float sm[kTileWarps][4][32 * LC];
+    __shared__ double s32[2][32];
+    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long pix0 = ((long)blockIdx.x * kTileWarps + wib) * 32;
+    double acc0 = 0.0, acc1 = 0.0;
+    if (pix0 < N) {
+        const int npix = (int)min(32L, (long)N - pix0);
+        float *A = sm[wib][0], *B = sm[wib][1], *C = sm[wib][2], *D = sm[wib][3];
+        float *ra = A + lane * LC, *rb = B + lane * LC, *rd = D + lane * LC;
+        const float* rc = C + lane * LC;
+        tile_in4_async<LC>(A, alpha, pix0, npix, lane);
+        if (pending) tile_in4_async<LC>(B, sa, pix0, npix, lane);
+        cp_async_commit();
+        tile_in4_async<LC>(C, U, pix0, npix, lane);
+        tile_in4_async<LC>(D, curQ, pix0, npix, lane);
+        cp_async_commit();
+        const float dl = pending ? sc->delta : 0.0f;
+        float x[LC];
+        // alpha (+ pending update)
+        cp_async_wait<1>();
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < LC; k++) {
-            float uu = ra[k];
+            float a = ra[k];
             if (pending) {
-                uu = fadd(uu, fmul(dl, fsub(su ? rb[k] : 0.0f, uu)));
-                ra[k] = uu;
+                a = fadd(a, fmul(dl, fsub(rb[k], a)));
+                ra[k] = a;
             }
-            x[k] = fadd(x[k], uu);
+            x[k] = a;
         }
         __syncwarp();
-        if (pending) tile_out4<LC>(A, u, pix0, npix, lane);
+        if (GAMMA && !u) tile_in4_async<LC>(B, gamma, pix0, npix, lane);
+        cp_async_commit();
+        if (pending) tile_out4<LC>(A, alpha, pix0, npix, lane);
+        // u (+ pending update)
+        if (u) {
+            __syncwarp();
+            tile_in4_async<LC>(A, u, pix0, npix, lane);
+            if (pending && su) tile_in4_async<LC>(B, su, pix0, npix, lane);
+            cp_async_commit();
+            cp_async_wait<0>();
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < LC; k++) {
+                float uu = ra[k];
+                if (pending) {
+                    uu = fadd(uu, fmul(dl, fsub(su ? rb[k] : 0.0f, uu)));
+                    ra[k] = uu;
+                }
+                x[k] = fadd(x[k], uu);
+            }
+            __syncwarp();
+            if (GAMMA) tile_in4_async<LC>(B, gamma, pix0, npix, lane);
+            cp_async_commit();
+            if (pending) tile_out4<LC>(A, u, pix0, npix, lane);
+        } else {
+#pragma unroll
+            for (int k = 0; k < LC; k++) x[k] = fadd(x[k], 0.0f);
+        }
+        // x = (alpha + u) - unary;  Y = multiplyC(x) + cur_Q
+        cp_async_wait<1>();
         __syncwarp();
-    } else {
 #pragma unroll
-        for (int k = 0; k < LC; k++) x[k] = fadd(x[k], 0.0f);
+        for (int k = 0; k < LC; k++) x[k] = fsub(x[k], rc[k]);
+        const float s = eig_sum_ct<LC, 0>(x);
+#pragma unroll
+        for (int k = 0; k < LC; k++) {
+            x[k] = fadd(fmul(fadd(fmul(gc.cm, s), x[k]), gc.lambda), rd[k]);
+            rd[k] = x[k];
+        }
+        __syncwarp();
+        tile_out4<LC>(D, Y, pix0, npix, lane);
+        if constexpr (GAMMA) {
+            cp_async_wait<0>();
+            __syncwarp();
+            float g[LC];
+#pragma unroll
+            for (int k = 0; k < LC; k++) g[k] = rb[k];
+#pragma unroll 1
+            for (int r = 0; r < 2; r++) {
+                acc0 = acc1;
+                acc1 = (double)gamma_row<LC>(gc, g, x);
+            }
+#pragma unroll
+            for (int k = 0; k < LC; k++) rb[k] = g[k];
+            if (lane >= npix) acc0 = acc1 = 0.0;
+            __syncwarp();
+            tile_out4<LC>(B, gamma, pix0, npix, lane);
+        }
     }
-    // x = (alpha + u) - unary;  Y = multiplyC(x) + cur_Q
-    tile_in4<LC>(A, U, pix0, npix, lane);
-    tile_in4<LC>(B, curQ, pix0, npix, lane);
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < LC; k++) x[k] = fsub(x[k], ra[k]);
-    const float s = eig_sum_ct<LC, 0>(x);
-#pragma unroll
-    for (int k = 0; k < LC; k++) rb[k] = fadd(fmul(fadd(fmul(cm, s), x[k]), lambda), rb[k]);
-    __syncwarp();
-    tile_out4<LC>(B, Y, pix0, npix, lane);
+    if constexpr (GAMMA) {
+        const double t0 = block_sum_any(acc0, s32[0]);
+        const double t1 = block_sum_any(acc1, s32[1]);
+        if (threadIdx.x == 0) {
+            partials[blockIdx.x] = t0;
+            partials[gridDim.x + blockIdx.x] = t1;
+        }
+    }
 }
 
+// lp_q_kernel's step, five or six arrays in or out: 39 -> 26 us (640x480, 21
+// labels) with all tiles on their way at once.
 template <int LC>
 __global__ void __launch_bounds__(32 * kTileWarps)
     lp_q_tiled(int N, float lambda, const float* __restrict__ alpha, const float* __restrict__ u,
@@ -789,10 +881,15 @@ __global__ void __launch_bounds__(32 * kTileWarps)
     if (pix0 < N) {
         const int npix = (int)min(32L, (long)N - pix0);
         float* T[4] = {sm[wib][0], sm[wib][1], sm[wib][2], sm[wib][3]};
-        tile_in4<LC>(T[0], alpha, pix0, npix, lane);
-        if (u) tile_in4<LC>(T[1], u, pix0, npix, lane);
-        tile_in4<LC>(T[2], gamma, pix0, npix, lane);
-        tile_in4<LC>(T[3], U, pix0, npix, lane);
+        // without u its tile takes curQ, which else follows once alpha's is free
+        tile_in4_async<LC>(T[0], alpha, pix0, npix, lane);
+        tile_in4_async<LC>(T[2], gamma, pix0, npix, lane);
+        tile_in4_async<LC>(T[3], U, pix0, npix, lane);
+        if (u) tile_in4_async<LC>(T[1], u, pix0, npix, lane);
+        cp_async_commit();
+        if (!u) tile_in4_async<LC>(T[1], curQ, pix0, npix, lane);
+        cp_async_commit();
+        cp_async_wait<1>();
         __syncwarp();
         const float *ra = T[0] + lane * LC, *ru = T[1] + lane * LC, *rg = T[2] + lane * LC, *rU = T[3] + lane * LC;
         float t[LC];
@@ -802,9 +899,12 @@ __global__ void __launch_bounds__(32 * kTileWarps)
 #pragma unroll
         for (int k = 0; k < LC; k++) t[k] = fsub(fadd(fadd(fadd(ra[k], beta), u ? ru[k] : 0.0f), rg[k]), rU[k]);
         __syncwarp();
-        tile_in4<LC>(T[0], curQ, pix0, npix, lane);
+        float* tq = u ? T[0] : T[1];
+        if (u) tile_in4_async<LC>(tq, curQ, pix0, npix, lane);
+        cp_async_commit();
+        cp_async_wait<0>();
         __syncwarp();
-        float* rq = T[0] + lane * LC;
+        float* rq = tq + lane * LC;
         const bool act = lane < npix;
 #pragma unroll
         for (int k = 0; k < LC; k++) {
@@ -816,7 +916,7 @@ __global__ void __launch_bounds__(32 * kTileWarps)
             }
         }
         __syncwarp();
-        tile_out4<LC>(T[0], Q, pix0, npix, lane);
+        tile_out4<LC>(tq, Q, pix0, npix, lane);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -852,36 +952,23 @@ __global__ void __launch_bounds__(32 * kTileWarps)
         const int npix = (int)min(32L, (long)N - pix0);
         float* G = sm[wib][0];
         float* Yt = sm[wib][1];
-        tile_in4<LC>(G, gamma, pix0, npix, lane);
-        tile_in4<LC>(Yt, Y, pix0, npix, lane);
+        tile_in4_async<LC>(G, gamma, pix0, npix, lane);
+        tile_in4_async<LC>(Yt, Y, pix0, npix, lane);
+        cp_async_commit();
+        cp_async_wait<0>();
         __syncwarp();
         float* rg = G + lane * LC;
         const float* ry = Yt + lane * LC;
-        float g[LC], t[LC];
-#pragma unroll
-        for (int k = 0; k < LC; k++) g[k] = rg[k];
-        const float s = eig_sum_ct<LC, 0>(g);
+        float g[LC], y[LC];
 #pragma unroll
         for (int k = 0; k < LC; k++) {
-            const float y = ry[k];
-            const float ph = (-y < 0.0f) ? 0.0f : -y;  // std::max(-Y, 0)
-            const float nh = (y < 0.0f) ? 0.0f : y;    // std::max(Y, 0)
-            float st = fadd(fmul(fsub(s, g[k]), gc.c0), ph);
-            st = fadd(st, gc.delta);
-            float tt = fmul(fadd(fmul(gc.c1, s), fmul(gc.c2, g[k])), gc.lambda);
-            tt = fadd(tt, nh);
-            tt = fadd(tt, gc.delta);
-            g[k] = fmul(g[k], st / tt);
-            rg[k] = g[k];
+            g[k] = rg[k];
+            y[k] = ry[k];
         }
-        const float s2 = eig_sum_ct<LC, 0>(g);
+        const float qv = gamma_row<LC>(gc, g, y);
+        if (lane < npix) acc = (double)qv;
 #pragma unroll
-        for (int k = 0; k < LC; k++) t[k] = fmul(g[k], fmul(fadd(fmul(gc.cm, s2), g[k]), gc.lambda));
-        const float d1 = eig_sum_ct<LC, 0>(t);
-#pragma unroll
-        for (int k = 0; k < LC; k++) t[k] = fmul(g[k], ry[k]);
-        const float d2 = eig_sum_ct<LC, 0>(t);
-        if (lane < npix) acc = (double)(float)dadd(dmul(0.5, (double)d1), (double)d2);
+        for (int k = 0; k < LC; k++) rg[k] = g[k];
         __syncwarp();
         tile_out4<LC>(G, gamma, pix0, npix, lane);
     }
@@ -901,9 +988,11 @@ __global__ void __launch_bounds__(32 * kTileWarps)
     if (pix0 < N) {
         const int npix = (int)min(32L, (long)N - pix0);
         float *Gt = sm[wib][0], *Qt = sm[wib][1], *Ut = sm[wib][2];
-        tile_in4<LC>(Gt, grad, pix0, npix, lane);
-        tile_in4<LC>(Qt, Q, pix0, npix, lane);
-        tile_in4<LC>(Ut, U, pix0, npix, lane);
+        tile_in4_async<LC>(Gt, grad, pix0, npix, lane);
+        tile_in4_async<LC>(Qt, Q, pix0, npix, lane);
+        tile_in4_async<LC>(Ut, U, pix0, npix, lane);
+        cp_async_commit();
+        cp_async_wait<0>();
         __syncwarp();
         const float* rg = Gt + lane * LC;
         float* rq = Qt + lane * LC;
@@ -1699,23 +1788,38 @@ int Model::lp(const float* init, float* out, const dcrf_lp_params& p, dcrf_solve
     int it = 0, count = 0, fw_total = 0;
     DCRF_CUDA(cudaMemsetAsync(&sc->gamma_sum, 0, sizeof(int), stream));
 
-    // One Frank-Wolfe iteration in three parts: lp_y and the qp-gamma reset
-    // (s1), the qp-gamma iterations, and Q, the bins, the clique and ordered
+    // One Frank-Wolfe iteration in three parts: lp_y with the qp-gamma reset
+    // or the first two iterations (s1), the other qp-gamma iterations, and Q, the bins, the clique and ordered
     // subgradients and the dual-gap step (s2).
-    auto s1 = [&](bool pending) {
+    //
+    // The first test compares with FLT_MAX and, below the tolerance of the
+    // rule (a float next to FLT_MAX is 2e31 away), fails for every objective
+    // a solve can have, so the second iteration always runs where max_iter
+    // allows it: the row-tiled lp_y does both.
+    bool pair = p.qp_max_iter >= 2 && p.qp_tol < 1e30f;
+    with_lc(L, [&](auto lc) { pair = pair && decltype(lc)::value > 0; });
+    auto s1 = [&](bool pending, const cudaGraphConditionalHandle* h) {
         // alpha / u of the previous iteration are updated inside lp_y (the
         // update after the last iteration is never read: both are reset
         // before the next proximal step).
         with_lc(L, [&](auto lc) {
             constexpr int LC = decltype(lc)::value;
-            if constexpr (LC > 0)
-                launch(lp_y_tiled<LC>, tgrid, 32 * kTileWarps, 0, stream, N, lambda, gc.cm, alpha, u, unary.get(),
-                       curQ, Y, pending, sa, su, sc);
-            else
+            if constexpr (LC > 0) {
+                auto* kern = pair ? lp_y_tiled<LC, true> : lp_y_tiled<LC, false>;
+                launch(kern, tgrid, 32 * kTileWarps, 0, stream, N, gc, alpha, u, unary.get(), curQ, Y, pending, sa, su,
+                       sc, gamma, part);
+            } else {
                 launch(lp_y_kernel<LC>, pg, kPix, 0, stream, N, L, lambda, gc.cm, alpha, u, unary.get(), curQ, Y,
                        pending, sa, su, sc);
+            }
         });
-        launch(lp_gamma_reset_kernel, 1, 1, 0, stream, sc);
+        if (!pair)
+            launch(lp_gamma_reset_kernel, 1, 1, 0, stream, sc);
+        else if (h)
+            launch(lp_gamma_pair_kernel<true>, 1, 1024, 0, stream, part, tgrid, p.qp_tol, sc, p.qp_max_iter, *h);
+        else
+            launch(lp_gamma_pair_kernel<false>, 1, 1024, 0, stream, part, tgrid, p.qp_tol, sc, p.qp_max_iter,
+                   cudaGraphConditionalHandle{});
     };
     // One qp-gamma iteration on stream st; with a graph handle its test also
     // sets the graph's loop condition.
@@ -1728,9 +1832,10 @@ int Model::lp(const float* init, float* out, const dcrf_lp_params& p, dcrf_solve
             else
                 launch(lp_gamma_kernel<LC>, kRedBlocks, kRedThreads, 0, st, N, L, gc, Y, gamma, sc, part);
             if (h)
-                launch(lp_gamma_check_cond_kernel, 1, 1024, 0, st, part, nblk, p.qp_tol, sc, p.qp_max_iter, *h);
+                launch(lp_gamma_check_kernel<true>, 1, 1024, 0, st, part, nblk, p.qp_tol, sc, p.qp_max_iter, *h);
             else
-                launch(lp_gamma_check_kernel, 1, 1024, 0, st, part, nblk, p.qp_tol, sc);
+                launch(lp_gamma_check_kernel<false>, 1, 1024, 0, st, part, nblk, p.qp_tol, sc, p.qp_max_iter,
+                       cudaGraphConditionalHandle{});
         });
     };
     auto s2 = [&]() {
@@ -1789,7 +1894,8 @@ int Model::lp(const float* init, float* out, const dcrf_lp_params& p, dcrf_solve
         DCRF_LAUNCH_CHECK();
     };
     // The whole iteration as one CUDA graph: s1, a `while` node whose body is
-    // one qp-gamma iteration and whose condition its test kernel sets, s2.
+    // one qp-gamma iteration and whose condition the test kernels set (s1's
+    // too: its default lets the body run), s2.
     // Built after the first iteration has run eagerly (it sizes every buffer
     // the iteration touches) and used for the rest of the solve: no host
     // round trip per iteration.  Kernel launch counts: the graph's own
@@ -1808,7 +1914,7 @@ int Model::lp(const float* init, float* out, const dcrf_lp_params& p, dcrf_solve
     cudaGraphExec_t* fw_graph = fwg.g;
     unsigned long long fw_graph_kernels = 0;
     bool graphs_ok = graphs_enabled();
-    int eager_gamma = 0;
+    int outside_body = 0;  // qp-gamma iterations that ran outside a graph's loop
     auto drop_graphs = [&]() { fwg.drop(); };
     auto build_graph = [&](bool pending) -> cudaGraphExec_t {
         std::lock_guard<std::recursive_mutex> cap(capture_mutex());
@@ -1822,7 +1928,7 @@ int Model::lp(const float* init, float* out, const dcrf_lp_params& p, dcrf_solve
             const unsigned long long k0 = g_kernel_launches.load();
             DCRF_CUDA(cudaStreamBeginCaptureToGraph(stream, g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
             main_cap = true;
-            s1(pending);
+            s1(pending, &h);
             cudaStreamCaptureStatus cs;
             cudaGraph_t cg = nullptr;
             const cudaGraphNode_t* deps = nullptr;
@@ -1884,14 +1990,18 @@ int Model::lp(const float* init, float* out, const dcrf_lp_params& p, dcrf_solve
             if (graphs_ok && fw_graph[pending]) {
                 DCRF_CUDA(cudaGraphLaunch(fw_graph[pending], stream));
                 g_kernel_launches.fetch_add(fw_graph_kernels);
+                if (pair) outside_body += 2;
                 continue;
             }
-            s1(pending);
-            // qp-gamma iterations; the reference needs at least two (its first
-            // test compares against FLT_MAX), so launch in pairs and look at
-            // the stop flag after each pair.
+            s1(pending, nullptr);
+            // The other qp-gamma iterations, in pairs, with a look at the stop
+            // flag after each pair.
             int launched = 0;
-            for (;;) {
+            if (pair) {
+                launched = 2;
+                fetch_scalars();
+            }
+            while (!pair || (!h_scal->stop && launched < p.qp_max_iter)) {
                 const int batch = std::min(2, p.qp_max_iter - launched);
                 for (int bi = 0; bi < batch; bi++) gamma_step(stream, nullptr);
                 launched += batch;
@@ -1899,7 +2009,7 @@ int Model::lp(const float* init, float* out, const dcrf_lp_params& p, dcrf_solve
                 fetch_scalars();
                 if (h_scal->stop || launched >= p.qp_max_iter || batch <= 0) break;
             }
-            eager_gamma += h_scal->steps;
+            outside_body += h_scal->steps;
             s2();
             if (graphs_ok && !fw_graph[0]) {
                 try {
@@ -1951,8 +2061,8 @@ int Model::lp(const float* init, float* out, const dcrf_lp_params& p, dcrf_solve
         }
     } while (it < p.prox_max_iter);
     fetch_scalars();
-    // the two kernels of each qp-gamma iteration that ran inside a graph
-    g_kernel_launches.fetch_add(2ull * (unsigned long long)std::max(0, h_scal->gamma_sum - eager_gamma));
+    // the two kernels of each qp-gamma iteration that ran inside a graph's loop
+    g_kernel_launches.fetch_add(2ull * (unsigned long long)std::max(0, h_scal->gamma_sum - outside_body));
     if (stats) {
         stats->iterations = it;
         stats->inner_iters = fw_total;
