@@ -99,7 +99,7 @@ __device__ __forceinline__ float2 ord_bin_pair(float q) {
 __device__ __forceinline__ int ord_lower_of(float2 b) { return (int)b.x; }
 __device__ __forceinline__ int ord_upper_of(float2 b) { return (int)b.y; }
 
-inline bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+__host__ __device__ inline bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
 }  // namespace
 

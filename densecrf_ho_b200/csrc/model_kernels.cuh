@@ -82,7 +82,13 @@ __device__ __forceinline__ void tile_in4_async(float* buf, const float* __restri
             if (idx < 8 * LC) cp_async16(reinterpret_cast<float4*>(buf) + idx, src + idx);
         }
     } else {
-        tile_in<LC>(buf, g, pix0, npix, lane);
+        const float* src = g + pix0 * LC;
+        const int n = npix * LC;
+#pragma unroll
+        for (int j = 0; j < LC; j++) {
+            const int idx = j * 32 + lane;
+            if (idx < n) cp_async4(buf + idx, src + idx);
+        }
     }
 }
 template <int LC>
