@@ -1,5 +1,5 @@
 """Lattice construction around the tile and class limits of its sort: pixel
-counts on both sides of the 4096-entry sort tile and of multiples of 4 (padding
+counts on both sides of the sort's tiles (2048 entries) and of multiples of 4 (padding
 pixels), every compile-time and run-time dimension, vertices only padding
 touches; every table equal to the oracle's, and the splat lists through the
 filter."""
