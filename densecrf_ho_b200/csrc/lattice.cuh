@@ -189,6 +189,8 @@ struct Lattice {
     void compute_noalloc(float* out, const float* in, int L, bool reverse);
     // Ordered (upper minus lower, 10-bin) filter of Q in [0,1]; out = epilogue(v).
     void compute_ord(float* out, const float* Q, int L, const SliceEpilogue& ep);
+    bool ord_dense(int L) const;
+    void compute_ord_dense(float* out, const float* Q, int L, const SliceEpilogue& ep);
     // The same from packed bins in two phases: splat + blur (leaves the vertex
     // values in ord_vals), then the slice.  Other work may run between them.
     void ord_splat_blur(const unsigned short* bins, int L);

@@ -31,12 +31,13 @@ namespace {
 // Programmatic dependent launches (launch_chained) pay while the filter's
 // kernels are short (64x48: 59 -> 47 us a call, 320x240 with 5 labels 105 ->
 // 91), and cost on long ones, whose successors' early blocks crowd them
-// (320x240 with 40 labels 228 -> 247, 640x480 269 -> 304 us; 393 -> 622 where
-// the bins are spread): chained up to 2^20 (pixel, label) values.
+// (320x240 with 12 labels 67 -> 74 us, with 40 labels 228 -> 247, 640x480 269
+// -> 304; 393 -> 622 where the bins are spread): chained up to 2^19 (pixel,
+// label) values.
 template <typename... KArgs, typename... Args>
 void launch_ord(long values, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                 Args&&... args) {
-    if (values <= 1L << 20) launch_chained(kernel, grid, block, smem, st, std::forward<Args>(args)...);
+    if (values <= 1L << 19) launch_chained(kernel, grid, block, smem, st, std::forward<Args>(args)...);
     else launch(kernel, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
@@ -585,7 +586,8 @@ __device__ __forceinline__ void quad_if(float4& r, const float4* p, bool stored)
 // where the quad does not exist), contiguous over labels; up[9] = T beside
 // pair 8; and behind a label's last stored quad one more of (0, T, 0, T), so
 // that up[c] of an entry in bin c is there whichever quad it falls in.
-// NWC: mask words as a compile-time constant (4: L = 20 .. 25), or 0.
+// NWC: mask words as a compile-time constant (1 .. 4: up to 6, 12, 19, 25 labels),
+// or 0 (two at a time).  152x71, 18 labels: 5.6 us as a loop over single words.
 constexpr int kOrdBlurThreads = 256;
 constexpr int kOrdBlurBlocks = 3;  // per SM
 template <int NWC, bool LAST>
@@ -671,20 +673,59 @@ __global__ void __launch_bounds__(kOrdBlurThreads, kOrdBlurBlocks)
             store(q1, v, 3, m.w, m.z, cT);
         }
     } else {
+        constexpr int C = NWC ? NWC : 2;  // words at a time: all of them, or two
+        unsigned a[C], b[C], c[C];
+        Sources s;
+        float Tl = 0.0f;
+        auto masks = [&](int vv, int2 nb, int r0) {
+#pragma unroll
+            for (int i = 0; i < C; i++) {
+                const bool in = NWC || r0 + i < NW;
+                a[i] = in ? act[(long)(vv + 1) * NW + r0 + i] : 0u;
+                b[i] = in ? act[(long)nb.x * NW + r0 + i] : 0u;
+                c[i] = in ? act[(long)nb.y * NW + r0 + i] : 0u;
+            }
+        };
+        auto fetch = [&](int vv, int2 nb) {  // the first masks, T and row pointers of vertex vv
+            masks(vv, nb, 0);
+            s.T0 = T[vv + 1];
+            s.T1 = T[nb.x];
+            s.T2 = T[nb.y];
+            if (LAST) Tl = Tn[vv + 1];
+            s.p0 = src + (long)(vv + 1) * row4 + lane;
+            s.p1 = src + (long)nb.x * row4 + lane;
+            s.p2 = src + (long)nb.y * row4 + lane;
+        };
+        if (v >= M) return;
+        int2 nb = nbr[v];
+        fetch(v, nb);
+        int2 nn = nbr[min(v + nw, M - 1)];
         for (; v < M; v += nw) {
-            const int2 nb = nbr[v];
-            const unsigned *m0 = act + (long)(v + 1) * NW, *m1 = act + (long)nb.x * NW, *m2 = act + (long)nb.y * NW;
-            const Sources s{src + (long)(v + 1) * row4 + lane, src + (long)nb.x * row4 + lane,
-                            src + (long)nb.y * row4 + lane,    T[v + 1], T[nb.x], T[nb.y]};
-            const float Tl = LAST ? Tn[v + 1] : 0.0f;
+            const Sources cur = s;
+            const float cT = Tl;
             unsigned before = 0u;
-            for (int r = 0; r < NW; r++) {
-                const unsigned a = m0[r], b = m1[r], c = m2[r], m = a | b | c;
-                Quads q;
-                load(s, r, a, b, c, q);
-                if (!LAST && lane == 0) act2[(long)(v + 1) * NW + r] = m;
-                store(q, v, r, m, before, Tl);
-                before = m;
+            for (int r0 = 0; r0 < NW; r0 += C) {
+                unsigned m[C];
+                Quads q[C];
+#pragma unroll
+                for (int i = 0; i < C; i++) {
+                    m[i] = a[i] | b[i] | c[i];
+                    load(cur, r0 + i, a[i], b[i], c[i], q[i]);
+                }
+                if (r0 + C < NW) {  // the next masks: this vertex's or the next one's
+                    masks(v, nb, r0 + C);
+                } else {
+                    nb = nn;
+                    fetch(min(v + nw, M - 1), nb);
+                    nn = nbr[min(v + 2 * nw, M - 1)];
+                }
+#pragma unroll
+                for (int i = 0; i < C; i++) {
+                    if (!NWC && r0 + i >= NW) break;
+                    if (!LAST && lane == 0) act2[(long)(v + 1) * NW + r0 + i] = m[i];
+                    store(q[i], v, r0 + i, m[i], before, cT);
+                    before = m[i];
+                }
             }
         }
     }
@@ -941,12 +982,13 @@ void launch_slice(float* out, const unsigned short* bins, int L, const Lattice& 
     auto pick = [&](auto g) {
         constexpr bool GAP = decltype(g)::value;
         if constexpr (NT == 2) {
-            return L == 21 && a.d == 2 && b.d == 5 ? ord_slice_kernel<GAP, NT, 21, 2, 5>
-                                                   : ord_slice_kernel<GAP, NT, 0, 0, 0>;
+            return a.d != 2 || b.d != 5 ? ord_slice_kernel<GAP, NT, 0, 0, 0>
+                   : L == 21            ? ord_slice_kernel<GAP, NT, 21, 2, 5>
+                                        : ord_slice_kernel<GAP, NT, 0, 2, 5>;
         } else {
-            return L == 21 && a.d == 5   ? ord_slice_kernel<GAP, NT, 21, 5, 0>
-                   : L == 21 && a.d == 2 ? ord_slice_kernel<GAP, NT, 21, 2, 0>
-                                         : ord_slice_kernel<GAP, NT, 0, 0, 0>;
+            return a.d == 5   ? (L == 21 ? ord_slice_kernel<GAP, NT, 21, 5, 0> : ord_slice_kernel<GAP, NT, 0, 5, 0>)
+                   : a.d == 2 ? (L == 21 ? ord_slice_kernel<GAP, NT, 21, 2, 0> : ord_slice_kernel<GAP, NT, 0, 2, 0>)
+                              : ord_slice_kernel<GAP, NT, 0, 0, 0>;
         }
     };
     auto kern = gap ? pick(std::true_type{}) : pick(std::false_type{});
@@ -979,6 +1021,10 @@ void ordered_bins(unsigned short* bins, const float* Q, int N, int L, const floa
 
 void Lattice::compute_ord(float* out, const float* Q, int L, const SliceEpilogue& ep) {
     require(L >= 1 && L <= kOrdMaxL, DCRF_E_ARG, "compute_ord: label count out of range");
+    if (ord_dense(L)) {
+        compute_ord_dense(out, Q, L, ep);
+        return;
+    }
     unsigned short* bins = obins.ensure(ordered_bins_size(N, L));
     ordered_bins(bins, Q, N, L, nullptr, stream);
     ord_splat_blur(bins, L);
@@ -1012,8 +1058,15 @@ void Lattice::ord_splat_blur(const unsigned short* bins, int L) {
                    (int)ht, (int)lt, L, NW, vorder.get(), seg_start.get(), seg.get(), b4, pm, as, ad, src, bytes);
     for (int j = 0; j <= d; j++) {
         const float* T = ord_T.get() + (long)j * (M + 1);
-        auto kern = j == d ? (NW == 4 ? ord_blur_kernel<4, true> : ord_blur_kernel<0, true>)
-                           : (NW == 4 ? ord_blur_kernel<4, false> : ord_blur_kernel<0, false>);
+        auto pick = [&](auto last) {
+            constexpr bool LAST = decltype(last)::value;
+            return NW == 1   ? ord_blur_kernel<1, LAST>
+                   : NW == 2 ? ord_blur_kernel<2, LAST>
+                   : NW == 3 ? ord_blur_kernel<3, LAST>
+                   : NW == 4 ? ord_blur_kernel<4, LAST>
+                             : ord_blur_kernel<0, LAST>;
+        };
+        auto kern = j == d ? pick(std::true_type{}) : pick(std::false_type{});
         launch_ord((long)N * L, kern, std::min(ceil_div(M, kOrdBlurThreads / 32), sm_count() * kOrdBlurBlocks), kOrdBlurThreads, 0, st, M, L, NW,
                        nbr.get() + (long)j * M, T, T + M + 1, reinterpret_cast<const float4*>(src),
                        reinterpret_cast<float4*>(dst), as, ad, plane);
@@ -1077,6 +1130,107 @@ void pair_bins(float2* bins, const float* Q, long n, cudaStream_t st) {
     }
 }
 
+// ---------------------------------------------------------------------------
+// The dense form: every bin of every label, nothing skipped (ord_dense).  Its
+// kernels leave most of the chip's registers and all of its shared memory to
+// other streams, and where no list is long they touch little more than the
+// quads that exist.
+//
+// The single masks of ord_step2: [cl >= b] and [b >= cu] as 0.0 / 1.0.
+__device__ __forceinline__ float ord_mask_lower(float cl, int b) {
+    float m;
+    asm("add.rn.sat.f32 %0, %1, %2;" : "=f"(m) : "f"(cl), "f"(1.0f - (float)b));
+    return m;
+}
+__device__ __forceinline__ float ord_mask_upper(float cu, int b) {
+    float m;
+    asm("sub.rn.sat.f32 %0, %1, %2;" : "=f"(m) : "f"((float)b + 1.0f), "f"(cu));
+    return m;
+}
+
+// Splat, one thread per (vertex, label), both passes in registers: lower bin 0
+// and upper bin 9 take every entry, the other 18 bins an FMA with a mask of
+// exactly 0 or 1 (fma(1, w, acc) is acc + w rounded once).  Also clears the
+// absent neighbour's row in both buffers.
+__global__ void ord_dense_splat_kernel(int M, int L, const int* __restrict__ seg_start, const int2* __restrict__ seg,
+                                       const float2* __restrict__ bins, float* __restrict__ vals,
+                                       float* __restrict__ other) {
+    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    for (long z = t; z < (long)kOrdW * L; z += (long)gridDim.x * blockDim.x) vals[z] = other[z] = 0.0f;
+    if (t >= (long)M * L) return;
+    const int v = (int)(t / L), k = (int)(t - (long)v * L);
+    const int s0 = seg_start[v], s1 = seg_start[v + 1];
+    float lo[kRes], up[kRes];
+#pragma unroll
+    for (int b = 0; b < kRes; b++) lo[b] = up[b] = 0.0f;
+#pragma unroll 2
+    for (int s = s0; s < s1; s++) {
+        const int2 en = seg[s];
+        const float2 x = bins[(long)en.x * L + k];
+        const float w = entry_w(en);
+        lo[0] = fadd(lo[0], w);
+#pragma unroll
+        for (int b = 1; b < kRes; b++) lo[b] = __fmaf_rn(ord_mask_lower(x.x, b), w, lo[b]);
+#pragma unroll
+        for (int b = 0; b < kRes - 1; b++) up[b] = __fmaf_rn(ord_mask_upper(x.y, b), w, up[b]);
+        up[kRes - 1] = fadd(up[kRes - 1], w);
+    }
+    float* row = vals + (long)(v + 1) * kOrdW * L + k;
+#pragma unroll
+    for (int b = 0; b < kRes; b++) {
+        row[(long)b * L] = lo[b];
+        row[(long)(kRes + b) * L] = up[b];
+    }
+}
+
+// One axis, one thread per four values.  R4: a row's float4 at compile time (0: row4r).
+template <int R4>
+__global__ void ord_dense_blur_kernel(int M, int row4r, const int2* __restrict__ nbr, const float4* __restrict__ src,
+                                      float4* __restrict__ dst) {
+    const int row4 = R4 ? R4 : row4r;
+    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long)M * row4) return;
+    const int v = (int)(t / row4), c = (int)(t - (long)v * row4);
+    const int2 nb = nbr[v];
+    const float4 a = src[(long)(v + 1) * row4 + c];
+    const float4 p = src[(long)nb.x * row4 + c];
+    const float4 q = src[(long)nb.y * row4 + c];
+    float4 r;
+    r.x = fadd(a.x, fmul(0.5f, fadd(p.x, q.x)));
+    r.y = fadd(a.y, fmul(0.5f, fadd(p.y, q.y)));
+    r.z = fadd(a.z, fmul(0.5f, fadd(p.z, q.z)));
+    r.w = fadd(a.w, fmul(0.5f, fadd(p.w, q.w)));
+    dst[(long)(v + 1) * row4 + c] = r;
+}
+
+// Slice, one thread per (pixel, label): the lower pass, then the upper.
+template <int DC, int LC>
+__global__ void __launch_bounds__(kTB, 8)
+    ord_dense_slice_kernel(int N, int Lrt, int drt, const int* __restrict__ offset, const float* __restrict__ bary,
+                           const float* __restrict__ vals, const float2* __restrict__ bins, float alpha, float* out,
+                           SliceEpilogue ep) {
+    const int L = LC ? LC : Lrt, d = DC ? DC : drt;
+    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long)N * L) return;
+    const int i = (int)(t / L), k = (int)(t - (long)i * L), d1 = d + 1;
+    const float2 bp = bins[t];
+    const int cl = ord_lower_of(bp), cu = ord_upper_of(bp);
+    float acc = 0.0f;
+#pragma unroll
+    for (int j = 0; j <= d; j++) {
+        const int o = offset[(long)i * d1 + j];
+        const float w = bary[(long)i * d1 + j];
+        acc = fadd(acc, fmul(vals[((long)(o + 1) * kOrdW + cl) * L + k], fmul(-w, alpha)));
+    }
+#pragma unroll
+    for (int j = 0; j <= d; j++) {
+        const int o = offset[(long)i * d1 + j];
+        const float w = bary[(long)i * d1 + j];
+        acc = fadd(acc, fmul(vals[((long)(o + 1) * kOrdW + kRes + cu) * L + k], fmul(w, alpha)));
+    }
+    out[t] = apply_epilogue(acc, t, i, k, ep);
+}
+
 // One entry into the bin-b pair (lower, upper) of packed accumulators:
 // acc = fma({[cl >= b], [b >= cu]}, w2, acc) with one f32x2 FMA, which rounds
 // each half exactly as fma.rn.f32 does.  w2 holds (w, w).  The bins are
@@ -1095,6 +1249,41 @@ __device__ __forceinline__ void ord_step2(unsigned long long& acc, float cl, flo
         : "f"(cl), "f"(cu), "f"(lo_c), "f"(up_c), "l"(w2));
 }
 }  // namespace
+
+// Whether a single filter takes the dense form: two features at most, no long
+// list and more than 2^19 (pixel, label) values.  Three calls in flight, the
+// quad form -> the dense one, us: d = 2, 21 labels, 640x480 215 -> 178, 300x200
+// 44.2 -> 31.6, 554x90 33.1 -> 26.6; 640x480 with 3 labels 56.2 -> 30.1; below the line,
+// 200x150 with 21 labels 21.9 -> 21.1, 320x240 with 2 labels 16.2 -> 18.7.
+// More features have long lists of mostly empty bins, where the quad form wins
+// (d = 5, 640x480, one call after the other: 340 -> 274).  The LP's fused slice needs the quad form.
+bool Lattice::ord_dense(int L) const { return d <= 2 && n_long == 0 && (long)N * L > 1L << 19; }
+
+void Lattice::compute_ord_dense(float* out, const float* Q, int L, const SliceEpilogue& ep) {
+    const size_t row = (size_t)L * kOrdW;
+    ensure_values(row);
+    cudaStream_t st = stream;
+    const long NL = (long)N * L;
+    float2* bins = r_ebins.ensure((size_t)NL);
+    pair_bins(bins, Q, NL, st);
+    float *src = va.get(), *dst = vb.get();
+    launch(ord_dense_splat_kernel, ceil_div((long)M * L, kTB), kTB, 0, st, M, L, (const int*)seg_start.get(),
+           (const int2*)seg.get(), (const float2*)bins, src, dst);
+    const int row4 = (int)(row / 4);
+    for (int j = 0; j <= d; j++) {
+        launch(row4 == 105 ? ord_dense_blur_kernel<105> : ord_dense_blur_kernel<0>, ceil_div((long)M * row4, kTB), kTB,
+               0, st, M, row4, (const int2*)(nbr.get() + (long)j * M), reinterpret_cast<const float4*>(src),
+               reinterpret_cast<float4*>(dst));
+        std::swap(src, dst);
+    }
+    const float alpha = 1.0f / (1.0f + std::pow(2.0f, (float)-d));
+    auto slice = d == 2 ? (L == 21 ? ord_dense_slice_kernel<2, 21> : ord_dense_slice_kernel<2, 0>)
+                        : ord_dense_slice_kernel<0, 0>;
+    launch(slice, ceil_div(NL, kTB), kTB, 0, st, N, L, d, (const int*)offset.get(), (const float*)bary.get(),
+           (const float*)src, (const float2*)bins, alpha, out, ep);
+    DCRF_LAUNCH_CHECK();
+    ord_vals = nullptr;  // the buffers hold no quads
+}
 
 // ---------------------------------------------------------------------------
 // The restricted ordered filter (seqCompute_upper_minus_lower_ord_restricted,
