@@ -792,6 +792,30 @@ constexpr int kOsThreads = 128;
 constexpr int kOsPer = 4;  // elements per thread; 1 where L < 8: the pixels' data would not fit
 constexpr int kSliceElems = kOsPer * kOsThreads;
 __host__ __device__ constexpr int slice_elems(int L) { return L < 8 ? kOsThreads : kSliceElems; }
+// A block's dual-gap sums.
+__device__ __forceinline__ void gap_store(double g0, double g1, const GapFusion& gf) {
+    __shared__ double p0[kOsThreads / 32], p1[kOsThreads / 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        g0 += __shfl_down_sync(0xffffffffu, g0, o);
+        g1 += __shfl_down_sync(0xffffffffu, g1, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        p0[threadIdx.x >> 5] = g0;
+        p1[threadIdx.x >> 5] = g1;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double a = 0.0, c = 0.0;
+        for (int w = 0; w < kOsThreads / 32; w++) {
+            a += p0[w];
+            c += p1[w];
+        }
+        gf.partials[blockIdx.x] = a;
+        gf.partials[gridDim.x + blockIdx.x] = c;
+    }
+}
+
 template <bool GAP, int NT, int LC, int D0, int D1>
 __global__ void __launch_bounds__(kOsThreads)
     ord_slice_kernel(int N, int Lrt, int P, OrdSliceTerm t0, OrdSliceTerm t1, const unsigned short* __restrict__ bins,
@@ -941,28 +965,58 @@ __global__ void __launch_bounds__(kOsThreads)
             }
         }
     }
-    if (GAP) {
-        __shared__ double p0[kOsThreads / 32], p1[kOsThreads / 32];
+    if (GAP) gap_store(g0, g1, gf);
+}
+
+// The slice where a pixel's labels are too few to share its sums, or the
+// elements too few to hide the phases above behind one another: one thread per
+// element (kOsPer of them in turn; the same blocks, for the same partial sums),
+// every vertex's float gathered (ord_slice_sum).
+template <int D>
+__device__ __forceinline__ float ord_slice_direct(const OrdSliceTerm& s, int i, int k, unsigned c, int L) {
+    int2 ow[D + 1];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            g0 += __shfl_down_sync(0xffffffffu, g0, o);
-            g1 += __shfl_down_sync(0xffffffffu, g1, o);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            p0[threadIdx.x >> 5] = g0;
-            p1[threadIdx.x >> 5] = g1;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double a = 0.0, c = 0.0;
-            for (int w = 0; w < kOsThreads / 32; w++) {
-                a += p0[w];
-                c += p1[w];
+    for (int j = 0; j <= D; j++)
+        ow[j] = make_int2(s.offset[(long)i * (D + 1) + j] + 1,
+                          __float_as_int(fmul(s.bary[(long)i * (D + 1) + j], s.alpha)));
+    return ord_slice_sum<D>(s, ow, k, c >> 8, c & 255, L);
+}
+template <bool GAP, int NT, int D0, int D1>
+__global__ void __launch_bounds__(kOsThreads)
+    ord_slice_direct_kernel(int N, int L, OrdSliceTerm t0, OrdSliceTerm t1, const unsigned short* __restrict__ bins,
+                            float* out, GapFusion gf) {
+    const int elems = slice_elems(L), Lb = ord_bin_row(L);
+    const long NL = (long)N * L, tb = (long)blockIdx.x * elems;
+    const int ne = (int)min((long)elems, NL - tb);
+    double g0 = 0.0, g1 = 0.0;
+    grid_release();
+    grid_wait();
+#pragma unroll
+    for (int r = 0; r < kOsPer; r++) {
+        const int e = r * kOsThreads + threadIdx.x;
+        if (e < ne) {
+            const long t = tb + e;
+            const int i = (int)(t / L), k = (int)(t - (long)i * L);
+            const unsigned c = bins[(long)i * Lb + k];
+            float v = apply_epilogue(ord_slice_direct<D0>(t0, i, k, c, L), t, i, k, t0.ep);
+            if (NT == 2) {
+                float s1 = ord_slice_direct<D1>(t1, i, k, c, L);
+                if (t1.ep.potts) {
+                    if (t1.ep.norm) s1 = fmul(s1, t1.ep.norm[i]);
+                    s1 = t1.ep.scale_vec ? fmul(t1.ep.scale_vec[k], s1) : fmul(t1.ep.scale, s1);
+                }
+                v = fadd(v, fmul(t1.ep.coef, s1));
             }
-            gf.partials[blockIdx.x] = a;
-            gf.partials[gridDim.x + blockIdx.x] = c;
+            out[t] = v;
+            if (GAP) {
+                const float al = fadd(gf.alpha[t], gf.u ? gf.u[t] : 0.0f);
+                const float tmp = fsub(al, fadd(v, gf.su ? gf.su[t] : 0.0f));
+                g0 += (double)tmp * (double)gf.Q[t];
+                g1 += (double)tmp * (double)tmp;
+            }
         }
     }
+    if (GAP) gap_store(g0, g1, gf);
 }
 
 OrdSliceTerm slice_term(const Lattice& l, const SliceEpilogue& ep) {
@@ -976,6 +1030,27 @@ void launch_slice(float* out, const unsigned short* bins, int L, const Lattice& 
     const long NL = (long)a.N * L;
     const OrdSliceTerm t0 = slice_term(a, ea), t1 = slice_term(b, eb);
     const int elems = slice_elems(L);
+    // One thread per element, us: 640x480, five features, 4 labels, three calls
+    // in flight 119 -> 106; the small LP (64x48, 21 labels, 6 steps) 6465 ->
+    // 6252; from 2^17 values on it loses: the LP at 152x71 with 18 labels
+    // 12430 -> 12640, at 200x120 with 21 labels 8340 -> 8800.
+    const bool known = NT == 2 ? a.d == 2 && b.d == 5 : a.d == 2 || a.d == 5;
+    if (known && (L < 8 || NL <= 1L << 17)) {
+        auto direct = [&](auto kern) {
+            launch_ord(NL, kern, ceil_div(NL, elems), kOsThreads, 0, st, a.N, L, t0, t1, bins, out,
+                       gap ? *gap : GapFusion{});
+        };
+        auto by_d = [&](auto g) {
+            constexpr bool GAP = decltype(g)::value;
+            if constexpr (NT == 2) direct(ord_slice_direct_kernel<GAP, 2, 2, 5>);
+            else if (a.d == 5) direct(ord_slice_direct_kernel<GAP, 1, 5, 5>);
+            else direct(ord_slice_direct_kernel<GAP, 1, 2, 2>);
+        };
+        if (gap) by_d(std::true_type{});
+        else by_d(std::false_type{});
+        DCRF_LAUNCH_CHECK();
+        return;
+    }
     const int P = std::min(elems / L + 2, elems);  // pixels that a block touches at most
     size_t smem = (sizeof(int2) + sizeof(float)) * P * (a.d + 1) + sizeof(float) * 4 * P;
     if (NT == 2) smem += (sizeof(int2) + sizeof(float)) * P * (b.d + 1);
