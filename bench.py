@@ -70,8 +70,8 @@ def parse():
     ap.add_argument("--only-batch-filter", action="store_true",
                     help="time only the batched lattice filter over the 64-image concatenated lattices")
     ap.add_argument("--splat-form", type=int, default=None,
-                    help="pin the 21-label plain filter's splat form (0-5, dcrf_batch_set_filter_shape) in the "
-                         "batched filter and batched QP legs instead of autotuning it")
+                    help="pass a splat form (0-5, dcrf_batch_set_filter_shape) in the batched filter and batched QP "
+                         "legs: accepted, without effect (one form is left); it also keeps the blur untuned")
     ap.add_argument("--all-splat-forms", action="store_true",
                     help="with --only-batch-filter: time the batched filter with every splat form pinned")
     ap.add_argument("--only-ho", action="store_true",
