@@ -1067,7 +1067,7 @@ __global__ void __launch_bounds__(32 * kSliceWarps)
         }
         cp_async_commit();
         for (int e = lane; e < np * d1; e += 32)
-            s_ow[e] = make_int2((offset[p0 * d1 + e] + 1) * Qn, __float_as_int(fmul(bary[p0 * d1 + e], alpha)));
+            s_ow[e] = make_int2(offset[p0 * d1 + e] + 1, __float_as_int(fmul(bary[p0 * d1 + e], alpha)));
         if (use_norm)
             for (int e = lane; e < np; e += 32) s_nrm[e] = ep.norm[p0 + e];
         cp_async_wait<0>();
@@ -1077,7 +1077,8 @@ __global__ void __launch_bounds__(32 * kSliceWarps)
             const float4* vq = vals + q;
             unsigned long long a0 = 0ull, a1 = 0ull;
             auto add = [&](int2 e) {
-                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(vq + e.x);
+                // 64-bit product: (M + 1) Q reaches 2^31 in value buffers of 34 GB
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(vq + (long)e.x * Qn);
                 const float wa = __int_as_float(e.y);
                 a0 = add_mul2(a0, wa, v.x);
                 a1 = add_mul2(a1, wa, v.y);
