@@ -45,7 +45,9 @@ struct GapFusion {
 // qminmax[0..1] (null: Q itself), packed (see ordered.cu); their element count.
 void ordered_bins(unsigned short* bins, const float* Q, int N, int L, const float* qminmax, cudaStream_t st);
 size_t ordered_bins_size(long N, int L);
-constexpr int kOrdMaxL = 1 << 20;  // label counts of the ordered filter (int products stay in range)
+// Label counts of the ordered filter: the five quads a label has are counted in
+// an int.  One pixel of one feature takes 190 GB of value buffers there.
+constexpr int kOrdMaxL = 400000000;
 // Blocks (GapFusion partials) of an ordered slice.
 int ord_slice_grid(int N, int L);
 // Capacity, in floats, of the fixed scratch array of compute_noalloc.

@@ -65,6 +65,8 @@ __device__ __forceinline__ int quads_of(int cmax) { return (cmax + 1) >> 1; }
 // pixel's bins reach, as mask words [N][NW]; a vertex's mask is the or of its
 // entries'.
 constexpr int kBinTile = 32;
+constexpr int kBinTileMaxL = 96;  // four warps' tiles in 48 KB (97 labels, 320x240: 479 us by tiles, 484 wide)
+
 template <bool RESCALE>
 __global__ void __launch_bounds__(kOrdThreads)
     ord_bins_kernel(int N, int L, const float* __restrict__ Q, const float* __restrict__ qmm,
@@ -127,6 +129,38 @@ __global__ void __launch_bounds__(kOrdThreads)
             w[i] = lo | hi << 16;
         }
         bins[p0 * G + it] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+// Bins of Q for any number of labels, without shared memory: a warp per pixel,
+// 32 labels at a time (lane = label, their 160 mask bits five words of their
+// own), the label blocks shared by gridDim.y warps where the pixels are few.
+// The whole filter with the tiles above in up to 227 KB, which ended at 454
+// labels, -> this: 320x240, five features, 150 labels 660 -> 651 us, 300 1218 ->
+// 1147; 160x120, 454 labels 803 -> 765; 64x48, 128 labels 131 -> 123.
+__global__ void __launch_bounds__(kOrdThreads)
+    ord_bins_wide_kernel(int N, int L, const float* __restrict__ Q, unsigned short* __restrict__ bins,
+                         unsigned* __restrict__ pmask) {
+    const int lane = threadIdx.x & 31, nblk = (L + 31) / 32, Lb = ord_bin_row(L), NW = ord_words(L);
+    grid_release();
+    grid_wait();
+    const long i = (long)blockIdx.x * kOrdWarps + (threadIdx.x >> 5);
+    if (i >= N) return;  // warp-uniform
+    const int at = kQuads * lane & 31, word = kQuads * lane >> 5;  // this lane's mask bits
+    for (int blk = blockIdx.y; blk < nblk; blk += gridDim.y) {
+        const int k = 32 * blk + lane;
+        const float q = k < L ? Q[i * L + k] : 0.0f;
+        const int cl = bin_lower(q);
+        if (k < Lb) bins[i * Lb + k] = (unsigned short)(cl << 8 | bin_upper(q));
+        const unsigned long long bits = (unsigned long long)((1u << quads_of(cl)) - 1u) << at;
+        const unsigned lo = (unsigned)bits, hi = (unsigned)(bits >> 32);
+        unsigned mine = 0;
+#pragma unroll
+        for (int r = 0; r < kQuads; r++) {
+            const unsigned w = __reduce_or_sync(0xffffffffu, word == r ? lo : word + 1 == r ? hi : 0u);
+            if (lane == r) mine = w;
+        }
+        if (lane < kQuads && kQuads * blk + lane < NW) pmask[i * NW + kQuads * blk + lane] = mine;
     }
 }
 
@@ -747,14 +781,18 @@ struct OrdSliceTerm {
 // One term's value of element (pixel, k) in any bin: the lower pass with weight
 // -w alpha, then the upper with w alpha (:639-650, :687-696), one float per
 // vertex and pass from the row its bin selects: T (lower bin 0), the plane up[0]
-// (upper bin 0) or its pair -- the pixel's own vertices hold it.
+// (upper bin 0) or its pair -- the pixel's own vertices hold it.  A row's bytes
+// fit an int up to kOrdIntL labels, beyond which launch_slice takes DC = 0.
+constexpr int kOrdIntL = 1 << 24;
 template <int DC>
 __device__ __forceinline__ float ord_slice_sum(const OrdSliceTerm& s, const int2* ow, int k, int cl, int cu, int L) {
-    const int d1 = (DC ? DC : s.d) + 1, row = (int)sizeof(float) * kOrdW * L;
-    const char* lo = reinterpret_cast<const char*>(cl ? s.vals + k * kOrdW + 2 * (cl - 1) : s.T);
-    const char* up = reinterpret_cast<const char*>(cu ? s.vals + k * kOrdW + 2 * cu + 1 : s.plane + k);
-    const int ls = cl ? row : (int)sizeof(float), us = cu ? row : (int)sizeof(float) * ord_plane_row(L);  // bytes
-    auto at = [](const char* b, int r, int stride) {
+    using S = std::conditional_t<DC != 0, int, long>;
+    const int d1 = (DC ? DC : s.d) + 1;
+    const S one = sizeof(float), row = one * kOrdW * L;
+    const char* lo = reinterpret_cast<const char*>(cl ? s.vals + S(k) * kOrdW + 2 * (cl - 1) : s.T);
+    const char* up = reinterpret_cast<const char*>(cu ? s.vals + S(k) * kOrdW + 2 * cu + 1 : s.plane + k);
+    const S ls = cl ? row : one, us = cu ? row : one * ord_plane_row(L);  // bytes
+    auto at = [](const char* b, int r, S stride) {
         return *reinterpret_cast<const float*>(b + (long)r * (long)stride);
     };
     float a = 0.0f;
@@ -904,9 +942,11 @@ __global__ void __launch_bounds__(kOsThreads)
         return v;
     };
     const bool dense = s_dense;
-    for (int it = threadIdx.x; !dense && it < np * Q; it += blockDim.x) {
+    // from the first element's group of four to the last one's: the block
+    // shares its outer pixels with its neighbours
+    const int ll = (ne - 1 + first) / L, last = ll * Q + (ne - 1 + first - ll * L) / 4;
+    for (int it = first / 4 + threadIdx.x; !dense && it <= last; it += blockDim.x) {
         const int li = it / Q, q = it - li * Q, e0 = li * L + 4 * q - first;
-        if (e0 + 3 < 0 || e0 >= ne) continue;  // a pixel the block shares with its neighbours
         const uint2 c = *reinterpret_cast<const uint2*>(bins + (long)(pf + li) * Lb + 4 * q);
         float a[NT][4];
 #pragma unroll
@@ -1034,7 +1074,7 @@ void launch_slice(float* out, const unsigned short* bins, int L, const Lattice& 
     // in flight 119 -> 106; the small LP (64x48, 21 labels, 6 steps) 6465 ->
     // 6252; from 2^17 values on it loses: the LP at 152x71 with 18 labels
     // 12430 -> 12640, at 200x120 with 21 labels 8340 -> 8800.
-    const bool known = NT == 2 ? a.d == 2 && b.d == 5 : a.d == 2 || a.d == 5;
+    const bool known = L <= kOrdIntL && (NT == 2 ? a.d == 2 && b.d == 5 : a.d == 2 || a.d == 5);
     if (known && (L < 8 || NL <= 1L << 17)) {
         auto direct = [&](auto kern) {
             launch_ord(NL, kern, ceil_div(NL, elems), kOsThreads, 0, st, a.N, L, t0, t1, bins, out,
@@ -1057,13 +1097,13 @@ void launch_slice(float* out, const unsigned short* bins, int L, const Lattice& 
     auto pick = [&](auto g) {
         constexpr bool GAP = decltype(g)::value;
         if constexpr (NT == 2) {
-            return a.d != 2 || b.d != 5 ? ord_slice_kernel<GAP, NT, 0, 0, 0>
-                   : L == 21            ? ord_slice_kernel<GAP, NT, 21, 2, 5>
-                                        : ord_slice_kernel<GAP, NT, 0, 2, 5>;
+            return !known    ? ord_slice_kernel<GAP, NT, 0, 0, 0>
+                   : L == 21 ? ord_slice_kernel<GAP, NT, 21, 2, 5>
+                             : ord_slice_kernel<GAP, NT, 0, 2, 5>;
         } else {
-            return a.d == 5   ? (L == 21 ? ord_slice_kernel<GAP, NT, 21, 5, 0> : ord_slice_kernel<GAP, NT, 0, 5, 0>)
-                   : a.d == 2 ? (L == 21 ? ord_slice_kernel<GAP, NT, 21, 2, 0> : ord_slice_kernel<GAP, NT, 0, 2, 0>)
-                              : ord_slice_kernel<GAP, NT, 0, 0, 0>;
+            return !known     ? ord_slice_kernel<GAP, NT, 0, 0, 0>
+                   : a.d == 5 ? (L == 21 ? ord_slice_kernel<GAP, NT, 21, 5, 0> : ord_slice_kernel<GAP, NT, 0, 5, 0>)
+                              : (L == 21 ? ord_slice_kernel<GAP, NT, 21, 2, 0> : ord_slice_kernel<GAP, NT, 0, 2, 0>);
         }
     };
     auto kern = gap ? pick(std::true_type{}) : pick(std::false_type{});
@@ -1085,12 +1125,17 @@ static unsigned* bin_masks(const unsigned short* bins, long N, int L) {
 }
 
 void ordered_bins(unsigned short* bins, const float* Q, int N, int L, const float* qminmax, cudaStream_t st) {
-    const size_t smem = sizeof(float) * kOrdWarps * (size_t)((kBinTile * L + 3) & ~3);
-    auto kern = qminmax ? ord_bins_kernel<true> : ord_bins_kernel<false>;
-    if (smem > 48 * 1024)  // opt-in size: a per-device function attribute, set on every such call
-        DCRF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    launch_ord((long)N * L, kern, ceil_div(N, kBinTile * kOrdWarps), kOrdThreads, smem, st, N, L, Q, qminmax,
-                   reinterpret_cast<uint4*>(bins), bin_masks(bins, N, L), (int)aligned16(Q));
+    const long NL = (long)N * L;
+    unsigned* pm = bin_masks(bins, N, L);
+    if (L <= kBinTileMaxL) {
+        launch_ord(NL, qminmax ? ord_bins_kernel<true> : ord_bins_kernel<false>, ceil_div(N, kBinTile * kOrdWarps),
+                   kOrdThreads, sizeof(float) * kOrdWarps * ((kBinTile * L + 3) & ~3), st, N, L, Q, qminmax,
+                   reinterpret_cast<uint4*>(bins), pm, (int)aligned16(Q));
+    } else {  // a lattice's own call: a model, the only one to rescale, has 64 labels at most
+        require(!qminmax, DCRF_E_ARG, "ordered_bins: too many labels to rescale");
+        const int split = std::max(1, std::min((L + 31) / 32, (1 << 14) / N));
+        launch_ord(NL, ord_bins_wide_kernel, dim3(ceil_div(N, kOrdWarps), split), kOrdThreads, 0, st, N, L, Q, bins, pm);
+    }
     DCRF_LAUNCH_CHECK();
 }
 
