@@ -37,6 +37,8 @@ namespace {
 
 thread_local std::string g_err;
 
+// A failed call leaves no error pending in the CUDA runtime: the next call's
+// launch checks would take it for their own.
 template <typename F>
 dcrf_status guard(F&& f) {
     try {
@@ -44,12 +46,15 @@ dcrf_status guard(F&& f) {
         return DCRF_OK;
     } catch (const Error& e) {
         g_err = e.what();
+        cudaGetLastError();
         return e.code;
     } catch (const std::bad_alloc&) {
         g_err = "host allocation failed";
+        cudaGetLastError();
         return DCRF_E_NOMEM;
     } catch (const std::exception& e) {
         g_err = e.what();
+        cudaGetLastError();
         return DCRF_E_CUDA;
     }
 }
