@@ -1211,7 +1211,6 @@ void build_impl(Lattice& L, const float* d_features) {
     L.visiting_order(nl);
     L.n_long = nl[0];
     L.n_huge = nl[1];
-    L.va_floats = 0;
     L.ord_T_ready = false;
 }
 
@@ -1490,7 +1489,6 @@ void Lattice::concat(const std::vector<const Lattice*>& parts) {
     DCRF_CUDA(cudaMemcpyAsync(db, hb.data(), sizeof(long) * hb.size(), cudaMemcpyHostToDevice, st));
     DCRF_CUDA(cudaStreamSynchronize(st));  // hb is the copy's source
     dom_tile = 0;
-    va_floats = 0;
     ord_T_ready = false;
     concatenated = true;
 }
@@ -1521,11 +1519,8 @@ void Lattice::build(const float* d_features, int d_, int N_) {
 
 void Lattice::ensure_values(size_t row_width) {
     const size_t need = (size_t)(M + 1) * row_width;
-    if (need > va_floats) {
-        va.ensure(need);
-        vb.ensure(need);
-        va_floats = need;
-    }
+    va.ensure(need);
+    vb.ensure(need);
 }
 
 // ---------------------------------------------------------------------------

@@ -134,7 +134,6 @@ struct Lattice {
     DevBuf<float> ord_plane, ord_T;
     bool ord_T_ready = false;
     void ensure_ord_totals();
-    size_t va_floats = 0;    // rows (M+1) * width currently zero-headed
 
     // build scratch
     DevBuf<int4> ekeys;
