@@ -644,8 +644,8 @@ Batch::~Batch() {
 // Term t's lattice over all images: every image's own lattice, built from
 // the term's features, concatenated (Lattice::concat).
 void Batch::build_lattice(Term& t) {
-    t.lat = std::make_unique<Lattice>();
-    t.lat->stream = stream;
+    auto lat = std::make_unique<Lattice>();  // the term's once it is complete
+    lat->stream = stream;
     std::vector<std::unique_ptr<Lattice>> parts;
     std::vector<const Lattice*> views;
     for (int i = 0; i < B; i++) {
@@ -655,7 +655,8 @@ void Batch::build_lattice(Term& t) {
         views.push_back(p.get());
         parts.push_back(std::move(p));
     }
-    t.lat->concat(views);
+    lat->concat(views);
+    t.lat = std::move(lat);
 }  // the per-image lattices are released here
 
 void Batch::ensure_lattices() {

@@ -1211,7 +1211,6 @@ void build_impl(Lattice& L, const float* d_features) {
     L.visiting_order(nl);
     L.n_long = nl[0];
     L.n_huge = nl[1];
-    L.ord_T_ready = false;
 }
 
 }  // namespace
@@ -1400,6 +1399,7 @@ void Lattice::visiting_order(int (&nl)[2]) {
 void Lattice::concat(const std::vector<const Lattice*>& parts) {
     require(!parts.empty(), DCRF_E_ARG, "lattice concat: no parts");
     cudaStream_t st = stream;
+    forget();
     d = parts[0]->d;
     const int d1 = d + 1;
     long Nt = 0, Mt = 0;
@@ -1489,7 +1489,6 @@ void Lattice::concat(const std::vector<const Lattice*>& parts) {
     DCRF_CUDA(cudaMemcpyAsync(db, hb.data(), sizeof(long) * hb.size(), cudaMemcpyHostToDevice, st));
     DCRF_CUDA(cudaStreamSynchronize(st));  // hb is the copy's source
     dom_tile = 0;
-    ord_T_ready = false;
     concatenated = true;
 }
 
@@ -1509,12 +1508,27 @@ void Lattice::prepare_live(int L) {
 void Lattice::build(const float* d_features, int d_, int N_) {
     require(N_ > 0, DCRF_E_ARG, "lattice: N must be positive");
     require(d_ >= 1 && d_ <= 16, DCRF_E_ARG, "lattice: feature dimension must be in [1, 16]");
+    forget();
     N = N_;
     d = d_;
-    if (d <= 2) build_impl<2>(*this, d_features);
-    else if (d <= 5) build_impl<5>(*this, d_features);
-    else if (d <= 8) build_impl<8>(*this, d_features);
-    else build_impl<16>(*this, d_features);
+    try {
+        if (d <= 2) build_impl<2>(*this, d_features);
+        else if (d <= 5) build_impl<5>(*this, d_features);
+        else if (d <= 8) build_impl<8>(*this, d_features);
+        else build_impl<16>(*this, d_features);
+    } catch (...) {
+        forget();
+        throw;
+    }
+}
+
+// No lattice: N = 0 until one is built, and nothing that was computed on the
+// former one is taken for this one's.
+void Lattice::forget() {
+    N = M = 0;
+    plain_vals = ord_vals = nullptr;
+    plain_L = r_L = 0;
+    ord_T_ready = false;
 }
 
 void Lattice::ensure_values(size_t row_width) {

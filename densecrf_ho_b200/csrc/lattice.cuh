@@ -170,6 +170,7 @@ struct Lattice {
 
     // features: device [N][d]
     void build(const float* d_features, int d_, int N_);
+    void forget();
     // Several images' lattices as one (see Lattice::concat in lattice.cu).
     void concat(const std::vector<const Lattice*>& parts);
     // out/in: device [N][L]; out may alias in.

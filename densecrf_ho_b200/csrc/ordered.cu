@@ -1531,6 +1531,7 @@ void Lattice::compute_ord_restricted(float* rout, const float* rQ, const int* pI
             "compute_ord_restricted: no stored splat for this label count (call with store first)");
     require(!store || Q, DCRF_E_ARG, "compute_ord_restricted: store needs Q");
     cudaStream_t st = stream;
+    if (store) r_L = 0;  // until this call has stored its splat
     const long row = (long)L * kOrdW, cells = (long)(M + 1) * row;
     float* stored = r_stored.ensure((size_t)cells);
     float* a = r_a.ensure((size_t)cells);
@@ -1548,7 +1549,6 @@ void Lattice::compute_ord_restricted(float* rout, const float* rQ, const int* pI
         float2* e = r_ebins.ensure((size_t)N * L);
         pair_bins(e, Q, (long)N * L, st);
         eb = e;
-        r_L = 0;  // until this call has stored its splat
     }
     DCRF_CUDA(cudaMemsetAsync(a, 0, sizeof(float) * row, st));      // row 0: the absent neighbour
     DCRF_CUDA(cudaMemsetAsync(b, 0, sizeof(float) * cells, st));    // new_values_ starts zeroed
