@@ -513,6 +513,22 @@ __global__ void __launch_bounds__(32 * kPadWarps)
     }
 }
 
+// The same where a pixel's row does not fit a warp's tile (row_tiles): a thread
+// per 16-byte group, blockIdx.y walking the pixels.  The whole filter at the
+// line, 64x48 and five features: 437 us with 3056 labels by tiles, 423 with
+// 3057 by these.
+__global__ void __launch_bounds__(kTB)
+    pad_wide_kernel(int N, int L, int Q, const float* __restrict__ in, float4* __restrict__ rows) {
+    const int q = blockIdx.x * kTB + threadIdx.x, n = L - 4 * q;
+    grid_release();
+    grid_wait();
+    if (q >= Q) return;
+    for (long i = blockIdx.y; i < N; i += gridDim.y) {
+        const float* x = in + i * L + 4 * q;
+        rows[i * Q + q] = make_float4(x[0], n > 1 ? x[1] : 0.0f, n > 2 ? x[2] : 0.0f, n > 3 ? x[3] : 0.0f);
+    }
+}
+
 // The lists a splat launch covers: positions [first, first + count) of
 // `order`, or the live images' positions of the domain behind lv.
 struct SplatRange {
@@ -1150,6 +1166,32 @@ __global__ void __launch_bounds__(32 * kSliceWarps)
     }
 }
 
+// The slice of rows that do not fit a warp's tile (row_tiles), split as
+// pad_wide_kernel: the same sums, no epilogue.
+__global__ void __launch_bounds__(kTB)
+    slice_wide_kernel(int N, int L, int Q, int d1, const int* __restrict__ offset, const float* __restrict__ bary,
+                      const float4* __restrict__ vals, float alpha, float* __restrict__ out) {
+    const int q = blockIdx.x * kTB + threadIdx.x, n = L - 4 * q;
+    grid_release();
+    grid_wait();
+    if (q >= Q) return;
+    for (long i = blockIdx.y; i < N; i += gridDim.y) {
+        unsigned long long a0 = 0ull, a1 = 0ull;
+        for (int j = 0; j < d1; j++) {
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(vals + (long)(offset[i * d1 + j] + 1) * Q + q);
+            const float wa = fmul(bary[i * d1 + j], alpha);
+            a0 = add_mul2(a0, wa, v.x);
+            a1 = add_mul2(a1, wa, v.y);
+        }
+        const float2 lo = unpack2(a0), hi = unpack2(a1);
+        float* o = out + i * L + 4 * q;
+        o[0] = lo.x;
+        if (n > 1) o[1] = lo.y;
+        if (n > 2) o[2] = hi.x;
+        if (n > 3) o[3] = hi.y;
+    }
+}
+
 int bits_for(int n) {  // bits needed to hold values 0..n-1
     int b = 0;
     while ((1LL << b) < (long long)n) b++;
@@ -1633,6 +1675,10 @@ static int slice_tile_max(int tile, int d, int L) {
     while (tile > 1 && slice_warp_bytes(tile, d, L) > (size_t)kSliceSmem) tile = tile > 4 ? (tile / 2) & ~3 : tile - 1;
     return tile;
 }
+// Whether four warps' tiles of one pixel fit a block's 48 KB: up to some 3050
+// labels.  Only a lattice's own calls can have more (a model's limit is 64).
+static bool row_tiles(int d, int L) { return kSliceWarps * slice_warp_bytes(1, d, L) <= (48 << 10); }
+static dim3 wide_grid(int N, int Q) { return dim3(ceil_div(Q, kTB), std::min(N, 65535)); }
 
 // Splats `in` [N][L] (times pre_norm) into vals: rows of Q float4 (L > 2) or
 // of L floats.  With live images only their lists (and pixels).
@@ -1656,11 +1702,17 @@ void Lattice::splat(const float* in, int L, const float* pre_norm, float* vals) 
     float4* rw = reinterpret_cast<float4*>(rows.ensure((size_t)N * Q * 4));
     const int tile = live ? dom_tile : slice_tile_for(L);
     require(tile > 0, DCRF_E_STATE, "splat: live images without prepare_live");
-    const size_t psmem = sizeof(float) * kPadWarps * (size_t)((tile * L + 3) & ~3);
-    launch_chained(Q == 6 ? pad_rows_kernel<6> : pad_rows_kernel<0>,
-                   unit_grid(N, tile * kPadWarps, live, 32 * kPadWarps), 32 * kPadWarps, psmem, st, N, L, Q, tile, in,
-                   pre_norm, rw, live_of(kDomTile),
-                   live ? (const long*)(dom_base.get() + (long)kDomPix * (images + 1)) : nullptr, (int)aligned16(in));
+    if (!row_tiles(d, L)) {
+        require(!live && !pre_norm, DCRF_E_ARG, "splat: too many labels");
+        launch_chained(pad_wide_kernel, wide_grid(N, Q), kTB, 0, st, N, L, Q, in, rw);
+    } else {
+        const size_t psmem = sizeof(float) * kPadWarps * (size_t)((tile * L + 3) & ~3);
+        launch_chained(Q == 6 ? pad_rows_kernel<6> : pad_rows_kernel<0>,
+                       unit_grid(N, tile * kPadWarps, live, 32 * kPadWarps), 32 * kPadWarps, psmem, st, N, L, Q, tile,
+                       in, pre_norm, rw, live_of(kDomTile),
+                       live ? (const long*)(dom_base.get() + (long)kDomPix * (images + 1)) : nullptr,
+                       (int)aligned16(in));
+    }
     const int hb = !concatenated && n_huge <= kHugePerSM * sm_count() ? n_huge : 0;
     const SplatRange rl{hb, n_long - hb, live_of(kDomLong)};
     const int lb = rl.count ? unit_grid(rl.count, kSplatWarps, live, kSplatThreads) : 0;
@@ -1815,6 +1867,11 @@ void Lattice::slice(float* out, int L, const SliceEpilogue& ep) {
     if (L <= 2) {
         launch_chained(slice_kernel<true, 0, 0>, unit_grid(NL, kTB, live, kTB), kTB, 0, st, N, L, d, offset.get(),
                        bary.get(), src, alpha, out, ep, live_of(kDomPix));
+    } else if (!row_tiles(d, L)) {
+        require(!live && !ep.potts && !ep.base && !ep.zero_base, DCRF_E_ARG, "slice: too many labels");
+        const int Q = value_row(L) / 4;
+        launch_chained(slice_wide_kernel, wide_grid(N, Q), kTB, 0, st, N, L, Q, d + 1, offset.get(), bary.get(),
+                       reinterpret_cast<const float4*>(src), alpha, out);
     } else {
         const int Q = value_row(L) / 4;
         // live images: tiles of each image's pixels, the size prepare_live fixed
