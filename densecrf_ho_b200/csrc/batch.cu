@@ -628,9 +628,9 @@ Batch::Batch(int n, const int* widths, const int* heights, int L_) : B(n), L(L_)
     require(Ntot * (long)L < (1L << 31), DCRF_E_ARG, "batch: too many pixel-labels");
     DCRF_CUDA(cudaGetDevice(&device));
     DCRF_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-    long* po = d_pix_off.ensure(n + 1);
+    long* po = own(d_pix_off, n + 1);
     DCRF_CUDA(cudaMemcpyAsync(po, pix_off.data(), sizeof(long) * (n + 1), cudaMemcpyHostToDevice, stream));
-    partials.ensure((size_t)kRedBlocks * 2);
+    own(partials, (size_t)kRedBlocks * 2);
     DCRF_CUDA(cudaStreamSynchronize(stream));
 }
 
@@ -656,6 +656,7 @@ void Batch::build_lattice(Term& t) {
         parts.push_back(std::move(p));
     }
     lat->concat(views);
+    lat->give_back_others = [this] { return give_back_rows(); };
     t.lat = std::move(lat);
 }  // the per-image lattices are released here
 
@@ -722,10 +723,10 @@ int Batch::qp(const float* init, float* out, int max_iter, int* steps, double* e
     float* psi = buf(2);
     float* tmp = buf(3);
     const int nt = (int)terms.size();
-    SolverScalars* sc = bsc.ensure(B);
-    int* done = bdone.ensure(B);
-    int* flags = bflags.ensure(2);  // [0] iterations of the current launch, [1] some image runs
-    double* part = bpart.ensure((size_t)B * kBPart);
+    SolverScalars* sc = own(bsc, B);
+    int* done = own(bdone, B);
+    int* flags = own(bflags, 2);  // [0] iterations of the current launch, [1] some image runs
+    double* part = own(bpart, (size_t)B * kBPart);
     const bool tiled = L == 21;
     if (tiled && btiles == 0) {  // row-tile blocks of the direction kernel, image after image
         std::vector<int> toff(B + 1, 0);
@@ -736,22 +737,22 @@ int Batch::qp(const float* init, float* out, int max_iter, int* steps, double* e
             tbase[i + 1] = toff[i + 1];
         }
         btiles = toff[B];
-        DCRF_CUDA(cudaMemcpyAsync(btile_off.ensure(B + 1), toff.data(), sizeof(int) * (B + 1), cudaMemcpyHostToDevice,
+        DCRF_CUDA(cudaMemcpyAsync(own(btile_off, B + 1), toff.data(), sizeof(int) * (B + 1), cudaMemcpyHostToDevice,
                                   stream));
-        DCRF_CUDA(cudaMemcpyAsync(btile_base.ensure(B + 1), tbase.data(), sizeof(long) * (B + 1),
+        DCRF_CUDA(cudaMemcpyAsync(own(btile_base, B + 1), tbase.data(), sizeof(long) * (B + 1),
                                   cudaMemcpyHostToDevice, stream));
         DCRF_CUDA(cudaStreamSynchronize(stream));  // the host vectors are the copies' sources
     }
-    double* part_dir = tiled ? bpart_dir.ensure(btiles) : nullptr;
+    double* part_dir = tiled ? own(bpart_dir, btiles) : nullptr;
     // The live images and each domain's live prefix, rebuilt at the start of
     // every iteration: kDomains domains per term (its lattice's lists,
     // vertices, slice tiles and pixels), then the direction kernel's tiles.
     const int nt_l = (int)terms.size();
     require(nt_l * Lattice::kDomains + 1 <= kMaxLiveDoms, DCRF_E_ARG, "batch qp: too many pairwise terms");
-    int* live_buf = blive.ensure(B + 1);
+    int* live_buf = own(blive, B + 1);
     const int* live_n = live_buf;
     const int* live_img = live_buf + 1;
-    long* lpre = blive_pre.ensure((size_t)(nt_l * Lattice::kDomains + 1) * (B + 1));
+    long* lpre = own(blive_pre, (size_t)(nt_l * Lattice::kDomains + 1) * (B + 1));
     LiveDoms doms{};
     for (int k = 0; k < nt_l; k++) {
         Lattice& lat = *terms[k]->lat;
@@ -1000,10 +1001,10 @@ void Batch::meanfield(int iterations, float* Q) {
     const long NL = Ntot * L;
     mf_T = iterations;
     const int slots = iterations / ck_every + 1 + (iterations % ck_every ? 1 : 0);
-    float* ck = mf_ck.ensure((size_t)slots * NL);
+    float* ck = own(mf_ck, (size_t)slots * NL);
     float* negU = buf(4);
     float* logits = buf(5);
-    float* x[2] = {mf_x0.ensure(ck_every > 1 ? NL : 1), mf_x1.ensure(ck_every > 1 ? NL : 1)};
+    float* x[2] = {own(mf_x0, ck_every > 1 ? NL : 1), own(mf_x1, ck_every > 1 ? NL : 1)};
     launch(negate_kernel, ceil_div(NL, 256), 256, 0, stream, NL, unary.get(), negU);
     unary_init(ck);  // Q_0 = softmax(-U)
     const float* q = ck;
@@ -1027,14 +1028,14 @@ void Batch::meanfield_backward(const float* grad_Q, float* grad_U, double* grad_
     const long NL = Ntot * L;
     const int nt = (int)terms.size();
     const float* ck = mf_ck.get();
-    float* g = mf_g0.ensure(NL);
-    float* gn = mf_g1.ensure(NL);
-    float* ga = mf_ga.ensure(NL);
-    float* seg = ck_every > 1 ? mf_seg.ensure((size_t)(ck_every - 1) * NL) : nullptr;
+    float* g = own(mf_g0, NL);
+    float* gn = own(mf_g1, NL);
+    float* ga = own(mf_ga, NL);
+    float* seg = ck_every > 1 ? own(mf_seg, (size_t)(ck_every - 1) * NL) : nullptr;
     float* negU = buf(4);
     float* logits = buf(5);
-    double* dw = mf_dw.ensure(std::max(nt, 1));
-    double* part = partials.ensure(std::max((size_t)kRedBlocks * 2, (size_t)Lattice::dot_partials()));
+    double* dw = own(mf_dw, std::max(nt, 1));
+    double* part = own(partials, std::max((size_t)kRedBlocks * 2, (size_t)Lattice::dot_partials()));
     if (ck_every > 1) launch(negate_kernel, ceil_div(NL, 256), 256, 0, stream, NL, unary.get(), negU);
     const float* gq = grad_Q;  // dL/dQ_{t+1}
     if (nt) DCRF_CUDA(cudaMemsetAsync(dw, 0, sizeof(double) * nt, stream));
@@ -1079,7 +1080,7 @@ void Batch::meanfield_backward(const float* grad_Q, float* grad_U, double* grad_
             if (L > 2) {
                 np = t.lat->slice_dot(ga, part, L, ep);
             } else {
-                float* m = mf_m.ensure(NL);
+                float* m = own(mf_m, NL);
                 t.lat->slice(m, L, ep);
                 launch(dot_kernel, kRedBlocks, kRedThreads, 0, stream, NL, ga, m, part);
                 np = kRedBlocks;

@@ -41,7 +41,18 @@ struct Batch {
     Batch(int n, const int* widths, const int* heights, int L_);
     ~Batch();
 
-    float* buf(int i) { return b[i].ensure((size_t)Ntot * L); }
+    // A buffer of the batch; its lattices' padded rows go first where memory is short.
+    template <typename T>
+    T* own(DevBuf<T>& buffer, size_t count) {
+        return ensure_after(buffer, count, [&] { return give_back_rows(); });
+    }
+    bool give_back_rows() {
+        bool any = false;
+        for (auto& t : terms)
+            if (t->lat) any |= t->lat->give_back_rows();
+        return any;
+    }
+    float* buf(int i) { return own(b[i], (size_t)Ntot * L); }
     // d_features: device [Ntot][d], image after image
     void add_term(const float* d_features, int d, float w);
     void apply(int k, float* out, const float* in, const float* base = nullptr, float coef = 1.0f,

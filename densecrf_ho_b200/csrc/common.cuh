@@ -91,6 +91,19 @@ struct DevBuf {
     T* get() const { return p; }
 };
 
+// b.ensure(count), tried again after give_back() -- true if it released
+// anything -- where memory is short.
+template <typename T, typename F>
+T* ensure_after(DevBuf<T>& b, size_t count, F&& give_back) {
+    try {
+        return b.ensure(count);
+    } catch (const Error& e) {
+        if (e.code != DCRF_E_NOMEM || !give_back()) throw;
+    }
+    cudaGetLastError();
+    return b.ensure(count);
+}
+
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 // The solver loops run as CUDA graphs with device-side while nodes unless the

@@ -343,14 +343,25 @@ __global__ void seg_fill_kernel(int E, int M, int d1, const int* __restrict__ so
 // in a batched solve, the units of the images still running (Live) with a
 // grid sized for the device.
 
+// The lists a splat launch covers: positions [first, first + count) of
+// `order`, or the live images' positions of the domain behind lv.
+struct SplatRange {
+    int first = 0, count = 0;
+    Live lv;
+};
+__device__ __forceinline__ int splat_vertex(const SplatRange& r, const int* __restrict__ order, long u) {
+    return order[r.lv.n ? live_unit(r.lv, u) : r.first + u];
+}
+
 // Streams the list [s0, s1) of one vertex through the per-warp ring:
-// `vals_of(slot, e)` is this lane's staged word for entry e, and
-// consume(slot, n) is called once per chunk, in order.
-template <typename T, typename Consume>
+// ring[slot][e] holds this chunk's entries' values, mw[slot] their weights and,
+// with a norm, mn[slot] their factors; consume(slot, n) is called once per
+// chunk, in order.
+template <typename Consume>
 __device__ __forceinline__ void stream_list(int s0, int s1, int L, int k, bool act, int lane,
-                                            const int2* __restrict__ seg,
-                                            const T* __restrict__ src, T (*ring)[kChunk][32], float (*mw)[kChunk],
-                                            Consume&& consume) {
+                                            const int2* __restrict__ seg, const float* __restrict__ src,
+                                            const float* __restrict__ norm, float (*ring)[kChunk][32],
+                                            float (*mw)[kChunk], float (*mn)[kChunk], Consume&& consume) {
     const int nch = (s1 - s0 + kChunk - 1) / kChunk;
     auto pix_of = [&](int c) {
         const int base = s0 + c * kChunk;
@@ -359,6 +370,7 @@ __device__ __forceinline__ void stream_list(int s0, int s1, int L, int k, bool a
     auto issue = [&](int c, int pc) {
         const int slot = c % kStages, base = s0 + c * kChunk, n = min(kChunk, s1 - base);
         if (lane < n) cp_async4(&mw[slot][lane], &seg[base + lane].y);
+        if (norm && lane < n) cp_async4(&mn[slot][lane], norm + pc);
         for (int e = 0; e < n; e++) {
             const int p = __shfl_sync(0xffffffffu, pc, e);
             if (act) cp_async4(&ring[slot][e][lane], src + (long)p * L + k);
@@ -387,44 +399,59 @@ __device__ __forceinline__ void stream_list(int s0, int s1, int L, int k, bool a
     __syncwarp();
 }
 
-// The allocation-free filter's splat of the long lists (it may not hold the
-// padded rows of the splat below): rows as they are, one warp per vertex.
+// The splat of input rows as they are, for the allocation-free filter and where
+// memory is short: neither holds the padded copy of the splat below.  The long
+// lists, one warp per vertex; rows of Lp values, those past L zero.
 __global__ void __launch_bounds__(32 * kStageWarps)
-    splat_kernel(int M, int L, const int* __restrict__ order, const int* __restrict__ seg_start,
-                 const int2* __restrict__ seg, const float* __restrict__ in,
+    splat_kernel(SplatRange r, int L, int Lp, const int* __restrict__ order, const int* __restrict__ seg_start,
+                 const int2* __restrict__ seg, const float* __restrict__ in, const float* __restrict__ norm,
                  float* __restrict__ vals) {
     __shared__ float ring[kStageWarps][kStages][kChunk][32];
-    __shared__ float mw[kStageWarps][kStages][kChunk];
+    __shared__ float mw[kStageWarps][kStages][kChunk], mn[kStageWarps][kStages][kChunk];
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int unit = blockIdx.x * kStageWarps + wib;
-    if (unit >= M) return;  // warp-uniform
-    const int v = order[unit];
-    const int s0 = seg_start[v], s1 = seg_start[v + 1];
-    for (int kb = 0; kb < L; kb += 32) {
-        const int k = kb + lane;
-        const bool act = k < L;
-        float acc = 0.0f;
-        stream_list<float>(s0, s1, L, k, act, lane, seg, in, ring[wib], mw[wib], [&](int slot, int n) {
+    const long total = live_total(r.lv, r.count);
+    for (long unit = (long)blockIdx.x * kStageWarps + wib; unit < total; unit += (long)gridDim.x * kStageWarps) {
+        const int v = splat_vertex(r, order, unit);  // warp-uniform
+        const int s0 = seg_start[v], s1 = seg_start[v + 1];
+        for (int kb = 0; kb < L; kb += 32) {
+            const int k = kb + lane;
+            const bool act = k < L;
+            float acc = 0.0f;
+            stream_list(s0, s1, L, k, act, lane, seg, in, norm, ring[wib], mw[wib], mn[wib], [&](int slot, int n) {
 #pragma unroll 4
-            for (int e = 0; e < n; e++) acc = fadd(acc, fmul(mw[wib][slot][e], ring[wib][slot][e][lane]));
-        });
-        if (act) vals[(long)(v + 1) * L + k] = acc;
+                for (int e = 0; e < n; e++) {
+                    const float x = ring[wib][slot][e][lane];
+                    acc = fadd(acc, fmul(mw[wib][slot][e], norm ? fmul(x, mn[wib][slot][e]) : x));
+                }
+            });
+            if (k < Lp) vals[(long)(v + 1) * Lp + k] = act ? acc : 0.0f;
+        }
     }
 }
 
-// ... and of the short lists: one thread per (vertex, label).
-__global__ void splat_short_kernel(int n_short, int L, const int* __restrict__ order,
-                                   const int* __restrict__ seg_start, const int2* __restrict__ seg, const float* __restrict__ in,
-                                   float* __restrict__ vals) {
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)n_short * L) return;
-    const int u = (int)(t / L), k = (int)(t - (long)u * L);
-    const int v = order[u];
-    const int s0 = seg_start[v], s1 = seg_start[v + 1];
-    float acc = 0.0f;
+// ... and the short ones: one thread per (vertex, label).  Also row 0 of both
+// value buffers, which absent neighbours read.
+__global__ void splat_short_kernel(SplatRange r, int L, int Lp, const int* __restrict__ order,
+                                   const int* __restrict__ seg_start, const int2* __restrict__ seg,
+                                   const float* __restrict__ in, const float* __restrict__ norm,
+                                   float* __restrict__ vals, float* __restrict__ other) {
+    const long t0 = (long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long)gridDim.x * blockDim.x;
+    for (long t = t0; t < Lp; t += nt) vals[t] = other[t] = 0.0f;
+    const long total = live_total(r.lv, r.count) * Lp;
+    for (long t = t0; t < total; t += nt) {
+        const long u = t / Lp;
+        const int k = (int)(t - u * Lp);
+        const int v = splat_vertex(r, order, u);
+        const int s0 = seg_start[v], s1 = k < L ? seg_start[v + 1] : s0;
+        float acc = 0.0f;
 #pragma unroll 4
-    for (int s = s0; s < s1; s++) acc = fadd(acc, fmul(entry_w(seg[s]), in[(long)seg[s].x * L + k]));
-    vals[(long)(v + 1) * L + k] = acc;
+        for (int s = s0; s < s1; s++) {
+            const int2 e = seg[s];
+            const float x = in[(long)e.x * L + k];
+            acc = fadd(acc, fmul(entry_w(e), norm ? fmul(x, norm[e.x]) : x));
+        }
+        vals[(long)(v + 1) * Lp + k] = acc;
+    }
 }
 
 // ----------------------------------------------------------- row splat --
@@ -527,16 +554,6 @@ __global__ void __launch_bounds__(kTB)
         const float* x = in + i * L + 4 * q;
         rows[i * Q + q] = make_float4(x[0], n > 1 ? x[1] : 0.0f, n > 2 ? x[2] : 0.0f, n > 3 ? x[3] : 0.0f);
     }
-}
-
-// The lists a splat launch covers: positions [first, first + count) of
-// `order`, or the live images' positions of the domain behind lv.
-struct SplatRange {
-    int first = 0, count = 0;
-    Live lv;
-};
-__device__ __forceinline__ int splat_vertex(const SplatRange& r, const int* __restrict__ order, long u) {
-    return order[r.lv.n ? live_unit(r.lv, u) : r.first + u];
 }
 
 // Thread t of nt of the short lists' part.
@@ -1575,8 +1592,8 @@ void Lattice::forget() {
 
 void Lattice::ensure_values(size_t row_width) {
     const size_t need = (size_t)(M + 1) * row_width;
-    va.ensure(need);
-    vb.ensure(need);
+    own(va, need);
+    own(vb, need);
 }
 
 // ---------------------------------------------------------------------------
@@ -1627,19 +1644,11 @@ void Lattice::compute_noalloc(float* out, const float* in, int L, bool reverse) 
     float* base = noalloc_scratch();
     float *src = base, *dst = base + (size_t)(M + 1) * L;
     cudaStream_t st = stream;
-    // The array keeps the previous call's contents: only the zero rows that
-    // absent neighbours read must be cleared; every other row read below is
-    // written first.
-    DCRF_CUDA(cudaMemsetAsync(src, 0, sizeof(float) * L, st));
-    DCRF_CUDA(cudaMemsetAsync(dst, 0, sizeof(float) * L, st));
+    // The array keeps the previous call's contents: the splat clears the zero
+    // rows that absent neighbours read; every other row read below is written
+    // first.
     const long ML = (long)M * L, NL = (long)N * L;
-    const int n_short = M - n_long;
-    if (n_long)
-        launch(splat_kernel, ceil_div(n_long, kStageWarps), 32 * kStageWarps, 0, st, n_long, L, vorder.get(),
-               seg_start.get(), seg.get(), in, src);
-    if (n_short)
-        launch(splat_short_kernel, ceil_div((long)n_short * L, kTB), kTB, 0, st, n_short, L,
-               (const int*)vorder.get() + n_long, seg_start.get(), seg.get(), in, src);
+    splat_plain(in, L, L, nullptr, src, dst);
     const bool seq = L <= 2;
     for (int jj = 0; jj <= d; jj++) {
         const int j = reverse ? d - jj : jj;
@@ -1680,6 +1689,35 @@ static int slice_tile_max(int tile, int d, int L) {
 static bool row_tiles(int d, int L) { return kSliceWarps * slice_warp_bytes(1, d, L) <= (48 << 10); }
 static dim3 wide_grid(int N, int Q) { return dim3(ceil_div(Q, kTB), std::min(N, 65535)); }
 
+// The splat without the padded rows, into rows of Lp floats.
+void Lattice::splat_plain(const float* in, int L, int Lp, const float* pre_norm, float* vals, float* other) {
+    const bool live = live_n != nullptr;
+    const int n_short = M - n_long;
+    if (n_long)
+        launch(splat_kernel, unit_grid(n_long, kStageWarps, live, 32 * kStageWarps), 32 * kStageWarps, 0, stream,
+               SplatRange{0, n_long, live_of(kDomLong)}, L, Lp, vorder.get(), seg_start.get(), seg.get(), in, pre_norm,
+               vals);
+    launch(splat_short_kernel, unit_grid((long)n_short * Lp, kTB, live, kTB), kTB, 0, stream,
+           SplatRange{n_long, n_short, live_of(kDomShort)}, L, Lp, vorder.get(), seg_start.get(), seg.get(), in,
+           pre_norm, vals, other);
+}
+
+// The padded rows, or null where there is no memory for them.  Not asked for
+// inside a capture, which must not wait for the device.
+float* Lattice::rows_or_null(size_t floats) {
+    if (rows.n >= floats) return rows.get();
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    DCRF_CUDA(cudaStreamIsCapturing(stream, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return nullptr;
+    try {
+        return rows.ensure(floats);
+    } catch (const Error& e) {
+        if (e.code != DCRF_E_NOMEM) throw;
+        cudaGetLastError();
+        return nullptr;
+    }
+}
+
 // Splats `in` [N][L] (times pre_norm) into vals: rows of Q float4 (L > 2) or
 // of L floats.  With live images only their lists (and pixels).
 void Lattice::splat(const float* in, int L, const float* pre_norm, float* vals) {
@@ -1699,7 +1737,11 @@ void Lattice::splat(const float* in, int L, const float* pre_norm, float* vals) 
         return;
     }
     const int Q = value_row(L) / 4;
-    float4* rw = reinterpret_cast<float4*>(rows.ensure((size_t)N * Q * 4));
+    float4* rw = reinterpret_cast<float4*>(rows_or_null((size_t)N * Q * 4));
+    if (!rw) {
+        splat_plain(in, L, 4 * Q, pre_norm, vals, other);
+        return;
+    }
     const int tile = live ? dom_tile : slice_tile_for(L);
     require(tile > 0, DCRF_E_STATE, "splat: live images without prepare_live");
     if (!row_tiles(d, L)) {
@@ -1809,7 +1851,7 @@ void Lattice::ensure_ord_totals() {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     DCRF_CUDA(cudaStreamIsCapturing(stream, &cs));
     const long rowT = M + 1;
-    float* T = ord_T.ensure((size_t)(d + 2) * rowT);
+    float* T = own(ord_T, (size_t)(d + 2) * rowT);
     DCRF_CUDA(cudaMemsetAsync(T, 0, sizeof(float) * (d + 2) * rowT, stream));
     const int n_short = M - n_long;
     const SplatRange rl{0, n_long, Live{}}, rs{n_long, n_short, Live{}};

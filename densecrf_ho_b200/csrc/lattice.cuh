@@ -17,6 +17,7 @@
 #include "common.cuh"
 #include "primitives.cuh"
 
+#include <functional>
 #include <vector>
 
 namespace dcrf {
@@ -125,7 +126,21 @@ struct Lattice {
     DevBuf<int16_t> vkeys;
     DevBuf<int2> nbr;
     DevBuf<float> va, vb;    // filter value buffers
-    DevBuf<float> rows;      // the plain splat's input in rows of 16-byte groups, norm applied
+    // The plain splat's input in rows of 16-byte groups, norm applied: an aid that
+    // is given back where another buffer of the handle finds no memory, and done
+    // without where it finds none itself (splat_plain).
+    DevBuf<float> rows;
+    float* rows_or_null(size_t floats);
+    bool give_back_rows() {
+        const bool had = rows.get() != nullptr;
+        rows.release();
+        return had;
+    }
+    std::function<bool()> give_back_others;  // the same of the other lattices of a model or batch
+    template <typename T>
+    T* own(DevBuf<T>& b, size_t count) {
+        return ensure_after(b, count, [&] { return give_back_rows() | (give_back_others && give_back_others()); });
+    }
     // Ordered filter (see ordered.cu): packed bins, masks of the stored quads,
     // the up[0] plane, and per axis the blurred sums of each vertex's weights
     // (T, a property of the lattice: computed on its first ordered call).
@@ -229,6 +244,7 @@ struct Lattice {
     void tune_shape(int L);
     // The splat of `in` [N][L] into the value buffer vals.
     void splat(const float* in, int L, const float* pre_norm, float* vals);
+    void splat_plain(const float* in, int L, int Lp, const float* pre_norm, float* vals, float* other);
 
     Lattice() = default;
     Lattice(const Lattice&) = delete;

@@ -217,10 +217,10 @@ __global__ void fill_ones_kernel(long n, float* x) {
 Model::Model(int W_, int H_, int L_) : W(W_), H(H_), N(W_ * H_), L(L_) {
     DCRF_CUDA(cudaGetDevice(&device));
     DCRF_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-    scal.ensure(1);
+    own(scal, 1);
     // per-block partials: fixed-grid reductions, and the per-pixel / per-element
     // kernels that fold a reduction in (two values per block)
-    partials.ensure(std::max<size_t>((size_t)kRedBlocks * 16,
+    own(partials, std::max<size_t>((size_t)kRedBlocks * 16,
                                      2 * (size_t)std::max(ceil_div((long)N * L, 256), ord_slice_grid(N, L)) + 64));
     static_assert(sizeof(SolverScalars) <= kPinnedSlot, "one slot per model");
     h_scal = static_cast<SolverScalars*>(pinned_alloc());
@@ -252,6 +252,7 @@ void Model::add_term(const float* d_features, int d, float w) {
     auto t = std::make_unique<Term>();
     t->lat = std::make_unique<Lattice>();
     t->lat->stream = stream;
+    t->lat->give_back_others = [this] { return give_back_rows(); };
     t->lat->build(d_features, d, N);
     t->w = w;
     t->d = d;
@@ -320,6 +321,7 @@ void Model::set_kernel_parameters(int k, const float* p) {
     DCRF_LAUNCH_CHECK();
     auto lat = std::make_unique<Lattice>();
     lat->stream = stream;
+    lat->give_back_others = [this] { return give_back_rows(); };
     lat->build(scaled, t.d, N);
     if (!t.twin) t.twin = std::move(t.lat);
     t.lat = std::move(lat);
@@ -345,9 +347,9 @@ int Model::kernel_gradient(int k, const float* b, const float* Q, float* out) {
     const long NL = (long)N * L;
     const int d = t.d, g = ceil_div(NL, 256);
     float *lbl = buf(8), *bn = buf(9), *ln = buf(10), *fa = buf(11), *fb = buf(12), *X = buf(13);
-    float* ones = this->b[7].ensure((size_t)NL);
-    float* r = this->b[14].ensure((size_t)N * d);
-    float* gg = this->b[15].ensure((size_t)N * d);
+    float* ones = own(this->b[7], (size_t)NL);
+    float* r = own(this->b[14], (size_t)N * d);
+    float* gg = own(this->b[15], (size_t)N * d);
     const float* nrm = t.norm.get();
     if (t.compat == kPotts)
         launch(scale_cols_kernel, g, 256, 0, stream, NL, L, Q, (const float*)nullptr, -t.w, lbl);
@@ -387,7 +389,7 @@ int Model::kernel_gradient(int k, const float* b, const float* Q, float* out) {
         }
     }
     const int nb = 64, nout = t.ktype == kDiagKernel ? d : d * d;
-    double* part = partials.ensure((size_t)nb * nout);
+    double* part = own(partials, (size_t)nb * nout);
     launch(feature_grad_partial_kernel, dim3(nb, nout), 256, 0, stream, N, d, (int)(t.ktype == kFullKernel),
            (const float*)t.feat.get(), has_r ? (const float*)r : nullptr, (const float*)gg, part);
     DCRF_LAUNCH_CHECK();
@@ -433,7 +435,7 @@ int Model::compat_gradient(int k, const float* b, const float* Q, float* out) {
     const bool diag = t.compat == kDiagonal;
     const int pairs = diag ? L : L * L;
     const int nb = 32;
-    part = partials.ensure((size_t)nb * pairs);
+    part = own(partials, (size_t)nb * pairs);
     launch(label_outer_partial_kernel, dim3(nb, pairs), 256, 0, stream, N, L, b, (const float*)fq, (int)diag, part);
     DCRF_LAUNCH_CHECK();
     std::vector<double> h((size_t)nb * pairs);
@@ -456,7 +458,7 @@ int Model::compat_gradient(int k, const float* b, const float* Q, float* out) {
 void Model::set_unary_logistic(const float* lw, const float* lf, int F) {
     require(F >= 1, DCRF_E_ARG, "logistic unary: F must be >= 1");
     logit_F = F;
-    DCRF_CUDA(cudaMemcpyAsync(logit_f.ensure((size_t)F * N), lf, sizeof(float) * F * N, cudaMemcpyHostToDevice,
+    DCRF_CUDA(cudaMemcpyAsync(own(logit_f, (size_t)F * N), lf, sizeof(float) * F * N, cudaMemcpyHostToDevice,
                               stream));
     set_unary_parameters(lw);
 }
@@ -468,11 +470,11 @@ void Model::set_unary_parameters(const float* lw) {
     if (logit_F == 0) return;  // UnaryEnergy::setParameters is a no-op
     const size_t nw = (size_t)L * logit_F;
     h_logit_w.assign(lw, lw + nw);
-    DCRF_CUDA(cudaMemcpyAsync(logit_w.ensure(nw), h_logit_w.data(), sizeof(float) * nw, cudaMemcpyHostToDevice,
+    DCRF_CUDA(cudaMemcpyAsync(own(logit_w, nw), h_logit_w.data(), sizeof(float) * nw, cudaMemcpyHostToDevice,
                               stream));
     const long NL = (long)N * L;
     launch(logistic_unary_kernel, ceil_div(NL, 256), 256, 0, stream, NL, L, logit_F, (const float*)logit_w.get(),
-           (const float*)logit_f.get(), unary.ensure((size_t)NL));
+           (const float*)logit_f.get(), own(unary, (size_t)NL));
     DCRF_LAUNCH_CHECK();
     has_unary = true;
     sync();
@@ -482,7 +484,7 @@ void Model::set_unary_parameters(const float* lw) {
 int Model::unary_gradient(const float* b, float* out) {
     if (logit_F == 0) return 0;  // UnaryEnergy::gradient: empty
     const int F = logit_F, pairs = L * F, nb = 32;
-    double* part = partials.ensure((size_t)nb * pairs);
+    double* part = own(partials, (size_t)nb * pairs);
     launch(logistic_grad_partial_kernel, dim3(nb, pairs), 256, 0, stream, N, L, F, b, (const float*)logit_f.get(),
            part);
     DCRF_LAUNCH_CHECK();
@@ -559,11 +561,11 @@ void Model::set_cliques(int R_, const int* off, const int* idx, const float* exp
     std::vector<int> bs((size_t)clique_max + 2, 0);
     for (int r = 0; r < R; r++) bs[packed[2 * R + 1 + r] + 1]++;
     for (size_t s = 1; s < bs.size(); s++) bs[s] += bs[s - 1];
-    int* dbs = cl_bstart.ensure(bs.size());
+    int* dbs = own(cl_bstart, bs.size());
     DCRF_CUDA(cudaMemcpyAsync(dbs, bs.data(), sizeof(int) * bs.size(), cudaMemcpyHostToDevice, stream));
-    int* doff = cl_off.ensure(packed.size());
+    int* doff = own(cl_off, packed.size());
     DCRF_CUDA(cudaMemcpyAsync(doff, packed.data(), sizeof(int) * packed.size(), cudaMemcpyHostToDevice, stream));
-    int* didx = cl_idx.ensure(std::max(clique_total, 1));
+    int* didx = own(cl_idx, std::max(clique_total, 1));
     if (clique_total)
         DCRF_CUDA(cudaMemcpyAsync(didx, idx, sizeof(int) * clique_total, cudaMemcpyHostToDevice, stream));
     // the chunked clique kernels' units: chunks of kCliqueChunk pixels per clique, L units each
@@ -577,14 +579,14 @@ void Model::set_cliques(int R_, const int* off, const int* idx, const float* exp
         }
         uc_nchunks = (int)ch.size();
         uc_units = ub[R];
-        int2* dch = uc_chunks.ensure(std::max<size_t>(ch.size(), 1));
+        int2* dch = own(uc_chunks, std::max<size_t>(ch.size(), 1));
         if (!ch.empty())
             DCRF_CUDA(cudaMemcpyAsync(dch, ch.data(), sizeof(int2) * ch.size(), cudaMemcpyHostToDevice, stream));
-        int* dub = uc_base.ensure(ub.size());
+        int* dub = own(uc_base, ub.size());
         DCRF_CUDA(cudaMemcpyAsync(dub, ub.data(), sizeof(int) * ub.size(), cudaMemcpyHostToDevice, stream));
     }
-    float* de = cl_exp.ensure(std::max(R, 1));
-    float* dc = cl_const.ensure(std::max(R, 1));
+    float* de = own(cl_exp, std::max(R, 1));
+    float* dc = own(cl_const, std::max(R, 1));
     if (R) {
         DCRF_CUDA(cudaMemcpyAsync(de, expw, sizeof(float) * R, cudaMemcpyHostToDevice, stream));
         DCRF_CUDA(cudaMemcpyAsync(dc, cst, sizeof(float) * R, cudaMemcpyHostToDevice, stream));
@@ -610,7 +612,7 @@ static CompatRoute route_compat(Model& m, const Term& t, SliceEpilogue& ep, floa
     const int kind = potts_only ? (int)kPotts : t.compat;
     if (kind == kMatrix) {
         ep.scale = 1.0f;
-        return {m.compat_tmp.ensure((size_t)m.N * m.L), true};
+        return {m.own(m.compat_tmp, (size_t)m.N * m.L), true};
     }
     if (kind == kDiagonal) {
         ep.scale = 1.0f;
@@ -844,7 +846,7 @@ double Model::energy_true(const int16_t* d_lab, bool ho) {
     require(has_unary, DCRF_E_STATE, "energy: no unary energy set");
     float* qc = buf(10);
     float* o = buf(11);
-    float* pw = b[12].ensure(N);
+    float* pw = own(b[12], N);
     launch(onehot_complement_kernel, ceil_div((long)N * L, 256), 256, 0, stream, N, L, d_lab, qc);
     for (size_t k = 0; k < terms.size(); k++) {
         apply((int)k, true, o, qc);
@@ -854,7 +856,7 @@ double Model::energy_true(const int16_t* d_lab, bool ho) {
     launch(energy_sum_kernel, kRedBlocks, kRedThreads, 0, stream, N, L, d_lab, unary.get(), pw, partials.get());
     launch(finalize_sums_kernel, 1, 32, 0, stream, partials.get(), kRedBlocks, 1, 0, scal.get());
     if (ho && R > 0) {
-        int* flags = ipart.ensure(std::max(R, 1));
+        int* flags = own(ipart, std::max(R, 1));
         launch(clique_label_change_kernel, R, 256, 0, stream, cl_off.get(), cl_idx.get(), d_lab, flags);
         launch(energy_ho_finish_kernel, 1, 1, 0, stream, R, flags, cl_exp.get(), scal.get());
     }
@@ -877,8 +879,8 @@ double Model::energy_lp(const float* Q) {
         launch(finalize_sums_kernel, 1, 32, 0, stream, partials.get(), kRedBlocks, 1, 1 + (int)k, scal.get());
     }
     if (R > 0) {
-        float* diffs = b[13].ensure(std::max(R, 1));
-        float2* part = reinterpret_cast<float2*>(uc_scan.ensure(std::max<size_t>(3 * (size_t)uc_units, 1)));
+        float* diffs = own(b[13], std::max(R, 1));
+        float2* part = reinterpret_cast<float2*>(own(uc_scan, std::max<size_t>(3 * (size_t)uc_units, 1)));
         if (uc_nchunks > 0)
             launch(clique_maxdiff_chunk_kernel, uc_nchunks, 256, 0, stream, uc_chunks.get(), cl_off.get(),
                    cl_idx.get(), uc_base.get(), L, Q, part);

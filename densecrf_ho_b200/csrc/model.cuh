@@ -135,7 +135,20 @@ struct Model {
     Model(int W_, int H_, int L_);
     ~Model();
 
-    float* buf(int i) { return b[i].ensure((size_t)N * L); }
+    // A buffer of the model; its lattices' padded rows go first where memory is short.
+    template <typename T>
+    T* own(DevBuf<T>& buffer, size_t count) {
+        return ensure_after(buffer, count, [&] { return give_back_rows(); });
+    }
+    bool give_back_rows() {
+        bool any = false;
+        for (auto& t : terms) {
+            any |= t->lat->give_back_rows();
+            if (t->twin) any |= t->twin->give_back_rows();
+        }
+        return any;
+    }
+    float* buf(int i) { return own(b[i], (size_t)N * L); }
     void add_term(const float* d_features, int d, float w);
     void set_cliques(int R, const int* off, const int* idx, const float* expw, const float* cst);
 

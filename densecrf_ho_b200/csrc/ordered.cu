@@ -1145,7 +1145,7 @@ void Lattice::compute_ord(float* out, const float* Q, int L, const SliceEpilogue
         compute_ord_dense(out, Q, L, ep);
         return;
     }
-    unsigned short* bins = obins.ensure(ordered_bins_size(N, L));
+    unsigned short* bins = own(obins, ordered_bins_size(N, L));
     ordered_bins(bins, Q, N, L, nullptr, stream);
     ord_splat_blur(bins, L);
     ord_slice(out, bins, L, ep, nullptr);
@@ -1159,8 +1159,8 @@ void Lattice::ord_splat_blur(const unsigned short* bins, int L) {
     const int NW = ord_words(L), nblk = (L + 31) / 32, n_short = M - n_long;
     const int nc = std::min(4, ord_bin_row(L) / 8);
     float *src = va.get(), *dst = vb.get();
-    unsigned *as = ord_a.ensure((size_t)(M + 1) * NW), *ad = ord_b.ensure((size_t)(M + 1) * NW);
-    float* plane = ord_plane.ensure((size_t)(M + 1) * ord_plane_row(L));
+    unsigned *as = own(ord_a, (size_t)(M + 1) * NW), *ad = own(ord_b, (size_t)(M + 1) * NW);
+    float* plane = own(ord_plane, (size_t)(M + 1) * ord_plane_row(L));
     const uint4* b4 = reinterpret_cast<const uint4*>(bins);
     const unsigned* pm = bin_masks(bins, N, L);
     if (n_long)
@@ -1384,7 +1384,7 @@ void Lattice::compute_ord_dense(float* out, const float* Q, int L, const SliceEp
     ensure_values(row);
     cudaStream_t st = stream;
     const long NL = (long)N * L;
-    float2* bins = r_ebins.ensure((size_t)NL);
+    float2* bins = own(r_ebins, (size_t)NL);
     pair_bins(bins, Q, NL, st);
     float *src = va.get(), *dst = vb.get();
     launch(ord_dense_splat_kernel, ceil_div((long)M * L, kTB), kTB, 0, st, M, L, (const int*)seg_start.get(),
@@ -1533,12 +1533,12 @@ void Lattice::compute_ord_restricted(float* rout, const float* rQ, const int* pI
     cudaStream_t st = stream;
     if (store) r_L = 0;  // until this call has stored its splat
     const long row = (long)L * kOrdW, cells = (long)(M + 1) * row;
-    float* stored = r_stored.ensure((size_t)cells);
-    float* a = r_a.ensure((size_t)cells);
-    float* b = r_b.ensure((size_t)cells);
-    unsigned char* active = r_active.ensure((size_t)std::max(M, 1));
-    int* pos = r_pos.ensure((size_t)N);
-    float2* rb = r_bins.ensure((size_t)std::max<long>((long)nP * L, 1));
+    float* stored = own(r_stored, (size_t)cells);
+    float* a = own(r_a, (size_t)cells);
+    float* b = own(r_b, (size_t)cells);
+    unsigned char* active = own(r_active, (size_t)std::max(M, 1));
+    int* pos = own(r_pos, (size_t)N);
+    float2* rb = own(r_bins, (size_t)std::max<long>((long)nP * L, 1));
     launch(fill_int_kernel, ceil_div(N, kTB), kTB, 0, st, (long)N, -1, pos);
     if (nP) {
         launch(scatter_pos_kernel, ceil_div(nP, kTB), kTB, 0, st, nP, pI, pos);
@@ -1546,7 +1546,7 @@ void Lattice::compute_ord_restricted(float* rout, const float* rQ, const int* pI
     }
     const float2* eb = nullptr;
     if (store) {
-        float2* e = r_ebins.ensure((size_t)N * L);
+        float2* e = own(r_ebins, (size_t)N * L);
         pair_bins(e, Q, (long)N * L, st);
         eb = e;
     }

@@ -1483,9 +1483,9 @@ double Model::energy_qp_ho(const float* Q) {
         const int* base = cl_off.get();
         const CliqueView cv{base, base + R + 1, base + 2 * R + 1, cl_idx.get(), cl_exp.get(), cl_const.get(), R,
                             clique_max, cl_bstart.get()};
-        float* small = b[14].ensure((size_t)8 * LR);
+        float* small = own(b[14], (size_t)8 * LR);
         float *zc = small + 6 * LR, *omz = small + 7 * LR;
-        double* preQ = ho_pre.ensure((size_t)2 * LR);
+        double* preQ = own(ho_pre, (size_t)2 * LR);
         launch(clear_step_flags_kernel, 1, 1, 0, stream, sc);
         launch(ho_zterm_prep_kernel, 1, 256, 0, stream, cv, L, (const float*)z_last.get(), zc, omz, sc);
         launch(eig_sum_kernel, 1, kHoThreads, 0, stream, (const float*)zc, LR, 8, sc, 2);
@@ -1610,9 +1610,9 @@ int Model::qp(const float* init, float* out, int max_iter, double* energy_out) {
         const int* base = cl_off.get();
         cv = CliqueView{base, base + R + 1, base + 2 * R + 1, cl_idx.get(), cl_exp.get(), cl_const.get(), R, clique_max,
                         cl_bstart.get()};
-        float* small = b[14].ensure((size_t)8 * LR);
-        pre32 = b[15].ensure((size_t)LR);
-        double* dpre = ho_pre.ensure((size_t)2 * LR);
+        float* small = own(b[14], (size_t)8 * LR);
+        pre32 = own(b[15], (size_t)LR);
+        double* dpre = own(ho_pre, (size_t)2 * LR);
         preQ = dpre;
         preS = dpre + LR;
         gz = small;
@@ -1732,7 +1732,7 @@ int Model::qp(const float* init, float* out, int max_iter, double* energy_out) {
         }
     }
     if (R > 0) {  // z_labels_ = z (src/densecrf.cpp:439)
-        DCRF_CUDA(cudaMemcpyAsync(z_last.ensure((size_t)LR), z, sizeof(float) * LR, cudaMemcpyDeviceToDevice,
+        DCRF_CUDA(cudaMemcpyAsync(own(z_last, (size_t)LR), z, sizeof(float) * LR, cudaMemcpyDeviceToDevice,
                                   stream));
         sync();
     }
@@ -1753,9 +1753,9 @@ int Model::lp(const float* init, float* out, const dcrf_lp_params& p, dcrf_solve
     float* su = R > 0 ? buf(4) : nullptr;
     float* gamma = buf(5);
     float* curQ = buf(6);
-    unsigned short* bins = lp_bins.ensure(ordered_bins_size(N, L));
+    unsigned short* bins = own(lp_bins, ordered_bins_size(N, L));
     float* Y = buf(8);
-    int16_t* lab = labels.ensure(N);
+    int16_t* lab = own(labels, N);
     SolverScalars* sc = scal.get();
     double* part = partials.get();
     const int nt = (int)terms.size();
@@ -1798,9 +1798,9 @@ int Model::lp(const float* init, float* out, const dcrf_lp_params& p, dcrf_solve
         const int* base = cl_off.get();
         cv = CliqueView{base, base + R + 1, base + 2 * R + 1, cl_idx.get(), cl_exp.get(), cl_const.get(), R, clique_max,
                         cl_bstart.get()};
-        upos = ipart.ensure(4 * (size_t)R);  // [2R] selected positions, [2R] write targets
+        upos = own(ipart, 4 * (size_t)R);  // [2R] selected positions, [2R] write targets
         if (!lp_win.get()) {
-            int* w = lp_win.ensure((size_t)N * L);
+            int* w = own(lp_win, (size_t)N * L);
             DCRF_CUDA(cudaMemsetAsync(w, 0xff, sizeof(int) * (size_t)N * L, stream));  // -1: no claim
         }
     }
@@ -1881,7 +1881,7 @@ int Model::lp(const float* init, float* out, const dcrf_lp_params& p, dcrf_solve
             const int nw = 2 * R;
             int* tgt = upos + 2 * R;
             DCRF_CUDA(cudaMemsetAsync(su, 0, sizeof(float) * NL, stream));
-            int2* ucp = uc_scan.ensure(std::max<size_t>(3 * (size_t)uc_units, 1));
+            int2* ucp = own(uc_scan, std::max<size_t>(3 * (size_t)uc_units, 1));
             if (uc_nchunks > 0) {
                 launch(ucond_minmax_kernel, uc_nchunks, 256, 0, stream, uc_chunks.get(), cl_off.get(), cl_idx.get(),
                        uc_base.get(), L, Q, ucp);
