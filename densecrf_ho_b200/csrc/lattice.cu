@@ -1768,8 +1768,11 @@ void Lattice::splat(const float* in, int L, const float* pre_norm, float* vals) 
     const int sb = n_short ? unit_grid((long)n_short * Q, kSplatThreads, live, kSplatThreads) : 0;
     const size_t smem = hb + lb ? (size_t)kSplatWarps * splat_ring_bytes(std::min(Q, 8)) : 0;
     auto kern = Q == 6 ? splat_rows_kernel<6> : splat_rows_kernel<0>;
-    if (smem > 48 * 1024)  // opt-in size: a per-device function attribute, set on every such call
-        DCRF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // The opt-in is an attribute of the kernel that all threads share: always the
+    // largest size there is (eight groups a row).
+    if (smem > 48 * 1024)
+        DCRF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       kSplatWarps * splat_ring_bytes(8)));
     if (hb + lb + sb)
         launch_chained(kern, hb + lb + sb, kSplatThreads, smem, st, rl, rs, hb, lb, Q, vorder.get(),
                        seg_start.get(), seg.get(), (const float4*)rw,

@@ -1092,8 +1092,10 @@ void launch_slice(float* out, const unsigned short* bins, int L, const Lattice& 
         return;
     }
     const int P = std::min(elems / L + 2, elems);  // pixels that a block touches at most
-    size_t smem = (sizeof(int2) + sizeof(float)) * P * (a.d + 1) + sizeof(float) * 4 * P;
-    if (NT == 2) smem += (sizeof(int2) + sizeof(float)) * P * (b.d + 1);
+    auto bytes = [](int pixels, int d0, int d1) {
+        return (sizeof(int2) + sizeof(float)) * pixels * (d0 + 1 + (NT == 2 ? d1 + 1 : 0)) + sizeof(float) * 4 * pixels;
+    };
+    const size_t smem = bytes(P, a.d, b.d);
     auto pick = [&](auto g) {
         constexpr bool GAP = decltype(g)::value;
         if constexpr (NT == 2) {
@@ -1107,8 +1109,11 @@ void launch_slice(float* out, const unsigned short* bins, int L, const Lattice& 
         }
     };
     auto kern = gap ? pick(std::true_type{}) : pick(std::false_type{});
-    if (smem > 40 * 1024)  // opt-in size: a per-device function attribute, set on every such call
-        DCRF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // The opt-in is an attribute of the kernel that all threads share: always the
+    // largest size there is (one label, two terms of 16 features: 53 KB).
+    if (smem > 40 * 1024)
+        DCRF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)bytes(slice_elems(1), 16, 16)));
     launch_ord(NL, kern, ceil_div(NL, elems), kOsThreads, smem, st, a.N, L, P, t0, t1, bins, out, gap ? *gap : GapFusion{});
     DCRF_LAUNCH_CHECK();
 }
@@ -1171,9 +1176,9 @@ void Lattice::ord_splat_blur(const unsigned short* bins, int L) {
     require(ht + lt < (1L << 30), DCRF_E_ARG, "compute_ord: too many labels");
     int bytes = std::max(n_long ? ord_ring_bytes(nc) + 2 * kUnitList : 0, ord_group_bytes(nc));
     bytes = (bytes + 15) & ~15;
+    static_assert(kOrdWarps * (ord_ring_bytes(4) + 2 * kUnitList) <= (48 << 10) &&
+                      kOrdWarps * ord_group_bytes(4) <= (48 << 10), "no opt-in to more shared memory");
     auto splat = L == 21 ? ord_splat_kernel<3, 4> : ord_splat_kernel<0, 0>;
-    if (bytes * kOrdWarps > 48 * 1024)  // opt-in size: a per-device function attribute, set on every such call
-        DCRF_CUDA(cudaFuncSetAttribute(splat, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes * kOrdWarps));
     launch_ord((long)N * L, splat, ceil_div(tasks, kOrdWarps), kOrdThreads, (size_t)bytes * kOrdWarps, st, M, n_long, n_huge,
                    (int)ht, (int)lt, L, NW, vorder.get(), seg_start.get(), seg.get(), b4, pm, as, ad, src, bytes);
     for (int j = 0; j <= d; j++) {
