@@ -1037,7 +1037,14 @@ void Batch::meanfield_backward(const float* grad_Q, float* grad_U, double* grad_
     double* dw = own(mf_dw, std::max(nt, 1));
     double* part = own(partials, std::max((size_t)kRedBlocks * 2, (size_t)Lattice::dot_partials()));
     if (ck_every > 1) launch(negate_kernel, ceil_div(NL, 256), 256, 0, stream, NL, unary.get(), negU);
-    const float* gq = grad_Q;  // dL/dQ_{t+1}
+    // dL/dQ_{t+1}; from a copy where the caller's grad_U lies over grad_Q: the
+    // softmax's adjoint writes the one while other warps still read the other.
+    const float* gq = grad_Q;
+    const uintptr_t uq = reinterpret_cast<uintptr_t>(grad_Q), uu = reinterpret_cast<uintptr_t>(grad_U);
+    if ((uq > uu ? uq - uu : uu - uq) < sizeof(float) * NL) {
+        DCRF_CUDA(cudaMemcpyAsync(g, grad_Q, sizeof(float) * NL, cudaMemcpyDeviceToDevice, stream));
+        gq = g;
+    }
     if (nt) DCRF_CUDA(cudaMemsetAsync(dw, 0, sizeof(double) * nt, stream));
     auto softmax_bwd = [&](const float* q, int first) {
         with_lc(L, [&](auto lc) {
