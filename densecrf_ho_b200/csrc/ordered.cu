@@ -942,11 +942,16 @@ __global__ void __launch_bounds__(kOsThreads)
         return v;
     };
     const bool dense = s_dense;
-    // from the first element's group of four to the last one's: the block
-    // shares its outer pixels with its neighbours
+    // The block shares its outer pixels with its neighbours.  With the labels at
+    // compile time it walks all groups of its pixels and skips those outside, else
+    // (a pixel may be many blocks') from the first element's group to the last's.
+    // The whole filter, 640x480, five features: 21 labels 269 us by the former, 277
+    // by the latter; 40 labels 562 and 546.
     const int ll = (ne - 1 + first) / L, last = ll * Q + (ne - 1 + first - ll * L) / 4;
-    for (int it = first / 4 + threadIdx.x; !dense && it <= last; it += blockDim.x) {
+    const int it0 = LC ? 0 : first / 4, it1 = LC ? np * Q : last + 1;
+    for (int it = it0 + threadIdx.x; !dense && it < it1; it += blockDim.x) {
         const int li = it / Q, q = it - li * Q, e0 = li * L + 4 * q - first;
+        if (LC && (e0 + 3 < 0 || e0 >= ne)) continue;
         const uint2 c = *reinterpret_cast<const uint2*>(bins + (long)(pf + li) * Lb + 4 * q);
         float a[NT][4];
 #pragma unroll
