@@ -36,8 +36,6 @@ constexpr int kEmpty = -1;
 constexpr int kStageWarps = 2;   // warps (splat lists) per splat block
 constexpr int kStages = 3;       // shared-memory ring depth, in chunks
 constexpr int kChunk = 32;       // entries per chunk (13 KB of ring per warp: 16 warps / SM)
-constexpr int kMaxOrderKey = (1 << 24) - 1;
-constexpr int kHugeLabels = 12;  // labels per block for those lists (120 threads)
 
 template <int KW>
 struct Key {

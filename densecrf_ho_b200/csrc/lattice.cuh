@@ -118,6 +118,10 @@ struct Lattice {
     int n_long = 0;  // vertices whose splat list exceeds the staging threshold
     int n_huge = 0;  // ... and the (leading) ones whose list is very long
     cudaStream_t stream = nullptr;  // borrowed
+    // side stream (highest priority) of the dense ordered splat's longest lists
+    cudaStream_t aux = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    void ensure_aux();
 
     DevBuf<int> offset, rank, seg_start;
     DevBuf<int2> seg;
@@ -249,6 +253,7 @@ struct Lattice {
     Lattice() = default;
     Lattice(const Lattice&) = delete;
     Lattice& operator=(const Lattice&) = delete;
+    ~Lattice();
 };
 
 }  // namespace dcrf

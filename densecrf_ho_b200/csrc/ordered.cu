@@ -1261,11 +1261,30 @@ void pair_bins(float2* bins, const float* Q, long n, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------
-// The dense form: every bin of every label, nothing skipped (ord_dense).  Its
-// kernels leave most of the chip's registers and all of its shared memory to
-// other streams, and where no list is long they touch little more than the
-// quads that exist.
-//
+// The dense form: every bin of every label, nothing skipped (ord_dense); a
+// vertex row holds 20 bins x L labels, bin-major ([v][bin][label]; bins [0,10)
+// lower, [10,20) upper) so that the slice's per-label bin reads coalesce.  Where no
+// list is long its kernels touch little more than the quads that exist and leave
+// most of the chip's registers and all of its shared memory to other streams.
+
+// One entry into the bin-b pair (lower, upper) of packed accumulators:
+// acc = fma({[cl >= b], [b >= cu]}, w2, acc) with one f32x2 FMA, which rounds
+// each half exactly as fma.rn.f32 does.  w2 holds (w, w).  The bins are
+// small integers, so the masks are saturated sums: cl + (1 - b) and
+// (b + 1) - cu are exact integers, clamped to [0, 1] they are exactly the
+// comparisons (and a NaN would clamp to +0).  One `add.sat` per mask.
+__device__ __forceinline__ void ord_step2(unsigned long long& acc, float cl, float cu, float b,
+                                          unsigned long long w2) {
+    const float lo_c = 1.0f - b, up_c = b + 1.0f;  // exact; hoisted out of the entry loops
+    asm("{\n\t.reg .f32 ml, mu;\n\t.reg .b64 m;\n\t"
+        "add.rn.sat.f32 ml, %1, %3;\n\t"
+        "sub.rn.sat.f32 mu, %4, %2;\n\t"
+        "mov.b64 m, {ml, mu};\n\t"
+        "fma.rn.f32x2 %0, m, %5, %0;\n\t}"
+        : "+l"(acc)
+        : "f"(cl), "f"(cu), "f"(lo_c), "f"(up_c), "l"(w2));
+}
+
 // The single masks of ord_step2: [cl >= b] and [b >= cu] as 0.0 / 1.0.
 __device__ __forceinline__ float ord_mask_lower(float cl, int b) {
     float m;
@@ -1278,17 +1297,210 @@ __device__ __forceinline__ float ord_mask_upper(float cu, int b) {
     return m;
 }
 
-// Splat, one thread per (vertex, label), both passes in registers: lower bin 0
+// Its long lists, by blocks.  The 20 x L bin sums of a
+// vertex are 20 L independent in-order chains; thread (k, g) carries the
+// chains of label k, bins g*NB .. g*NB+NB-1, both passes, so a block shares
+// a long list's work and the longest lists no longer set the kernel's
+// length.
+//
+// The list streams through shared memory in chunks of kOE entries: the
+// pixel ids and weights of chunk c + 2 kODX and the (c_lower, c_upper) bins
+// of chunk c + kODX are copied with cp.async while chunk c is summed, one
+// block barrier per chunk.  Ring rows are label-major ([k][entry][lower,
+// upper], padded to an odd number of 16-byte units) so a thread reads two
+// entries per 16-byte load and eight consecutive labels hit distinct banks.
+// Weights are staged as (w, w) pairs; entries past the end of the list get
+// weight 0, which leaves every accumulator unchanged (the masks are 0 or 1
+// for any stale bin value).
+constexpr int kHugeLabels = 12;         // labels per block for the lists over kHugeList
+constexpr int kOE = 32;                 // entries per chunk
+constexpr int kODX = 4;                 // bins are copied kODX chunks ahead of use, pixel ids 2 kODX
+constexpr int kOXS = kODX + 1;          // bin ring slots (chunks c .. c+kODX)
+constexpr int kOPS = 2 * kODX + 1;      // pixel / weight ring slots (chunks c .. c+2 kODX)
+constexpr int kORow = 2 * kOE + 4;      // floats per ring row: 17 x 16 bytes
+constexpr int kOrdBlockMaxL = 160;      // larger L: the quad form (shared-memory ring size)
+constexpr int kGroupChoices[] = {1, 2, 3, 5, 10};
+
+// Bin split with the fewest warp instructions per list entry: warps x (three
+// instructions per bin slot -- two masks and one f32x2 FMA -- + about two
+// for the shared-memory loads).
+int ord_groups_cheapest(int L) {
+    int best = 1;
+    long best_cost = -1;
+    for (int G : kGroupChoices) {
+        if (L * G > 1024) break;
+        const long warps = (L * G + 31) / 32, nb = (kRes + G - 1) / G;
+        const long cost = warps * (3 * nb + 2);
+        if (best_cost < 0 || cost <= best_cost) {
+            best = G;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
+size_t ord_block_smem(int kb) {
+    return sizeof(float) * ((size_t)kOXS * kb * kORow + (size_t)kOPS * kOE * 2) + sizeof(int) * kOPS * kOE;
+}
+
+// G bin groups per label, NB = ceil(10 / G) bin slots per thread; slots past
+// bin 9 (when G does not divide 10) run on a dummy bin that is not stored.
+// Block b covers labels [k0, k0 + nk) of vertex order[b / kblocks], k0 =
+// (b % kblocks) * kb: a very long list can be shared by several blocks.
+// Compute threads are label-major (t = k * G + g), so the G threads reading
+// one label's bins sit in one warp and their shared-memory loads broadcast;
+// staging threads are entry-major (t = g * nk + k) so one warp's copies read
+// consecutive labels of one pixel.
+template <int G>
+__global__ void __launch_bounds__(kOrdBlockMaxL * G < 1024 ? kOrdBlockMaxL * G : 1024)
+    ord_dense_long_kernel(int L, int kb, int kblocks, const int* __restrict__ order,
+                           const int* __restrict__ seg_start, const int2* __restrict__ seg,
+                           const float2* __restrict__ bins, float* __restrict__ vals) {
+    extern __shared__ __align__(16) float osm[];
+    float* xr = osm;                            // [kOXS][kb][kORow]
+    float* wr = xr + (size_t)kOXS * kb * kORow;  // [kOPS][kOE][2]
+    int* pr = reinterpret_cast<int*>(wr + kOPS * kOE * 2);  // [kOPS][kOE]
+    constexpr int NB = (kRes + G - 1) / G;
+    const int t = threadIdx.x;
+    const int v = order[blockIdx.x / kblocks];
+    const int k0 = (blockIdx.x % kblocks) * kb, nk = min(kb, L - k0);
+    const int s0 = seg_start[v], s1 = seg_start[v + 1];
+    const int nch = (s1 - s0 + kOE - 1) / kOE;
+    const bool worker = t < nk * G;
+    const int k = t / G, g = t - k * G;      // compute role
+    const int sk = t % nk, sg = t / nk;      // staging role (sg < G for workers)
+
+    auto stage_pw = [&](int c) {  // pixel ids and weights of chunk c
+        if (c < nch && t < kOE) {
+            const int slot = c % kOPS, e = s0 + c * kOE + t;
+            if (e < s1) {
+                cp_async4(&pr[slot * kOE + t], &seg[e].x);
+                cp_async4(&wr[(slot * kOE + t) * 2], &seg[e].y);
+                cp_async4(&wr[(slot * kOE + t) * 2 + 1], &seg[e].y);
+            } else {
+                pr[slot * kOE + t] = 0;
+                wr[(slot * kOE + t) * 2] = 0.0f;
+                wr[(slot * kOE + t) * 2 + 1] = 0.0f;
+            }
+        }
+    };
+    // (c_lower, c_upper) of chunk c; needs chunk c's pixel ids in place.
+    // Staging thread (sk, sg) copies label k0 + sk of entries sg, sg + G, ...
+    // All pixel ids are read before the first copy is issued (the copies'
+    // memory clobber would otherwise order each read after the last copy).
+    auto stage_x = [&](int c) {
+        if (c >= nch || !worker) return;
+        constexpr int MX = (kOE + G - 1) / G;
+        const int slot = c % kOXS, ps = c % kOPS;
+        const int n = min(kOE, s1 - (s0 + c * kOE));
+        float* dst = &xr[((size_t)slot * kb + sk) * kORow];
+        const float2* src = bins + k0 + sk;
+        int pix[MX];
+#pragma unroll
+        for (int i = 0; i < MX; i++) {
+            const int e = sg + i * G;
+            pix[i] = e < n ? pr[ps * kOE + e] : 0;
+        }
+#pragma unroll
+        for (int i = 0; i < MX; i++) {
+            const int e = sg + i * G;
+            if (e < n) cp_async8(dst + 2 * e, src + (long)pix[i] * L);
+        }
+    };
+
+    // Group j (committed at iteration j; j < 0 in the prologue) holds the
+    // bins of chunk j + kODX and the pixel ids / weights of chunk j + 2 kODX.
+#pragma unroll
+    for (int c = 0; c < kODX; c++) stage_pw(c);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < kODX; c++) {
+        stage_x(c);
+        stage_pw(c + kODX);
+        cp_async_commit();
+    }
+
+    // Bin g*NB + i's (lower, upper) sums as one packed pair: ord_step2 adds
+    // an entry to both with one f32x2 FMA (each half rounded as fma.rn.f32).
+    unsigned long long acc[NB];
+    float bf[NB];
+#pragma unroll
+    for (int i = 0; i < NB; i++) {
+        acc[i] = 0ull;
+        bf[i] = (float)(g * NB + i);
+    }
+    for (int c = 0; c < nch; c++) {
+        cp_async_wait<kODX - 1>();  // group c - kODX: bins of chunk c, pixel ids of chunk c + kODX
+        __syncthreads();            // ... everyone's copies; and chunk c-1's slots are free
+        stage_x(c + kODX);
+        stage_pw(c + 2 * kODX);
+        cp_async_commit();
+        if (worker) {
+            const float4* xs = reinterpret_cast<const float4*>(&xr[((size_t)(c % kOXS) * kb + k) * kORow]);
+            const ulonglong2* ws = reinterpret_cast<const ulonglong2*>(&wr[(c % kOPS) * kOE * 2]);
+            const int n2 = (min(kOE, s1 - (s0 + c * kOE)) + 1) >> 1;
+            // Batches of eight entries, the next batch's loads issued before
+            // this batch is summed.  A batch may run past n2 into the chunk's
+            // zero-weight tail (the ring rows hold kOE entries).
+            float4 x[4];      // (c_lower, c_upper) of entries 2 j, 2 j + 1
+            ulonglong2 w[4];  // ((w, w), (w, w)) of the same entries
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                x[j] = xs[j];
+                w[j] = ws[j];
+            }
+            for (int b0 = 0; b0 < n2; b0 += 4) {
+                float4 xn[4];
+                ulonglong2 wn[4];
+                const int nb0 = b0 + 4 < kOE / 2 ? b0 + 4 : b0;  // stays inside the ring row
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    xn[j] = xs[nb0 + j];
+                    wn[j] = ws[nb0 + j];
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+#pragma unroll
+                    for (int i = 0; i < NB; i++) ord_step2(acc[i], x[j].x, x[j].y, bf[i], w[j].x);
+#pragma unroll
+                    for (int i = 0; i < NB; i++) ord_step2(acc[i], x[j].z, x[j].w, bf[i], w[j].y);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    x[j] = xn[j];
+                    w[j] = wn[j];
+                }
+            }
+        }
+    }
+    cp_async_wait<0>();
+    if (worker) {
+        float* row = vals + (long)(v + 1) * kOrdW * L + k0 + k;
+#pragma unroll
+        for (int i = 0; i < NB; i++) {
+            if (g * NB + i >= kRes) break;
+            const float2 r = unpack2(acc[i]);
+            row[(long)(g * NB + i) * L] = r.x;
+            row[(long)(kRes + g * NB + i) * L] = r.y;
+        }
+    }
+}
+
+// Splat of the short lists (order: those past the long ones; null: every list), one
+// thread per (vertex, label), both passes in registers: lower bin 0
 // and upper bin 9 take every entry, the other 18 bins an FMA with a mask of
 // exactly 0 or 1 (fma(1, w, acc) is acc + w rounded once).  Also clears the
 // absent neighbour's row in both buffers.
-__global__ void ord_dense_splat_kernel(int M, int L, const int* __restrict__ seg_start, const int2* __restrict__ seg,
+__global__ void ord_dense_splat_kernel(int n_short, int L, const int* __restrict__ order,
+                                       const int* __restrict__ seg_start, const int2* __restrict__ seg,
                                        const float2* __restrict__ bins, float* __restrict__ vals,
                                        float* __restrict__ other) {
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     for (long z = t; z < (long)kOrdW * L; z += (long)gridDim.x * blockDim.x) vals[z] = other[z] = 0.0f;
-    if (t >= (long)M * L) return;
-    const int v = (int)(t / L), k = (int)(t - (long)v * L);
+    if (t >= (long)n_short * L) return;
+    const int u = (int)(t / L), k = (int)(t - (long)u * L), v = order ? order[u] : u;
     const int s0 = seg_start[v], s1 = seg_start[v + 1];
     float lo[kRes], up[kRes];
 #pragma unroll
@@ -1360,34 +1572,54 @@ __global__ void __launch_bounds__(kTB, 8)
     }
     out[t] = apply_epilogue(acc, t, i, k, ep);
 }
-
-// One entry into the bin-b pair (lower, upper) of packed accumulators:
-// acc = fma({[cl >= b], [b >= cu]}, w2, acc) with one f32x2 FMA, which rounds
-// each half exactly as fma.rn.f32 does.  w2 holds (w, w).  The bins are
-// small integers, so the masks are saturated sums: cl + (1 - b) and
-// (b + 1) - cu are exact integers, clamped to [0, 1] they are exactly the
-// comparisons (and a NaN would clamp to +0).  One `add.sat` per mask.
-__device__ __forceinline__ void ord_step2(unsigned long long& acc, float cl, float cu, float b,
-                                          unsigned long long w2) {
-    const float lo_c = 1.0f - b, up_c = b + 1.0f;  // exact; hoisted out of the entry loops
-    asm("{\n\t.reg .f32 ml, mu;\n\t.reg .b64 m;\n\t"
-        "add.rn.sat.f32 ml, %1, %3;\n\t"
-        "sub.rn.sat.f32 mu, %4, %2;\n\t"
-        "mov.b64 m, {ml, mu};\n\t"
-        "fma.rn.f32x2 %0, m, %5, %0;\n\t}"
-        : "+l"(acc)
-        : "f"(cl), "f"(cu), "f"(lo_c), "f"(up_c), "l"(w2));
-}
 }  // namespace
 
-// Whether a single filter takes the dense form: two features at most, no long
-// list and more than 2^19 (pixel, label) values.  Three calls in flight, the
-// quad form -> the dense one, us: d = 2, 21 labels, 640x480 215 -> 178, 300x200
-// 44.2 -> 31.6, 554x90 33.1 -> 26.6; 640x480 with 3 labels 56.2 -> 30.1; below the line,
-// 200x150 with 21 labels 21.9 -> 21.1, 320x240 with 2 labels 16.2 -> 18.7.
-// More features have long lists of mostly empty bins, where the quad form wins
-// (d = 5, 640x480, one call after the other: 340 -> 274).  The LP's fused slice needs the quad form.
-bool Lattice::ord_dense(int L) const { return d <= 2 && n_long == 0 && (long)N * L > 1L << 19; }
+void Lattice::ensure_aux() {
+    if (aux) return;
+    int lo = 0, hi = 0;
+    DCRF_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+    DCRF_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
+    DCRF_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
+    DCRF_CUDA(cudaStreamCreateWithPriority(&aux, cudaStreamNonBlocking, hi));
+}
+
+Lattice::~Lattice() {
+    if (aux) {
+        cudaStreamSynchronize(aux);
+        cudaStreamDestroy(aux);
+    }
+    if (ev_join) cudaEventDestroy(ev_join);
+    if (ev_fork) cudaEventDestroy(ev_fork);
+}
+
+// Whether a single filter takes the dense form (the LP's fused slice needs the
+// quad form).  The lines lie where the two cross on a solver's kind of values
+// (softmax of normal logits); one call after the other, us, quad form -> dense.
+//   No long list, two features at most: from 2^19 (pixel, label) values or 2^18
+//   pixels on; from 20 labels on where there are pixels to fill the chip, and
+//   above 28 labels, whose masks are read in a loop.  640x480 with one label 59 ->
+//   37, 21 labels 205 -> 207, and 215 -> 178 with three calls in flight; 160x120
+//   with 22 labels 41.5 -> 39.9, 97x83 with 32 49 -> 36; below the lines 320x240
+//   with 2 labels 29 -> 34, 97x83 with 21 30 -> 37.
+//   Else the quad form wins where long lists leave most quads empty (five
+//   features, 640x480, 21 labels 272 -> 362), and loses with few labels: a list's
+//   sums fill few lanes (640x480: 2 labels 143 -> 107, 8 192 -> 182, 12 232 ->
+//   231, 16 259 -> 289; 320x240, whose splat does not fill the chip: 12 labels
+//   123 -> 112, 20 146 -> 142, 26 180 -> 207; smaller ones win throughout), and a
+//   vertex's mask costs its blur a warp whatever the labels: a noisy image
+//   640x480, 650 thousand vertices, one label 1186 -> 254, 21 labels 3918 -> 3638,
+//   28 4728 -> 4923; 97x83, 25 thousand, 4 labels 66 -> 55, 12 70 -> 82.
+// On evenly spread values, where all quads exist, the quad form loses everywhere
+// (five features, 640x480, 21 labels 379 -> 350): a single filter of those is
+// slower than the dense form would be.
+bool Lattice::ord_dense(int L) const {
+    if (n_long && L > kOrdBlockMaxL) return false;
+    if (d <= 2 && n_long == 0)
+        return (long)N * L > 1L << 19 || N > 1 << 18 || L > 28 || (L >= 20 && N >= 1 << 14);
+    const bool long_lists = (long)N * (d + 1) >= 32L * M;  // on average
+    const int by_lists = !long_lists ? 0 : N > 1 << 18 ? 12 : N > 1 << 16 ? 20 : 0;
+    return L <= std::max((double)by_lists, 4.0 * std::log2((double)M) - 50.0);
+}
 
 void Lattice::compute_ord_dense(float* out, const float* Q, int L, const SliceEpilogue& ep) {
     const size_t row = (size_t)L * kOrdW;
@@ -1397,8 +1629,39 @@ void Lattice::compute_ord_dense(float* out, const float* Q, int L, const SliceEp
     float2* bins = own(r_ebins, (size_t)NL);
     pair_bins(bins, Q, NL, st);
     float *src = va.get(), *dst = vb.get();
-    launch(ord_dense_splat_kernel, ceil_div((long)M * L, kTB), kTB, 0, st, M, L, (const int*)seg_start.get(),
-           (const int2*)seg.get(), (const float2*)bins, src, dst);
+    const int n_short = M - n_long;
+    auto long_lists = [&](int G, int kb, int first, int count, cudaStream_t ls) {
+        if (count <= 0) return;
+        const int kblocks = (L + kb - 1) / kb;
+        const size_t smem = ord_block_smem(kb);
+        auto kern = G == 10 ? ord_dense_long_kernel<10>
+                  : G == 5  ? ord_dense_long_kernel<5>
+                  : G == 3  ? ord_dense_long_kernel<3>
+                  : G == 2  ? ord_dense_long_kernel<2>
+                            : ord_dense_long_kernel<1>;
+        // an attribute of the kernel that all threads share: always its largest size
+        if (smem > 48 * 1024)
+            DCRF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)ord_block_smem(kOrdBlockMaxL)));
+        launch(kern, count * kblocks, (kb * G + 31) / 32 * 32, smem, ls, L, kb, kblocks,
+               (const int*)vorder.get() + first, (const int*)seg_start.get(), (const int2*)seg.get(),
+               (const float2*)bins, src);
+    };
+    // The very long lists set the length of their kernel and leave most SMs
+    // idle: on a stream of their own, joined before the blur, beside the others
+    // (other rows of src).
+    if (n_huge) {
+        ensure_aux();
+        DCRF_CUDA(cudaEventRecord(ev_fork, st));
+        DCRF_CUDA(cudaStreamWaitEvent(aux, ev_fork, 0));
+        long_lists(10, std::min(L, kHugeLabels), 0, n_huge, aux);
+        DCRF_CUDA(cudaEventRecord(ev_join, aux));
+    }
+    if (n_long > n_huge) long_lists(ord_groups_cheapest(L), L, n_huge, n_long - n_huge, st);
+    launch(ord_dense_splat_kernel, std::max(1, ceil_div((long)n_short * L, kTB)), kTB, 0, st, n_short, L,
+           n_long ? (const int*)vorder.get() + n_long : nullptr, (const int*)seg_start.get(), (const int2*)seg.get(),
+           (const float2*)bins, src, dst);
+    if (n_huge) DCRF_CUDA(cudaStreamWaitEvent(st, ev_join, 0));
     const int row4 = (int)(row / 4);
     for (int j = 0; j <= d; j++) {
         launch(row4 == 105 ? ord_dense_blur_kernel<105> : ord_dense_blur_kernel<0>, ceil_div((long)M * row4, kTB), kTB,
