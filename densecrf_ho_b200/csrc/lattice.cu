@@ -1059,13 +1059,13 @@ __global__ void slice_kernel(int N, int Lrt, int drt, const int* __restrict__ of
 // alpha) * value_j, from +0.
 // DOT: `out` is not written; the warp's FP64 sum of dot[e] * v[e] goes to
 // partials[warp] instead.
-// A row's first group has a 64-bit index (value buffers of 34 GB have 2^31
-// groups); with Q at compile time it is staged as an unsigned product, which
-// holds below 2^32 groups (staged_rows) and spares the gathers a multiplication
-// each: 16 images of 512x512 50.4 ms against 50.6, 64 images' QP 27.8 against 28.1.
+// S32: a row's first group (row times Q) is staged as an unsigned product, below
+// 2^32 groups (staged_rows); value buffers of 69 GB take the kernel that stages
+// the row and multiplies at the gather in 64 bits (the whole filter, 320x240, three
+// features, 12 labels: 80 us staged, 86 multiplied).
 constexpr int kSliceWarps = 4;
 constexpr int kSliceTile = 20;  // pixels per warp tile (4 rounds of 5 at L = 21)
-template <int DC, int Q, int LC, bool DOT>
+template <int DC, int Q, int LC, bool DOT, bool S32 = true>
 __global__ void __launch_bounds__(32 * kSliceWarps)
     slice_rows_kernel(int N, int Lrt, int Qrt, int drt, int tile, const int* __restrict__ offset,
                       const float* __restrict__ bary, const float4* __restrict__ vals, float alpha, float* out,
@@ -1102,7 +1102,7 @@ __global__ void __launch_bounds__(32 * kSliceWarps)
         }
         cp_async_commit();
         for (int e = lane; e < np * d1; e += 32)
-            s_ow[e] = make_int2((int)((unsigned)(offset[p0 * d1 + e] + 1) * (Q ? Q : 1)),
+            s_ow[e] = make_int2((int)((unsigned)(offset[p0 * d1 + e] + 1) * (S32 ? Qn : 1)),
                                 __float_as_int(fmul(bary[p0 * d1 + e], alpha)));
         if (use_norm)
             for (int e = lane; e < np; e += 32) s_nrm[e] = ep.norm[p0 + e];
@@ -1113,7 +1113,7 @@ __global__ void __launch_bounds__(32 * kSliceWarps)
             const float4* vq = vals + q;
             unsigned long long a0 = 0ull, a1 = 0ull;
             auto add = [&](int2 e) {
-                const long row = Q ? (long)(unsigned)e.x : (long)e.x * Qn;
+                const long row = S32 ? (long)(unsigned)e.x : (long)e.x * Qn;
                 const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(vq + row);
                 const float wa = __int_as_float(e.y);
                 a0 = add_mul2(a0, wa, v.x);
@@ -1935,8 +1935,9 @@ void Lattice::slice(float* out, int L, const SliceEpilogue& ep) {
                            L, Q, d, tile, offset.get(), bary.get(), reinterpret_cast<const float4*>(src), alpha, out,
                            ep, live_of(kDomTile), pix_base, vec, (const float*)nullptr, (double*)nullptr);
         };
-        const bool l21 = L == 21 && staged_rows(M, Q);
-        if (d == 5 && l21) sl(slice_rows_kernel<5, 6, 21, false>);
+        const bool l21 = L == 21;
+        if (!staged_rows(M, Q)) sl(slice_rows_kernel<0, 0, 0, false, false>);
+        else if (d == 5 && l21) sl(slice_rows_kernel<5, 6, 21, false>);
         else if (d == 2 && l21) sl(slice_rows_kernel<2, 6, 21, false>);
         else if (d == 5) sl(slice_rows_kernel<5, 0, 0, false>);
         else if (d == 2) sl(slice_rows_kernel<2, 0, 0, false>);
@@ -1958,8 +1959,9 @@ int Lattice::slice_dot(const float* dot, double* partials, int L, const SliceEpi
                        tile, offset.get(), bary.get(), reinterpret_cast<const float4*>(plain_vals), alpha,
                        (float*)nullptr, ep, Live{}, (const long*)nullptr, (int)aligned16(dot), dot, partials);
     };
-    const bool l21 = L == 21 && staged_rows(M, Q);
-    if (d == 5 && l21) sl(slice_rows_kernel<5, 6, 21, true>);
+    const bool l21 = L == 21;
+    if (!staged_rows(M, Q)) sl(slice_rows_kernel<0, 0, 0, true, false>);
+    else if (d == 5 && l21) sl(slice_rows_kernel<5, 6, 21, true>);
     else if (d == 2 && l21) sl(slice_rows_kernel<2, 6, 21, true>);
     else sl(slice_rows_kernel<0, 0, 0, true>);
     DCRF_LAUNCH_CHECK();
