@@ -1059,13 +1059,13 @@ __global__ void slice_kernel(int N, int Lrt, int drt, const int* __restrict__ of
 // alpha) * value_j, from +0.
 // DOT: `out` is not written; the warp's FP64 sum of dot[e] * v[e] goes to
 // partials[warp] instead.
-// S32: a row's first group (row times Q) is staged as an unsigned product, below
-// 2^32 groups (staged_rows); value buffers of 69 GB take the kernel that stages
-// the row and multiplies at the gather in 64 bits (the whole filter, 320x240, three
-// features, 12 labels: 80 us staged, 86 multiplied).
+// A row's first group (row times Q) is staged as an unsigned product: two value
+// buffers of 2^32 groups, 64 GiB each, do not fit the device, and a 64-bit
+// multiplication at the gather costs (the whole filter, 320x240, three features,
+// 12 labels: 80 us staged, 86 multiplied).
 constexpr int kSliceWarps = 4;
 constexpr int kSliceTile = 20;  // pixels per warp tile (4 rounds of 5 at L = 21)
-template <int DC, int Q, int LC, bool DOT, bool S32 = true>
+template <int DC, int Q, int LC, bool DOT>
 __global__ void __launch_bounds__(32 * kSliceWarps)
     slice_rows_kernel(int N, int Lrt, int Qrt, int drt, int tile, const int* __restrict__ offset,
                       const float* __restrict__ bary, const float4* __restrict__ vals, float alpha, float* out,
@@ -1102,7 +1102,7 @@ __global__ void __launch_bounds__(32 * kSliceWarps)
         }
         cp_async_commit();
         for (int e = lane; e < np * d1; e += 32)
-            s_ow[e] = make_int2((int)((unsigned)(offset[p0 * d1 + e] + 1) * (S32 ? Qn : 1)),
+            s_ow[e] = make_int2((int)((unsigned)(offset[p0 * d1 + e] + 1) * Qn),
                                 __float_as_int(fmul(bary[p0 * d1 + e], alpha)));
         if (use_norm)
             for (int e = lane; e < np; e += 32) s_nrm[e] = ep.norm[p0 + e];
@@ -1113,7 +1113,7 @@ __global__ void __launch_bounds__(32 * kSliceWarps)
             const float4* vq = vals + q;
             unsigned long long a0 = 0ull, a1 = 0ull;
             auto add = [&](int2 e) {
-                const long row = S32 ? (long)(unsigned)e.x : (long)e.x * Qn;
+                const long row = (long)(unsigned)e.x;
                 const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(vq + row);
                 const float wa = __int_as_float(e.y);
                 a0 = add_mul2(a0, wa, v.x);
@@ -1690,8 +1690,6 @@ static int slice_tile_max(int tile, int d, int L) {
 // Whether four warps' tiles of one pixel fit a block's 48 KB: up to some 3050
 // labels.  Only a lattice's own calls can have more (a model's limit is 64).
 static bool row_tiles(int d, int L) { return kSliceWarps * slice_warp_bytes(1, d, L) <= (48 << 10); }
-// Whether the rows' groups can be counted in 32 bits.
-static bool staged_rows(int M, int Q) { return (long)(M + 1) * Q < 1L << 32; }
 static dim3 wide_grid(int N, int Q) { return dim3(ceil_div(Q, kTB), std::min(N, 65535)); }
 
 // The splat without the padded rows, into rows of Lp floats.
@@ -1876,6 +1874,8 @@ void Lattice::ensure_ord_totals() {
 void Lattice::splat_blur(const float* in, int L, bool reverse, const float* pre_norm) {
     require(L >= 1, DCRF_E_ARG, "compute: L must be >= 1");
     const int Lp = value_row(L);
+    // slice_rows_kernel's row index; ensure_values would find no memory either
+    require((long)(M + 1) * (Lp / 4) < 1L << 32, DCRF_E_NOMEM, "compute: value buffers over 64 GiB");
     ensure_values((size_t)Lp);
     if (L == 21 && shape_L != L) tune_shape(L);
     cudaStream_t st = stream;
@@ -1936,8 +1936,7 @@ void Lattice::slice(float* out, int L, const SliceEpilogue& ep) {
                            ep, live_of(kDomTile), pix_base, vec, (const float*)nullptr, (double*)nullptr);
         };
         const bool l21 = L == 21;
-        if (!staged_rows(M, Q)) sl(slice_rows_kernel<0, 0, 0, false, false>);
-        else if (d == 5 && l21) sl(slice_rows_kernel<5, 6, 21, false>);
+        if (d == 5 && l21) sl(slice_rows_kernel<5, 6, 21, false>);
         else if (d == 2 && l21) sl(slice_rows_kernel<2, 6, 21, false>);
         else if (d == 5) sl(slice_rows_kernel<5, 0, 0, false>);
         else if (d == 2) sl(slice_rows_kernel<2, 0, 0, false>);
@@ -1960,8 +1959,7 @@ int Lattice::slice_dot(const float* dot, double* partials, int L, const SliceEpi
                        (float*)nullptr, ep, Live{}, (const long*)nullptr, (int)aligned16(dot), dot, partials);
     };
     const bool l21 = L == 21;
-    if (!staged_rows(M, Q)) sl(slice_rows_kernel<0, 0, 0, true, false>);
-    else if (d == 5 && l21) sl(slice_rows_kernel<5, 6, 21, true>);
+    if (d == 5 && l21) sl(slice_rows_kernel<5, 6, 21, true>);
     else if (d == 2 && l21) sl(slice_rows_kernel<2, 6, 21, true>);
     else sl(slice_rows_kernel<0, 0, 0, true>);
     DCRF_LAUNCH_CHECK();
