@@ -18,11 +18,15 @@ struct dcrf_lattice_s {
     cudaStream_t stream = nullptr;
     DevBuf<float> feat, in, out;
     DevBuf<int> ipi;
+    template <typename T>
+    T* own(DevBuf<T>& b, size_t n) { return lat.own(b, n); }
 };
 
 struct dcrf_batch_s {
     dcrf::Batch* b = nullptr;
     DevBuf<float> io0, io1, feat;
+    template <typename T>
+    T* own(DevBuf<T>& buffer, size_t n) { return b->own(buffer, n); }
 };
 
 struct dcrf_model_s {
@@ -31,6 +35,8 @@ struct dcrf_model_s {
     DevBuf<int> ipi;
     DevBuf<uint8_t> img;
     DevBuf<int16_t> lab;
+    template <typename T>
+    T* own(DevBuf<T>& b, size_t n) { return m->own(b, n); }
 };
 
 namespace {
@@ -66,9 +72,10 @@ void check_device() {
         throw Error(DCRF_E_CUDA, std::string("no usable CUDA device: ") + cudaGetErrorString(e));
 }
 
-template <typename T>
-T* upload(DevBuf<T>& b, const T* h, size_t n, cudaStream_t st) {
-    T* d = b.ensure(n);
+// To a buffer of the handle.
+template <typename H, typename T>
+T* upload(H handle, DevBuf<T>& b, const T* h, size_t n, cudaStream_t st) {
+    T* d = handle->own(b, n);
     DCRF_CUDA(cudaMemcpyAsync(d, h, sizeof(T) * n, cudaMemcpyHostToDevice, st));
     return d;
 }
@@ -157,7 +164,7 @@ dcrf_status dcrf_lattice_init(dcrf_lattice h, const float* features, int d, int 
         need(h, "lattice");
         need(features, "features");
         if (d < 1 || N < 1) throw Error(DCRF_E_ARG, "invalid feature shape");
-        const float* df = upload(h->feat, features, (size_t)d * N, h->stream);
+        const float* df = upload(h, h->feat, features, (size_t)d * N, h->stream);
         h->lat.build(df, d, N);
         DCRF_CUDA(cudaStreamSynchronize(h->stream));
     });
@@ -201,8 +208,8 @@ dcrf_status dcrf_lattice_compute(dcrf_lattice h, float* out, const float* in, in
         if (h->lat.N == 0) throw Error(DCRF_E_STATE, "lattice not initialised");
         if (L < 1) throw Error(DCRF_E_ARG, "L must be >= 1");
         const size_t n = (size_t)L * h->lat.N;
-        float* di = upload(h->in, in, n, h->stream);
-        float* dout = h->out.ensure(n);
+        float* di = upload(h, h->in, in, n, h->stream);
+        float* dout = h->own(h->out, n);
         dcrf::SliceEpilogue ep;
         h->lat.compute(dout, di, L, reverse != 0, ep);
         download(out, dout, n, h->stream);
@@ -229,9 +236,9 @@ dcrf_status dcrf_lattice_gradient(dcrf_lattice h, float* df, const float* a, con
         if (h->lat.N == 0) throw Error(DCRF_E_STATE, "lattice not initialised");
         if (L < 1) throw Error(DCRF_E_ARG, "L must be >= 1");
         const size_t n = (size_t)L * h->lat.N;
-        float* da = upload(h->in, a, n, h->stream);
-        float* db = upload(h->feat, b, n, h->stream);
-        float* ddf = h->out.ensure((size_t)h->lat.N * h->lat.d);
+        float* da = upload(h, h->in, a, n, h->stream);
+        float* db = upload(h, h->feat, b, n, h->stream);
+        float* ddf = h->own(h->out, (size_t)h->lat.N * h->lat.d);
         h->lat.gradient(ddf, da, db, L);
         download(df, ddf, (size_t)h->lat.N * h->lat.d, h->stream);
     });
@@ -258,8 +265,8 @@ dcrf_status dcrf_lattice_compute_ord(dcrf_lattice h, float* out, const float* Q,
         const size_t n = (size_t)L * h->lat.N;
         for (size_t i = 0; i < n; i++)  // the reference asserts 0 <= Q <= 1 here
             if (!(Q[i] >= 0.0f && Q[i] <= 1.0f)) throw Error(DCRF_E_RANGE, "Value out of bounds");
-        float* dq = upload(h->in, Q, n, h->stream);
-        float* dout = h->out.ensure(n);
+        float* dq = upload(h, h->in, Q, n, h->stream);
+        float* dout = h->own(h->out, n);
         dcrf::SliceEpilogue ep;
         h->lat.compute_ord(dout, dq, L, ep);
         download(out, dout, n, h->stream);
@@ -295,10 +302,10 @@ dcrf_status dcrf_lattice_compute_ord_restricted(dcrf_lattice h, float* rout, con
         check_restricted(h->lat.N, L, pI, nP, rQ, Q, store);
         if (nP) need(rout, "rout");
         const size_t n = (size_t)nP * L;
-        const float* drq = n ? upload(h->in, rQ, n, h->stream) : nullptr;
-        const float* dq = store ? upload(h->feat, Q, (size_t)h->lat.N * L, h->stream) : nullptr;
-        const int* dpi = nP ? upload(h->ipi, pI, (size_t)nP, h->stream) : nullptr;
-        float* dout = h->out.ensure(std::max<size_t>(n, 1));
+        const float* drq = n ? upload(h, h->in, rQ, n, h->stream) : nullptr;
+        const float* dq = store ? upload(h, h->feat, Q, (size_t)h->lat.N * L, h->stream) : nullptr;
+        const int* dpi = nP ? upload(h, h->ipi, pI, (size_t)nP, h->stream) : nullptr;
+        float* dout = h->own(h->out, std::max<size_t>(n, 1));
         dcrf::SliceEpilogue ep;
         h->lat.compute_ord_restricted(dout, drq, dpi, nP, dq, L, store != 0, ep);
         if (n) download(rout, dout, n, h->stream);
@@ -431,7 +438,7 @@ dcrf_status dcrf_model_set_unary_dev(dcrf_model h, const float* d_unary) {
     return guard([&] {
         auto& m = M(h);
         need(d_unary, "unary");
-        float* u = m.unary.ensure((size_t)m.N * m.L);
+        float* u = m.own(m.unary, (size_t)m.N * m.L);
         DCRF_CUDA(cudaMemcpyAsync(u, d_unary, sizeof(float) * m.N * m.L, cudaMemcpyDeviceToDevice, m.stream));
         m.has_unary = true;
         m.logit_F = 0;  // a constant unary replaces the unary energy
@@ -443,7 +450,7 @@ dcrf_status dcrf_model_set_unary(dcrf_model h, const float* unary) {
     return guard([&] {
         auto& m = M(h);
         need(unary, "unary");
-        upload(m.unary, unary, (size_t)m.N * m.L, m.stream);
+        upload(h, m.unary, unary, (size_t)m.N * m.L, m.stream);
         m.has_unary = true;
         m.logit_F = 0;  // a constant unary replaces the unary energy
         m.gen++;
@@ -492,7 +499,7 @@ dcrf_status dcrf_model_unary_gradient(dcrf_model h, const float* b, float* grad,
         need(b, "b");
         if (n) *n = m.L * m.logit_F;
         if (m.logit_F == 0 || !grad) return;  // grad NULL: query the count
-        const float* db = upload(h->io0, b, (size_t)m.N * m.L, m.stream);
+        const float* db = upload(h, h->io0, b, (size_t)m.N * m.L, m.stream);
         m.unary_gradient(db, grad);
     });
 }
@@ -502,7 +509,7 @@ dcrf_status dcrf_model_add_pairwise(dcrf_model h, const float* features, int d, 
         auto& m = M(h);
         need(features, "features");
         if (d < 1 || d > 16) throw Error(DCRF_E_ARG, "feature dimension must be in [1, 16]");
-        const float* df = upload(h->feat, features, (size_t)d * m.N, m.stream);
+        const float* df = upload(h, h->feat, features, (size_t)d * m.N, m.stream);
         m.add_term(df, d, w_potts);
         m.sync();
     });
@@ -517,7 +524,7 @@ dcrf_status dcrf_model_add_gaussian(dcrf_model h, float sx, float sy, float w_po
                 f[2 * ((size_t)j * m.W + i)] = i / sx;
                 f[2 * ((size_t)j * m.W + i) + 1] = j / sy;
             }
-        const float* df = upload(h->feat, f.data(), f.size(), m.stream);
+        const float* df = upload(h, h->feat, f.data(), f.size(), m.stream);
         m.add_term(df, 2, w_potts);
         m.sync();
     });
@@ -538,7 +545,7 @@ dcrf_status dcrf_model_add_bilateral(dcrf_model h, float sx, float sy, float sr,
                 f[5 * p + 3] = rgb[3 * p + 1] / sg;
                 f[5 * p + 4] = rgb[3 * p + 2] / sb;
             }
-        const float* df = upload(h->feat, f.data(), f.size(), m.stream);
+        const float* df = upload(h, h->feat, f.data(), f.size(), m.stream);
         m.add_term(df, 5, w_potts);
         m.sync();
     });
@@ -703,7 +710,7 @@ dcrf_status dcrf_model_unary_init(dcrf_model h, float* Q) {
         auto& m = M(h);
         need(Q, "Q");
         const size_t n = (size_t)m.N * m.L;
-        float* d = h->io0.ensure(n);
+        float* d = h->own(h->io0, n);
         m.unary_init(d);
         download(Q, d, n, m.stream);
     });
@@ -726,8 +733,8 @@ dcrf_status dcrf_model_pairwise_apply(dcrf_model h, int k, int nonorm, float* ou
         need(out, "out");
         need(in, "in");
         const size_t n = (size_t)m.N * m.L;
-        float* di = upload(h->io0, in, n, m.stream);
-        float* dout = h->io1.ensure(n);
+        float* di = upload(h, h->io0, in, n, m.stream);
+        float* dout = h->own(h->io1, n);
         m.apply(k, nonorm != 0, dout, di);
         download(out, dout, n, m.stream);
     });
@@ -740,9 +747,9 @@ dcrf_status dcrf_model_pairwise_apply_ord(dcrf_model h, int k, float* out, const
         need(out, "out");
         need(Q, "Q");
         const size_t n = (size_t)m.N * m.L;
-        float* dq = upload(h->io0, Q, n, m.stream);
+        float* dq = upload(h, h->io0, Q, n, m.stream);
         m.check_unit_range(dq);
-        float* dout = h->io1.ensure(n);
+        float* dout = h->own(h->io1, n);
         m.apply_ord(k, dout, dq);
         download(out, dout, n, m.stream);
     });
@@ -756,10 +763,10 @@ dcrf_status dcrf_model_pairwise_apply_ord_restricted(dcrf_model h, int k, float*
         check_restricted(m.N, m.L, pI, nP, rQ, Q, store);
         if (nP) need(rout, "rout");
         const size_t n = (size_t)nP * m.L;
-        const float* drq = n ? upload(h->io0, rQ, n, m.stream) : nullptr;
-        const float* dq = store ? upload(h->io2, Q, (size_t)m.N * m.L, m.stream) : nullptr;
-        const int* dpi = nP ? upload(h->ipi, pI, (size_t)nP, m.stream) : nullptr;
-        float* dout = h->io1.ensure(std::max<size_t>(n, 1));
+        const float* drq = n ? upload(h, h->io0, rQ, n, m.stream) : nullptr;
+        const float* dq = store ? upload(h, h->io2, Q, (size_t)m.N * m.L, m.stream) : nullptr;
+        const int* dpi = nP ? upload(h, h->ipi, pI, (size_t)nP, m.stream) : nullptr;
+        float* dout = h->own(h->io1, std::max<size_t>(n, 1));
         m.apply_ord_restricted(k, dout, drq, dpi, nP, dq, store != 0);
         if (n) download(rout, dout, n, m.stream);
         else DCRF_CUDA(cudaStreamSynchronize(m.stream));
@@ -783,8 +790,8 @@ dcrf_status dcrf_model_pairwise_apply_bf(dcrf_model h, int k, int nonorm, float*
         need(out, "out");
         need(Q, "Q");
         const size_t n = (size_t)m.N * m.L;
-        const float* dq = upload(h->io0, Q, n, m.stream);
-        float* dout = h->io1.ensure(n);
+        const float* dq = upload(h, h->io0, Q, n, m.stream);
+        float* dout = h->own(h->io1, n);
         m.apply_bf(k, nonorm != 0, dout, dq);
         download(out, dout, n, m.stream);
     });
@@ -798,8 +805,8 @@ dcrf_status dcrf_model_pairwise_apply_upper_minus_lower_bf(dcrf_model h, int k, 
         need(out, "out");
         check_ind(m, ind);
         const size_t n = (size_t)m.N * m.L;
-        const int* di = upload(h->ipi, ind, n, m.stream);
-        float* dout = h->io1.ensure(n);
+        const int* di = upload(h, h->ipi, ind, n, m.stream);
+        float* dout = h->own(h->io1, n);
         m.apply_upper_minus_lower_bf(k, nonorm != 0, dout, di, nullptr);
         download(out, dout, n, m.stream);
     });
@@ -814,9 +821,9 @@ dcrf_status dcrf_model_pairwise_apply_upper_minus_lower_bf_ord(dcrf_model h, int
         need(Q, "Q");
         check_ind(m, ind);
         const size_t n = (size_t)m.N * m.L;
-        const int* di = upload(h->ipi, ind, n, m.stream);
-        const float* dq = upload(h->io0, Q, n, m.stream);
-        float* dout = h->io1.ensure(n);
+        const int* di = upload(h, h->ipi, ind, n, m.stream);
+        const float* dq = upload(h, h->io0, Q, n, m.stream);
+        float* dout = h->own(h->io1, n);
         m.apply_upper_minus_lower_bf(k, nonorm != 0, dout, di, dq);
         download(out, dout, n, m.stream);
     });
@@ -830,8 +837,8 @@ dcrf_status dcrf_model_pairwise_apply_upper_minus_lower_dc(dcrf_model h, int k, 
         need(out, "out");
         check_ind(m, ind);
         const size_t n = (size_t)m.N * m.L;
-        const int* di = upload(h->ipi, ind, n, m.stream);
-        float* dout = h->io1.ensure(n);
+        const int* di = upload(h, h->ipi, ind, n, m.stream);
+        float* dout = h->own(h->io1, n);
         m.apply_upper_minus_lower_dc(k, nonorm != 0, dout, di);
         download(out, dout, n, m.stream);
     });
@@ -862,8 +869,8 @@ dcrf_status dcrf_model_qp(dcrf_model h, const float* init, float* out, const dcr
         need(init, "init");
         need(out, "out");
         const size_t n = (size_t)m.N * m.L;
-        float* di = upload(h->io0, init, n, m.stream);
-        float* dout = h->io1.ensure(n);
+        float* di = upload(h, h->io0, init, n, m.stream);
+        float* dout = h->own(h->io1, n);
         const int max_iter = params ? params->max_iter : 0;
         if (max_iter < 0) throw Error(DCRF_E_ARG, "max_iter must be >= 0");
         double e = 0.0;
@@ -909,8 +916,8 @@ dcrf_status dcrf_model_lp(dcrf_model h, const float* init, float* out, const dcr
         else dcrf_lp_params_default(&p);
         check_lp_params(p);
         const size_t n = (size_t)m.N * m.L;
-        float* di = upload(h->io0, init, n, m.stream);
-        float* dout = h->io1.ensure(n);
+        float* di = upload(h, h->io0, init, n, m.stream);
+        float* dout = h->own(h->io1, n);
         dcrf_solve_stats s{};
         m.lp(di, dout, p, &s);
         download(out, dout, n, m.stream);
@@ -923,8 +930,8 @@ dcrf_status dcrf_model_current_map(dcrf_model h, const float* Q, int16_t* labels
         auto& m = M(h);
         need(Q, "Q");
         need(labels, "labels");
-        float* dq = upload(h->io0, Q, (size_t)m.N * m.L, m.stream);
-        int16_t* dl = h->lab.ensure(m.N);
+        float* dq = upload(h, h->io0, Q, (size_t)m.N * m.L, m.stream);
+        int16_t* dl = h->own(h->lab, m.N);
         m.current_map(dq, dl);
         download(labels, dl, m.N, m.stream);
     });
@@ -935,7 +942,7 @@ dcrf_status dcrf_model_energy_true(dcrf_model h, const int16_t* labels, double* 
         auto& m = M(h);
         need(labels, "labels");
         need(energy, "energy");
-        int16_t* dl = upload(h->lab, labels, m.N, m.stream);
+        int16_t* dl = upload(h, h->lab, labels, m.N, m.stream);
         *energy = m.energy_true(dl, false);
     });
 }
@@ -945,7 +952,7 @@ dcrf_status dcrf_model_energy_ho(dcrf_model h, const int16_t* labels, double* en
         auto& m = M(h);
         need(labels, "labels");
         need(energy, "energy");
-        int16_t* dl = upload(h->lab, labels, m.N, m.stream);
+        int16_t* dl = upload(h, h->lab, labels, m.N, m.stream);
         *energy = m.energy_true(dl, true);
     });
 }
@@ -955,7 +962,7 @@ dcrf_status dcrf_model_energy_lp(dcrf_model h, const float* Q, double* energy) {
         auto& m = M(h);
         need(Q, "Q");
         need(energy, "energy");
-        float* dq = upload(h->io0, Q, (size_t)m.N * m.L, m.stream);
+        float* dq = upload(h, h->io0, Q, (size_t)m.N * m.L, m.stream);
         *energy = m.energy_lp(dq);
     });
 }
@@ -965,7 +972,7 @@ dcrf_status dcrf_model_lr_qp_value(dcrf_model h, const float* Q, double* energy)
         auto& m = M(h);
         need(Q, "Q");
         need(energy, "energy");
-        float* dq = upload(h->io0, Q, (size_t)m.N * m.L, m.stream);
+        float* dq = upload(h, h->io0, Q, (size_t)m.N * m.L, m.stream);
         *energy = m.lr_qp_value(dq);
     });
 }
@@ -976,8 +983,8 @@ dcrf_status dcrf_model_lr_qp_value_diag(dcrf_model h, const float* Q, const floa
         need(Q, "Q");
         need(energy, "energy");
         const size_t n = (size_t)m.N * m.L;
-        float* dq = upload(h->io0, Q, n, m.stream);
-        const float* dd = diag_dom ? upload(h->io1, diag_dom, n, m.stream) : nullptr;
+        float* dq = upload(h, h->io0, Q, n, m.stream);
+        const float* dd = diag_dom ? upload(h, h->io1, diag_dom, n, m.stream) : nullptr;
         *energy = m.lr_qp_value(dq, dd);
     });
 }
@@ -987,7 +994,7 @@ dcrf_status dcrf_model_energy_higher_order(dcrf_model h, const float* Q, double*
         auto& m = M(h);
         need(Q, "Q");
         need(energy, "energy");
-        float* dq = upload(h->io0, Q, (size_t)m.N * m.L, m.stream);
+        float* dq = upload(h, h->io0, Q, (size_t)m.N * m.L, m.stream);
         *energy = m.energy_qp_ho(dq);
     });
 }
@@ -997,8 +1004,8 @@ dcrf_status dcrf_model_unary_energy(dcrf_model h, const int16_t* labels, float* 
         auto& m = M(h);
         need(labels, "labels");
         need(out, "out");
-        int16_t* dl = upload(h->lab, labels, m.N, m.stream);
-        float* dout = h->io1.ensure((size_t)m.N);
+        int16_t* dl = upload(h, h->lab, labels, m.N, m.stream);
+        float* dout = h->own(h->io1, (size_t)m.N);
         m.unary_energy(dl, dout);
         download(out, dout, (size_t)m.N, m.stream);
     });
@@ -1009,8 +1016,8 @@ dcrf_status dcrf_model_pairwise_energy(dcrf_model h, const int16_t* labels, int 
         auto& m = M(h);
         need(labels, "labels");
         need(out, "out");
-        int16_t* dl = upload(h->lab, labels, m.N, m.stream);
-        float* dout = h->io2.ensure((size_t)m.N);
+        int16_t* dl = upload(h, h->lab, labels, m.N, m.stream);
+        float* dout = h->own(h->io2, (size_t)m.N);
         m.pairwise_energy(dl, term, dout);
         download(out, dout, (size_t)m.N, m.stream);
     });
@@ -1022,7 +1029,7 @@ dcrf_status dcrf_model_max_rounding(dcrf_model h, const float* Q, float* out) {
         need(Q, "Q");
         need(out, "out");
         const size_t n = (size_t)m.N * m.L;
-        float* dq = upload(h->io0, Q, n, m.stream);
+        float* dq = upload(h, h->io0, Q, n, m.stream);
         m.max_rounding(dq, dq);
         download(out, dq, n, m.stream);
     });
@@ -1058,8 +1065,8 @@ dcrf_status dcrf_model_pairwise_kernel_gradient(dcrf_model h, int k, const float
         need(b, "b");
         need(Q, "Q");
         const size_t n = (size_t)m.N * m.L;
-        const float* db = upload(h->io0, b, n, m.stream);
-        const float* dq = upload(h->io1, Q, n, m.stream);
+        const float* db = upload(h, h->io0, b, n, m.stream);
+        const float* dq = upload(h, h->io1, Q, n, m.stream);
         m.kernel_gradient(k, db, dq, grad);
     });
 }
@@ -1072,8 +1079,8 @@ dcrf_status dcrf_model_pairwise_gradient(dcrf_model h, int k, const float* b, co
         need(Q, "Q");
         need(grad, "grad");
         const size_t n = (size_t)m.N * m.L;
-        const float* db = upload(h->io0, b, n, m.stream);
-        const float* dq = upload(h->io1, Q, n, m.stream);
+        const float* db = upload(h, h->io0, b, n, m.stream);
+        const float* dq = upload(h, h->io1, Q, n, m.stream);
         m.compat_gradient(k, db, dq, grad);
     });
 }
@@ -1149,7 +1156,7 @@ dcrf_status dcrf_batch_set_unary_dev(dcrf_batch h, const float* d_unary) {
     return guard([&] {
         auto& b = BT(h);
         need(d_unary, "unary");
-        float* u = b.unary.ensure((size_t)b.Ntot * b.L);
+        float* u = b.own(b.unary, (size_t)b.Ntot * b.L);
         b.unary_gen++;
         DCRF_CUDA(cudaMemcpyAsync(u, d_unary, sizeof(float) * b.Ntot * b.L, cudaMemcpyDeviceToDevice, b.stream));
         b.has_unary = true;
@@ -1160,7 +1167,7 @@ dcrf_status dcrf_batch_set_unary(dcrf_batch h, const float* unary) {
     return guard([&] {
         auto& b = BT(h);
         need(unary, "unary");
-        upload(b.unary, unary, (size_t)b.Ntot * b.L, b.stream);
+        upload(h, b.unary, unary, (size_t)b.Ntot * b.L, b.stream);
         b.unary_gen++;
         DCRF_CUDA(cudaStreamSynchronize(b.stream));
         b.has_unary = true;
@@ -1178,7 +1185,7 @@ dcrf_status dcrf_batch_add_gaussian(dcrf_batch h, float sx, float sy, float w_po
                     f[2 * p] = i / sx;
                     f[2 * p + 1] = j / sy;
                 }
-        const float* df = upload(h->feat, f.data(), f.size(), b.stream);
+        const float* df = upload(h, h->feat, f.data(), f.size(), b.stream);
         b.add_term(df, 2, w_potts);
         DCRF_CUDA(cudaStreamSynchronize(b.stream));
     });
@@ -1200,7 +1207,7 @@ dcrf_status dcrf_batch_add_bilateral(dcrf_batch h, float sx, float sy, float sr,
                     f[5 * p + 3] = rgb[3 * p + 1] / sg;
                     f[5 * p + 4] = rgb[3 * p + 2] / sb;
                 }
-        const float* df = upload(h->feat, f.data(), f.size(), b.stream);
+        const float* df = upload(h, h->feat, f.data(), f.size(), b.stream);
         b.add_term(df, 5, w_potts);
         DCRF_CUDA(cudaStreamSynchronize(b.stream));
     });
@@ -1211,7 +1218,7 @@ dcrf_status dcrf_batch_unary_init(dcrf_batch h, float* Q) {
         auto& b = BT(h);
         need(Q, "Q");
         const size_t n = (size_t)b.Ntot * b.L;
-        float* d = h->io0.ensure(n);
+        float* d = h->own(h->io0, n);
         b.unary_init(d);
         download(Q, d, n, b.stream);
     });
@@ -1249,8 +1256,8 @@ dcrf_status dcrf_batch_qp(dcrf_batch h, const float* init, float* out, const dcr
         need(init, "init");
         need(out, "out");
         const size_t n = (size_t)b.Ntot * b.L;
-        float* di = upload(h->io0, init, n, b.stream);
-        float* dout = h->io1.ensure(n);
+        float* di = upload(h, h->io0, init, n, b.stream);
+        float* dout = h->own(h->io1, n);
         batch_qp(b, di, dout, params, stats);
         download(out, dout, n, b.stream);
     });
@@ -1264,7 +1271,7 @@ dcrf_status dcrf_batch_meanfield(dcrf_batch h, int iterations, float* Q) {
     return guard([&] {
         auto& b = BT(h);
         const size_t n = (size_t)b.Ntot * b.L;
-        float* d = Q ? h->io1.ensure(n) : nullptr;
+        float* d = Q ? h->own(h->io1, n) : nullptr;
         b.meanfield(iterations, d);
         if (Q) download(Q, d, n, b.stream);
         DCRF_CUDA(cudaStreamSynchronize(b.stream));
@@ -1289,8 +1296,8 @@ dcrf_status dcrf_batch_meanfield_backward(dcrf_batch h, const float* grad_Q, flo
         need(grad_U, "grad_U");
         if (!b.terms.empty()) need(grad_w, "grad_w");
         const size_t n = (size_t)b.Ntot * b.L;
-        const float* dg = upload(h->io0, grad_Q, n, b.stream);
-        float* du = h->io1.ensure(n);
+        const float* dg = upload(h, h->io0, grad_Q, n, b.stream);
+        float* du = h->own(h->io1, n);
         b.meanfield_backward(dg, du, grad_w);
         download(grad_U, du, n, b.stream);
     });
@@ -1336,8 +1343,8 @@ dcrf_status dcrf_batch_pairwise_apply(dcrf_batch h, int k, float* out, const flo
         need(in, "in");
         dcrf::require(k >= 0 && k < (int)b.terms.size(), DCRF_E_ARG, "pairwise term index out of range");
         const size_t n = (size_t)b.Ntot * b.L;
-        upload(h->io0, in, n, b.stream);
-        float* d = h->io1.ensure(n);
+        upload(h, h->io0, in, n, b.stream);
+        float* d = h->own(h->io1, n);
         b.apply(k, d, h->io0.get());
         download(out, d, n, b.stream);
         DCRF_CUDA(cudaStreamSynchronize(b.stream));

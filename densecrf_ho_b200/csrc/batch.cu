@@ -646,17 +646,18 @@ Batch::~Batch() {
 void Batch::build_lattice(Term& t) {
     auto lat = std::make_unique<Lattice>();  // the term's once it is complete
     lat->stream = stream;
+    lat->give_back_others = [this] { return give_back(); };
     std::vector<std::unique_ptr<Lattice>> parts;
     std::vector<const Lattice*> views;
     for (int i = 0; i < B; i++) {
         auto p = std::make_unique<Lattice>();
         p->stream = stream;
+        p->give_back_others = lat->give_back_others;
         p->build(t.feat.get() + pix_off[i] * t.d, t.d, W[i] * H[i]);
         views.push_back(p.get());
         parts.push_back(std::move(p));
     }
     lat->concat(views);
-    lat->give_back_others = [this] { return give_back_rows(); };
     t.lat = std::move(lat);
 }  // the per-image lattices are released here
 
@@ -669,12 +670,12 @@ void Batch::add_term(const float* d_features, int d, float w) {
     weights_gen++;
     ensure_lattices();
     auto t = std::make_unique<Term>();
-    DCRF_CUDA(cudaMemcpyAsync(t->feat.ensure((size_t)Ntot * d), d_features, sizeof(float) * Ntot * d,
+    DCRF_CUDA(cudaMemcpyAsync(own(t->feat, (size_t)Ntot * d), d_features, sizeof(float) * Ntot * d,
                               cudaMemcpyDeviceToDevice, stream));
     t->d = d;
     build_lattice(*t);
     t->w = w;
-    float* nrm = t->norm.ensure(Ntot);
+    float* nrm = own(t->norm, Ntot);
     launch(bfill_kernel, ceil_div(Ntot, 256), 256, 0, stream, Ntot, 1.0f, nrm);
     SliceEpilogue ep;
     t->lat->compute(nrm, nrm, 1, false, ep);

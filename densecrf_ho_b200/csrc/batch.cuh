@@ -41,15 +41,15 @@ struct Batch {
     Batch(int n, const int* widths, const int* heights, int L_);
     ~Batch();
 
-    // A buffer of the batch; its lattices' padded rows go first where memory is short.
+    // A buffer of the batch; what its lattices can do without goes first where memory is short.
     template <typename T>
     T* own(DevBuf<T>& buffer, size_t count) {
-        return ensure_after(buffer, count, [&] { return give_back_rows(); });
+        return ensure_after(buffer, count, [&] { return give_back(); });
     }
-    bool give_back_rows() {
+    bool give_back() {
         bool any = false;
         for (auto& t : terms)
-            if (t->lat) any |= t->lat->give_back_rows();
+            if (t->lat) any |= t->lat->give_back();
         return any;
     }
     float* buf(int i) { return own(b[i], (size_t)Ntot * L); }

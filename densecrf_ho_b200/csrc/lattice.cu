@@ -1060,9 +1060,9 @@ __global__ void slice_kernel(int N, int Lrt, int drt, const int* __restrict__ of
 // DOT: `out` is not written; the warp's FP64 sum of dot[e] * v[e] goes to
 // partials[warp] instead.
 // A row's first group (row times Q) is staged as an unsigned product: two value
-// buffers of 2^32 groups, 64 GiB each, do not fit the device, and a 64-bit
-// multiplication at the gather costs (the whole filter, 320x240, three features,
-// 12 labels: 80 us staged, 86 multiplied).
+// buffers of more than 2^32 groups (64 GiB, in blocks of 96) do not fit the
+// device, and a 64-bit multiplication at the gather costs (the whole filter,
+// 320x240, three features, 12 labels: 80 us staged, 86 multiplied).
 constexpr int kSliceWarps = 4;
 constexpr int kSliceTile = 20;  // pixels per warp tile (4 rounds of 5 at L = 21)
 template <int DC, int Q, int LC, bool DOT>
@@ -1458,10 +1458,9 @@ void Lattice::visiting_order(int (&nl)[2]) {
     DCRF_CUDA(cudaStreamSynchronize(stream));
 }
 
-void Lattice::concat(const std::vector<const Lattice*>& parts) {
+void Lattice::concat_parts(const std::vector<const Lattice*>& parts) {
     require(!parts.empty(), DCRF_E_ARG, "lattice concat: no parts");
     cudaStream_t st = stream;
-    forget();
     d = parts[0]->d;
     const int d1 = d + 1;
     long Nt = 0, Mt = 0;
@@ -1570,18 +1569,58 @@ void Lattice::prepare_live(int L) {
 void Lattice::build(const float* d_features, int d_, int N_) {
     require(N_ > 0, DCRF_E_ARG, "lattice: N must be positive");
     require(d_ >= 1 && d_ <= 16, DCRF_E_ARG, "lattice: feature dimension must be in [1, 16]");
-    forget();
-    N = N_;
-    d = d_;
-    try {
+    build_in([&] {
+        N = N_;
+        d = d_;
         if (d <= 2) build_impl<2>(*this, d_features);
         else if (d <= 5) build_impl<5>(*this, d_features);
         else if (d <= 8) build_impl<8>(*this, d_features);
         else build_impl<16>(*this, d_features);
-    } catch (...) {
-        forget();
-        throw;
+    });
+}
+
+void Lattice::concat(const std::vector<const Lattice*>& parts) {
+    build_in([&] { concat_parts(parts); });
+}
+
+template <typename F>
+void Lattice::build_in(F&& build) {
+    forget();
+    for (bool again = false;; again = true) {
+        try {
+            build();
+            return;
+        } catch (const Error& e) {
+            forget();
+            if (again || e.code != DCRF_E_NOMEM ||
+                !(give_back() | give_back_quads() | (give_back_others && give_back_others())))
+                throw;
+            cudaGetLastError();
+        } catch (...) {
+            forget();
+            throw;
+        }
     }
+}
+
+static bool release_all() { return false; }
+template <typename T, typename... Rest>
+static bool release_all(DevBuf<T>& b, Rest&... rest) {
+    const bool had = b.get() != nullptr;
+    b.release();
+    return release_all(rest...) | had;
+}
+
+bool Lattice::give_back() {
+    return release_all(rows, ekeys, table, entry_slot, flags, slot_vid, sort_keys, sort_vals, vorder_keys, scan.block_sums,
+                       sort.keys_alt, sort.vals_alt, sort.hist, sort.scan.block_sums);
+}
+
+// The ordered filter's buffers beside the value buffers.
+bool Lattice::give_back_quads() {
+    ord_vals = nullptr;
+    ord_T_ready = false;
+    return release_all(obins, ord_a, ord_b, ord_plane, ord_T);
 }
 
 // No lattice: N = 0 until one is built, and nothing that was computed on the

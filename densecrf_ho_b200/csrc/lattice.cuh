@@ -131,20 +131,21 @@ struct Lattice {
     DevBuf<int2> nbr;
     DevBuf<float> va, vb;    // filter value buffers
     // The plain splat's input in rows of 16-byte groups, norm applied: an aid that
-    // is given back where another buffer of the handle finds no memory, and done
-    // without where it finds none itself (splat_plain).
+    // is done without where it finds no memory (splat_plain).
     DevBuf<float> rows;
     float* rows_or_null(size_t floats);
-    bool give_back_rows() {
-        const bool had = rows.get() != nullptr;
-        rows.release();
-        return had;
-    }
+    // Releases what a complete lattice can do without, the rows and the scratch of
+    // its build: where another buffer of the handle finds no memory.
+    bool give_back();
     std::function<bool()> give_back_others;  // the same of the other lattices of a model or batch
     template <typename T>
     T* own(DevBuf<T>& b, size_t count) {
-        return ensure_after(b, count, [&] { return give_back_rows() | (give_back_others && give_back_others()); });
+        return ensure_after(b, count, [&] { return give_back() | (give_back_others && give_back_others()); });
     }
+    // A build, done again where it found no memory at first and a filter's buffers,
+    // the other lattices' included, could be released.
+    template <typename F>
+    void build_in(F&& build);
     // Ordered filter (see ordered.cu): packed bins, masks of the stored quads,
     // the up[0] plane, and per axis the blurred sums of each vertex's weights
     // (T, a property of the lattice: computed on its first ordered call).
@@ -153,6 +154,7 @@ struct Lattice {
     DevBuf<float> ord_plane, ord_T;
     bool ord_T_ready = false;
     void ensure_ord_totals();
+    bool give_back_quads();
 
     // build scratch
     DevBuf<int4> ekeys;
@@ -192,6 +194,7 @@ struct Lattice {
     void forget();
     // Several images' lattices as one (see Lattice::concat in lattice.cu).
     void concat(const std::vector<const Lattice*>& parts);
+    void concat_parts(const std::vector<const Lattice*>& parts);
     // out/in: device [N][L]; out may alias in.
     void compute(float* out, const float* in, int L, bool reverse, const SliceEpilogue& ep,
                  const float* pre_norm = nullptr);

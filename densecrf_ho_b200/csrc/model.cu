@@ -252,11 +252,11 @@ void Model::add_term(const float* d_features, int d, float w) {
     auto t = std::make_unique<Term>();
     t->lat = std::make_unique<Lattice>();
     t->lat->stream = stream;
-    t->lat->give_back_others = [this] { return give_back_rows(); };
+    t->lat->give_back_others = [this] { return give_back(); };
     t->lat->build(d_features, d, N);
     t->w = w;
     t->d = d;
-    float* tf = t->feat.ensure((size_t)N * d);
+    float* tf = own(t->feat, (size_t)N * d);
     DCRF_CUDA(cudaMemcpyAsync(tf, d_features, sizeof(float) * (size_t)N * d, cudaMemcpyDeviceToDevice, stream));
     t->kparams.assign(d, 1.0f);
     compute_norm(*t);
@@ -267,7 +267,7 @@ void Model::add_term(const float* d_features, int d, float w) {
 // the term's lattice, then per NormalizationType.
 void Model::compute_norm(Term& t) {
     if (t.ntype == kNoNorm) return;
-    float* nrm = t.norm.ensure(N);
+    float* nrm = own(t.norm, N);
     launch(fill_kernel, ceil_div(N, 256), 256, 0, stream, N, 1.0f, nrm);
     SliceEpilogue ep;  // plain output
     t.lat->compute(nrm, nrm, 1, false, ep);
@@ -314,14 +314,14 @@ void Model::set_kernel_parameters(int k, const float* p) {
     const size_t np = full ? (size_t)t.d * t.d : (size_t)t.d;
     t.kparams.assign(p, p + np);
     DevBuf<float> dp, sf;
-    DCRF_CUDA(cudaMemcpyAsync(dp.ensure(np), p, sizeof(float) * np, cudaMemcpyHostToDevice, stream));
-    float* scaled = sf.ensure((size_t)N * t.d);
+    DCRF_CUDA(cudaMemcpyAsync(own(dp, np), p, sizeof(float) * np, cudaMemcpyHostToDevice, stream));
+    float* scaled = own(sf, (size_t)N * t.d);
     launch(scale_features_kernel, ceil_div((long)N * t.d, 256), 256, 0, stream, N, t.d, (const float*)t.feat.get(),
            (const float*)dp.get(), (int)full, scaled);
     DCRF_LAUNCH_CHECK();
     auto lat = std::make_unique<Lattice>();
     lat->stream = stream;
-    lat->give_back_others = [this] { return give_back_rows(); };
+    lat->give_back_others = [this] { return give_back(); };
     lat->build(scaled, t.d, N);
     if (!t.twin) t.twin = std::move(t.lat);
     t.lat = std::move(lat);
@@ -671,7 +671,7 @@ void Model::set_compat(int k, int kind, const float* params) {
             for (int r = 0; r < L; r++) h[(size_t)c * L + r] = (params[(size_t)c * L + r] + params[(size_t)r * L + c]) * 0.5f;
     }
     t.hcw = h;
-    float* d = t.cw.ensure(h.size());
+    float* d = own(t.cw, h.size());
     DCRF_CUDA(cudaMemcpyAsync(d, h.data(), sizeof(float) * h.size(), cudaMemcpyHostToDevice, stream));
     sync();
     t.compat = kind;

@@ -135,16 +135,16 @@ struct Model {
     Model(int W_, int H_, int L_);
     ~Model();
 
-    // A buffer of the model; its lattices' padded rows go first where memory is short.
+    // A buffer of the model; what its lattices can do without goes first where memory is short.
     template <typename T>
     T* own(DevBuf<T>& buffer, size_t count) {
-        return ensure_after(buffer, count, [&] { return give_back_rows(); });
+        return ensure_after(buffer, count, [&] { return give_back(); });
     }
-    bool give_back_rows() {
+    bool give_back() {
         bool any = false;
         for (auto& t : terms) {
-            any |= t->lat->give_back_rows();
-            if (t->twin) any |= t->twin->give_back_rows();
+            any |= t->lat->give_back();
+            if (t->twin) any |= t->twin->give_back();
         }
         return any;
     }

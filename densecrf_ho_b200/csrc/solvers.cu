@@ -366,15 +366,15 @@ static void ho_prefix32(cudaStream_t stream, int L, const CliqueView& cv, const 
 
 // FP64 clique prefixes of p (minus one when asked) into out64 [R][L]:
 // segment totals, then the segments' prefixes with their carries.
-static void ho_prefix64(cudaStream_t stream, DevBuf<double>& seg_buf, int clique_max, int L, const CliqueView& cv,
-                        const float* p, int minus_one, double* out64, const SolverScalars* sc, int skip_on_zero_step) {
+static void ho_prefix64(Model& m, int clique_max, int L, const CliqueView& cv, const float* p, int minus_one, double* out64, const SolverScalars* sc, int skip_on_zero_step) {
     const int nseg = (clique_max + kHoSeg - 1) / kHoSeg;
+    cudaStream_t stream = m.stream;
     if (nseg == 0) {  // only empty cliques: their zeros
         launch(ho_seg_prefix_kernel, 1, 64, 0, stream, cv, L, p, minus_one, (const double*)nullptr, out64, sc,
                skip_on_zero_step);
         return;
     }
-    double* tot = seg_buf.ensure((size_t)nseg * L);
+    double* tot = m.own(m.ho_seg, (size_t)nseg * L);
     launch(ho_seg_total_kernel, nseg, 64, 0, stream, cv, L, p, minus_one, tot, sc, skip_on_zero_step);
     launch(ho_seg_prefix_kernel, nseg, 64, 0, stream, cv, L, p, minus_one, (const double*)tot, out64, sc,
            skip_on_zero_step);
@@ -1489,7 +1489,7 @@ double Model::energy_qp_ho(const float* Q) {
         launch(clear_step_flags_kernel, 1, 1, 0, stream, sc);
         launch(ho_zterm_prep_kernel, 1, 256, 0, stream, cv, L, (const float*)z_last.get(), zc, omz, sc);
         launch(eig_sum_kernel, 1, kHoThreads, 0, stream, (const float*)zc, LR, 8, sc, 2);
-        ho_prefix64(stream, ho_seg, clique_max, L, cv, Q, 1, preQ, nullptr, 0);
+        ho_prefix64(*this, clique_max, L, cv, Q, 1, preQ, nullptr, 0);
         launch(ho_scalar_kernel, 1, kLMax, 0, stream, cv, L, (const float*)omz, (const double*)preQ, 8, sc, 1);
     }
     launch(ho_energy_finish_kernel, 1, 1, 0, stream, nt, sc, (int)(R > 0));
@@ -1628,7 +1628,7 @@ int Model::qp(const float* init, float* out, int max_iter, double* energy_out) {
         DCRF_CUDA(cudaMemsetAsync(ho, 0, sizeof(float) * NL, stream));
         // the float chain of Q - 1 (sequential, as the reference sums it) and its FP64 prefixes
         ho_prefix32(stream, L, cv, Q, 1, pre32, nullptr, 0);
-        ho_prefix64(stream, ho_seg, clique_max, L, cv, Q, 1, preQ, nullptr, 0);
+        ho_prefix64(*this, clique_max, L, cv, Q, 1, preQ, nullptr, 0);
         launch(ho_regions_kernel, ceil_div(LR, 256), 256, 0, stream, cv, L, pre32, gz, 0, nullptr);
     }
     // grad_y = unary + sum_k 2 A_k Q; energy terms Q . A_k Q (same applies).
@@ -1669,7 +1669,7 @@ int Model::qp(const float* init, float* out, int max_iter, double* energy_out) {
         if (R > 0) {
             launch(ho_direction_kernel, 1, 256, 0, stream, cv, L, gz, z, sxz, t1, t2, cz, sc);
             launch(eig_sum_kernel, 1, kHoThreads, 0, stream, sxz, LR, 5, sc, 0);
-            ho_prefix64(stream, ho_seg, clique_max, L, cv, sx, 0, preS, sc, 0);
+            ho_prefix64(*this, clique_max, L, cv, sx, 0, preS, sc, 0);
             launch(ho_scalar_kernel, 1, kLMax, 0, stream, cv, L, t1, preQ, 3, sc, 0);    // a
             launch(ho_scalar_kernel, 1, kLMax, 0, stream, cv, L, t2, preS, 4, sc, 0);   // b
             launch(ho_scalar_kernel, 1, kLMax, 0, stream, cv, L, t1, preS, 6, sc, 0);   // denom term
@@ -1688,7 +1688,7 @@ int Model::qp(const float* init, float* out, int max_iter, double* energy_out) {
             // the prefixes of the updated Q - 1 (after a zero step Q is
             // unchanged, and so is the float chain)
             ho_prefix32(stream, L, cv, Q, 1, pre32, sc, 1);
-            ho_prefix64(stream, ho_seg, clique_max, L, cv, Q, 1, preQ, nullptr, 0);
+            ho_prefix64(*this, clique_max, L, cv, Q, 1, preQ, nullptr, 0);
             launch(ho_regions_kernel, ceil_div(LR, 256), 256, 0, stream, cv, L, pre32, gz, 1, sc);
             launch(ho_zterm_prep_kernel, 1, 256, 0, stream, cv, L, z, zc, omz, sc);
             launch(eig_sum_kernel, 1, kHoThreads, 0, stream, zc, LR, 8, sc, 2);
