@@ -45,6 +45,7 @@ constexpr int kQuads = 5;        // 16-byte quads (two pairs) per label
 constexpr int kPairs = 9;        // pairs (lo[b+1], up[b])
 constexpr int kOrdWarps = 4;     // warps per block of the splat and bins kernels
 constexpr int kOrdThreads = 32 * kOrdWarps;
+constexpr int kOrdBlockMaxL = 160;  // labels of the dense form's long lists at most (its ring's shared memory)
 
 // Mask words per vertex; labels 32 j .. 32 j + 31 are words 5 j .. 5 j + 4.
 __host__ __device__ constexpr int ord_words(int L) { return (kQuads * L + 31) / 32; }
@@ -1151,14 +1152,20 @@ void ordered_bins(unsigned short* bins, const float* Q, int N, int L, const floa
 
 void Lattice::compute_ord(float* out, const float* Q, int L, const SliceEpilogue& ep) {
     require(L >= 1 && L <= kOrdMaxL, DCRF_E_ARG, "compute_ord: label count out of range");
-    if (ord_dense(L)) {
-        compute_ord_dense(out, Q, L, ep);
-        return;
+    if (!ord_dense(L)) {
+        try {
+            unsigned short* bins = own(obins, ordered_bins_size(N, L));
+            ordered_bins(bins, Q, N, L, nullptr, stream);
+            ord_splat_blur(bins, L);
+            ord_slice(out, bins, L, ep, nullptr);
+            return;
+        } catch (const Error& e) {  // the dense form's buffers beside the value buffers are fewer
+            if (e.code != DCRF_E_NOMEM || (n_long && L > kOrdBlockMaxL)) throw;
+            cudaGetLastError();
+            give_back_quads();
+        }
     }
-    unsigned short* bins = own(obins, ordered_bins_size(N, L));
-    ordered_bins(bins, Q, N, L, nullptr, stream);
-    ord_splat_blur(bins, L);
-    ord_slice(out, bins, L, ep, nullptr);
+    compute_ord_dense(out, Q, L, ep);
 }
 
 void Lattice::ord_splat_blur(const unsigned short* bins, int L) {
@@ -1318,7 +1325,6 @@ constexpr int kODX = 4;                 // bins are copied kODX chunks ahead of 
 constexpr int kOXS = kODX + 1;          // bin ring slots (chunks c .. c+kODX)
 constexpr int kOPS = 2 * kODX + 1;      // pixel / weight ring slots (chunks c .. c+2 kODX)
 constexpr int kORow = 2 * kOE + 4;      // floats per ring row: 17 x 16 bytes
-constexpr int kOrdBlockMaxL = 160;      // larger L: the quad form (shared-memory ring size)
 constexpr int kGroupChoices[] = {1, 2, 3, 5, 10};
 
 // Bin split with the fewest warp instructions per list entry: warps x (three

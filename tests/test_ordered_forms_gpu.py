@@ -1,12 +1,17 @@
 """The single ordered filter on both sides of each line between its quad and its
 dense form: few labels over long and huge lists, many vertices, many pixels; bit
 for bit against the oracle."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
-from densecrf_ho_b200 import Permutohedral, synth
+from densecrf_ho_b200 import Permutohedral, device_memory_stats, lib, set_device_memory_limit, synth
+from densecrf_ho_b200._lib import DCRFError, check
 
 pytestmark = pytest.mark.gpu
+
+DCRF_E_NOMEM = 5
 
 
 def _features(W, H, d, kind):
@@ -69,3 +74,48 @@ def test_restricted_and_plain_between_the_forms(oracle_mod):
         assert np.array_equal(lat.compute(q), plain)
         assert np.array_equal(lat.compute_upper_minus_lower_ord(q), full)
         assert np.array_equal(lat.compute_upper_minus_lower_ord_restricted(rq2, pI, None, False), want2)
+
+
+def _dev_filter(lat, x, entry, *args):
+    import torch
+    out = torch.full_like(x, float("nan"))
+    torch.cuda.synchronize()
+    check(entry(lat._h, C.c_void_p(out.data_ptr()), C.c_void_p(x.data_ptr()), x.shape[1], *args))
+    torch.cuda.synchronize()
+    return out.cpu().numpy()
+
+
+def _block(n):  # device blocks: powers of two split in quarters
+    p = 512
+    while p < n:
+        p *= 2
+    return p if p == 512 else -(-n // (p // 4)) * (p // 4)
+
+
+@pytest.mark.parametrize("W,H,kind,L", [(97, 83, "noisy", 21), (97, 83, "photo", 21), (161, 120, "grid", 5)])
+def test_without_memory_for_the_quads(W, H, kind, L):
+    """Budgets below what a call of the quad form's range takes: the same bits or
+    no memory, and never the latter where the dense form has room."""
+    import torch
+    N = W * H
+    f = _features(W, H, 2 if kind == "grid" else 5, kind)
+    x = torch.rand(N, L, generator=torch.Generator(device="cuda").manual_seed(L), device="cuda")
+    entry = lib().dcrf_lattice_compute_ord_dev
+    lat = Permutohedral().init(f)
+    before = device_memory_stats()[0]
+    want = _dev_filter(lat, x, entry)
+    took = device_memory_stats()[0] - before
+    dense = 2 * _block(80 * (lat.M + 1) * L) + _block(8 * N * L)
+    del lat
+    for budget in [took * k // 24 for k in range(25)] + [dense, took - 1]:
+        lat = Permutohedral().init(f)
+        set_device_memory_limit(device_memory_stats()[0] + budget)
+        try:
+            for _ in range(2):
+                assert np.array_equal(_dev_filter(lat, x, entry), want)
+        except DCRFError as e:
+            assert e.code == DCRF_E_NOMEM and budget < dense
+        finally:
+            set_device_memory_limit(0)
+        assert np.array_equal(_dev_filter(lat, x, entry), want)
+        del lat
