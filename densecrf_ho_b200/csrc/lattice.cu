@@ -399,11 +399,19 @@ __device__ __forceinline__ void stream_list(int s0, int s1, int L, int k, bool a
 
 // The splat of input rows as they are, for the allocation-free filter and where
 // memory is short: neither holds the padded copy of the splat below.  The long
-// lists, one warp per vertex; rows of Lp values, those past L zero.
+// lists, one warp per vertex; rows of Lp values, those past L zero.  PLAIN: no
+// norm, no live images and rows of L values (the allocation-free filter, 640x480,
+// two features, 100 labels: 402 us so, 424 with those at run time).
+template <bool PLAIN>
 __global__ void __launch_bounds__(32 * kStageWarps)
     splat_kernel(SplatRange r, int L, int Lp, const int* __restrict__ order, const int* __restrict__ seg_start,
-                 const int2* __restrict__ seg, const float* __restrict__ in, const float* __restrict__ norm,
+                 const int2* __restrict__ seg, const float* __restrict__ in, const float* __restrict__ norm_,
                  float* __restrict__ vals) {
+    const float* norm = PLAIN ? nullptr : norm_;
+    if (PLAIN) {
+        Lp = L;
+        r.lv = Live{};
+    }
     __shared__ float ring[kStageWarps][kStages][kChunk][32];
     __shared__ float mw[kStageWarps][kStages][kChunk], mn[kStageWarps][kStages][kChunk];
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -429,10 +437,16 @@ __global__ void __launch_bounds__(32 * kStageWarps)
 
 // ... and the short ones: one thread per (vertex, label).  Also row 0 of both
 // value buffers, which absent neighbours read.
+template <bool PLAIN>
 __global__ void splat_short_kernel(SplatRange r, int L, int Lp, const int* __restrict__ order,
                                    const int* __restrict__ seg_start, const int2* __restrict__ seg,
-                                   const float* __restrict__ in, const float* __restrict__ norm,
+                                   const float* __restrict__ in, const float* __restrict__ norm_,
                                    float* __restrict__ vals, float* __restrict__ other) {
+    const float* norm = PLAIN ? nullptr : norm_;
+    if (PLAIN) {
+        Lp = L;
+        r.lv = Live{};
+    }
     const long t0 = (long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long)gridDim.x * blockDim.x;
     for (long t = t0; t < Lp; t += nt) vals[t] = other[t] = 0.0f;
     const long total = live_total(r.lv, r.count) * Lp;
@@ -1733,13 +1747,14 @@ static dim3 wide_grid(int N, int Q) { return dim3(ceil_div(Q, kTB), std::min(N, 
 
 // The splat without the padded rows, into rows of Lp floats.
 void Lattice::splat_plain(const float* in, int L, int Lp, const float* pre_norm, float* vals, float* other) {
-    const bool live = live_n != nullptr;
+    const bool live = live_n != nullptr, plain = !live && !pre_norm && Lp == L;
     const int n_short = M - n_long;
     if (n_long)
-        launch(splat_kernel, unit_grid(n_long, kStageWarps, live, 32 * kStageWarps), 32 * kStageWarps, 0, stream,
-               SplatRange{0, n_long, live_of(kDomLong)}, L, Lp, vorder.get(), seg_start.get(), seg.get(), in, pre_norm,
-               vals);
-    launch(splat_short_kernel, unit_grid((long)n_short * Lp, kTB, live, kTB), kTB, 0, stream,
+        launch(plain ? splat_kernel<true> : splat_kernel<false>, unit_grid(n_long, kStageWarps, live, 32 * kStageWarps),
+               32 * kStageWarps, 0, stream, SplatRange{0, n_long, live_of(kDomLong)}, L, Lp, vorder.get(),
+               seg_start.get(), seg.get(), in, pre_norm, vals);
+    launch(plain ? splat_short_kernel<true> : splat_short_kernel<false>,
+           unit_grid((long)n_short * Lp, kTB, live, kTB), kTB, 0, stream,
            SplatRange{n_long, n_short, live_of(kDomShort)}, L, Lp, vorder.get(), seg_start.get(), seg.get(), in,
            pre_norm, vals, other);
 }
