@@ -567,11 +567,44 @@ __device__ __forceinline__ void ord_splat_group(int first, int count, int L, int
     }
 }
 
+// Very short lists: a thread per (list, label), all nine pairs in registers, the
+// next entry's loads in flight; thread k < NW of a list also finds mask word k.  A
+// group of four lists of three entries each leaves its warp mostly idle (a noisy
+// 640x480 image: one label 447 -> 263 us the filter, 4 1069 -> 929; 320x240, 12
+// labels 589 -> 571).
+__device__ __forceinline__ void ord_splat_few(long t, int n_short, int L, int NW, const int* __restrict__ order,
+                                              const int* __restrict__ seg_start, const int2* __restrict__ seg,
+                                              const unsigned short* __restrict__ bins,
+                                              const unsigned* __restrict__ pmask, unsigned* __restrict__ act,
+                                              float* __restrict__ vals) {
+    if (t >= (long)n_short * L) return;
+    const int u = (int)(t / L), k = (int)(t - (long)u * L), Lb = ord_bin_row(L);
+    const int v = order[u], s0 = seg_start[v], s1 = seg_start[v + 1];
+    PairSums<kPairs> ps;
+    ps.init(0);
+    unsigned m = 0;
+    int cmax = 0;
+#pragma unroll 2
+    for (int s = s0; s < s1; s++) {
+        const int2 e = seg[s];
+        const unsigned c = bins[(long)e.x * Lb + k];
+        if (k < NW) m |= pmask[(long)e.x * NW + k];
+        cmax = max(cmax, (int)(c >> 8));
+        ps.add(c, pack2(entry_w(e), entry_w(e)));
+    }
+    if (k < NW) act[(long)(v + 1) * NW + k] = m;
+    unsigned long long* label = reinterpret_cast<unsigned long long*>(vals + (long)(v + 1) * kOrdW * L + (long)k * kOrdW);
+    const int n = 2 * quads_of(cmax);
+#pragma unroll
+    for (int i = 0; i < kPairs; i++)
+        if (i < n) label[i] = ps.acc[i];
+}
+
 // One launch: warps [0, huge_tasks) the lists over kHugeList entries, the next
 // long_tasks the other long ones (longest first), the rest groups of short
-// lists.  Row 0 of both masks (the absent neighbour) is cleared here: none of
+// lists, or (FEW) 32 (list, label) of them each.  Row 0 of both masks (the absent neighbour) is cleared here: none of
 // its quads exists, and its T is 0.
-template <int NC, int NWC>
+template <int NC, int NWC, bool FEW>
 __global__ void __launch_bounds__(kOrdThreads, 6)
     ord_splat_kernel(int M, int n_long, int n_huge, int huge_tasks, int long_tasks, int L, int NW,
                      const int* __restrict__ order, const int* __restrict__ seg_start, const int2* __restrict__ seg,
@@ -596,6 +629,11 @@ __global__ void __launch_bounds__(kOrdThreads, 6)
         return;
     }
     t -= long_tasks;
+    if (FEW) {
+        ord_splat_few(32 * t + lane, M - n_long, L, NW, order + n_long, seg_start, seg,
+                      reinterpret_cast<const unsigned short*>(bins), pmask, act, vals);
+        return;
+    }
     const long first = n_long + t * kGroup;
     if (first < M)
         ord_splat_group<NC, NWC>((int)first, (int)min((long)kGroup, M - first), L, NW, order, seg_start, seg, bins,
@@ -764,6 +802,48 @@ __global__ void __launch_bounds__(kOrdBlurThreads, kOrdBlurBlocks)
             }
         }
     }
+}
+
+// The same with a thread per (vertex, quad), where the quads of one mask word (up to
+// 6 labels) leave a warp's lanes idle.  The whole filter in the quad form, a warp a
+// vertex -> this, us: 640x480, five features, 2 labels 143 -> 131, a noisy image
+// (650 thousand vertices) with one label 1185 -> 447, with 4 1191 -> 1069; with 8
+// labels this loses, 6 to 12 %.
+template <bool LAST>
+__global__ void __launch_bounds__(kOrdBlurThreads)
+    ord_blur_few_kernel(int M, int L, int NW, const int2* __restrict__ nbr, const float* __restrict__ T,
+                        const float* __restrict__ Tn, const float4* __restrict__ src, float4* __restrict__ dst,
+                        const unsigned* __restrict__ act, unsigned* __restrict__ act2, float* __restrict__ plane) {
+    const int row4 = kQuads * L;
+    const long t = (long)blockIdx.x * kOrdBlurThreads + threadIdx.x;
+    grid_release();
+    grid_wait();
+    if (t >= (long)M * row4) return;
+    const int v = (int)(t / row4), idx = (int)(t - (long)v * row4), r = idx >> 5, bit = idx & 31;
+    const int k = idx / kQuads, j = idx - k * kQuads;
+    const int2 nb = nbr[v];
+    const unsigned *pa = act + (long)(v + 1) * NW + r, *pb = act + (long)nb.x * NW + r, *pc = act + (long)nb.y * NW + r;
+    const unsigned a = *pa, b = *pb, c = *pc, m = a | b | c;
+    if (!LAST && bit == 0) act2[(long)(v + 1) * NW + r] = m;
+    bool on = m >> bit & 1u;
+    if (LAST && j > 0)  // behind a stored quad
+        on = on || (bit ? m >> (bit - 1) & 1u : (pa[-1] | pb[-1] | pc[-1]) >> 31);
+    if (!on && !(LAST && j == 0)) return;
+    const float T0 = T[v + 1], T1 = T[nb.x], T2 = T[nb.y];
+    float4 x = make_float4(0.0f, T0, 0.0f, T0), y = make_float4(0.0f, T1, 0.0f, T1), z = make_float4(0.0f, T2, 0.0f, T2);
+    quad_if(x, src + (long)(v + 1) * row4 + idx, a >> bit & 1u);
+    quad_if(y, src + (long)nb.x * row4 + idx, b >> bit & 1u);
+    quad_if(z, src + (long)nb.y * row4 + idx, c >> bit & 1u);
+    float4 q;
+    q.x = fadd(x.x, fmul(0.5f, fadd(y.x, z.x)));
+    q.y = fadd(x.y, fmul(0.5f, fadd(y.y, z.y)));
+    q.z = fadd(x.z, fmul(0.5f, fadd(y.z, z.z)));
+    q.w = fadd(x.w, fmul(0.5f, fadd(y.w, z.w)));
+    if (LAST) {
+        if (j == kQuads - 1) q.w = Tn[v + 1];
+        if (j == 0) plane[(long)(v + 1) * ord_plane_row(L) + k] = q.y;
+    }
+    if (on) dst[(long)(v + 1) * row4 + idx] = q;
 }
 
 // --------------------------------------------------------------- slice --
@@ -1184,29 +1264,36 @@ void Lattice::ord_splat_blur(const unsigned short* bins, int L) {
         launch_ord((long)N * L, NW == 4 ? ord_mask_kernel<4> : ord_mask_kernel<0>, n_long, 32 * kMaskWarps, 0, st, NW,
                        vorder.get(), seg_start.get(), seg.get(), pm, as);
     const long ht = (long)n_huge * nblk * kPairs, lt = (long)(n_long - n_huge) * nblk * kLongRounds;
-    const long tasks = ht + lt + (n_short + kGroup - 1) / kGroup;
+    // Groups of lists or a thread per list and label: the latter where the lists have
+    // few entries on average and are many; with many labels and vertices the group's
+    // skipped quads win (noisy 640x480, 21 labels: an LP 101 ms by groups, 103 else).
+    const bool few_lists = (long)N * (d + 1) < 8L * M && M >= 1 << 12 && (L <= 16 || M < 1 << 16);
+    const long tasks = ht + lt + (few_lists ? ((long)n_short * L + 31) / 32 : (n_short + kGroup - 1) / kGroup);
     require(ht + lt < (1L << 30), DCRF_E_ARG, "compute_ord: too many labels");
-    int bytes = std::max(n_long ? ord_ring_bytes(nc) + 2 * kUnitList : 0, ord_group_bytes(nc));
+    int bytes = std::max(n_long ? ord_ring_bytes(nc) + 2 * kUnitList : 0, few_lists ? 0 : ord_group_bytes(nc));
     bytes = (bytes + 15) & ~15;
     static_assert(kOrdWarps * (ord_ring_bytes(4) + 2 * kUnitList) <= (48 << 10) &&
                       kOrdWarps * ord_group_bytes(4) <= (48 << 10), "no opt-in to more shared memory");
-    auto splat = L == 21 ? ord_splat_kernel<3, 4> : ord_splat_kernel<0, 0>;
+    auto splat = few_lists ? (L == 21 ? ord_splat_kernel<3, 4, true> : ord_splat_kernel<0, 0, true>)
+                           : (L == 21 ? ord_splat_kernel<3, 4, false> : ord_splat_kernel<0, 0, false>);
     launch_ord((long)N * L, splat, ceil_div(tasks, kOrdWarps), kOrdThreads, (size_t)bytes * kOrdWarps, st, M, n_long, n_huge,
                    (int)ht, (int)lt, L, NW, vorder.get(), seg_start.get(), seg.get(), b4, pm, as, ad, src, bytes);
+    const bool few = NW == 1;
     for (int j = 0; j <= d; j++) {
         const float* T = ord_T.get() + (long)j * (M + 1);
         auto pick = [&](auto last) {
             constexpr bool LAST = decltype(last)::value;
-            return NW == 1   ? ord_blur_kernel<1, LAST>
+            return few       ? ord_blur_few_kernel<LAST>
                    : NW == 2 ? ord_blur_kernel<2, LAST>
                    : NW == 3 ? ord_blur_kernel<3, LAST>
                    : NW == 4 ? ord_blur_kernel<4, LAST>
                              : ord_blur_kernel<0, LAST>;
         };
         auto kern = j == d ? pick(std::true_type{}) : pick(std::false_type{});
-        launch_ord((long)N * L, kern, std::min(ceil_div(M, kOrdBlurThreads / 32), sm_count() * kOrdBlurBlocks), kOrdBlurThreads, 0, st, M, L, NW,
-                       nbr.get() + (long)j * M, T, T + M + 1, reinterpret_cast<const float4*>(src),
-                       reinterpret_cast<float4*>(dst), as, ad, plane);
+        const int grid = few ? ceil_div((long)M * kQuads * L, kOrdBlurThreads)
+                             : std::min(ceil_div(M, kOrdBlurThreads / 32), sm_count() * kOrdBlurBlocks);
+        launch_ord((long)N * L, kern, grid, kOrdBlurThreads, 0, st, M, L, NW, nbr.get() + (long)j * M, T, T + M + 1,
+                   reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), as, ad, plane);
         std::swap(src, dst);
         std::swap(as, ad);
     }
@@ -1603,18 +1690,19 @@ Lattice::~Lattice() {
 // (softmax of normal logits); one call after the other, us, quad form -> dense.
 //   No long list, two features at most: from 2^19 (pixel, label) values or 2^18
 //   pixels on; from 20 labels on where there are pixels to fill the chip, and
-//   above 28 labels, whose masks are read in a loop.  640x480 with one label 59 ->
-//   37, 21 labels 205 -> 207, and 215 -> 178 with three calls in flight; 160x120
+//   above 28 labels, whose masks are read in a loop.  640x480 with 3 labels 70 ->
+//   51, 21 labels 205 -> 207, and 215 -> 178 with three calls in flight; 160x120
 //   with 22 labels 41.5 -> 39.9, 97x83 with 32 49 -> 36; below the lines 320x240
-//   with 2 labels 29 -> 34, 97x83 with 21 30 -> 37.
+//   with 2 labels 25 -> 34, 97x83 with 21 30 -> 37.
 //   Else the quad form wins where long lists leave most quads empty (five
 //   features, 640x480, 21 labels 272 -> 362), and loses with few labels: a list's
-//   sums fill few lanes (640x480: 2 labels 143 -> 107, 8 192 -> 182, 12 232 ->
+//   sums fill few lanes (640x480: 2 labels 131 -> 107, 8 192 -> 182, 12 232 ->
 //   231, 16 259 -> 289; 320x240, whose splat does not fill the chip: 12 labels
-//   123 -> 112, 20 146 -> 142, 26 180 -> 207; smaller ones win throughout), and a
-//   vertex's mask costs its blur a warp whatever the labels: a noisy image
-//   640x480, 650 thousand vertices, one label 1186 -> 254, 21 labels 3918 -> 3638,
-//   28 4728 -> 4923; 97x83, 25 thousand, 4 labels 66 -> 55, 12 70 -> 82.
+//   123 -> 112, 20 146 -> 142, 26 180 -> 207; smaller ones win throughout), and its
+//   masks cost by the vertex whatever the labels: a noisy image 640x480, 650
+//   thousand vertices, 2 labels 496 -> 409, 4 929 -> 709, 21 3949 -> 3659, 32 5159
+//   -> 5482; 320x240, 178 thousand, 4 labels 255 -> 215, 20 902 -> 916; 160x120, 52
+//   thousand, 4 labels 64 -> 70.
 // On evenly spread values, where all quads exist, the quad form loses everywhere
 // (five features, 640x480, 21 labels 379 -> 350): a single filter of those is
 // slower than the dense form would be.
@@ -1624,7 +1712,7 @@ bool Lattice::ord_dense(int L) const {
         return (long)N * L > 1L << 19 || N > 1 << 18 || L > 28 || (L >= 20 && N >= 1 << 14);
     const bool long_lists = (long)N * (d + 1) >= 32L * M;  // on average
     const int by_lists = !long_lists ? 0 : N > 1 << 18 ? 12 : N > 1 << 16 ? 20 : 0;
-    return L <= std::max((double)by_lists, 4.0 * std::log2((double)M) - 50.0);
+    return L <= std::max((double)by_lists, 8.0 * std::log2((double)M) - 127.0);
 }
 
 void Lattice::compute_ord_dense(float* out, const float* Q, int L, const SliceEpilogue& ep) {

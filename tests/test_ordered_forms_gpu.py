@@ -39,8 +39,9 @@ def _iterate(N, L, rng, spread):
     (256, 256, 5, "wide", (20, 21)),
     (513, 512, 5, "photo", (12, 13)),   # more than 2^18
     (257, 256, 3, "photo", (6, 20)),
-    (97, 83, 5, "noisy", (1, 8, 9)),    # some 25 thousand vertices
-    (61, 47, 5, "noisy", (1, 2, 3, 4)),
+    (97, 83, 5, "noisy", (1, 2, 6, 7, 12, 16, 17, 21, 33)),  # some 25 thousand vertices of few entries
+    (200, 150, 5, "noisy", (1, 3, 4, 16, 17)),               # and 77 thousand
+    (61, 47, 5, "noisy", (1, 2, 3, 4)), (31, 7, 3, "noisy", (1, 6, 7)),
     (512, 513, 2, "grid", (1,)), (512, 512, 2, "grid", (1, 2)),
     (128, 128, 2, "grid", (19, 20)), (127, 129, 2, "grid", (19, 20, 28, 29)),
     (31, 7, 2, "grid", (28, 29, 161)), (61, 47, 1, "line", (29,)),
