@@ -805,7 +805,8 @@ __global__ void __launch_bounds__(kOrdBlurThreads, kOrdBlurBlocks)
 }
 
 // The same with a thread per (vertex, quad), where the quads of one mask word (up to
-// 6 labels) leave a warp's lanes idle.  The whole filter in the quad form, a warp a
+// 6 labels) leave a warp's lanes idle and the vertices fill the chip (from 4096 on;
+// 97x83, 1100 vertices, 3 labels 16.5 us by warps, 18.8 so).  The whole filter in the quad form, a warp a
 // vertex -> this, us: 640x480, five features, 2 labels 143 -> 131, a noisy image
 // (650 thousand vertices) with one label 1185 -> 447, with 4 1191 -> 1069; with 8
 // labels this loses, 6 to 12 %.
@@ -862,12 +863,11 @@ struct OrdSliceTerm {
 // One term's value of element (pixel, k) in any bin: the lower pass with weight
 // -w alpha, then the upper with w alpha (:639-650, :687-696), one float per
 // vertex and pass from the row its bin selects: T (lower bin 0), the plane up[0]
-// (upper bin 0) or its pair -- the pixel's own vertices hold it.  A row's bytes
-// fit an int up to kOrdIntL labels, beyond which launch_slice takes DC = 0.
-constexpr int kOrdIntL = 1 << 24;
-template <int DC>
+// (upper bin 0) or its pair -- the pixel's own vertices hold it.  WIDE: a row's
+// bytes may not fit an int.
+template <int DC, bool WIDE = false>
 __device__ __forceinline__ float ord_slice_sum(const OrdSliceTerm& s, const int2* ow, int k, int cl, int cu, int L) {
-    using S = std::conditional_t<DC != 0, int, long>;
+    using S = std::conditional_t<WIDE, long, int>;
     const int d1 = (DC ? DC : s.d) + 1;
     const S one = sizeof(float), row = one * kOrdW * L;
     const char* lo = reinterpret_cast<const char*>(cl ? s.vals + S(k) * kOrdW + 2 * (cl - 1) : s.T);
@@ -943,7 +943,9 @@ __global__ void __launch_bounds__(kOsThreads)
     __shared__ int n_hot, s_dense;
     __shared__ float s_val[kSliceElems];
     __shared__ unsigned s_hot[kSliceElems];  // element | bins << 16
-    const int L = LC ? LC : Lrt, elems = slice_elems(L), Lb = ord_bin_row(L), Q = ord_plane_row(L) / 4;
+    constexpr bool kWide = LC < 0;  // more labels than a block has elements, at run time as with 0
+    constexpr bool kSkip = LC > 0 || (LC == 0 && D0 == 0);
+    const int L = LC > 0 ? LC : Lrt, elems = slice_elems(L), Lb = ord_bin_row(L), Q = ord_plane_row(L) / 4;
     const long NL = (long)N * L, tb = (long)blockIdx.x * elems;
     const int pf = (int)(tb / L), first = (int)(tb - (long)pf * L), np = min(P, N - pf);
     const int ne = (int)min((long)elems, NL - tb);
@@ -1024,15 +1026,16 @@ __global__ void __launch_bounds__(kOsThreads)
     };
     const bool dense = s_dense;
     // The block shares its outer pixels with its neighbours.  With the labels at
-    // compile time it walks all groups of its pixels and skips those outside, else
-    // (a pixel may be many blocks') from the first element's group to the last's.
-    // The whole filter, 640x480, five features: 21 labels 269 us by the former, 277
-    // by the latter; 40 labels 562 and 546.
+    // compile time, or neither them nor the features, it walks all groups of its
+    // pixels and skips those outside (kSkip), else (a pixel may be many blocks') from
+    // the first element's group to the last's.  The whole filter, 640x480, by the
+    // former and the latter: five features, 21 labels 269 us and 277, 40 labels 562
+    // and 546; three features, 21 labels 221 and 231.
     const int ll = (ne - 1 + first) / L, last = ll * Q + (ne - 1 + first - ll * L) / 4;
-    const int it0 = LC ? 0 : first / 4, it1 = LC ? np * Q : last + 1;
+    const int it0 = kSkip ? 0 : first / 4, it1 = kSkip ? np * Q : last + 1;
     for (int it = it0 + threadIdx.x; !dense && it < it1; it += blockDim.x) {
         const int li = it / Q, q = it - li * Q, e0 = li * L + 4 * q - first;
-        if (LC && (e0 + 3 < 0 || e0 >= ne)) continue;
+        if (kSkip && (e0 + 3 < 0 || e0 >= ne)) continue;
         const uint2 c = *reinterpret_cast<const uint2*>(bins + (long)(pf + li) * Lb + 4 * q);
         float a[NT][4];
 #pragma unroll
@@ -1072,8 +1075,8 @@ __global__ void __launch_bounds__(kOsThreads)
     for (int n = threadIdx.x; n < items; n += blockDim.x) {
         const unsigned h = dense ? n | bin_of(n) << 16 : s_hot[n], c = h >> 16;
         const int e = h & 0xffff, f = e + first, li = f / L, k = f - li * L;
-        const float a0 = ord_slice_sum<D0>(t0, s_ow[0] + li * da, k, c >> 8, c & 255, L);
-        const float a1 = NT == 2 ? ord_slice_sum<D1>(t1, s_ow[1] + li * db, k, c >> 8, c & 255, L) : 0.0f;
+        const float a0 = ord_slice_sum<D0, kWide>(t0, s_ow[0] + li * da, k, c >> 8, c & 255, L);
+        const float a1 = NT == 2 ? ord_slice_sum<D1, kWide>(t1, s_ow[1] + li * db, k, c >> 8, c & 255, L) : 0.0f;
         s_val[e] = finish(a0, a1, li, k);
     }
     __syncthreads();
@@ -1160,7 +1163,9 @@ void launch_slice(float* out, const unsigned short* bins, int L, const Lattice& 
     // in flight 119 -> 106; the small LP (64x48, 21 labels, 6 steps) 6465 ->
     // 6252; from 2^17 values on it loses: the LP at 152x71 with 18 labels
     // 12430 -> 12640, at 200x120 with 21 labels 8340 -> 8800.
-    const bool known = L <= kOrdIntL && (NT == 2 ? a.d == 2 && b.d == 5 : a.d == 2 || a.d == 5);
+    const bool wide = L > kSliceElems;  // one term's only: a model has 64 labels at most
+    require(!wide || (NT == 1 && !gap), DCRF_E_ARG, "ord_slice: too many labels");
+    const bool known = !wide && (NT == 2 ? a.d == 2 && b.d == 5 : a.d == 2 || a.d == 5);
     if (known && (L < 8 || NL <= 1L << 17)) {
         auto direct = [&](auto kern) {
             launch_ord(NL, kern, ceil_div(NL, elems), kOsThreads, 0, st, a.N, L, t0, t1, bins, out,
@@ -1189,7 +1194,8 @@ void launch_slice(float* out, const unsigned short* bins, int L, const Lattice& 
                    : L == 21 ? ord_slice_kernel<GAP, NT, 21, 2, 5>
                              : ord_slice_kernel<GAP, NT, 0, 2, 5>;
         } else {
-            return !known     ? ord_slice_kernel<GAP, NT, 0, 0, 0>
+            return wide       ? ord_slice_kernel<false, 1, -1, 0, 0>
+                   : !known   ? ord_slice_kernel<GAP, NT, 0, 0, 0>
                    : a.d == 5 ? (L == 21 ? ord_slice_kernel<GAP, NT, 21, 5, 0> : ord_slice_kernel<GAP, NT, 0, 5, 0>)
                               : (L == 21 ? ord_slice_kernel<GAP, NT, 21, 2, 0> : ord_slice_kernel<GAP, NT, 0, 2, 0>);
         }
@@ -1278,12 +1284,13 @@ void Lattice::ord_splat_blur(const unsigned short* bins, int L) {
                            : (L == 21 ? ord_splat_kernel<3, 4, false> : ord_splat_kernel<0, 0, false>);
     launch_ord((long)N * L, splat, ceil_div(tasks, kOrdWarps), kOrdThreads, (size_t)bytes * kOrdWarps, st, M, n_long, n_huge,
                    (int)ht, (int)lt, L, NW, vorder.get(), seg_start.get(), seg.get(), b4, pm, as, ad, src, bytes);
-    const bool few = NW == 1;
+    const bool few = NW == 1 && M >= 1 << 12;
     for (int j = 0; j <= d; j++) {
         const float* T = ord_T.get() + (long)j * (M + 1);
         auto pick = [&](auto last) {
             constexpr bool LAST = decltype(last)::value;
             return few       ? ord_blur_few_kernel<LAST>
+                   : NW == 1 ? ord_blur_kernel<1, LAST>
                    : NW == 2 ? ord_blur_kernel<2, LAST>
                    : NW == 3 ? ord_blur_kernel<3, LAST>
                    : NW == 4 ? ord_blur_kernel<4, LAST>
