@@ -980,10 +980,9 @@ __global__ void order_key_kernel(int M, const int* __restrict__ seg_start, int* 
 
 // One blur pass along one lattice axis: new = old + 1/2 (n1 + n2).  seqCompute
 // evaluates it in double (0.5 is a double literal there, :518).
-template <bool SEQ, int LC = 0>
-__global__ void blur_kernel(int M, int Lrt, const int2* __restrict__ nbr,
+template <bool SEQ>
+__global__ void blur_kernel(int M, int L, const int2* __restrict__ nbr,
                             const float* __restrict__ src, float* __restrict__ dst, Live lv) {
-    const int L = LC ? LC : Lrt;
     grid_release();
     grid_wait();
     const long total = live_total(lv, M) * L;
@@ -1033,11 +1032,10 @@ __global__ void blur4_kernel(int M, int Qrt, const int2* __restrict__ nbr, const
 
 // Slice: out(i, k) = sum_j (bary_ij * alpha) * value(o_ij, k) (sseCompute,
 // :1046-1051) or sum_j (bary_ij * value) * alpha (seqCompute, :529-534).
-template <bool SEQ, int DC, int LC>
-__global__ void slice_kernel(int N, int Lrt, int drt, const int* __restrict__ offset,
+template <bool SEQ>
+__global__ void slice_kernel(int N, int L, int d, const int* __restrict__ offset,
                              const float* __restrict__ bary, const float* __restrict__ vals,
                              float alpha, float* out, SliceEpilogue ep, Live lv) {
-    const int L = LC ? LC : Lrt, d = DC ? DC : drt;
     const int d1 = d + 1;
     grid_release();
     grid_wait();
@@ -1717,10 +1715,10 @@ void Lattice::compute_noalloc(float* out, const float* in, int L, bool reverse) 
     const float alpha = 1.0f / (1.0f + std::pow(2.0f, (float)-d));
     const SliceEpilogue ep;
     if (seq)
-        launch(slice_kernel<true, 0, 0>, ceil_div(NL, kTB), kTB, 0, st, N, L, d, offset.get(), bary.get(), src, alpha,
+        launch(slice_kernel<true>, ceil_div(NL, kTB), kTB, 0, st, N, L, d, offset.get(), bary.get(), src, alpha,
                out, ep, Live{});
     else
-        launch(slice_kernel<false, 0, 0>, ceil_div(NL, kTB), kTB, 0, st, N, L, d, offset.get(), bary.get(), src, alpha,
+        launch(slice_kernel<false>, ceil_div(NL, kTB), kTB, 0, st, N, L, d, offset.get(), bary.get(), src, alpha,
                out, ep, Live{});
     DCRF_LAUNCH_CHECK();
 }
@@ -1969,7 +1967,7 @@ void Lattice::slice(float* out, int L, const SliceEpilogue& ep) {
     const float alpha = 1.0f / (1.0f + std::pow(2.0f, (float)-d));
     const bool live = live_n != nullptr;
     if (L <= 2) {
-        launch_chained(slice_kernel<true, 0, 0>, unit_grid(NL, kTB, live, kTB), kTB, 0, st, N, L, d, offset.get(),
+        launch_chained(slice_kernel<true>, unit_grid(NL, kTB, live, kTB), kTB, 0, st, N, L, d, offset.get(),
                        bary.get(), src, alpha, out, ep, live_of(kDomPix));
     } else if (!row_tiles(d, L)) {
         require(!live && !ep.potts && !ep.base && !ep.zero_base, DCRF_E_ARG, "slice: too many labels");
