@@ -69,11 +69,6 @@ def parse():
                     help="time only the batched QP, without the sequential comparison (a short command for ncu)")
     ap.add_argument("--only-batch-filter", action="store_true",
                     help="time only the batched lattice filter over the 64-image concatenated lattices")
-    ap.add_argument("--splat-form", type=int, default=None,
-                    help="pass a splat form (0-5, dcrf_batch_set_filter_shape) in the batched filter and batched QP "
-                         "legs: accepted, without effect (one form is left); it also keeps the blur untuned")
-    ap.add_argument("--all-splat-forms", action="store_true",
-                    help="with --only-batch-filter: time the batched filter with every splat form pinned")
     ap.add_argument("--only-ho", action="store_true",
                     help="time only qp_sp / lp_sp at 640x480 (no CPU reference)")
     ap.add_argument("--batch-images", type=int, default=64,
@@ -613,17 +608,7 @@ def measure_ho(W=640, H=480, seed=2, cpu=True):
     return out
 
 
-def pin_splat_form(b, form):
-    """Pins both terms' launch shapes of a batch: the default blur / slice
-    shapes with splat form `form` (no autotuning)."""
-    for k in range(b.n_terms()):
-        b.set_filter_shape(k, (4, 256, 128, int(form)))
-
-
-SPLAT_FORMS = ("staged", "warp_long", "warp_all", "tiled_all", "staged_long_tiled_short", "bulk_all")
-
-
-def measure_batch(n=64, max_iter=100, reps=3, sequential=True, splat_form=None):
+def measure_batch(n=64, max_iter=100, reps=3, sequential=True):
     """Config 4: the plain QP (as config 1, up to 100 Frank-Wolfe iterations)
     of n images of uneven sizes (H ~ U[240, 500], W ~ U[320, 500], seeded),
     solved as one batch (dcrf_batch_qp_dev: concatenated lattices, per-image
@@ -644,8 +629,6 @@ def measure_batch(n=64, max_iter=100, reps=3, sequential=True, splat_form=None):
     b.addPairwiseBilateral(BILAT[0], BILAT[0], BILAT[1], BILAT[1], BILAT[1],
                            np.concatenate([im["rgb"] for im in imgs]), BILAT[2])
     setup_ms = (time.perf_counter() - t0) * 1e3
-    if splat_form is not None:
-        pin_splat_form(b, splat_form)
     q0 = b.unary_init()
     init = torch.from_numpy(q0).cuda()
     out = torch.empty_like(init)
@@ -718,7 +701,7 @@ def measure_batch(n=64, max_iter=100, reps=3, sequential=True, splat_form=None):
             "outputs_match_sequential": same}
 
 
-def measure_batch_filter(n=64, reps=10, splat_form=None, all_forms=False):
+def measure_batch_filter(n=64, reps=10):
     """The batched lattice filter: PairwisePotential::apply of each pairwise
     term (normalised Potts filter, pre- and post-scaled by the norm) over the
     term's concatenated lattice of the config-4 batch (n images, H ~ U[240,
@@ -737,35 +720,12 @@ def measure_batch_filter(n=64, reps=10, splat_form=None, all_forms=False):
     b.addPairwiseBilateral(BILAT[0], BILAT[0], BILAT[1], BILAT[1], BILAT[1],
                            np.concatenate([im["rgb"] for im in imgs]), BILAT[2])
     N = int(b.N)
-    if splat_form is not None:
-        pin_splat_form(b, splat_form)
     x = torch.rand((N, L), device="cuda", generator=torch.Generator("cuda").manual_seed(1))
     y = torch.empty_like(x)
     sptr = C.c_void_p()
     check(Ls.dcrf_batch_stream(b._h, C.byref(sptr)))
     bs = torch.cuda.ExternalStream(sptr.value)
     peak, peak_kind = measured_peaks()
-    if all_forms:  # every splat form pinned in turn; outputs must not change
-        forms = {}
-        for k, name in enumerate(("gaussian", "bilateral")):
-            ref = None
-            for f, fname in enumerate(SPLAT_FORMS):
-                b.set_filter_shape(k, (4, 256, 128, f))
-                run = lambda: check(Ls.dcrf_batch_pairwise_apply_dev(b._h, k, C.c_void_p(y.data_ptr()),
-                                                                     C.c_void_p(x.data_ptr())))
-                for _ in range(3):
-                    run()
-                torch.cuda.synchronize()
-                e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-                e0.record(bs)
-                for _ in range(reps):
-                    run()
-                e1.record(bs)
-                torch.cuda.synchronize()
-                if ref is None:
-                    ref = y.clone()
-                forms[f"{name}_{fname}"] = {"ms": e0.elapsed_time(e1) / reps, "same_output": bool(torch.equal(ref, y))}
-        return {"images": n, "pixels": N, "forms": forms}
     out = {"workload": f"PairwisePotential::apply over the concatenated lattice of {n} images "
                        f"H~U[240,500] W~U[320,500] (seeded), L={L}, device-resident",
            "images": n, "pixels": N, "peak_gbs": peak, "peak_kind": peak_kind}
@@ -790,9 +750,7 @@ def measure_batch_filter(n=64, reps=10, splat_form=None, all_forms=False):
         out[name] = {"M": M, "d": d, "ms": t * 1e3, "bytes": fb, "gbs": fb / t / 1e9, "frac": fb / t / 1e9 / peak,
                      "gpix_label_s": N * L / t / 1e9,
                      "launches_per_call": int((Ls.dcrf_kernel_launches() - l0) // reps),
-                     "tuned_shape": {"splat_form": SPLAT_FORMS[shp[3]],
-                                     "splat_vertices_per_block": shp[0], "blur_threads": shp[1],
-                                     "slice_pixels_per_block": shp[2]}}
+                     "blur_threads": shp[1]}
     return out
 
 
@@ -1119,14 +1077,13 @@ def run_ours(args):
         print(json.dumps(measure_filters(W, H, img, reps=3)))
         return
     if args.only_batch_filter:
-        print(json.dumps(measure_batch_filter(n=args.batch_images, splat_form=args.splat_form,
-                                              all_forms=args.all_splat_forms)))
+        print(json.dumps(measure_batch_filter(n=args.batch_images)))
         return
     if args.only_ho:
         print(json.dumps(measure_ho(cpu=False)))
         return
     if args.only_batch_qp:
-        print(json.dumps(measure_batch(n=args.batch_images, reps=1, sequential=False, splat_form=args.splat_form)))
+        print(json.dumps(measure_batch(n=args.batch_images, reps=1, sequential=False)))
         return
     if args.only_batch:
         print(json.dumps(measure_ho()))
