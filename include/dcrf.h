@@ -53,7 +53,10 @@ typedef struct dcrf_model_s* dcrf_model;
 dcrf_status dcrf_release_cached_memory(void);
 /* A budget on the device memory the library holds for live models, lattices
  * and batches (bytes; 0 = none, the default).  A request beyond it fails with
- * DCRF_E_NOMEM before any device call.  No counterpart in the reference. */
+ * DCRF_E_NOMEM before any device call, once the handle has given back what it
+ * can do without (the plain filter's input in padded rows, 16 ceil(L / 4) bytes
+ * a pixel and lattice, and the scratch of a complete build; other handles'
+ * are not touched).  No counterpart in the reference. */
 dcrf_status dcrf_set_device_memory_limit(uint64_t bytes);
 /* Bytes held by live models / lattices / batches, bytes kept in the cache,
  * and the number of cudaMalloc calls the library has made (any may be NULL).
