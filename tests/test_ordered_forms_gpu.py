@@ -22,6 +22,10 @@ def _features(W, H, d, kind):
     rgb = synth.make_image(W, H, 21, 5)["rgb"]
     if kind == "noisy":
         rgb = np.random.default_rng(0).integers(0, 256, size=rgb.shape).astype(np.uint8)
+    if kind == "half":  # noise beside one colour: many vertices and long lists
+        rgb = np.random.default_rng(0).integers(0, 256, size=(H, W, 3)).astype(np.uint8)
+        rgb[:, W // 2:] = 100
+        rgb = rgb.reshape(-1, 3)
     s = 8 if kind == "wide" else 1  # wide: huge lists
     return np.ascontiguousarray(synth.bilateral_features(W, H, 50 * s, 50 * s, *[15 * s] * 3, rgb)[:, :d])
 
@@ -93,7 +97,8 @@ def _block(n):  # device blocks: powers of two split in quarters
     return p if p == 512 else -(-n // (p // 4)) * (p // 4)
 
 
-@pytest.mark.parametrize("W,H,kind,L", [(97, 83, "noisy", 21), (97, 83, "photo", 21), (161, 120, "grid", 5)])
+@pytest.mark.parametrize("W,H,kind,L", [(97, 83, "noisy", 21), (97, 83, "photo", 21), (161, 120, "grid", 5),
+                                        (97, 83, "half", 40), (97, 83, "half", 100)])
 def test_without_memory_for_the_quads(W, H, kind, L):
     """Budgets below what a call of the quad form's range takes: the same bits or
     no memory, and never the latter where the dense form has room."""
@@ -120,3 +125,56 @@ def test_without_memory_for_the_quads(W, H, kind, L):
             set_device_memory_limit(0)
         assert np.array_equal(_dev_filter(lat, x, entry), want)
         del lat
+
+
+@pytest.mark.parametrize("W,H,kind,L", [(257, 256, "wide", 4), (257, 256, "wide", 21), (200, 150, "noisy", 3)])
+def test_captured_in_a_caller_s_graph(W, H, kind, L):
+    """A call captured on the lattice's stream and replayed on other values."""
+    import torch
+    f = _features(W, H, 5, kind)
+    gen = torch.Generator(device="cuda").manual_seed(L)
+    x, y = (torch.rand(W * H, L, generator=gen, device="cuda") for _ in range(2))
+    entry = lib().dcrf_lattice_compute_ord_dev
+    lat = Permutohedral().init(f)
+    wants = [_dev_filter(lat, v, entry) for v in (x, y)]
+    sp = C.c_void_p()
+    check(lib().dcrf_lattice_stream(lat._h, C.byref(sp)))
+    src, out = x.clone(), torch.empty_like(x)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(sp.value), capture_error_mode="thread_local"):
+        check(entry(lat._h, C.c_void_p(out.data_ptr()), C.c_void_p(src.data_ptr()), L))
+    for v, want in zip((y, x), wants[::-1]):
+        src.copy_(v)
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(out.cpu().numpy(), want)
+    graph.reset()
+
+
+def test_threads_with_lattices_of_their_own():
+    """Both forms from several threads at once, each with its handle."""
+    import threading
+
+    import torch
+    f, g = _features(257, 256, 5, "wide"), _features(97, 83, 5, "noisy")
+    entry = lib().dcrf_lattice_compute_ord_dev
+    jobs = []
+    for L, feat in ((2, f), (12, f), (21, f), (1, g), (21, g)):
+        x = torch.rand(len(feat), L, device="cuda", generator=torch.Generator(device="cuda").manual_seed(L))
+        lat = Permutohedral().init(feat)
+        jobs.append((lat, x, _dev_filter(lat, x, entry)))
+    bad = []
+
+    def work(lat, x, want):
+        for _ in range(20):
+            if not np.array_equal(_dev_filter(lat, x, entry), want):
+                bad.append(x.shape)
+
+    threads = [threading.Thread(target=work, args=j) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
