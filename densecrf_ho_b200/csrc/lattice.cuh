@@ -214,6 +214,7 @@ struct Lattice {
     // Ordered (upper minus lower, 10-bin) filter of Q in [0,1]; out = epilogue(v).
     void compute_ord(float* out, const float* Q, int L, const SliceEpilogue& ep);
     bool ord_dense(int L) const;
+    bool ord_many(int L) const;
     void compute_ord_dense(float* out, const float* Q, int L, const SliceEpilogue& ep);
     // The same from packed bins in two phases: splat + blur (leaves the vertex
     // values in ord_vals), then the slice.  Other work may run between them.

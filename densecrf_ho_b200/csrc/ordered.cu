@@ -1718,8 +1718,13 @@ bool Lattice::ord_dense(int L) const {
     if (d <= 2 && n_long == 0)
         return (long)N * L > 1L << 19 || N > 1 << 18 || L > 28 || (L >= 20 && N >= 1 << 14);
     const bool long_lists = (long)N * (d + 1) >= 32L * M;  // on average
-    const int by_lists = !long_lists ? 0 : N > 1 << 18 ? 12 : N > 1 << 16 ? 20 : 0;
-    return L <= std::max((double)by_lists, 8.0 * std::log2((double)M) - 127.0);
+    return L <= (!long_lists ? 0 : N > 1 << 18 ? 12 : N > 1 << 16 ? 20 : 0) || ord_many(L);
+}
+
+// ... for the number of its vertices: from 60 thousand on for one label, eight more
+// with each doubling.
+bool Lattice::ord_many(int L) const {
+    return (d > 2 || n_long) && L <= kOrdBlockMaxL && L <= 8.0 * std::log2((double)M) - 127.0;
 }
 
 void Lattice::compute_ord_dense(float* out, const float* Q, int L, const SliceEpilogue& ep) {
